@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(CH) attention_plain_kernel(const DkAttnParams 
   long long* voff = (long long*)(scratch + 34 + ((p.hd + CH + 34) & 1));  // CH, 8-byte aligned
   const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int row = p.tok_row[t], pos = p.tok_pos[t];
+  if (p.row_filter == 1 && p.row_q_len[row] != 1) return;      // rows that bring several tokens are another kernel's
   const int hd = p.hd, ps = p.ps, KV = p.KV;
   const int g = h / (p.H / KV);
   const T* q = (const T*)p.q + (size_t)t * p.q_stride + (size_t)h * hd;
@@ -116,6 +117,7 @@ extern "C" int dk_attention_plain(const DkAttnParams* pp, cudaStream_t stream) {
   DK_REQUIRE(p.sel_pages == nullptr || (p.sel_count != nullptr && p.row_flags != nullptr && p.row_slot != nullptr),
              "attention: chosen pages are given without their counts, row flags or slots");
   DK_REQUIRE(p.dump == nullptr || p.row_flags != nullptr, "attention: a score dump is asked for without row flags");
+  DK_REQUIRE(p.row_filter != 1 || p.row_q_len != nullptr, "attention: rows of one token are asked for without the rows' lengths");
   const size_t smem = (size_t)(p.hd + CH + 36) * sizeof(float) + (size_t)CH * sizeof(long long);
   dim3 grid(p.T, p.H);
   if (p.dtype == DK_F32) attention_plain_kernel<float><<<grid, CH, smem, stream>>>(p);

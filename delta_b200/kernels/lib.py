@@ -71,6 +71,8 @@ _SIGNATURES = {
     "dk_silu_mul": [P, P, I, I, I, P],
     "dk_rope_append": [P, P, P, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P],
     "dk_gemm_nt_plain": [P, P, P, I, I, I, I, I, I, I, I, P],
+    "dk_attention_f32_supported": [I, I, I, I, I],
+    "dk_attention_f32": [C.POINTER(AttnParams), I, P],
     "dk_attention_plain": [C.POINTER(AttnParams), P],
     "dk_recent_pages": [P, P, P, P, P, P, I, I, I, D, I, P],
     "dk_page_scores": [P, P, P, P, P, P, P, I, I, I, I, I, I, D, I, P],

@@ -243,6 +243,17 @@ def attention_plain(params: AttnParams):
     _l.check(_l.load().dk_attention_plain(C.byref(params), _stream()), "attention_plain")
 
 
+def attention_f32_supported(dtype, H, KV, hd, q_stride) -> bool:
+    if dtype != torch.float32:
+        return False
+    return bool(_l.load().dk_attention_f32_supported(F32, H, KV, hd, int(q_stride)))
+
+
+def attention_f32(params: AttnParams, max_q_len: int):
+    """32-bit rows that bring several tokens (rows of one are taken too), 32 queries a block; no chosen pages, no score dump."""
+    _l.check(_l.load().dk_attention_f32(C.byref(params), int(max_q_len), _stream()), "attention_f32")
+
+
 def attention_decode_supported(dtype, H, KV, hd, ps) -> bool:
     if dtype != torch.bfloat16:
         return False

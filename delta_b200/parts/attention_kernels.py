@@ -124,6 +124,16 @@ def run(ctx, params, group: str) -> None:
     """Runs paged attention with the kernels that fit the batch.  ``group`` names the cache group
     of the layer (its block tables tell whether pages lie in runs)."""
     if plain(ctx):
+        # 32 bit: rows that bring several tokens share tiles of keys, rows of one token stay with the plain kernel whatever stands
+        # beside them, so that a row's sums are the same in every batch.  Chosen pages and score dumps are the plain kernel's.
+        if (not ctx.decode_only and "attention" not in ctx.plain_kernels and params.sel_pages is None and params.dump is None
+                and ops.attention_f32_supported(ctx.dtype, params.H, params.KV, params.hd, params.q_stride)):
+            if any(n == 1 for n in ctx.host["q_lens"]):
+                params.row_filter = 1
+                ops.attention_plain(params)
+                params.row_filter = 2
+            ops.attention_f32(params, ctx.max_q_len)
+            return
         ops.attention_plain(params)
         return
     dec_ok = ops.attention_decode_supported(ctx.dtype, params.H, params.KV, params.hd, params.ps)

@@ -1,0 +1,63 @@
+"""Kernels at the sizes where their tiles can go wrong: one row or key beside a tile's edge, sizes below a tile, rows of very different lengths."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, PagedCase, ops
+
+pytestmark = pytest.mark.gpu
+
+
+# 64 x 128, 32 x 64 and 32 x 32 sums a block, each with rows, columns and K beside the tiles' edges; the last two have no 16-byte rows
+@pytest.mark.parametrize("M, N, K", [(300, 11012, 36), (1025, 2049, 20), (130, 11008, 132), (33, 2048, 64), (1, 65, 16), (65, 130, 18), (7, 33, 3)])
+def test_gemm_f32_tiles(M, N, K):
+    o = ops()
+    torch.manual_seed(M + N)
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    out = torch.full((M + 1, N), 7.0, device=DEV)
+    o.gemm_nt_plain(a, w, out[:M])
+    ref = a.double() @ w.double().T
+    # a sum of K products, each rounded once: K / 2 units of 2^-24 of the sum of magnitudes bounds it by far
+    bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + 1e-30
+    assert bool(((out[:M].double() - ref).abs() <= bound).all()) and bool((out[M:] == 7.0).all())
+    one = torch.empty(1, N, device=DEV)
+    o.gemm_nt_plain(a[M - 1:].contiguous(), w, one)      # another tile size, the same order of the sum
+    assert torch.equal(one[0], out[M - 1])
+
+
+@pytest.mark.parametrize("H, KV, hd, ps", [(4, 2, 128, 16), (3, 3, 64, 8), (8, 1, 32, 64)])
+@pytest.mark.parametrize("window", [0, 1, 33, 100])
+def test_attention_f32_tiles(H, KV, hd, ps, window):
+    o = ops()
+    case = PagedCase(torch.float32, H, KV, hd, ps, seq_lens=[2, 31, 32, 33, 200, 129, 97, 300], q_lens=[2, 31, 32, 33, 64, 2, 65, 1], seed=H + window)
+    out, lse = torch.full((case.T, H * hd), 9.0, device=DEV), torch.empty(case.T, H, device=DEV)
+    o.attention_f32(case.params(out, lse=lse, window=window), max(case.q_lens))
+    ref, ref_lse, _ = case.reference(window=window)
+    # scores of about 6 at most in 32 bit: their rounding (hd 2^-24 |q| |k| scale) moves a weight by less than 1e-5
+    assert torch.allclose(out.cpu(), ref, atol=2e-5, rtol=2e-5)
+    assert torch.allclose(lse.cpu(), ref_lse, atol=2e-5, rtol=2e-5)
+    # the rows of one token are left to the plain kernel, the others give the same bits
+    again = torch.full_like(out, 9.0)
+    o.attention_f32(case.params(again, window=window, row_filter=2), max(case.q_lens))
+    assert torch.equal(again[:-1], out[:-1]) and bool((again[-1] == 9.0).all())
+    o.attention_plain(case.params(again, window=window, row_filter=1))
+    assert torch.allclose(again[-1], out[-1], atol=2e-5, rtol=2e-5) and torch.equal(again[:-1], out[:-1])
+
+
+def test_attention_f32_keeps_what_a_query_does_not_see_out_of_its_sums():
+    """A later token's infinite value reaches its own query and the ones behind it only; a page outside the pool is reported and left out."""
+    o = ops()
+    case = PagedCase(torch.float32, 2, 1, 64, 16, seq_lens=[40], q_lens=[40], seed=5)
+    page = int(case.bt[0, 1])
+    case.kv[page, 1, 0, 4, 3] = math.inf      # position 20
+    out = torch.empty(40, 128, device=DEV)
+    o.attention_f32(case.params(out), 40)
+    ref, _, _ = case.reference()
+    assert torch.allclose(out[:20].cpu(), ref[:20], atol=2e-5, rtol=2e-5) and not bool(torch.isfinite(out[20:, 3]).any())
+    case.bt[0, 1] = 1 << 20
+    err = o.new_error_record(DEV)
+    o.attention_f32(case.params(out, err=err), 40)
+    with pytest.raises(o.KernelError, match="page id"):
+        o.raise_if_error(err)
+    assert torch.allclose(out[:16].cpu(), ref[:16], atol=2e-5, rtol=2e-5)
