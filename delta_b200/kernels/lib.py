@@ -64,6 +64,7 @@ _SIGNATURES = {
     "dk_attention_rows_mma": [C.POINTER(RowAttnParams), I, I, P, P],
     "dk_attention_rows_tc_supported": [C.POINTER(RowAttnParams)],
     "dk_attention_rows_tc": [C.POINTER(RowAttnParams), I, P],
+    "dk_gemm_heads": [P, P, P, I, I, I, I, I, I, L, L, L, P],
     "dk_gemm_nt_plain_batched": [P, P, P, I, I, I, I, I, I, I, L, L, L, I, I, P],
     "dk_embedding": [P, P, P, I, I, I, I, P, P],
     "dk_rms_norm": [P, P, P, P, P, I, I, F, I, I, I, P],

@@ -617,6 +617,16 @@ def latent_prepare(src, tok_pos, tok_row, block_table, cache, qabs, *, norm_weig
         low.shape[1] if low is not None else 0, dtype_code(src.dtype), _ptr(err, "err", i32), _stream()), "latent_prepare")
 
 
+def gemm_heads_supported(M, K, lda, sa, sw, a_ptr, w_ptr) -> bool:
+    """Up to 16 rows whose operands begin on 16-byte boundaries, K a multiple of 32."""
+    return 0 < M <= 16 and K % 32 == 0 and lda % 8 == 0 and sa % 8 == 0 and sw % 8 == 0 and a_ptr % 16 == 0 and w_ptr % 16 == 0
+
+
+def gemm_heads(a_ptr, w_ptr, c_ptr, M, N, K, lda, ldc, batch, sa, sw, sc):
+    """C_b = A_b W_b^T for every b of a batch of small bfloat16 products (addresses; strides in elements; W_b's rows lie K apart)."""
+    _l.check(_l.load().dk_gemm_heads(a_ptr, w_ptr, c_ptr, M, N, K, lda, ldc, batch, sa, sw, sc, _stream()), "gemm_heads")
+
+
 def gemm_nt_plain_batched(a_ptr, w_ptr, c_ptr, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, in_dtype, out_dtype):
     """``batch`` products C_b[M,N] = A_b[M,K] W_b[N,K]^T on the FMA units with float accumulation; the operands of product b
     lie b*sa, b*sw and b*sc elements behind the given addresses (raw addresses: the operands may be interleaved views)."""

@@ -61,3 +61,21 @@ def test_attention_f32_keeps_what_a_query_does_not_see_out_of_its_sums():
     with pytest.raises(o.KernelError, match="page id"):
         o.raise_if_error(err)
     assert torch.allclose(out[:16].cpu(), ref[:16], atol=2e-5, rtol=2e-5)
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("N, K, heads", [(256, 128, 16), (128, 256, 3), (40, 32, 5), (16, 160, 1)])
+def test_gemm_heads(M, N, K, heads):
+    """Operands of a head between those of the others, as they lie in a layer's rows; columns beside a warp's 16, K beside a step of 128."""
+    o = ops()
+    torch.manual_seed(M + N)
+    a = torch.randn(M, heads, K + 8, device=DEV).bfloat16()
+    w = (torch.randn(heads, N, K, device=DEV) * 0.1).bfloat16()
+    c = torch.full((M, heads, N + 3), 5.0, dtype=torch.bfloat16, device=DEV)
+    o.gemm_heads(a.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K, heads * (K + 8), heads * (N + 3), heads, K + 8, N * K, N + 3)
+    ref = torch.einsum("mhk,hnk->mhn", a[:, :, :K].double(), w.double())
+    # one rounding to bfloat16 (2^-9 of the value) and the rounding of a 32-bit sum
+    assert bool(((c[:, :, :N].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()) and bool((c[:, :, N:] == 5.0).all())
+    assert not o.gemm_heads_supported(17, K, K, K, N * K, a.data_ptr(), w.data_ptr()) and not o.gemm_heads_supported(M, K, K, K, N * K, a.data_ptr() + 2, w.data_ptr())
+    with pytest.raises(o.KernelError, match="multiple of 32"):
+        o.gemm_heads(a.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K - 8, K, N, 1, K, N * K, N)
