@@ -1124,6 +1124,34 @@ def state_space_chunked(xbc, dt_ptr, dt_stride, A_log, dt_bias, D, state, out, w
     return out
 
 
+def state_space_mma_chunk() -> int:
+    return int(_l.load().dk_state_space_mma_chunk())
+
+
+def state_space_mma_supported(N, P, stride, dtype) -> bool:
+    return dtype == torch.bfloat16 and bool(_l.load().dk_state_space_mma_supported(int(N), int(P), int(stride)))
+
+
+def state_space_mma_floats(H, G) -> int:
+    return int(_l.load().dk_state_space_mma_floats(int(H), int(G)))
+
+
+def state_space_mma(xbc, dt_ptr, dt_stride, A_log, dt_bias, D, state, out, work, chunk_base, total_chunks, max_chunks, *, H, G, N, P,
+                        row_slot, row_q_start, row_q_len):
+    """``state_space_chunked`` for bfloat16 portions on the tensor cores, in chunks of ``state_space_mma_chunk`` tokens; ``work`` float32 with
+    total_chunks * ``state_space_mma_floats`` entries."""
+    if xbc.dtype != torch.bfloat16:
+        raise KernelError(f"state_space_mma takes bfloat16 rows, not {xbc.dtype}")
+    _check_shape(state, (H, P, N), "state_space_mma")
+    i32, f32 = torch.int32, torch.float32
+    _l.check(_l.load().dk_state_space_mma(
+        _ptr(xbc, "xbc"), xbc.shape[1], dt_ptr, int(dt_stride), _ptr(A_log, "A_log", f32), _ptr(dt_bias, "dt_bias", f32), _ptr(D, "D", f32),
+        _ptr(state, "state", f32), _ptr(out, "out", f32), _ptr(work, "work", f32), _ptr(row_slot, "row_slot", i32),
+        _ptr(row_q_start, "row_q_start", i32), _ptr(row_q_len, "row_q_len", i32), _ptr(chunk_base, "chunk_base", i32), row_slot.shape[0],
+        int(total_chunks), int(max_chunks), H, G, N, P, _stream()), "state_space_mma", 2)
+    return out
+
+
 def _check_shape(state, per_slot, who):
     if tuple(state.shape[1:]) != tuple(per_slot):
         raise KernelError(f"{who}: the state has shape {tuple(state.shape)}, expected [slots, {', '.join(str(n) for n in per_slot)}]")

@@ -11,7 +11,8 @@ pair per run of the layer; a step continues from what the request's earlier step
 
 W_in's rows are put into the order x | B | C | z | dt when they are bound, so that the convolution's inputs come first.  Step sizes,
 decays, the recurrence and the norm are 32 bit whatever the compute type (``csrc/state_space.cu``): steps of single tokens and short
-portions take the tokens in turn with the state in registers, long portions run in chunks of 32 tokens.
+portions take the tokens in turn with the state in registers, long portions run in chunks of 32 tokens, or, in bfloat16 with heads that
+fit the MMA tiles, of 64 (``csrc/state_space_mma.cu``).
 """
 from __future__ import annotations
 
@@ -78,7 +79,15 @@ class StateSpace(Mixer):
         y = torch.empty((T, C), dtype=torch.float32, device=x.device)
         args = (xbc, at(self.channels + C), src.shape[1], self.A_log, self.dt_bias, self.D, st[STATE], y)
         sizes = dict(H=H, G=G, N=N, P=P)
-        if not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM and ops.state_space_chunked_supported(N, P, x.dtype):
+        portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
+        if portions and ops.state_space_mma_supported(N, P, xbc.shape[1], x.dtype):
+            chunk = ops.state_space_mma_chunk()
+            base, total, most = chunk_layout(ctx, chunk)
+            per = ops.state_space_mma_floats(H, G)
+            bound = (-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per
+            work = ctx.scratch("state_space.chunks", (total * per,), torch.float32, bound=(bound,))
+            ops.state_space_mma(*args, work, base, total, most, **sizes, **rows)
+        elif portions and ops.state_space_chunked_supported(N, P, x.dtype):
             base, total, most = chunk_layout(ctx, ops.state_space_chunk())
             per = ops.state_space_chunk_floats(H, G)
             bound = (-(-ctx.max_step_tokens // ops.state_space_chunk()) + ctx.max_rows) * per

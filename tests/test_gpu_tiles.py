@@ -79,3 +79,54 @@ def test_gemm_heads(M, N, K, heads):
     assert not o.gemm_heads_supported(17, K, K, K, N * K, a.data_ptr(), w.data_ptr()) and not o.gemm_heads_supported(M, K, K, K, N * K, a.data_ptr() + 2, w.data_ptr())
     with pytest.raises(o.KernelError, match="multiple of 32"):
         o.gemm_heads(a.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K - 8, K, N, 1, K, N * K, N)
+
+
+def ssd_inputs(H, G, N, P, lens, slots, seed, decays):
+    g = torch.Generator().manual_seed(seed)
+    T = sum(lens)
+    xbc = torch.randn(T, H * P + 2 * G * N, generator=g).bfloat16()
+    dtraw = (torch.randn(T, H + 3, generator=g) * 2).bfloat16()
+    A_log, bias = {"weak": (torch.full((H,), -4.0), -4.0), "mixed": (torch.linspace(-2, 2, H), -1.0), "strong": (torch.full((H,), 3.0), 2.0)}[decays]
+    if decays == "mixed":
+        dtraw[::7] += 30.0
+    state = torch.randn(max(slots) + 2, H, P, N, generator=g)
+    return xbc, dtraw, A_log, torch.full((H,), bias), torch.randn(H, generator=g), state
+
+
+def ssd_reference(xbc, dtraw, A_log, dt_bias, D, S, H, G, N, P):
+    """One row in 64 bits on the device: (y [n, H, P], the state behind it [H, P, N])."""
+    n = xbc.shape[0]
+    x = xbc[:, :H * P].double().view(n, H, P)
+    B, C = (t.double().reshape(n, G, N).repeat_interleave(H // G, dim=1) for t in xbc[:, H * P:].split(G * N, dim=1))
+    z = dtraw[:, :H].double() + dt_bias.double()
+    dt = torch.where(z > 20, z, torch.log1p(torch.exp(z.clamp(max=20))))
+    A, out = torch.exp(A_log.double()), []
+    for t in range(n):
+        S = torch.exp(-A * dt[t])[:, None, None] * S + x[t][:, :, None] * (dt[t][:, None] * B[t])[:, None, :]
+        out.append(torch.einsum("hpn,hn->hp", S, C[t]) + D.double()[:, None] * x[t])
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("decays", ["weak", "mixed", "strong"])
+@pytest.mark.parametrize("H, G, N, P", [(4, 2, 128, 64), (3, 1, 64, 32), (40, 1, 128, 96)])
+def test_state_space_mma(H, G, N, P, decays):
+    """Chunks of 64: rows of one token, one beside a chunk's end on either side, several chunks; slots out of order; a slot of no row."""
+    o = ops()
+    lens, slots = [1, 63, 64, 65, 200], [2, 0, 4, 1, 5]
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    xbc, dtraw, A_log, dt_bias, D, state = (t.to(DEV) for t in ssd_inputs(H, G, N, P, lens, slots, H + N, decays))
+    st, out = state.clone(), torch.full((sum(lens), H * P), float("nan"), device=DEV)
+    assert o.state_space_mma_supported(N, P, xbc.shape[1], xbc.dtype) and not o.state_space_mma_supported(N, P, xbc.shape[1], torch.float32)
+    counts = [-(-n // o.state_space_mma_chunk()) for n in lens]
+    base = torch.tensor([sum(counts[:i]) for i in range(len(counts))], dtype=torch.int32, device=DEV)
+    work = torch.full((sum(counts) * o.state_space_mma_floats(H, G),), float("nan"), device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    o.state_space_mma(xbc, dtraw.data_ptr(), H + 3, A_log, dt_bias, D, st, out, work, base, sum(counts), max(counts), H=H, G=G, N=N, P=P,
+                      row_slot=i32(slots), row_q_start=i32(starts), row_q_len=i32(lens))
+    for r, n in enumerate(lens):
+        s = slice(starts[r], starts[r] + n)
+        y, S = ssd_reference(xbc[s], dtraw[s], A_log, dt_bias, D, state[slots[r]].double(), H, G, N, P)
+        # the bound of the 32-bit kernels' own test
+        assert (out[s].double().view(n, H, P) - y).abs().max() < 1e-5 * y.abs().max(), r
+        assert (st[slots[r]].double() - S).abs().max() < 1e-5 * S.abs().max(), r
+    assert torch.equal(st[3], state[3]) and torch.equal(st[6], state[6])
