@@ -104,6 +104,10 @@ _SIGNATURES = {
     "dk_decay_attention": [P, I, I, I, I, I, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "dk_decay_attention_chunk": [],
     "dk_decay_attention_chunked_supported": [I, I],
+    "dk_decay_attention_tiles_chunk": [],
+    "dk_decay_attention_tiles_supported": [I, I, I, I, I, I],
+    "dk_decay_attention_tiles_floats": [I, I],
+    "dk_decay_attention_tiles": [P, I, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
     "dk_decay_attention_chunked": [P, I, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "dk_decay_attention_step_supported": [I, I],
     "dk_decay_attention_step": [P, I, I, I, I, I, P, P, P, P, P, I, I, I, I, I, P],

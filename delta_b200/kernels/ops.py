@@ -870,6 +870,34 @@ def decay_attention_chunked(src, q_off, k_off, v_off, decays, state, out, work, 
     return out
 
 
+def decay_attention_tiles_chunk() -> int:
+    return int(_l.load().dk_decay_attention_tiles_chunk())
+
+
+def decay_attention_tiles_supported(dk, dv, stride, q_off, k_off, v_off) -> bool:
+    return bool(_l.load().dk_decay_attention_tiles_supported(int(dk), int(dv), int(stride), int(q_off), int(k_off), int(v_off)))
+
+
+def decay_attention_tiles_floats(dk, dv) -> int:
+    return int(_l.load().dk_decay_attention_tiles_floats(int(dk), int(dv)))
+
+
+def decay_attention_tiles(src, q_off, k_off, v_off, decays, state, out, work, chunk_base, total_chunks, max_chunks, *, H, dk, dv, row_slot,
+                          row_q_start, row_q_len, silu=True):
+    """``decay_attention_chunked`` for heads of 64 or 128 entries, in chunks of ``decay_attention_tiles_chunk`` tokens; ``work`` float32 with
+    room for total_chunks x H x ``decay_attention_tiles_floats``."""
+    if tuple(state.shape[1:]) != (H, dk, dv):
+        raise KernelError(f"decay_attention_tiles: the state has shape {tuple(state.shape)}, expected [slots, {H}, {dk}, {dv}]")
+    i32 = torch.int32
+    _l.check(_l.load().dk_decay_attention_tiles(
+        _ptr(src, "src"), src.shape[1], int(q_off), int(k_off), int(v_off), int(bool(silu)), _ptr(decays, "decays", torch.float64),
+        _ptr(state, "state", torch.float32), _ptr(out, "out", torch.float32), _ptr(work, "work", torch.float32),
+        _ptr(row_slot, "row_slot", i32), _ptr(row_q_start, "row_q_start", i32), _ptr(row_q_len, "row_q_len", i32),
+        _ptr(chunk_base, "chunk_base", i32), row_slot.shape[0], int(total_chunks), int(max_chunks), H, dk, dv, dtype_code(src.dtype), _stream()),
+        "decay_attention_tiles", 3)
+    return out
+
+
 def gated_rms_norm(o, gate_ptr, gate_stride, weight, out, eps, group=None, gate_first=False, gate_dtype=None):
     """out = o / sqrt(mean(o^2) + eps) * weight * sigmoid(gate) per token; ``o`` float32 [T, n]; the gate's n values of a token
     lie at ``gate_ptr`` + t * ``gate_stride`` elements of the type of ``out``.  ``group``: the mean is taken over every ``group``

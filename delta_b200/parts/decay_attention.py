@@ -7,7 +7,8 @@ With mixer input h, H heads, key size dk and value size dv:
 A request's state is S [H, dk, dv] in 32 bit, zero at its start, one per run of the layer; a step continues from what
 the request's earlier steps left, so a prompt may be cut anywhere.  The four projections are one product; the
 recurrence, its decays and the norm are 32 bit whatever the compute type.  Steps of single tokens stream the state through
-registers once; short portions run one block per (row, head) over the row's chunks in turn; long portions run their chunks in parallel (``csrc/decay_attention.cu``).
+registers once; short portions run one block per (row, head) over the row's chunks in turn; long portions run their chunks in parallel (``csrc/decay_attention.cu``;
+heads of 64 or 128 entries in chunks of 64 tokens, ``csrc/decay_attention_tiles.cu``).
 """
 from __future__ import annotations
 
@@ -16,6 +17,7 @@ import torch
 from ..kernels import ops
 from . import linear
 from .base import MIXERS, Mixer, StateSpec, TensorSpec
+from .chunks import chunk_layout
 
 STATE = "decay_attention"
 PARALLEL_FROM = 65      # portions of at least this many tokens run their chunks in parallel
@@ -56,8 +58,17 @@ class DecayAttention(Mixer):
         qkvg = linear.linear(ctx, x, self.w_in)                       # [T, 2 H dk + 2 H dv]: q | k | v | g, before activations
         o = torch.empty((T, H * dv), dtype=torch.float32, device=x.device)
         rows = dict(row_slot=ctx.row_slot, row_q_start=ctx.row_q_start, row_q_len=ctx.row_q_len)
-        if not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM and ops.decay_attention_chunked_supported(dk, dv):
-            # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
+        portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
+        # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
+        if portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk):
+            chunk = ops.decay_attention_tiles_chunk()
+            base, total, most = chunk_layout(ctx, chunk)
+            per = H * ops.decay_attention_tiles_floats(dk, dv)
+            bound = (-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per
+            work = ctx.scratch("decay_attention.chunks", (total * per,), torch.float32, bound=(bound,))
+            ops.decay_attention_tiles(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, total, most, H=H, dk=dk,
+                                      dv=dv, silu=True, **rows)
+        elif portions and ops.decay_attention_chunked_supported(dk, dv):
             chunk = ops.decay_attention_chunk()
 
             def layout():

@@ -130,3 +130,65 @@ def test_state_space_mma(H, G, N, P, decays):
         assert (out[s].double().view(n, H, P) - y).abs().max() < 1e-5 * y.abs().max(), r
         assert (st[slots[r]].double() - S).abs().max() < 1e-5 * S.abs().max(), r
     assert torch.equal(st[3], state[3]) and torch.equal(st[6], state[6])
+
+
+def decay_case(lens, slots, H, dk, dv, dtype, decays, seed):
+    g = torch.Generator().manual_seed(seed)
+    src = (torch.randn(sum(lens), 2 * H * dk + H * dv + 8, generator=g) * 0.8).to(dtype).to(DEV)
+    state = (torch.randn(max(slots) + 2, H, dk, dv, generator=g) * 0.3).to(DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    rows = dict(row_slot=i32(slots), row_q_start=i32([sum(lens[:i]) for i in range(len(lens))]), row_q_len=i32(lens))
+    return src, state, torch.tensor(decays, dtype=torch.float64, device=DEV), rows
+
+
+def decay_reference(src, S, decays, H, dk, dv):
+    """One row in 64 bits: (o [n, H, dv], the state behind it)."""
+    x = torch.nn.functional.silu(src.double())
+    n = x.shape[0]
+    q, k, v = x[:, :H * dk].view(n, H, dk), x[:, H * dk:2 * H * dk].view(n, H, dk), x[:, 2 * H * dk:2 * H * dk + H * dv].view(n, H, dv)
+    out = []
+    for t in range(n):
+        S = decays[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
+        out.append(torch.einsum("hkv,hk->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+def decay_tiles(o, src, state, decays, rows, lens, H, dk, dv):
+    counts = [-(-n // o.decay_attention_tiles_chunk()) for n in lens]
+    base = torch.tensor([sum(counts[:i]) for i in range(len(counts))], dtype=torch.int32, device=DEV)
+    work = torch.full((sum(counts) * H * o.decay_attention_tiles_floats(dk, dv),), float("nan"), device=DEV)
+    out = torch.full((sum(lens), H * dv), float("nan"), device=DEV)
+    o.decay_attention_tiles(src, 0, H * dk, 2 * H * dk, decays, state, out, work, base, sum(counts), max(counts), H=H, dk=dk, dv=dv, **rows)
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dk, dv", [(128, 128), (64, 64), (128, 64), (64, 128)])
+def test_decay_attention_tiles(dk, dv, dtype):
+    """Chunks of 64: rows of one token, beside a chunk's end on either side, of more chunks than the scan has under way; decays whose
+    powers underflow and close to one; from states that are not zero."""
+    o = ops()
+    H, lens, slots = 3, [1, 63, 64, 65, 389], [2, 0, 4, 1, 5]
+    src, state, decays, rows = decay_case(lens, slots, H, dk, dv, dtype, [0.999, 0.02, 0.7], dk + dv)
+    st = state.clone()
+    assert o.decay_attention_tiles_supported(dk, dv, src.shape[1], 0, H * dk, 2 * H * dk) and not o.decay_attention_tiles_supported(96, dv, 8, 0, 0, 0)
+    out = decay_tiles(o, src, st, decays, rows, lens, H, dk, dv)
+    at = 0
+    for r, n in enumerate(lens):
+        y, S = decay_reference(src[at:at + n], state[slots[r]].double(), decays, H, dk, dv)
+        # the bound of the chunked kernels' own test
+        assert (out[at:at + n].double().view(n, H, dv) - y).abs().max() < 2e-5 * y.abs().max(), r
+        assert (st[slots[r]].double() - S).abs().max() < 2e-5 * S.abs().max(), r
+        at += n
+    assert torch.equal(st[3], state[3]) and torch.equal(st[6], state[6])
+
+
+def test_decay_attention_tiles_keep_later_tokens_out():
+    """An infinite value reaches its own token's group of four and what lies behind it, nothing before."""
+    o = ops()
+    lens, H = [100], 2
+    src, state, decays, rows = decay_case(lens, [0], H, 128, 128, torch.bfloat16, [0.9, 0.5], 3)
+    clean = decay_tiles(o, src, state.clone(), decays, rows, lens, H, 128, 128)
+    src[30, 2 * H * 128 + 5] = math.inf
+    out = decay_tiles(o, src, state.clone(), decays, rows, lens, H, 128, 128)
+    assert torch.equal(out[:28], clean[:28]) and not bool(torch.isfinite(out[30:, 5]).any())
