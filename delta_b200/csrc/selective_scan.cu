@@ -63,50 +63,76 @@ __global__ void conv_state_kernel(const T* __restrict__ xin, int in_stride, floa
 }
 
 // The same for 2 to 4 taps, C a multiple of 8 and 16-byte aligned rows: a thread takes eight channels of CONV_TOKENS tokens that
-// follow one another and keeps the window of inputs in registers, so every input is read once per tile.
+// follow one another and keeps the window of inputs in registers, so every input is read once per tile.  Bound by latency: the tile's
+// inputs, taps and rows are all asked for before the first product.  2,048 tokens of 6,144 channels,
+// bfloat16, four taps: 53 -> 27 us (50 MB).
 // grid (ceil(tokens / CONV_TOKENS), ceil(C / 8 / blockDim))
 constexpr int CONV_TOKENS = 8;
+
+// Eight neighbouring entries as they lie in memory.
+template <typename T>
+struct Eight {
+  uint4 v[sizeof(T) / 2];
+  __device__ __forceinline__ void get(const T* p) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) v[i] = reinterpret_cast<const uint4*>(p)[i];
+  }
+  __device__ __forceinline__ void floats(float (&x)[8]) const { load8<T>(reinterpret_cast<const T*>(v), x); }
+};
+
 template <typename T, int TAPS>
-__global__ void conv_silu_vec_kernel(const T* __restrict__ xin, int in_stride, const float* __restrict__ w, const float* __restrict__ bias,
+__global__ void __launch_bounds__(128) conv_silu_vec_kernel(const T* __restrict__ xin, int in_stride, const float* __restrict__ w, const float* __restrict__ bias,
                                      const float* __restrict__ conv_state, T* __restrict__ out, const int* __restrict__ tok_row,
                                      const int* __restrict__ row_slot, const int* __restrict__ row_q_start, int tokens, int C, int act) {
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   if (c >= C) return;
-  const int t_from = blockIdx.x * CONV_TOKENS, t_to = min(t_from + CONV_TOKENS, tokens);
-  float wv[TAPS][8], b[8], win[TAPS - 1][8];
+  const int t_from = blockIdx.x * CONV_TOKENS, n = min(CONV_TOKENS, tokens - t_from);
+  Eight<T> raw[CONV_TOKENS];
+  int rows[CONV_TOKENS];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    b[e] = bias ? bias[c + e] : 0.f;
+  for (int i = 0; i < CONV_TOKENS; ++i) {
+    const int t = t_from + min(i, n - 1);
+    raw[i].get(xin + (size_t)t * in_stride + c);
+    rows[i] = tok_row[t];
+  }
+  float wv[8 * TAPS], b[8], win[TAPS - 1][8];      // wv[e TAPS + j]: a channel's taps side by side, as they lie
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j) wv[j][e] = w[(size_t)(c + e) * TAPS + j];
+  for (int e = 0; e < 2 * TAPS; ++e) *reinterpret_cast<float4*>(wv + 4 * e) = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + 4 * e);
+  if (bias != nullptr) {
+    load8<float>(bias + c, b);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) b[e] = 0.f;
   }
   int row = -1;
-  for (int t = t_from; t < t_to; ++t) {
-    if (tok_row[t] != row) {      // the first token of the tile, or of a row: the inputs before it
-      row = tok_row[t];
+#pragma unroll
+  for (int i = 0; i < CONV_TOKENS; ++i) {
+    if (i >= n) break;
+    if (rows[i] != row) {      // the first token of the tile, or of a row: the inputs before it
+      row = rows[i];
       const int q0 = row_q_start[row];
       const float* st = conv_state + (size_t)row_slot[row] * (TAPS - 1) * C;
 #pragma unroll
       for (int j = 0; j < TAPS - 1; ++j) {
-        const int k = t - q0 - (TAPS - 1) + j;
+        const int k = t_from + i - q0 - (TAPS - 1) + j;
         if (k >= 0) load8<T>(xin + (size_t)(q0 + k) * in_stride + c, win[j]);
         else load8<float>(st + (size_t)(TAPS - 1 + k) * C + c, win[j]);
       }
     }
     float x[8], o[8];
-    load8<T>(xin + (size_t)t * in_stride + c, x);
+    raw[i].floats(x);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float acc = b[e];
 #pragma unroll
-      for (int j = 0; j < TAPS - 1; ++j) acc = fmaf(wv[j][e], win[j][e], acc);
-      acc = fmaf(wv[TAPS - 1][e], x[e], acc);
+      for (int j = 0; j < TAPS - 1; ++j) acc = fmaf(wv[e * TAPS + j], win[j][e], acc);
+      acc = fmaf(wv[e * TAPS + TAPS - 1], x[e], acc);
       o[e] = act ? acc / (1.f + expf(-acc)) : acc;
 #pragma unroll
       for (int j = 0; j + 1 < TAPS - 1; ++j) win[j][e] = win[j + 1][e];
       win[TAPS - 2][e] = x[e];
     }
-    store8<T>(out + (size_t)t * C + c, o);
+    store8<T>(out + (size_t)(t_from + i) * C + c, o);
   }
 }
 
@@ -309,7 +335,7 @@ extern "C" int dk_conv_silu(const void* xin, int in_stride, const float* w, cons
     return dk_check_launch("conv_silu");
   }
   if (taps >= 2 && taps <= 4 && in_bias == nullptr && C % 8 == 0 && in_stride % 8 == 0 && ((uintptr_t)xin % 16) == 0 && ((uintptr_t)out % 16) == 0 &&
-      ((uintptr_t)conv_state % 16) == 0) {
+      (((uintptr_t)conv_state | (uintptr_t)w | (uintptr_t)bias) % 16) == 0) {
     const dim3 gv((T_ + CONV_TOKENS - 1) / CONV_TOKENS, (C / 8 + 127) / 128);
 #define VEC(T, TAPS)                                                                                                              \
   conv_silu_vec_kernel<T, TAPS><<<gv, 128, 0, stream>>>((const T*)xin, in_stride, w, bias, conv_state, (T*)out, tok_row, row_slot, row_q_start, \
