@@ -1,7 +1,6 @@
 // y[M,N] = x[M,K] W[N,K]^T on the fifth-generation tensor cores, for decode steps (M up to
 // 128 rows): the weights stream once through shared memory by TMA and never touch
-// registers.  More rows (prompt portions) are taken in chunks of up to 256 by one block per
-// (tile of W, chunk), as a measure of what the library's product is worth there.
+// registers.  More rows (prompt portions) are gemm_rows_tc.cu's.
 //
 // "Swap AB": a block owns 128 rows of W, which are the M side of a tcgen05.mma tile
 // (A operand), and all M activation rows, padded to a multiple of 16, are its N side (B
@@ -48,17 +47,7 @@ struct TcArgs {
   int swiglu;        // rows of the tile: 64 gate rows then the 64 up rows that belong to them
   int n_up;          // first up row in W (= columns of the output) when swiglu
   int tmem_cols;
-  int ksub;          // boxes of 64 elements of K per stage (4, or 2 or 1 when many rows leave less room)
-  int chunks;        // groups of mpad rows of x: block (tile, chunk) makes rows [chunk * mpad, ...) of the tile's columns
-  // grouped products (a mixture of experts): chunk c of x meets the matrix of expert chunk_expert[c], whose rows start at
-  // expert * expert_rows of W; chunks with a negative expert are left out.  row_map: output row of every row of x (negative:
-  // the row is not stored).  glu: the epilogue is the gated activation with clamped branches instead of silu(gate) * up.
-  const int* chunk_expert;
-  const int* row_map;
-  int expert_rows;
-  int glu;
-  float glu_limit, glu_alpha, glu_shift;
-  int relu_squared;  // the epilogue of a product of one branch: relu(y)^2 of the rounded product
+  int ksub;          // boxes of 64 elements of K per stage (4, or 2 when many rows leave less room)
 };
 
 __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,
@@ -77,17 +66,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
   cg::cluster_group cluster = cg::this_cluster();
   const int splits = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
-  // 128 rows of W (64 + 64 with the SwiGLU epilogue).  The chunks of one tile are neighbours in the grid, so that
-  // a tile of W is fetched from memory once and then found in the L2 by the blocks of the other chunks.
-  const int tile = blockIdx.x / a.chunks;
-  const int m0 = (blockIdx.x % a.chunks) * a.mpad;    // first row of x and of the output of this block
-  int w_row0 = 0;                                     // first row of this block's matrix in W
-  if (a.chunk_expert != nullptr) {
-    const int expert = a.chunk_expert[blockIdx.x % a.chunks];
-    if (expert < 0) return;                           // before anything is asked for or handed out: the whole block leaves
-    w_row0 = expert * a.expert_rows;
-  }
-  const int m_here = min(a.mpad, a.M - m0);
+  const int tile = blockIdx.x;      // 128 rows of W (64 + 64 with the SwiGLU epilogue)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rows_out = a.swiglu ? 64 : TILE_ROWS;    // output columns this tile makes
   const int n0 = tile * rows_out;
@@ -116,12 +95,12 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
       const int kc = ((ks_begin + i) * KSUB + sub) * KSTEP;     // past K the boxes are filled with zeros
       const uint32_t dst = dst0 + sub * a_bytes;
       if (a.swiglu) {
-        tma_load_2d(dst, &map_w, kc, w_row0 + n0, full0 + 8 * s);                           // 64 gate rows
-        tma_load_2d(dst + 64 * KSTEP * 2, &map_w, kc, w_row0 + a.n_up + n0, full0 + 8 * s);  // their 64 up rows
+        tma_load_2d(dst, &map_w, kc, n0, full0 + 8 * s);                           // 64 gate rows
+        tma_load_2d(dst + 64 * KSTEP * 2, &map_w, kc, a.n_up + n0, full0 + 8 * s);  // their 64 up rows
       } else {
-        tma_load_2d(dst, &map_w, kc, w_row0 + n0, full0 + 8 * s);
+        tma_load_2d(dst, &map_w, kc, n0, full0 + 8 * s);
       }
-      tma_load_2d(dst0 + KSUB * a_bytes + sub * b_bytes, &map_x, kc, m0, full0 + 8 * s);   // rows past M are zeros
+      tma_load_2d(dst0 + KSUB * a_bytes + sub * b_bytes, &map_x, kc, 0, full0 + 8 * s);   // rows past M are zeros
     }
   };
   // The first round of the ring needs nothing but the barriers this thread has just made: it is asked for
@@ -204,7 +183,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
   const float* parts[8];
 #pragma unroll
   for (int b = 0; b < 8; ++b) parts[b] = (b < splits && splits > 1) ? cluster.map_shared_rank(part, b) : part;
-  for (int item = tid; item < groups * m_here; item += TC_THREADS) {
+  for (int item = tid; item < groups * a.M; item += TC_THREADS) {
     const int m = item / groups, r = r_begin + (item % groups) * 8;
     float4 g0[8], g1[8], u0[8], u1[8];
 #pragma unroll
@@ -233,26 +212,12 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     }
     const int n = n0 + r;
     if (good && n < (a.swiglu ? a.n_up : a.N)) {     // N and the first up row are multiples of 8: a group is in or out as a whole
-      if (a.swiglu && a.glu) {      // both products rounded to bfloat16 first, as separate products would be
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          y[i] = dk_glu_value(__bfloat162float(__float2bfloat16_rn(y[i])), __bfloat162float(__float2bfloat16_rn(u[i])), a.glu_limit,
-                              a.glu_alpha, a.glu_shift);
-      } else if (a.swiglu) {
+      if (a.swiglu) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) y[i] = y[i] / (1.f + expf(-y[i])) * u[i];
-      } else if (a.relu_squared) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float v = fmaxf(__bfloat162float(__float2bfloat16_rn(y[i])), 0.f);
-          y[i] = v * v;
-        }
       }
-      long long out_row = m0 + m;
-      if (a.row_map != nullptr) out_row = a.row_map[m0 + m];
-      if (out_row < 0) continue;
       if (a.out_f32) {
-        float* dst = (float*)a.out + (size_t)out_row * a.ldc + n;
+        float* dst = (float*)a.out + (size_t)m * a.ldc + n;
         *reinterpret_cast<float4*>(dst) = make_float4(y[0], y[1], y[2], y[3]);
         *reinterpret_cast<float4*>(dst + 4) = make_float4(y[4], y[5], y[6], y[7]);
       } else {
@@ -263,7 +228,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         st.y = *reinterpret_cast<uint32_t*>(&p1);
         st.z = *reinterpret_cast<uint32_t*>(&p2);
         st.w = *reinterpret_cast<uint32_t*>(&p3);
-        *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + (size_t)out_row * a.ldc + n) = st;
+        *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + (size_t)m * a.ldc + n) = st;
       }
     }
   }
@@ -273,8 +238,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
   }
 }
 
-// The kernel's allowance of dynamic shared memory only ever grows, and both launchers below keep one record of it per
-// device: a second record would let one launcher lower what the other believes it has.
+// The kernel's allowance of dynamic shared memory only ever grows; one record of it per device.
 bool grant_shared_memory(size_t smem) {
   static size_t configured_on[DK_MAX_DEVICES] = {0};
   size_t& configured = configured_on[dk_current_device()];
@@ -303,13 +267,6 @@ extern "C" int dk_gemm_tc_supported(int M, int N, int K, int swiglu) {
   return 1;
 }
 
-// More than 128 rows (prompt portions): the same kernel with the rows of x in chunks of up to 256, one block per
-// (tile of W, chunk); K is not split and a block has the SM to itself.
-extern "C" int dk_gemm_tc_many_rows_supported(int M, int N, int K, int swiglu) {
-  if (M <= 128 || M > (1 << 20)) return 0;
-  return dk_gemm_tc_supported(128, N, K, swiglu);
-}
-
 // splits: blocks that share K as one cluster (1, 2, 4 or 8).  out_dtype DK_BF16 or DK_F32.
 // per_sm: 1, or 2 to size the ring of stages so that two blocks share an SM's shared memory (stages of half the
 // length): with more tiles than SMs but no more than twice as many (11,008 SwiGLU columns are 172 tiles), all
@@ -317,10 +274,7 @@ extern "C" int dk_gemm_tc_many_rows_supported(int M, int N, int K, int swiglu) {
 extern "C" int dk_gemm_tc(const void* x, const void* W, void* out, int M, int N, int K, int lda, int ldw, int ldc,
                           int out_dtype, int swiglu, int splits, int per_sm, int* err, cudaStream_t stream) {
   DK_REQUIRE(per_sm == 1 || per_sm == 2, "gemm_tc: per_sm must be 1 or 2, got %d", per_sm);
-  const bool many = M > 128;
-  DK_REQUIRE(many ? dk_gemm_tc_many_rows_supported(M, N, K, swiglu) : dk_gemm_tc_supported(M, N, K, swiglu),
-             "gemm_tc: sizes not taken: M=%d N=%d K=%d swiglu=%d", M, N, K, swiglu);
-  DK_REQUIRE(!many || (splits == 1 && per_sm == 1), "gemm_tc: more than 128 rows go with splits=1 and per_sm=1 (got %d, %d)", splits, per_sm);
+  DK_REQUIRE(dk_gemm_tc_supported(M, N, K, swiglu), "gemm_tc: sizes not taken: M=%d N=%d K=%d swiglu=%d", M, N, K, swiglu);
   DK_REQUIRE(splits == 1 || splits == 2 || splits == 4 || splits == 8, "gemm_tc: splits must be 1, 2, 4 or 8, got %d", splits);
   DK_REQUIRE((lda % 8) == 0 && (ldw % 8) == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)W % 16) == 0,
              "gemm_tc: operands must start on 16-byte boundaries with leading sizes that are multiples of 8");
@@ -328,24 +282,17 @@ extern "C" int dk_gemm_tc(const void* x, const void* W, void* out, int M, int N,
   DK_REQUIRE((ldc % 8) == 0 && ((uintptr_t)out % 16) == 0,
              "gemm_tc: the output must start on a 16-byte boundary with a leading size that is a multiple of 8");
   TcArgs a;
-  a.chunk_expert = nullptr;
-  a.row_map = nullptr;
-  a.expert_rows = 0;
-  a.glu = 0;
-  a.relu_squared = 0;
-  a.glu_limit = a.glu_alpha = a.glu_shift = 0.f;
   a.out = out;
   a.err = err;
   a.M = M; a.N = N; a.K = K; a.ldc = ldc;
-  a.mpad = M > 256 ? 256 : (M + 15) / 16 * 16;
-  a.chunks = (M + a.mpad - 1) / a.mpad;
+  a.mpad = (M + 15) / 16 * 16;
   a.out_f32 = out_dtype == DK_F32;
   a.swiglu = swiglu;
   a.n_up = swiglu ? N / 2 : 0;
-  a.tmem_cols = a.mpad <= 32 ? 32 : (a.mpad <= 64 ? 64 : (a.mpad <= 128 ? 128 : 256));
+  a.tmem_cols = a.mpad <= 32 ? 32 : (a.mpad <= 64 ? 64 : 128);
   const int a_bytes = TILE_ROWS * KSTEP * 2;
   const int b_bytes = a.mpad * KSTEP * 2;
-  a.ksub = per_sm == 2 ? 2 : (a.mpad <= 64 ? KSUB_MAX : (a.mpad <= 128 ? 2 : 1));
+  a.ksub = per_sm == 2 ? 2 : (a.mpad <= 64 ? KSUB_MAX : 2);
   const int stage_bytes = a.ksub * (a_bytes + b_bytes);
   const int part_bytes = a.mpad * TILE_ROWS * 4;
   int stages = ((224 * 1024) / per_sm - 2048) / stage_bytes;
@@ -366,8 +313,7 @@ extern "C" int dk_gemm_tc(const void* x, const void* W, void* out, int M, int N,
   const int n_out = swiglu ? N / 2 : N;
   const int tiles = (n_out + rows_out - 1) / rows_out;
   cudaLaunchConfig_t cfg = {};
-  DK_REQUIRE((long long)tiles * a.chunks < (1ll << 31), "gemm_tc: too many blocks");
-  cfg.gridDim = dim3(tiles * a.chunks, splits, 1);
+  cfg.gridDim = dim3(tiles, splits, 1);
   cfg.blockDim = dim3(TC_THREADS, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -384,83 +330,4 @@ extern "C" int dk_gemm_tc(const void* x, const void* W, void* out, int M, int N,
     return DK_ERR_LAUNCH;
   }
   return dk_check_launch("gemm_tc");
-}
-
-// Grouped products for a mixture of experts: x [M, K] holds the rows of all experts in tiles of `tile_m` (128 or 256) rows,
-// tile c belonging to expert chunk_expert[c] (negative: no rows); W [E * expert_rows, K] holds the experts' matrices one
-// after the other, [gate (n) | up (n)] rows each when `glu`, else n rows.  out[row_map ? row_map[r] : r][0..n) for every row
-// r of x (rows mapped to a negative number are not stored).  `glu` 2: n rows each and the epilogue relu(y)^2.  One block per (128 rows of an expert's matrix, tile of x).
-extern "C" int dk_experts_gemm_tc_supported(int n, int K, int glu) {
-  return dk_gemm_tc_supported(128, glu ? 2 * n : n, K, glu);
-}
-
-extern "C" int dk_experts_gemm_tc(const void* x, const void* W, void* out, const int* chunk_expert, const int* row_map, int M,
-                                  int tile_m, int n, int K, int E, int ldc, int out_dtype, int glu, float limit, float alpha,
-                                  float shift, int* err, cudaStream_t stream) {
-  if (M == 0) return 0;
-  const int relu_squared = glu == 2;      // glu: 0 the plain product, 1 the gated activation, 2 one branch through relu(y)^2
-  glu = glu == 1;
-  DK_REQUIRE(tile_m == 128 || tile_m == 256, "experts_gemm_tc: tiles of 128 or 256 rows, got %d", tile_m);
-  DK_REQUIRE(M > 0 && M % tile_m == 0 && E > 0, "experts_gemm_tc: %d rows are no whole tiles of %d", M, tile_m);
-  DK_REQUIRE(dk_experts_gemm_tc_supported(n, K, glu), "experts_gemm_tc: sizes not taken: n=%d K=%d glu=%d", n, K, glu);
-  DK_REQUIRE(((uintptr_t)x % 16) == 0 && ((uintptr_t)W % 16) == 0 && ((uintptr_t)out % 16) == 0 && (ldc % 8) == 0,
-             "experts_gemm_tc: operands must start on 16-byte boundaries with leading sizes that are multiples of 8");
-  DK_REQUIRE(out_dtype == DK_BF16 || out_dtype == DK_F32, "experts_gemm_tc: unknown output dtype %d", out_dtype);
-  DK_REQUIRE(chunk_expert != nullptr, "experts_gemm_tc: no tile map");
-  TcArgs a;
-  a.chunk_expert = chunk_expert;
-  a.row_map = row_map;
-  a.expert_rows = glu ? 2 * n : n;
-  a.glu = glu;
-  a.relu_squared = relu_squared;
-  a.glu_limit = limit; a.glu_alpha = alpha; a.glu_shift = shift;
-  a.out = out;
-  a.err = err;
-  a.M = M; a.N = n; a.K = K; a.ldc = ldc;
-  a.mpad = tile_m;
-  a.chunks = M / tile_m;
-  a.out_f32 = out_dtype == DK_F32;
-  a.swiglu = glu;
-  a.n_up = glu ? n : 0;
-  a.tmem_cols = tile_m;
-  const int a_bytes = TILE_ROWS * KSTEP * 2;
-  const int b_bytes = a.mpad * KSTEP * 2;
-  a.ksub = a.mpad <= 128 ? 2 : 1;
-  const int stage_bytes = a.ksub * (a_bytes + b_bytes);
-  const int part_bytes = a.mpad * TILE_ROWS * 4;
-  int stages = (224 * 1024 - 2048) / stage_bytes;
-  if (stages > 8) stages = 8;
-  DK_REQUIRE(stages >= 2, "experts_gemm_tc: no room for two stages");
-  a.stages = stages;
-  size_t smem = (size_t)stages * stage_bytes;
-  if (smem < (size_t)part_bytes) smem = part_bytes;
-  smem += 1024;
-  CUtensorMap map_w, map_x;
-  DK_REQUIRE(make_map(&map_w, W, (long long)E * a.expert_rows, K, K, glu ? 64 : TILE_ROWS), "experts_gemm_tc: cannot encode the tensor map of W");
-  DK_REQUIRE(make_map(&map_x, x, M, K, K, a.mpad), "experts_gemm_tc: cannot encode the tensor map of x");
-  if (!grant_shared_memory(smem)) {
-    dk_set_error("experts_gemm_tc: cannot get %zu bytes of shared memory", smem);
-    return DK_ERR_LAUNCH;
-  }
-  const int rows_out = glu ? 64 : TILE_ROWS;
-  const int tiles = (n + rows_out - 1) / rows_out;
-  cudaLaunchConfig_t cfg = {};
-  DK_REQUIRE((long long)tiles * a.chunks < (1ll << 31), "experts_gemm_tc: too many blocks");
-  cfg.gridDim = dim3(tiles * a.chunks, 1, 1);
-  cfg.blockDim = dim3(TC_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel, map_w, map_x, a);
-  if (e != cudaSuccess) {
-    dk_set_error("experts_gemm_tc: launch failed: %s", cudaGetErrorString(e));
-    return DK_ERR_LAUNCH;
-  }
-  return dk_check_launch("experts_gemm_tc");
 }

@@ -192,3 +192,20 @@ def test_decay_attention_tiles_keep_later_tokens_out():
     src[30, 2 * H * 128 + 5] = math.inf
     out = decay_tiles(o, src, state.clone(), decays, rows, lens, H, 128, 128)
     assert torch.equal(out[:28], clean[:28]) and not bool(torch.isfinite(out[30:, 5]).any())
+
+
+@pytest.mark.parametrize("M, N, K", [(700, 22016, 264), (129, 8, 64), (257, 136, 72), (5000, 264, 64), (1300, 4104, 520)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gemm_rows_tc_pieces(M, N, K, dtype):
+    """More pieces than both accumulators of every SM, a single piece, rows and columns beside a piece's edge, K that ends inside a box."""
+    o = ops()
+    torch.manual_seed(M + N)
+    err = o.new_error_record(DEV)
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn(N, K, device=DEV) * 0.1).bfloat16()
+    out = torch.full((M + 2, N), 9.0, dtype=dtype, device=DEV)
+    o.gemm_tc(x, w, out[:M], err=err)
+    o.raise_if_error(err)
+    ref = x.double() @ w.double().T
+    # products are exact in 32 bit; a sum of K of them, rounded at every step, and one rounding to bfloat16
+    bound = K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + (ref.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+    assert bool(((out[:M].double() - ref).abs() <= bound + 1e-6).all()) and bool((out[M:] == 9.0).all())
