@@ -656,6 +656,15 @@ def attention_rows_mma(params: RowAttnParams, max_m: int, splits: int = 1, scrat
                                              _stream()), "attention_rows_mma", 2 if splits > 1 else 1)
 
 
+def attention_rows_wide_supported(params: RowAttnParams) -> bool:
+    return bool(_l.load().dk_attention_rows_wide_supported(C.byref(params)))
+
+
+def attention_rows_wide(params: RowAttnParams, max_q_len: int):
+    """``attention_rows_tc`` for values that are the front part of their keys, keys of up to 320 and values of up to 256 entries."""
+    _l.check(_l.load().dk_attention_rows_wide(C.byref(params), int(max_q_len), _stream()), "attention_rows_wide")
+
+
 def attention_rows_tc_supported(params: RowAttnParams) -> bool:
     """True when the tcgen05 kernel of the family takes these sizes (bfloat16; key and value sizes multiples of 8 from 64 to 128; no shaped
     scores)."""

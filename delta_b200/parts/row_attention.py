@@ -85,11 +85,16 @@ def run(ctx, params) -> None:
     chosen from the step's host data."""
     singles = ctx.decode_only or any(n == 1 for n in ctx.host["q_lens"])
     several = not ctx.decode_only
-    tc = several and not plain(ctx) and ctx.max_q_len >= TC_MIN_TOKENS and ops.attention_rows_tc_supported(params)
+    tc = None      # the tcgen05 kernel that takes these sizes
+    if several and not plain(ctx) and ctx.max_q_len >= TC_MIN_TOKENS:
+        if ops.attention_rows_tc_supported(params):
+            tc = ops.attention_rows_tc
+        elif ops.attention_rows_wide_supported(params):
+            tc = ops.attention_rows_wide
     if plain(ctx) or not ops.attention_rows_mma_supported(params):
         params.row_filter = 0
-        if tc and not singles:
-            ops.attention_rows_tc(params, ctx.max_q_len)
+        if tc is not None and not singles:
+            tc(params, ctx.max_q_len)
         else:
             ops.attention_rows_plain(params)
         return
@@ -111,8 +116,8 @@ def run(ctx, params) -> None:
         ops.attention_rows_mma(params, group, splits, scratch)
     if several:
         params.row_filter = 2 if singles else 0
-        if tc:
-            ops.attention_rows_tc(params, ctx.max_q_len)
+        if tc is not None:
+            tc(params, ctx.max_q_len)
             return
         ops.attention_rows_mma(params, ctx.max_q_len * group, 1, None)
 
