@@ -209,3 +209,26 @@ def test_gemm_rows_tc_pieces(M, N, K, dtype):
     # products are exact in 32 bit; a sum of K of them, rounded at every step, and one rounding to bfloat16
     bound = K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + (ref.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
     assert bool(((out[:M].double() - ref).abs() <= bound + 1e-6).all()) and bool((out[M:] == 9.0).all())
+
+
+@pytest.mark.parametrize("scoring, correction, groups", [("softmax", False, None), ("sigmoid", True, (4, 2)), ("softmax_all", True, (4, 2)), ("sigmoid", False, None)])
+@pytest.mark.parametrize("T, rows, E, d", [(128, 17, 16, 64), (201, 20, 20, 2048), (2048, 16, 16, 1024), (130, 72, 64, 96)])
+def test_router_of_many_tokens(T, rows, E, d, scoring, correction, groups):
+    """Tiles of 16 tokens and 32 rows, the last ones partly filled; blocks of 32 entries that not every warp has."""
+    o = ops()
+    torch.manual_seed(T + rows)
+    x, w = torch.randn(T, d, device=DEV).bfloat16(), (torch.randn(rows, d, device=DEV) * 0.05).bfloat16()
+    cor = torch.rand(E, device=DEV) * 0.1 if correction else None
+    top = 4
+    z = torch.full((T + 1, rows), 9.0, device=DEV)
+    choice, weight = torch.full((T, top), -5, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    o.router(x, w, E, top, z[:T], choice, weight, scoring=scoring, correction=cor, scale=1.5, normalize=True, groups=groups)
+    ref = x.double() @ w.double().T
+    # exact products; their sum in 32 bit, rounded at every one of d steps at most
+    assert bool(((z[:T].double() - ref).abs() <= 2.0 ** -23 * d * (x.double().abs() @ w.double().abs().T) / 8 + 1e-7).all()) and bool((z[T] == 9.0).all())
+    assert (z[:T].double() - ref).norm() < 3e-7 * ref.norm()
+    # the same tokens one at a time: another kernel, the same choice wherever the scores are not a rounding apart
+    for t in range(0, T, 37):
+        z1, c1, w1 = torch.empty(1, rows, device=DEV), torch.empty(1, top, dtype=torch.int32, device=DEV), torch.empty(1, top, device=DEV)
+        o.router(x[t:t + 1].contiguous(), w, E, top, z1, c1, w1, scoring=scoring, correction=cor, scale=1.5, normalize=True, groups=groups)
+        assert torch.allclose(z1[0], z[t], atol=2e-6, rtol=2e-6) and torch.equal(c1[0], choice[t]) and torch.allclose(w1[0], weight[t], atol=1e-5, rtol=1e-5)
