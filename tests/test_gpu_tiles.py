@@ -232,3 +232,40 @@ def test_router_of_many_tokens(T, rows, E, d, scoring, correction, groups):
         z1, c1, w1 = torch.empty(1, rows, device=DEV), torch.empty(1, top, dtype=torch.int32, device=DEV), torch.empty(1, top, device=DEV)
         o.router(x[t:t + 1].contiguous(), w, E, top, z1, c1, w1, scoring=scoring, correction=cor, scale=1.5, normalize=True, groups=groups)
         assert torch.allclose(z1[0], z[t], atol=2e-6, rtol=2e-6) and torch.equal(c1[0], choice[t]) and torch.allclose(w1[0], weight[t], atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H, KV, dk, dv", [(16, 4, 128, 128), (3, 1, 64, 24), (5, 5, 8, 8), (4, 0, 32, 16), (2, 1, 256, 256)])
+@pytest.mark.parametrize("norm, rot, interleaved, unit, from_key, bias", [("whole", 0, False, False, False, True), ("head", 32, False, False, False, True),
+                                                                          (None, 16, True, True, True, False), (None, 8, True, False, False, False),
+                                                                          ("head", 16, False, True, True, True)])
+def test_rows_append_unit_wide_accesses(H, KV, dk, dv, dtype, norm, rot, interleaved, unit, from_key, bias):
+    """Rows that begin on 16-byte boundaries beside the same rows one element off, which the narrow kernel takes."""
+    o = ops()
+    if rot > dk or (from_key and dv > dk) or (rot and not interleaved and rot % 16):
+        pytest.skip("no such head")
+    g = torch.Generator().manual_seed(H * dk + dv)
+    T, ps = 37, 8
+    cols = (H + KV) * dk + (0 if from_key else KV * dv)
+    data = torch.randn(T, cols, generator=g).to(dtype)
+    f = lambda *s: torch.randn(*s, generator=g).to(DEV)      # noqa: E731
+    b = f((H + KV) * dk + (0 if from_key else KV * dv)) * 0.1 if bias else None
+    qn, kn = (f(H * dk if norm == "whole" else dk), f(max(KV, 1) * dk if norm == "whole" else dk) if KV else None) if norm else (None, None)
+    table = f(T, rot // 2, 2) if rot else None
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    pos, row, bt = i32(list(range(T))), i32([0] * T), i32([[4, 2, 0, 1, 3]])
+    got = []
+    for pad in (8, 9):
+        src = torch.zeros(T, cols + pad, dtype=dtype)
+        src[:, :cols] = data
+        src = src.to(DEV)
+        cache = torch.zeros(5, KV, ps, dk + dv, dtype=dtype, device=DEV) if KV else None
+        err = o.new_error_record(DEV)
+        o.rows_append_unit(src, pos, row, bt, cache, H=H, KV=KV, dk=dk, dv=dv, ps=ps, row_width=dk + dv, k_off=0, v_off=dk, table=table, rot_dims=rot,
+                           interleaved=interleaved, unit_eps=1e-5 if unit else None, value_from_key=from_key, bias=b, q_norm=qn, k_norm=kn,
+                           pre_eps=1e-5, norm_whole=norm == "whole", q_temp=(0.3, 5), err=err)
+        o.raise_if_error(err)
+        got.append((src[:, :cols].double(), cache.double() if KV else torch.zeros(1)))
+    tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8      # sums of squares in another order; in bfloat16 the last bit of the one rounding
+    for a, c in zip(*got):
+        assert (a - c).abs().max() <= tol * c.abs().max().clamp(min=1.0)
