@@ -39,6 +39,7 @@
 #include "common.cuh"
 #include "attention_params.h"
 #include "tcgen05_helpers.cuh"
+#include "attention_pieces.cuh"
 #include <cstdlib>
 
 namespace {
@@ -78,20 +79,29 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// One piece of work: 128 queries of one head of one row.  Pieces are numbered with the head fastest, then the rows,
-// then the query tiles of each row from its latest (which has the most keys) to its first: from long to short.
+// One piece of work: 128 queries of one head of one row.  Pieces are numbered with the head fastest, then as the block's list has them
+// (attention_pieces.cuh); without a list by the rows, then the query tiles of each row from its latest (which has the most keys) to its first.
 struct Piece {
   int row, h, qt, nq, t0, pos0, last_pos, kt_first, n_tiles, first_page, last_page;
   bool valid;
 };
 
-__device__ __forceinline__ Piece piece_of(const DkAttnParams& p, int index, int row_lo, int n_rows) {
+constexpr int LISTED = 64;      // pairs of row and query tile that the list holds
+
+__device__ __forceinline__ Piece piece_of(const DkAttnParams& p, int index, int row_lo, int n_rows, const uint32_t* list, int listed) {
   Piece w;
   w.h = index % p.H;
-  w.row = row_lo + (index / p.H) % n_rows;
-  const int yy = index / (p.H * n_rows);                // 0: the row's latest query tile, which has the most keys
-  const int q_len = p.row_q_len[w.row];
-  w.qt = (q_len + QT - 1) / QT - 1 - yy;
+  int q_len;
+  if (listed >= 0) {
+    const uint32_t pair = list[index / p.H];
+    w.row = (pair >> 9) & 511;
+    w.qt = pair & 511;
+    q_len = p.row_q_len[w.row];
+  } else {
+    w.row = row_lo + (index / p.H) % n_rows;
+    q_len = p.row_q_len[w.row];
+    w.qt = (q_len + QT - 1) / QT - 1 - index / (p.H * n_rows);      // 0: the row's latest query tile, which has the most keys
+  }
   const int q0 = w.qt * QT;
   w.valid = !(p.row_filter == 2 && q_len == 1) && w.qt >= 0;
   w.nq = min(QT, q_len - q0);
@@ -131,6 +141,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int failed;
   __shared__ int row_range[2];
+  __shared__ PieceList<LISTED> pieces;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ps = p.ps, G = p.H / p.KV;
@@ -180,12 +191,16 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
       row_range[1] = hi;
     }
   }
+  const int listed = list_pieces<LISTED>(pieces, p.row_q_len, p.rows, p.row_filter == 2, QT, [&](int row, int qt) {
+    const int pos0 = p.row_pos_start[row] + qt * QT, last = p.row_pos_start[row] + min(p.row_q_len[row], (qt + 1) * QT) - 1;
+    return last / KT - ((p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0) / KT + 1;
+  });
   if (warp == MMA_WARP) tmem_alloc(s2u(&tmem_slot), TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const int row_lo = row_range[0], n_rows = max(0, row_range[1] - row_range[0] + 1);
-  const int n_pieces = p.H * n_qt * n_rows;
+  const int n_pieces = p.H * (listed >= 0 ? listed : n_qt * n_rows);
   // The pieces a block takes: in rounds of gridDim.x pieces, forwards in the even rounds and backwards in the odd ones.
   // Pieces are numbered from long to short, so a block that got a long one in one round gets a short one in the next,
   // and all blocks end at about the same time without asking each other anything.
@@ -220,7 +235,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
     for (int round = 0; round * (int)gridDim.x < n_pieces && !failed; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece w = piece_of(p, index, row_lo, n_rows);
+      const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       const int kvh = w.h / G;
       if (kind == 0) {
@@ -293,7 +308,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
     for (int round = 0; ok && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece w = piece_of(p, index, row_lo, n_rows);
+      const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       ok = wait_all(q_full, n_done & 1);
       for (int j = 0; ok && j < w.n_tiles; ++j) {
@@ -328,7 +343,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
     for (int round = 0; ok && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece w = piece_of(p, index, row_lo, n_rows);
+      const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       for (int j = 0; ok && j < w.n_tiles; ++j) {
         const int c = j & 1, ord = (c ? had1 : had0) + j / 2;
@@ -367,7 +382,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
     for (int round = 0; good && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece pc = piece_of(p, index, row_lo, n_rows);
+      const Piece pc = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!pc.valid) continue;
       const int n_tiles = pc.n_tiles, pos0 = pc.pos0, last_pos = pc.last_pos, kt_first = pc.kt_first, nq = pc.nq, t0 = pc.t0, h = pc.h;
       const int qpos = pos0 + r;

@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "row_attention_params.h"
 #include "tcgen05_helpers.cuh"
+#include "attention_pieces.cuh"
 
 namespace {
 constexpr int QT = 128, KT = 64, DKP = 320, DVP = 256;
@@ -47,11 +48,14 @@ struct Piece {
   int row, h, nq, t0, pos0, kt_first, n_tiles, first_page, last_page;
 };
 
-// Pieces are numbered with the head fastest, then the rows, then a row's query tiles from its latest (which has the most keys) on.
-__device__ __forceinline__ bool piece_of(const DkRowAttnParams& p, int index, Piece& w) {
+constexpr int LISTED = 256;      // pairs of row and query tile that the list holds
+
+// Pieces are numbered with the head fastest, then as the block's list has them (attention_pieces.cuh); without a list by the rows, then a row's
+// query tiles from its latest (which has the most keys) on.
+__device__ __forceinline__ bool piece_of(const DkRowAttnParams& p, int index, const uint32_t* list, int listed, Piece& w) {
   w.h = index % p.H;
-  w.row = (index / p.H) % p.rows;
-  const int q_len = p.row_q_len[w.row], qt = (q_len + QT - 1) / QT - 1 - index / (p.H * p.rows);
+  w.row = listed >= 0 ? (list[index / p.H] >> 9) & 511 : (index / p.H) % p.rows;
+  const int q_len = p.row_q_len[w.row], qt = listed >= 0 ? (int)(list[index / p.H] & 511) : (q_len + QT - 1) / QT - 1 - index / (p.H * p.rows);
   if (qt < 0 || (p.row_filter == 2 && q_len == 1)) return false;
   w.nq = min(QT, q_len - qt * QT);
   w.t0 = p.row_q_start[w.row] + qt * QT;
@@ -71,12 +75,13 @@ struct Bars {
 
 __global__ void __launch_bounds__(THREADS, 1)
 attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                           const __grid_constant__ CUtensorMap map_k_run, const DkRowAttnParams p, const int n_pieces) {
+                           const __grid_constant__ CUtensorMap map_k_run, const DkRowAttnParams p, const int n_qt) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) Bars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int failed;
+  __shared__ PieceList<LISTED> pieces;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t q_full = s2u(&bars.q_full), q_empty = s2u(&bars.q_empty), k_full = s2u(bars.k_full), k_empty = s2u(bars.k_empty),
                  s_full = s2u(bars.s_full), p_full = s2u(bars.p_full), o_done = s2u(bars.o_done);
@@ -95,6 +100,11 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  const int listed = list_pieces<LISTED>(pieces, p.row_q_len, p.rows, p.row_filter == 2, QT, [&](int row, int qt) {
+    const int pos0 = p.row_pos_start[row] + qt * QT, last = p.row_pos_start[row] + min(p.row_q_len[row], (qt + 1) * QT) - 1;
+    return last / KT - row_first_key(p, pos0) / KT + 1;
+  });
+  const int n_pieces = p.H * (listed >= 0 ? listed : n_qt * p.rows);
   if (warp == 5) tmem_alloc(s2u(&tmem_slot), TMEM_COLS);
   tc_fence_before();
   __syncthreads();
@@ -112,7 +122,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const int ppt = KT / p.ps;      // pages of a tile
     for (int round = 0; round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
-      if (index >= n_pieces || !piece_of(p, index, w)) continue;
+      if (index >= n_pieces || !piece_of(p, index, pieces.sorted, listed, w)) continue;
       if (!together(done == 0 || mbar_wait(q_empty, (done - 1) & 1))) { failed = 1; break; }
       if (lane == 0) {
         mbar_expect_tx(q_full, BOXES * Q_BOX);
@@ -160,7 +170,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     bool ok = true;
     for (int round = 0; ok && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
-      if (index >= n_pieces || !piece_of(p, index, w)) continue;
+      if (index >= n_pieces || !piece_of(p, index, pieces.sorted, listed, w)) continue;
       ok = together(mbar_wait(q_full, done & 1));
       for (int j = 0; ok && j < w.n_tiles; ++j, ++g) {
         const int s = g % STAGES, c = g & 1;
@@ -187,7 +197,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     bool ok = true;
     for (int round = 0; ok && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
-      if (index >= n_pieces || !piece_of(p, index, w)) continue;
+      if (index >= n_pieces || !piece_of(p, index, pieces.sorted, listed, w)) continue;
       for (int j = 0; j < w.n_tiles; ++j, ++g) {
         const int s = g % STAGES, c = g & 1;
         ok = together(mbar_wait(k_full + 8 * s, (g / STAGES) & 1) && mbar_wait(p_full + 8 * c, (g >> 1) & 1));
@@ -217,7 +227,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll 1
     for (int round = 0; good && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
-      if (index >= n_pieces || !piece_of(p, index, w)) continue;
+      if (index >= n_pieces || !piece_of(p, index, pieces.sorted, listed, w)) continue;
       const int qpos = w.pos0 + r, last_pos = w.pos0 + w.nq - 1;
       const int q_first = row_first_key(p, qpos), last_first = row_first_key(p, last_pos);      // the first keys this and the last query see
       float m_used = -INFINITY, l_sum = 0.f;
@@ -366,6 +376,6 @@ extern "C" int dk_attention_rows_wide(const DkRowAttnParams* pp, int max_q_len, 
     ok = true;
   }
   const int sms = dk_sm_count();
-  attention_rows_wide_kernel<<<(int)(pieces < sms ? pieces : sms), THREADS, SMEM, stream>>>(map_q, map_k, map_k_run, p, (int)pieces);
+  attention_rows_wide_kernel<<<(int)(pieces < sms ? pieces : sms), THREADS, SMEM, stream>>>(map_q, map_k, map_k_run, p, (max_q_len + QT - 1) / QT);
   return dk_check_launch("attention_rows_wide");
 }
