@@ -14,6 +14,11 @@
 //     from there, so it costs no shared memory and no copy; the scores of the half's next tile wait for the products with P.
 //   * Pages of a tile that no query of the block sees (before the window or chunk, given back already, or behind the last token)
 //     are replaced by one that is there: their scores are masked, and what is multiplied by the zeros is finite.
+//   * Scores may be shaped first (an instance of its own): capped, s <- cap tanh(s / cap), and given a bias by distance and head.  Three
+//     special-function results a score instead of one.  The head's biases lie in shared memory in powers of two, a copy for each half, with
+//     as many entries before the first and behind the last distance as a tile can ask for, so that a score's bias is one load at a
+//     fixed offset; a tile whose keys all lie behind the last distance takes one bias.  Tables that do not fit are read where they lie.
+//     Prompts of 1,301, 700 and 47 tokens, 16 heads of 128: 68 us; warp-level MMA (attention_rows_mma.cu) 204 us.
 //
 //   warps 0-7   softmax: thread r of a half owns query r, which is lane r of the TMEM
 //   warps 8, 9  producers, one for keys and one for values
@@ -23,6 +28,7 @@
 #include "common.cuh"
 #include "row_attention_params.h"
 #include "tcgen05_helpers.cuh"
+#include "attention_pieces.cuh"
 
 namespace {
 constexpr int QT = 128;            // queries per block (rows of both MMAs)
@@ -32,6 +38,7 @@ constexpr int PRODUCER_WARP0 = 8, MMA_WARP = 10;   // warp 10 issues the score p
 constexpr int THREADS = (MMA_WARP + 2) * 32;
 constexpr int BOX_BYTES = 128 * 128;   // 128 rows of one 128-byte swizzle row each
 constexpr float RESCALE_STEP = 8.f;    // in powers of two
+constexpr int BIAS_BEFORE = KT + QT, BIAS_BEHIND = KT + QT;      // entries of a bias table in shared memory beside the distances 0 .. dist_max
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0, COL_O = 2 * KT;   // S_0, S_1, then O_0, O_1
 
@@ -56,25 +63,40 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+__device__ __forceinline__ float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// One piece of work: 128 queries of one head of one row.  Pieces are numbered with the head fastest, then the rows,
-// then the query tiles of each row from its latest (which has the most keys) to its first: from long to short.
+// One piece of work: 128 queries of one head of one row.  Pieces are numbered with the head fastest, then as the block's list has them
+// (attention_pieces.cuh); without a list by the rows, then the query tiles of each row from its latest (which has the most keys) to its first.
 struct Piece {
   int row, h, qt, nq, t0, pos0, last_pos, kt_first, n_tiles, first_page, last_page;
   bool valid;
 };
 
-__device__ __forceinline__ Piece piece_of(const DkRowAttnParams& p, int index, int row_lo, int n_rows) {
+constexpr int LISTED = 256;      // pairs of row and query tile that the list holds
+
+__device__ __forceinline__ Piece piece_of(const DkRowAttnParams& p, int index, int row_lo, int n_rows, const uint32_t* list, int listed) {
   Piece w;
   w.h = index % p.H;
-  w.row = row_lo + (index / p.H) % n_rows;
-  const int yy = index / (p.H * n_rows);                // 0: the row's latest query tile, which has the most keys
-  const int q_len = p.row_q_len[w.row];
-  w.qt = (q_len + QT - 1) / QT - 1 - yy;
+  int q_len;
+  if (listed >= 0) {
+    const uint32_t pair = list[index / p.H];
+    w.row = (pair >> 9) & 511;
+    w.qt = pair & 511;
+    q_len = p.row_q_len[w.row];
+  } else {
+    w.row = row_lo + (index / p.H) % n_rows;
+    q_len = p.row_q_len[w.row];
+    w.qt = (q_len + QT - 1) / QT - 1 - index / (p.H * n_rows);      // 0: the row's latest query tile, which has the most keys
+  }
   const int q0 = w.qt * QT;
   w.valid = !(p.row_filter == 2 && q_len == 1) && w.qt >= 0;
   w.nq = min(QT, q_len - q0);
@@ -95,25 +117,26 @@ __device__ __forceinline__ Piece piece_of(const DkRowAttnParams& p, int index, i
 // write the piece before.  Every barrier is used by the tiles of one parity (tile j of a piece by the barriers of
 // class j % 2, as is its stage of K and V), so what a wait needs is the number of tiles of that class the block
 // has had so far: `had[c]`, counted alike by every warp.
-template <int DKP, int DVP>
+template <int DKP, int DVP, bool SHAPED>
 __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                        const __grid_constant__ CUtensorMap map_k,
                                                                        const __grid_constant__ CUtensorMap map_k_run,
                                                                        const __grid_constant__ CUtensorMap map_v,
                                                                        const __grid_constant__ CUtensorMap map_v_run,
-                                                                       const DkRowAttnParams p, const int n_qt) {
+                                                                       const DkRowAttnParams p, const int n_qt, const int bias_floats) {
   using L = Layout<DKP, DVP>;
   constexpr int STAGES = L::STAGES;
   static_assert(STAGES == 2, "a stage belongs to the tiles of one parity");
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  // barriers: q_full, k_full[2], v_full[2], s_full[2], p_full[2], o_done[2], merge, piece_done
-  __shared__ __align__(8) unsigned long long bars[1 + 2 + 2 + 2 + 2 + 2 + 1 + 1];
+  // barriers: q_full, k_full[2], v_full[2], s_full[2], p_full[2], o_done[2], merge, piece_done, bias_full[2]
+  __shared__ __align__(8) unsigned long long bars[1 + 2 + 2 + 2 + 2 + 2 + 1 + 1 + 2];
   auto row_stat = [&](int w) { return reinterpret_cast<float2*>(smem + L::OFF_STAT + w * QT * 8); };     // maximum and sum of half w's tiles, per query
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int failed;
   __shared__ int row_range[2];
+  __shared__ PieceList<LISTED> pieces;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ps = p.ps, G = p.H / p.KV;
@@ -121,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
   const uint32_t bar0 = s2u(&bars[0]);
   const uint32_t q_full = bar0;
   const uint32_t k_full = bar0 + 8, v_full = k_full + 16, s_full = v_full + 16, p_full = s_full + 16, o_done = p_full + 16,
-                 merge_bar = o_done + 16, piece_done = merge_bar + 8;
+                 merge_bar = o_done + 16, piece_done = merge_bar + 8, bias_full = piece_done + 8;
   if (tid == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < STAGES; ++s) {
@@ -132,6 +155,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       mbar_init(s_full + 8 * w, 1);
       mbar_init(p_full + 8 * w, HALF_THREADS);
       mbar_init(o_done + 8 * w, 1);
+      mbar_init(bias_full + 8 * w, HALF_THREADS);
     }
     mbar_init(merge_bar, 2 * HALF_THREADS);
     mbar_init(piece_done, 2 * HALF_THREADS);
@@ -162,12 +186,16 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       row_range[1] = hi;
     }
   }
+  const int listed = list_pieces<LISTED>(pieces, p.row_q_len, p.rows, p.row_filter == 2, QT, [&](int row, int qt) {
+    const int pos0 = p.row_pos_start[row] + qt * QT, last = p.row_pos_start[row] + min(p.row_q_len[row], (qt + 1) * QT) - 1;
+    return last / KT - row_first_key(p, pos0) / KT + 1;
+  });
   if (warp == MMA_WARP) tmem_alloc(s2u(&tmem_slot), TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const int row_lo = row_range[0], n_rows = max(0, row_range[1] - row_range[0] + 1);
-  const int n_pieces = p.H * n_qt * n_rows;
+  const int n_pieces = p.H * (listed >= 0 ? listed : n_qt * n_rows);
   // The pieces a block takes: in rounds of gridDim.x pieces, forwards in the even rounds and backwards in the odd ones.
   // Pieces are numbered from long to short, so a block that got a long one in one round gets a short one in the next,
   // and all blocks end at about the same time without asking each other anything.
@@ -205,7 +233,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
     for (int round = 0; round * (int)gridDim.x < n_pieces && !failed; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece w = piece_of(p, index, row_lo, n_rows);
+      const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       const int kvh = w.h / G;
       if (kind == 0) {
@@ -279,7 +307,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
     for (int round = 0; ok && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece w = piece_of(p, index, row_lo, n_rows);
+      const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       ok = wait_all(q_full, n_done & 1);
       for (int j = 0; ok && j < w.n_tiles; ++j) {
@@ -314,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
     for (int round = 0; ok && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece w = piece_of(p, index, row_lo, n_rows);
+      const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       for (int j = 0; ok && j < w.n_tiles; ++j) {
         const int c = j & 1, ord = (c ? had1 : had0) + j / 2;
@@ -347,18 +375,31 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t t_s = tmem + lane_base + COL_S + w * KT;    // scores of this half
     const uint32_t t_o = tmem + lane_base + COL_O + w * DVP;
-    const float sl2 = p.scale * 1.4426950408889634f;
+    // scores in powers of two: a multiple of the product, or (shaped) what `shape` below makes of it
+    const float sl2 = SHAPED ? 1.f : p.scale * 1.4426950408889634f;
+    const float cap2 = SHAPED ? p.softcap * 1.4426950408889634f : 0.f;
+    const float to_tanh = SHAPED && p.softcap > 0.f ? p.scale / p.softcap * (2.f * 1.4426950408889634f) : 0.f;
     bool good = true;
     int had_w = 0;            // tiles of this half in the pieces before the current one
 #pragma unroll 1
     for (int round = 0; good && round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
-      const Piece pc = piece_of(p, index, row_lo, n_rows);
+      const Piece pc = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!pc.valid) continue;
       const int n_tiles = pc.n_tiles, pos0 = pc.pos0, last_pos = pc.last_pos, kt_first = pc.kt_first, nq = pc.nq, t0 = pc.t0, h = pc.h;
       const int qpos = pos0 + r;
       const int q_first = row_first_key(p, qpos), last_first = row_first_key(p, last_pos);      // the first keys this and the last query see
+      float* bias_sm = nullptr;
+      if (SHAPED && bias_floats > 0) {      // (this half's tiles of the piece before are done)
+        bias_sm = reinterpret_cast<float*>(smem + L::TOTAL - 1024) + w * bias_floats;
+        const float* bias = p.dist_bias + (size_t)h * (p.dist_max + 1);
+        for (int i = (warp & 3) * 32 + lane; i < bias_floats; i += HALF_THREADS)
+          bias_sm[i] = bias[min(max(i - BIAS_BEFORE, 0), p.dist_max)] * 1.4426950408889634f;
+        mbar_arrive(bias_full + 8 * w);
+        bool ok = mbar_wait(bias_full + 8 * w, n_done & 1);
+        if (!__all_sync(0xffffffffu, ok && !failed)) { failed = 1; good = false; break; }
+      }
       float m_used = -INFINITY, l_sum = 0.f;
       int mine = 0;                                       // tiles of this half in this piece so far
       // Before this half lets the P V product overwrite an accumulator, and before it leaves a maximum and sum again, both halves
@@ -379,6 +420,31 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
 #pragma unroll
         for (int c = 0; c < KT / 32; ++c) tmem_ld32_nowait(t_s + c * 32, v + c * 32);
         tmem_wait_ld();
+        if (SHAPED) {
+          if (p.softcap > 0.f) {      // cap tanh(t) = cap - 2 cap / (1 + e^(2t)): exact at both ends
+#pragma unroll
+            for (int i = 0; i < KT; ++i) v[i] = fmaf(-2.f * cap2, fast_rcp(1.f + fast_exp2(v[i] * to_tanh)), cap2);
+          } else {
+#pragma unroll
+            for (int i = 0; i < KT; ++i) v[i] *= p.scale * 1.4426950408889634f;
+          }
+          if (p.dist_bias != nullptr) {
+            const float* bias = p.dist_bias + (size_t)h * (p.dist_max + 1);
+            if (kbase + KT - 1 <= pos0 - p.dist_max) {
+              const float far = bias[p.dist_max] * 1.4426950408889634f;
+#pragma unroll
+              for (int i = 0; i < KT; ++i) v[i] += far;
+            } else if (bias_floats > 0) {
+              const float* at = bias_sm + BIAS_BEFORE + min(qpos - kbase, p.dist_max + BIAS_BEHIND - 1);
+#pragma unroll
+              for (int i = 0; i < KT; ++i) v[i] += at[-i];
+            } else {      // (a key behind the query is masked below: its huge unsigned distance takes the last entry)
+              const unsigned dist = (unsigned)(qpos - kbase);
+#pragma unroll
+              for (int i = 0; i < KT; ++i) v[i] = fmaf(bias[min(dist - (unsigned)i, (unsigned)p.dist_max)], 1.4426950408889634f, v[i]);
+            }
+          }
+        }
         if (edge) {
           const int hi = qpos - kbase, lo = q_first - kbase;
 #pragma unroll
@@ -506,8 +572,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
   if (warp == MMA_WARP) tmem_dealloc(tmem, TMEM_COLS);
 }
 
-template <int DKP, int DVP>
-int launch(const DkRowAttnParams& p, int max_q_len, cudaStream_t stream) {
+template <int DKP, int DVP, bool SHAPED>
+int launch_as(const DkRowAttnParams& p, int max_q_len, cudaStream_t stream) {
   using L = Layout<DKP, DVP>;
   CUtensorMap map_q, map_k, map_k_run, map_v, map_v_run;
   const long long rows = (long long)p.num_pages * p.KV * p.ps;
@@ -527,12 +593,16 @@ int launch(const DkRowAttnParams& p, int max_q_len, cudaStream_t stream) {
                make_tensor_map_bf16_4d(kind ? &map_v_run : &map_k_run, base, dims, strides, p.ps, KT / p.ps),
                "attention_rows_tc: cannot encode a tensor map of the cache");
   }
+  constexpr int MOST = SHAPED ? 224 * 1024 : L::TOTAL;
+  int bias_floats = SHAPED && p.dist_bias != nullptr ? (BIAS_BEFORE + p.dist_max + 1 + BIAS_BEHIND + 3) / 4 * 4 : 0;
+  if (L::TOTAL + 2LL * bias_floats * (int)sizeof(float) > MOST) bias_floats = 0;
+  const int smem = L::TOTAL + 2 * bias_floats * (int)sizeof(float);
   static bool configured_on[DK_MAX_DEVICES] = {false};
   bool& configured = configured_on[dk_current_device()];
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_rows_tc_kernel<DKP, DVP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(attention_rows_tc_kernel<DKP, DVP, SHAPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
     if (e != cudaSuccess) {
-      dk_set_error("attention_rows_tc: cannot get %d bytes of shared memory: %s", L::TOTAL, cudaGetErrorString(e));
+      dk_set_error("attention_rows_tc: cannot get %d bytes of shared memory: %s", MOST, cudaGetErrorString(e));
       return DK_ERR_LAUNCH;
     }
     configured = true;
@@ -541,8 +611,14 @@ int launch(const DkRowAttnParams& p, int max_q_len, cudaStream_t stream) {
   const long long pieces = (long long)p.H * n_qt * p.rows;
   DK_REQUIRE(pieces < (1ll << 30), "attention_rows_tc: too many pieces of work");
   const int sms = dk_sm_count();
-  attention_rows_tc_kernel<DKP, DVP><<<(int)(pieces < sms ? pieces : sms), THREADS, L::TOTAL, stream>>>(map_q, map_k, map_k_run, map_v, map_v_run, p, n_qt);
+  attention_rows_tc_kernel<DKP, DVP, SHAPED><<<(int)(pieces < sms ? pieces : sms), THREADS, smem, stream>>>(map_q, map_k, map_k_run, map_v, map_v_run, p,
+                                                                                                          n_qt, bias_floats);
   return dk_check_launch("attention_rows_tc");
+}
+
+template <int DKP, int DVP>
+int launch(const DkRowAttnParams& p, int max_q_len, cudaStream_t stream) {
+  return p.softcap > 0.f || p.dist_bias != nullptr ? launch_as<DKP, DVP, true>(p, max_q_len, stream) : launch_as<DKP, DVP, false>(p, max_q_len, stream);
 }
 }  // namespace
 
@@ -552,7 +628,7 @@ extern "C" int dk_attention_rows_tc_supported(const DkRowAttnParams* pp) {
   if (p.dk % 8 || p.dv % 8 || p.dk < 64 || p.dk > 128 || p.dv < 64 || p.dv > 128) return 0;
   if (p.row_width % 8 || p.k_off % 8 || p.v_off % 8 || p.q_stride % 8 || p.q_head_stride % 8) return 0;
   if (p.ps != 8 && p.ps != 16 && p.ps != 32 && p.ps != 64 && p.ps != 128) return 0;
-  if (p.softcap > 0.f || p.dist_bias != nullptr || !(p.scale > 0.f)) return 0;
+  if (!(p.scale > 0.f) || p.softcap < 0.f || (p.dist_bias != nullptr && p.dist_max < 0)) return 0;
   if (((uintptr_t)p.q % 16) || ((uintptr_t)p.cache % 16) || ((uintptr_t)p.out % 16)) return 0;
   return 1;
 }
@@ -562,7 +638,7 @@ extern "C" int dk_attention_rows_tc(const DkRowAttnParams* pp, int max_q_len, cu
   const DkRowAttnParams& p = *pp;
   if (p.T == 0 || p.rows == 0) return 0;
   DK_REQUIRE(dk_attention_rows_tc_supported(pp), "attention_rows_tc: sizes not taken (bfloat16; key and value sizes multiples of 8 from 64 to 128; "
-             "page size 8 to 128 and a power of two; offsets and strides multiples of 8; a positive scale; no shaped scores): dk=%d dv=%d width=%d "
+             "page size 8 to 128 and a power of two; offsets and strides multiples of 8; a positive scale): dk=%d dv=%d width=%d "
              "ps=%d", p.dk, p.dv, p.row_width, p.ps);
   DK_REQUIRE(max_q_len >= 1, "attention_rows_tc: max_q_len must be positive");
   DK_REQUIRE(p.window >= 0 && p.chunk >= 0, "attention_rows_tc: bad window %d or chunk %d", p.window, p.chunk);

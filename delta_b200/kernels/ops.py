@@ -666,8 +666,7 @@ def attention_rows_wide(params: RowAttnParams, max_q_len: int):
 
 
 def attention_rows_tc_supported(params: RowAttnParams) -> bool:
-    """True when the tcgen05 kernel of the family takes these sizes (bfloat16; key and value sizes multiples of 8 from 64 to 128; no shaped
-    scores)."""
+    """True when the tcgen05 kernel of the family takes these sizes (bfloat16; key and value sizes multiples of 8 from 64 to 128)."""
     return bool(_l.load().dk_attention_rows_tc_supported(C.byref(params)))
 
 

@@ -1,9 +1,11 @@
-"""The tcgen05 attention kernels over a cache of rows whose value is the front part of its key, at the edges of its tiles."""
+"""The tcgen05 attention kernels over a cache of rows whose value is the front part of its key, and with shaped scores, at the edges of their tiles."""
 import pytest
+import torch
 
 from test_gpu_row_attention import run_case
 
 pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
 
 
 @pytest.fixture
@@ -40,3 +42,45 @@ def test_wide_many_pieces_beside_single_tokens(wide_everywhere):
 @pytest.mark.parametrize("kp", [0, 15, 63, 64, 127, 128, 255, 298])
 def test_wide_one_key_that_matters(wide_everywhere, kp):
     run_case("bfloat16", False, (4, 1, 320, 256), [(150, 150)], latent=True, spikes=[(0, 149, kp)], seed=kp)
+
+
+@pytest.mark.parametrize("dk, dv", [(128, 128), (64, 128), (72, 104)])
+@pytest.mark.parametrize("cap, far", [(4.0, 37), (50.0, 400), (0.0, 64), (6.0, -1)])
+def test_shaped_portions(dk, dv, cap, far):
+    """Capped scores and biases by distance in the tcgen05 kernel (tiles beside, across and behind the table's last distance), beside the plain
+    kernel's answer for the same inputs in 32 bit."""
+    from delta_b200.kernels import ops
+    g = torch.Generator().manual_seed(dk + far)
+    H, KV, ps = 4, 2, 16
+    lens, before = [130, 64, 300], [0, 200, 500]
+    pages = [-(-(b + n) // ps) for b, n in zip(before, lens)]
+    bt = torch.full((3, max(pages)), -1, dtype=torch.int32)
+    order = torch.randperm(sum(pages), generator=g).to(torch.int32)
+    for r in range(3):
+        bt[r, :pages[r]] = order[sum(pages[:r]):sum(pages[:r + 1])]
+    cache = torch.randn(sum(pages), KV, ps, dk + dv, generator=g).bfloat16()
+    T = sum(lens)
+    q = (torch.randn(T, H * dk, generator=g) * 1.5).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)      # noqa: E731
+    sink = torch.randn(H, generator=g).to(DEV)
+    dist = (torch.randn(H, far + 1, generator=g) * 2).to(DEV) if far >= 0 else None
+    rows = dict(block_table=bt.to(DEV), tok_row=i32([r for r, n in enumerate(lens) for _ in range(n)]),
+                tok_pos=i32([b + j for b, n in zip(before, lens) for j in range(n)]), row_q_start=i32([sum(lens[:r]) for r in range(3)]),
+                row_q_len=i32(lens), row_pos_start=i32(before), sink=sink, dist_bias=dist)
+    got = {}
+    for dtype in (torch.bfloat16, torch.float32):
+        qd, cd = q.to(DEV).to(dtype), cache.to(DEV).to(dtype)
+        out = torch.full((T, H * dv), float("nan"), dtype=dtype, device=DEV)
+        err = ops.new_error_record(DEV)
+        params = ops.row_attn_params(q=qd, cache=cd, q_stride=H * dk, q_head_stride=dk, out=out, H=H, KV=KV, dk=dk, dv=dv, ps=ps, row_width=dk + dv,
+                                     k_off=0, v_off=dk, scale=0.1, softcap=cap, err=err, **rows)
+        if dtype == torch.float32:
+            ops.attention_rows_plain(params)
+        else:
+            assert ops.attention_rows_tc_supported(params)
+            ops.attention_rows_tc(params, max(lens))
+        ops.raise_if_error(err)
+        got[dtype] = out.double()
+    want = got[torch.float32]
+    # weights to 16 bits, one rounding of the output to bfloat16 (2^-9 of it); values are about one
+    assert (got[torch.bfloat16] - want).abs().max() < 2.0 ** -8 * want.abs().max()
