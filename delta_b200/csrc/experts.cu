@@ -391,24 +391,83 @@ router_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
            choice + (size_t)(t0 + k) * top, weight + (size_t)(t0 + k) * top, lane);
 }
 
-constexpr int ALIGN_HELD = 16;
+// The same for few tokens in bfloat16: a block takes one token, its warps share d, and sixteen rows of W are asked for at once.  Bound by latency:
+// behind a step that streamed its experts' weights W comes from the memory again, so one round of loads instead of eight.  8 tokens, 17
+// rows of 2,048, after 200 MB: 12.2 -> 6.2 us.
+constexpr int FEW_ROWS = 16;
+
+__global__ void __launch_bounds__(ROUTER_WARPS * 32)
+router_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, float* __restrict__ logits, int* __restrict__ choice,
+                  float* __restrict__ weight, int d, int n_rows, int E, int top, const float* __restrict__ correction, float route_scale, int scored,
+                  int groups, int keep, int group_top2) {
+  extern __shared__ float zs[];      // [n_rows], (scored: [E]), (groups: [groups]), then the warps' sums [warps][n_rows]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x;
+  float* score = zs + n_rows;
+  float* group = score + (scored ? E : 0);
+  float* part = group + groups;
+  for (int r0 = 0; r0 < n_rows; r0 += FEW_ROWS) {
+    float acc[FEW_ROWS];
+#pragma unroll
+    for (int q = 0; q < FEW_ROWS; ++q) acc[q] = 0.f;
+    for (int c = (warp * 32 + lane) * 8; c < d; c += ROUTER_WARPS * 256) {
+      uint4 raw[FEW_ROWS];      // (rows behind the last one repeat it)
+#pragma unroll
+      for (int q = 0; q < FEW_ROWS; ++q) raw[q] = __ldg(reinterpret_cast<const uint4*>(w + (size_t)min(r0 + q, n_rows - 1) * d + c));
+      float xv[8], wv[8];
+      load8<__nv_bfloat16>(x + (size_t)t * d + c, xv);
+#pragma unroll
+      for (int q = 0; q < FEW_ROWS; ++q) {
+        load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&raw[q]), wv);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[q] = fmaf(xv[i], wv[i], acc[q]);
+      }
+    }
+    // the lanes' sums: each step halves what a lane keeps, so a pair of lanes ends with one row
+#pragma unroll
+    for (int half = FEW_ROWS / 2, bit = 16; half > 0; half >>= 1, bit >>= 1) {
+      const bool upper = (lane & bit) != 0;
+#pragma unroll
+      for (int q = 0; q < FEW_ROWS / 2; ++q)
+        if (q < half) {
+          const float send = upper ? acc[q] : acc[q + half], mine = upper ? acc[q + half] : acc[q];
+          acc[q] = mine + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+    }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    if ((lane & 1) == 0 && r0 + lane / 2 < n_rows) part[(size_t)warp * n_rows + r0 + lane / 2] = acc[0];
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < n_rows; r += ROUTER_WARPS * 32) {
+    float v = 0.f;
+#pragma unroll
+    for (int q = 0; q < ROUTER_WARPS; ++q) v += part[(size_t)q * n_rows + r];
+    zs[r] = v;
+    logits[(size_t)t * n_rows + r] = v;
+  }
+  __syncthreads();
+  if (warp == 0)
+    choose(zs, score, group, E, top, correction, route_scale, scored, groups, keep, group_top2, choice + (size_t)t * top, weight + (size_t)t * top, lane);
+}
+
 
 // One block.  sorted[p] = slot (token * top + choice) or -1; tile_expert[tile] = expert or -1.
+// HELD: choices that a thread asks for at once (a load behind every atomic would wait for it).
+template <int HELD>
 __global__ void experts_align_kernel(const int* __restrict__ choice, int n_slots, int E, int* __restrict__ sorted, int capacity,
                                      int* __restrict__ tile_expert, int max_tiles, int tile_m) {
   __shared__ int count[MAX_EXPERTS], start[MAX_EXPERTS];
-  int held[ALIGN_HELD];      // a thread's first choices, all asked for at once (a load behind every atomic would wait for it)
+  int held[HELD];
 #pragma unroll
-  for (int i = 0; i < ALIGN_HELD; ++i) {
+  for (int i = 0; i < HELD; ++i) {
     const int s = threadIdx.x + i * blockDim.x;
     held[i] = s < n_slots ? choice[s] : -1;
   }
   for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < ALIGN_HELD; ++i)
+  for (int i = 0; i < HELD; ++i)
     if (held[i] >= 0 && held[i] < E) atomicAdd(&count[held[i]], 1);
-  for (int s = threadIdx.x + ALIGN_HELD * blockDim.x; s < n_slots; s += blockDim.x) {
+  for (int s = threadIdx.x + HELD * blockDim.x; s < n_slots; s += blockDim.x) {
     const int e = choice[s];
     if (e >= 0 && e < E) atomicAdd(&count[e], 1);
   }
@@ -428,9 +487,9 @@ __global__ void experts_align_kernel(const int* __restrict__ choice, int n_slots
   __syncthreads();
   // the order of an expert's rows is whatever the atomics give: every row is computed alone, so it changes no value
 #pragma unroll
-  for (int i = 0; i < ALIGN_HELD; ++i)
+  for (int i = 0; i < HELD; ++i)
     if (held[i] >= 0 && held[i] < E) sorted[start[held[i]] + atomicAdd(&count[held[i]], 1)] = threadIdx.x + i * blockDim.x;
-  for (int s = threadIdx.x + ALIGN_HELD * blockDim.x; s < n_slots; s += blockDim.x) {
+  for (int s = threadIdx.x + HELD * blockDim.x; s < n_slots; s += blockDim.x) {
     const int e = choice[s];
     if (e < 0 || e >= E) continue;
     sorted[start[e] + atomicAdd(&count[e], 1)] = s;
@@ -666,7 +725,7 @@ experts_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16
 }
 
 // rows[p] = x[sorted[p] / top] (zeros where sorted[p] < 0): the tokens in the sorted order, for products that want their rows
-// side by side (csrc/gemm_tc.cu).  K is a multiple of 8.
+// side by side (csrc/gemm_rows_tc.cu).  K is a multiple of 8.
 // row_scale (or null): rows[p] = row_scale[sorted[p]] * x[sorted[p] / top], rounded once: a choice's weight multiplies what its
 // expert reads.
 __global__ void experts_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted, int top,
@@ -836,6 +895,12 @@ extern "C" int dk_router(const void* x, const void* w, float* logits, int* choic
         group_top2);
     return dk_check_launch("router");
   }
+  const size_t few_smem = ((size_t)n_rows * (1 + ROUTER_WARPS) + (scored ? E : 0) + groups) * sizeof(float);
+  if (dtype == DK_BF16 && T_ < 128 && d % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && few_smem <= 48 * 1024) {
+    router_few_kernel<<<T_, ROUTER_WARPS * 32, few_smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, d, n_rows, E,
+                                                                  top, correction, route_scale, scored, groups, keep, group_top2);
+    return dk_check_launch("router");
+  }
   const int blocks = (T_ + tpb - 1) / tpb;
   const bool vec = d % 8 == 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)w % 16) == 0;
 #define LAUNCH(T, V) router_kernel<T, V><<<blocks, ROUTER_WARPS * 32, smem, stream>>>((const T*)x, (const T*)w, logits, choice, weight, T_, d, n_rows, E, top, tpb, correction, route_scale, scored, groups, keep, group_top2)
@@ -857,7 +922,8 @@ extern "C" int dk_experts_align(const int* choice, int n_slots, int E, int* sort
   DK_REQUIRE(n_slots > 0 && E > 0 && E <= MAX_EXPERTS, "experts_align: bad sizes slots=%d E=%d (at most %d experts)", n_slots, E, MAX_EXPERTS);
   DK_REQUIRE(tile_m > 0 && capacity % tile_m == 0 && max_tiles * tile_m == capacity && capacity >= n_slots + (tile_m - 1) * (E < n_slots ? E : n_slots),
              "experts_align: %d rows in %d tiles do not hold %d slots of %d experts", capacity, max_tiles, n_slots, E);
-  experts_align_kernel<<<1, 1024, 0, stream>>>(choice, n_slots, E, sorted, capacity, tile_expert, max_tiles, tile_m);
+  if (n_slots <= 1024) experts_align_kernel<1><<<1, 1024, 0, stream>>>(choice, n_slots, E, sorted, capacity, tile_expert, max_tiles, tile_m);
+  else experts_align_kernel<16><<<1, 1024, 0, stream>>>(choice, n_slots, E, sorted, capacity, tile_expert, max_tiles, tile_m);
   return dk_check_launch("experts_align");
 }
 

@@ -149,6 +149,8 @@ _SIGNATURES = {
     "dk_router": [P, P, P, P, P, I, I, I, I, I, P, F, I, I, I, I, I, P],
     "dk_experts_align": [P, I, I, P, I, P, I, I, P],
     "dk_experts_gather": [P, P, I, P, I, I, P, P],
+    "dk_experts_stream_supported": [I],
+    "dk_experts_stream": [P, P, P, P, P, I, I, I, I, I, F, F, F, P, I, P],
     "dk_experts_gemm_tc_supported": [I, I, I],
     "dk_experts_gemm_tc": [P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, F, P, P],
     "dk_experts_gemm": [P, P, P, P, P, I, I, I, I, I, F, F, F, P, I, P],

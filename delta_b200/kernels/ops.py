@@ -1310,6 +1310,24 @@ def experts_gemm(a, w, out, sorted_slots, tile_expert, *, top, n, k, act=False, 
                                        dtype_code(a.dtype), _stream()), "experts_gemm")
 
 
+def experts_stream_supported(dtype, *ks) -> bool:
+    return dtype == torch.bfloat16 and all(_l.load().dk_experts_stream_supported(int(k)) for k in ks)
+
+
+def experts_stream(a, w, out, sorted_slots, tile_expert, *, top, n, k, most, act=False, limit=-1.0, alpha=1.702, shift=1.0, row_scale=None):
+    """``experts_gemm`` for a handful of rows an expert (about ``most``): bfloat16 weights straight into the tensor cores' fragments."""
+    if row_scale is not None and not act:
+        raise KernelError("experts_stream: a scale per row belongs to the first product")
+    code = {False: 0, True: 1, "gated": 1, "relu_squared": 2}.get(act)
+    if code is None:
+        raise KernelError(f"experts_stream: unknown activation '{act}'")
+    bf = torch.bfloat16
+    _l.check(_l.load().dk_experts_stream(_ptr(a, "a", bf), _ptr(w, "w", bf), _ptr(out, "out", bf if code else torch.float32),
+                                         _ptr(sorted_slots, "sorted_slots", torch.int32), _ptr(tile_expert, "tile_expert", torch.int32),
+                                         tile_expert.numel(), int(top), int(n), int(k), code, float(limit), float(alpha), float(shift),
+                                         _ptr(row_scale, "row_scale", torch.float32), int(most), _stream()), "experts_stream")
+
+
 def experts_combine(z, weight, out, shared=None, gate_logit=None, gate_stride=0, top=None, identity=None):
     """out[t] = sum_j weight[t, j] z[t*top + j] (+ sigmoid(gate logit of t) * shared[t]; no gate logit: + shared[t]); ``gate_logit``: an
     address (float32).  ``weight`` None with ``top``: every weight is 1.  ``identity`` (x, choice, first): a choice from ``first`` on adds

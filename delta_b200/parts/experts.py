@@ -8,7 +8,7 @@
 Nothing about the routing is read on the host: the (token, choice) pairs are sorted by expert on the device into tiles of
 rows of one expert, and the two products of all experts are one launch each: warp-level MMA over tiles of 64 rows
 (``csrc/experts.cu``), or, when a step brings many rows an expert, the tcgen05 product over tiles of 128 rows gathered side
-by side (``csrc/gemm_tc.cu``).  The router's rows and
+by side (``csrc/gemm_rows_tc.cu``).  The router's rows and
 the shared expert's gate row are one matrix, so one product gives both.
 
 Options: ``scoring`` "softmax_all": as "sigmoid" below with s = the softmax over all of the router's logits.  ``groups`` (count, keep): the
@@ -34,6 +34,7 @@ from .feed_forward import ClampedGLU
 
 
 TC_TILE = 128               # rows of a tile on the tcgen05 path
+STREAM_TOKENS = 32          # up to this many tokens (so many rows an expert at most) the products are a stream over the experts' weights
 TC_ROWS_PER_EXPERT = 96     # from this many rows an expert on average, the products go to the tcgen05 kernel
 
 
@@ -138,6 +139,10 @@ class Experts(FeedForward):
             ops.experts_gemm_tc(rows, self.w1, y, tile_expert, tile, n=F, glu=True if self.gated else act, limit=self.limit, alpha=self.alpha, shift=self.shift,
                                 err=ctx.err)
             ops.experts_gemm_tc(y, self.w2, out_slots, tile_expert, tile, n=d, row_map=sorted_slots, err=ctx.err)
+        elif T <= STREAM_TOKENS and "products" not in ctx.plain_kernels and ops.experts_stream_supported(x.dtype, d, F):
+            ops.experts_stream(x, self.w1, y, sorted_slots, tile_expert, top=top, n=F, k=d, most=T, act=act, limit=self.limit, alpha=self.alpha,
+                               shift=self.shift, row_scale=row_scale)
+            ops.experts_stream(y, self.w2, out_slots, sorted_slots, tile_expert, top=top, n=d, k=F, most=T)
         else:
             ops.experts_gemm(x, self.w1, y, sorted_slots, tile_expert, top=top, n=F, k=d, act=act, limit=self.limit, alpha=self.alpha,
                              shift=self.shift, row_scale=row_scale)

@@ -269,3 +269,53 @@ def test_rows_append_unit_wide_accesses(H, KV, dk, dv, dtype, norm, rot, interle
     tol = 2e-6 if dtype == torch.float32 else 2.0 ** -8      # sums of squares in another order; in bfloat16 the last bit of the one rounding
     for a, c in zip(*got):
         assert (a - c).abs().max() <= tol * c.abs().max().clamp(min=1.0)
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 32, 70])
+@pytest.mark.parametrize("E, top, F, d", [(16, 4, 64, 256), (3, 2, 40, 72), (5, 5, 1056, 1032)])
+@pytest.mark.parametrize("act", ["gated", "relu_squared"])
+def test_experts_stream(T, E, top, F, d, act):
+    """The stream over the experts' weights beside the tiles of 64 rows on the same routing: rows beside a tile of eight, K and columns beside a
+    chunk and a block, an expert that nobody chooses, more rows than a round (T = 70 told as 32), weights on the inputs."""
+    o = ops()
+    g = torch.Generator().manual_seed(T + F)
+    x = torch.randn(T, d, generator=g).bfloat16().to(DEV)
+    w1 = (torch.randn(E, (2 if act == "gated" else 1) * F, d, generator=g) / d ** 0.5).bfloat16().to(DEV)
+    w2 = (torch.randn(E, d, F, generator=g) / F ** 0.5).bfloat16().to(DEV)
+    z = torch.randn(T, E, generator=g)
+    if E > top:
+        z[:, 1] -= 100.0
+    choice, weight = torch.empty(T, top, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    o.router_topk(z.to(DEV), E, top, choice, weight)
+    tile = o.experts_tile_rows()
+    cap = -(-(T * top + (tile - 1) * min(E, T * top)) // tile) * tile
+    ss, te = torch.empty(cap, dtype=torch.int32, device=DEV), torch.empty(cap // tile, dtype=torch.int32, device=DEV)
+    o.experts_align(choice, E, ss, te, tile)
+    scale = (torch.rand(T * top, generator=g) + 0.5).to(DEV) if act == "gated" else None
+    got = []
+    for stream in (False, True):
+        y, zs = torch.zeros(cap, F, dtype=torch.bfloat16, device=DEV), torch.full((T * top, d), float("nan"), device=DEV)
+        kw = dict(top=top, act=act, limit=0.9, row_scale=scale)
+        if stream:
+            o.experts_stream(x, w1, y, ss, te, n=F, k=d, most=min(T, 32), **kw)
+            o.experts_stream(y, w2, zs, ss, te, top=top, n=d, k=F, most=min(T, 32))
+        else:
+            o.experts_gemm(x, w1, y, ss, te, n=F, k=d, **kw)
+            o.experts_gemm(y, w2, zs, ss, te, top=top, n=d, k=F)
+        got.append((y.float(), zs))
+    # the same products in another order of the sums: the last bit of a bfloat16 in between, 2^-8 of a few entries' share
+    assert (got[0][0] - got[1][0]).abs().max() <= 2.0 ** -7 * got[0][0].abs().max()
+    assert bool(torch.isfinite(got[1][1]).all()) and (got[0][1] - got[1][1]).abs().max() <= 1e-2 * got[0][1].abs().max()
+
+
+@pytest.mark.parametrize("T, rows, E, d", [(1, 17, 16, 2048), (8, 20, 20, 1000), (127, 40, 33, 4096)])
+def test_router_of_few_tokens(T, rows, E, d):
+    o = ops()
+    torch.manual_seed(T + rows)
+    x, w = torch.randn(T, d, device=DEV).bfloat16(), (torch.randn(rows, d, device=DEV) * 0.05).bfloat16()
+    z, choice, weight = torch.empty(T, rows, device=DEV), torch.empty(T, 4, dtype=torch.int32, device=DEV), torch.empty(T, 4, device=DEV)
+    o.router(x, w, E, 4, z, choice, weight)
+    ref = x.double() @ w.double().T
+    assert (z.double() - ref).norm() < 3e-7 * ref.norm()      # exact products, sums of 32 bit
+    val, idx = torch.topk(z[:, :E], 4, dim=-1)
+    assert torch.equal(choice.long(), idx) and torch.allclose(weight, torch.softmax(val, -1), atol=1e-6)
