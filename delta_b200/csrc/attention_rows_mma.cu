@@ -36,9 +36,14 @@ __device__ __forceinline__ float tanh_by_exp(float t) {
 // RM: 16-row tiles of query rows per warp.  With two, every key and value fragment that a warp fetches from shared memory
 // feeds two products, which is what bounds this kernel (it moves 512 bytes of fragments for every 2 x 4,096 FLOP product).
 // SHAPED: scores are capped and take biases by distance (an instance of its own, so that the others keep their registers).
-template <int WARPS, int KT, int DVMAX, int RM, bool SHAPED>
-__global__ void __launch_bounds__(WARPS * 32) attention_rows_mma_kernel(const DkRowAttnParams p, float* __restrict__ part) {
-  constexpr int QT = 16 * WARPS * RM, THREADS = WARPS * 32, NT = DVMAX / 8, WR = 16 * RM;
+// KW > 1 (with one warp and one tile of query rows): that many warps take the key tiles in turn, each with stages, sums and a maximum of its own, and
+// are merged in shared memory at the end.  For single tokens with wide rows, whose tiles leave an SM room for four warps: more of them
+// per block mean fewer splits to merge.  8 tokens, 16 heads, keys of 320, values of 256, 2,048 keys:
+// 19 -> 13 us, the merge behind it 5.9 -> 4.4.
+template <int WARPS, int KT, int DVMAX, int RM, bool SHAPED, int KW>
+__global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(const DkRowAttnParams p, float* __restrict__ part) {
+  static_assert(KW == 1 || (WARPS == 1 && RM == 1), "key tiles are shared out over warps for one tile of query rows");
+  constexpr int QT = 16 * WARPS * RM, THREADS = WARPS * KW * 32, NT = DVMAX / 8, WR = 16 * RM;
   extern __shared__ __align__(128) unsigned char smem[];
   const int row = blockIdx.z / p.KV, g = blockIdx.z % p.KV;
   const int q_len = p.row_q_len[row];
@@ -47,13 +52,13 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_mma_kernel(const Dk
   const int M = q_len * G;
   const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * QT;      // late tiles have the most keys: start them first
   if (m0 >= M) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
+  const int tid = threadIdx.x, warp = KW > 1 ? 0 : tid >> 5, kw = KW > 1 ? tid >> 5 : 0, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int dk = p.dk, dv = p.dv, ps = p.ps;
   const int KB = dk / 16;
   const int ROWS = pad128(p.row_width * 2), QS = pad128(dk * 2);   // bytes between rows of a key tile / of the query tile
   const int CPR = p.row_width / 8;                                  // 16-byte chunks of a cached row
   unsigned char* q_smem = smem;
-  unsigned char* kv_smem = smem + QT * QS;
+  unsigned char* kv_smem = smem + QT * QS + (size_t)kw * PSTAGES * KT * ROWS;
   const int nrows = min(QT, M - m0);
   const int q_start = p.row_q_start[row], pos_start = p.row_pos_start[row];
   const int first_pos = pos_start + m0 / G, last_pos = pos_start + (m0 + nrows - 1) / G;
@@ -132,14 +137,19 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_mma_kernel(const Dk
   const int warp_lo = row_first_key(p, warp_first_pos);
   const int kc0 = p.k_off / 8, vc0 = p.v_off / 8;
 
-  if (kt_a < kt_b) load_tile(kt_a, 0);
+  if (kt_a + kw < kt_b) load_tile(kt_a + kw, 0);
   cp_async_commit();
-  for (int kt = kt_a; kt < kt_b; ++kt) {
-    if (kt + 1 < kt_b) load_tile(kt + 1, (kt + 1 - kt_a) % PSTAGES);
+  if (KW > 1) {      // everybody's queries
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+  for (int kt = kt_a + kw; kt < kt_b; kt += KW) {
+    if (kt + KW < kt_b) load_tile(kt + KW, ((kt - kt_a) / KW + 1) % PSTAGES);
     cp_async_commit();
     cp_async_wait<1>();
-    __syncthreads();
-    const uint32_t kbase = smem_u32(kv_smem + (size_t)((kt - kt_a) % PSTAGES) * KT * ROWS);
+    if (KW > 1) __syncwarp();
+    else __syncthreads();
+    const uint32_t kbase = smem_u32(kv_smem + (size_t)(((kt - kt_a) / KW) % PSTAGES) * KT * ROWS);
     const uint32_t qbase = smem_u32(q_smem);
     const int kt0 = kt * KT;
     const bool visible = warp * WR < nrows && kt0 <= warp_last_pos && kt0 + KT - 1 >= warp_lo;
@@ -270,9 +280,79 @@ __global__ void __launch_bounds__(WARPS * 32) attention_rows_mma_kernel(const Dk
         }
       }
     }
-    __syncthreads();   // every warp is done with this stage before the next load overwrites it
+    if (KW > 1) __syncwarp();
+    else __syncthreads();   // every warp is done with this stage before the next load overwrites it
   }
   cp_async_wait<0>();
+
+  if constexpr (KW > 1) {
+    // The warps' sums meet under the largest maximum: each leaves its own, scaled, where its stages were, and everybody adds.
+    __shared__ float stat[2][KW][16];
+    float* mine = reinterpret_cast<float*>(kv_smem);
+    const int LDO = dv + 4;
+    __syncwarp();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float ll = l_run[0][half];
+      ll += __shfl_xor_sync(0xffffffffu, ll, 1);
+      ll += __shfl_xor_sync(0xffffffffu, ll, 2);
+      if (tq == 0) {
+        stat[0][kw][gq + 8 * half] = m_run[0][half];
+        stat[1][kw][gq + 8 * half] = ll;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int r = gq + 8 * half;
+      float mm = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < KW; ++w) mm = fmaxf(mm, stat[0][w][r]);
+      const float f = m_run[0][half] == -INFINITY ? 0.f : exp2f(m_run[0][half] - mm);
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+        if (n * 8 < dv) *reinterpret_cast<float2*>(mine + r * LDO + n * 8 + 2 * tq) = make_float2(o[0][n][2 * half] * f, o[0][n][2 * half + 1] * f);
+    }
+    __syncthreads();
+    const float* all = reinterpret_cast<const float*>(smem + QT * QS);
+    const size_t next = (size_t)PSTAGES * KT * ROWS / sizeof(float);
+    for (int r = kw; r < nrows; r += KW) {
+      const int m = m0 + r, t = q_start + m / G, head = g * G + m % G;
+      float mm = -INFINITY, ll = 0.f;
+#pragma unroll
+      for (int w = 0; w < KW; ++w) mm = fmaxf(mm, stat[0][w][r]);
+#pragma unroll
+      for (int w = 0; w < KW; ++w) ll += stat[0][w][r] == -INFINITY ? 0.f : stat[1][w][r] * exp2f(stat[0][w][r] - mm);
+      float inv = 1.f;
+      if (splits == 1) {
+        float f = 1.f;
+        if (p.sink != nullptr) {      // the sink joins the denominator: a key with this logit and no value
+          const float s2 = p.sink[head] * LOG2E, mf = fmaxf(mm, s2);
+          f = mm == -INFINITY ? 0.f : exp2f(mm - mf);
+          ll = ll * f + exp2f(s2 - mf);
+        }
+        inv = ll > 0.f ? f * row_head_gate<__nv_bfloat16>(p, t, head) / ll : 0.f;
+      }
+      float* dst = part + (((size_t)t * p.H + head) * splits + split) * (dv + 2);
+      __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + ((size_t)t * p.H + head) * dv;
+      for (int d = lane * 2; d < dv; d += 64) {
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < KW; ++w) {
+          const float2 x = *reinterpret_cast<const float2*>(all + w * next + r * LDO + d);
+          v.x += x.x;
+          v.y += x.y;
+        }
+        if (splits > 1) *reinterpret_cast<float2*>(dst + d) = v;
+        else *reinterpret_cast<uint32_t*>(orow + d) = pack_bf16(v.x * inv, v.y * inv);
+      }
+      if (splits > 1 && lane == 0) {
+        dst[dv] = mm;
+        dst[dv + 1] = ll;
+      }
+    }
+    return;
+  }
 
 #pragma unroll
   for (int rm = 0; rm < RM; ++rm) {
@@ -359,10 +439,10 @@ __global__ void attention_rows_merge_kernel(const DkRowAttnParams p, const float
   }
 }
 
-template <int WARPS, int KT, int DVMAX, int RM, bool SHAPED>
+template <int WARPS, int KT, int DVMAX, int RM, bool SHAPED, int KW = 1>
 int launch_as(const DkRowAttnParams& p, int max_m, int splits, float* part, cudaStream_t stream) {
   const int m_tiles = (max_m + 16 * WARPS * RM - 1) / (16 * WARPS * RM);
-  const size_t smem = (size_t)16 * WARPS * RM * pad128(p.dk * 2) + (size_t)PSTAGES * KT * pad128(p.row_width * 2);
+  const size_t smem = (size_t)16 * WARPS * RM * pad128(p.dk * 2) + (size_t)KW * PSTAGES * KT * pad128(p.row_width * 2);
   if (smem > 220 * 1024) {
     dk_set_error("attention_rows_mma: rows of %d elements need more shared memory than a block has", p.row_width);
     return DK_ERR_ARG;
@@ -370,7 +450,7 @@ int launch_as(const DkRowAttnParams& p, int max_m, int splits, float* part, cuda
   static size_t configured_on[DK_MAX_DEVICES] = {0};
   size_t& configured = configured_on[dk_current_device()];
   if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_rows_mma_kernel<WARPS, KT, DVMAX, RM, SHAPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(attention_rows_mma_kernel<WARPS, KT, DVMAX, RM, SHAPED, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
       dk_set_error("attention_rows_mma: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
       return DK_ERR_LAUNCH;
@@ -378,15 +458,15 @@ int launch_as(const DkRowAttnParams& p, int max_m, int splits, float* part, cuda
     configured = smem;
   }
   dim3 grid(m_tiles, splits, p.rows * p.KV);
-  attention_rows_mma_kernel<WARPS, KT, DVMAX, RM, SHAPED><<<grid, WARPS * 32, smem, stream>>>(p, part);
+  attention_rows_mma_kernel<WARPS, KT, DVMAX, RM, SHAPED, KW><<<grid, WARPS * KW * 32, smem, stream>>>(p, part);
   return dk_check_launch("attention_rows_mma");
 }
 
 // RM_SHAPED: the 16-row tiles a warp takes when the scores are shaped (the shaping's registers leave room for fewer).
-template <int WARPS, int KT, int DVMAX, int RM, int RM_SHAPED = RM>
+template <int WARPS, int KT, int DVMAX, int RM, int RM_SHAPED = RM, int KW = 1>
 int launch(const DkRowAttnParams& p, int max_m, int splits, float* part, cudaStream_t stream) {
-  if (p.softcap > 0.f || p.dist_bias != nullptr) return launch_as<WARPS, KT, DVMAX, RM_SHAPED, true>(p, max_m, splits, part, stream);
-  return launch_as<WARPS, KT, DVMAX, RM, false>(p, max_m, splits, part, stream);
+  if (p.softcap > 0.f || p.dist_bias != nullptr) return launch_as<WARPS, KT, DVMAX, RM_SHAPED, true, KW>(p, max_m, splits, part, stream);
+  return launch_as<WARPS, KT, DVMAX, RM, false, KW>(p, max_m, splits, part, stream);
 }
 }  // namespace
 
@@ -403,6 +483,11 @@ extern "C" int dk_attention_rows_mma_supported(const DkRowAttnParams* pp) {
 // Floats of scratch that `splits` > 1 need.
 extern "C" long long dk_attention_rows_mma_scratch_floats(int T, int H, int dv, int splits) {
   return splits > 1 ? (long long)T * H * splits * (dv + 2) : 0;
+}
+
+// Warps of a block that share the key tiles (of 32) of a single token's group of up to 16 heads.
+extern "C" int dk_attention_rows_mma_key_warps(int dv, int row_width, int dk) {
+  return dv > 128 && (size_t)16 * pad128(dk * 2) + (size_t)4 * PSTAGES * 32 * pad128(row_width * 2) <= 200 * 1024 ? 4 : 1;
 }
 
 // max_m: the most query rows (tokens * heads of a group) any batch row brings among those the filter lets through.
@@ -423,6 +508,7 @@ extern "C" int dk_attention_rows_mma(const DkRowAttnParams* pp, int max_m, int s
   if (max_m <= 16) {
     if (p.dv <= 64) e = launch<1, 32, 64, 1>(p, max_m, splits, part, stream);
     else if (p.dv <= 128) e = launch<1, 32, 128, 1>(p, max_m, splits, part, stream);
+    else if (dk_attention_rows_mma_key_warps(p.dv, p.row_width, p.dk) == 4) e = launch<1, 32, 256, 1, 1, 4>(p, max_m, splits, part, stream);
     else e = launch<1, 32, 256, 1>(p, max_m, splits, part, stream);
   } else if (p.dv > 128) {
     // A wide value leaves room for one 16-row tile a warp, so the fragment loads are hidden by more warps instead: eight

@@ -60,6 +60,7 @@ _SIGNATURES = {
     "dk_attention_rows_plain": [C.POINTER(RowAttnParams), P],
     "dk_rows_append": [P, I, P, P, P, I, P, I, P, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P],
     "dk_latent_prepare": [P, I, P, P, P, I, P, I, P, I, I, I, P, F, P, I, I, I, I, I, I, P, I, I, P, P],
+    "dk_attention_rows_mma_key_warps": [I, I, I],
     "dk_attention_rows_mma_supported": [C.POINTER(RowAttnParams)],
     "dk_attention_rows_mma": [C.POINTER(RowAttnParams), I, I, P, P],
     "dk_attention_rows_wide_supported": [C.POINTER(RowAttnParams)],

@@ -640,6 +640,11 @@ def gemm_nt_plain_batched(a_ptr, w_ptr, c_ptr, M, N, K, lda, ldw, ldc, batch, sa
                                                 dtype_code(in_dtype), dtype_code(out_dtype), _stream()), "gemm_nt_plain_batched")
 
 
+def attention_rows_mma_key_warps(params: RowAttnParams) -> int:
+    """Warps of a block that share a single token's key tiles (up to 16 heads a group)."""
+    return int(_l.load().dk_attention_rows_mma_key_warps(params.dv, params.row_width, params.dk))
+
+
 def attention_rows_mma_supported(params: RowAttnParams) -> bool:
     """True when the tensor-core kernel of the family takes these sizes (bfloat16; key and value sizes multiples of 16)."""
     return bool(_l.load().dk_attention_rows_mma_supported(C.byref(params)))

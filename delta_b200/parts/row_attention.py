@@ -66,11 +66,14 @@ def plain(ctx) -> bool:
     return "attention" in ctx.plain_kernels or ctx.dtype != torch.bfloat16
 
 
-def decode_splits(rows: int, kv_heads: int, group: int, max_keys: int, sm_count: int) -> int:
+def decode_splits(rows: int, kv_heads: int, group: int, max_keys: int, sm_count: int, key_warps: int = 1) -> int:
     """Blocks that share the keys of a (row, key-value head) in a step of single tokens: enough to fill the device (a group of
     up to 16 heads is one warp a block, of which an SM holds about six; larger groups take four warps a block, two blocks an SM),
-    and so few that every block has two key tiles."""
+    and so few that every block has two key tiles.  With several ``key_warps`` (wide rows) a block has its SM to itself and a tile of 32
+    keys for each of its warps at least."""
     small = group <= 16
+    if small and key_warps > 1:
+        return max(1, min(sm_count // max(1, rows * kv_heads), -(-max_keys // (32 * key_warps)), MAX_SPLITS))
     blocks = max(1, rows * kv_heads * (1 if small else -(-group // 64)))
     tiles = max(1, -(-max_keys // (32 if small else 64)))
     return max(1, min((SINGLE_WARP_BLOCKS_PER_SM if small else 2) * sm_count // blocks, tiles // 2, MAX_SPLITS))
@@ -108,7 +111,7 @@ def run(ctx, params) -> None:
             reach = params.window or params.chunk
             max_keys = min(longest, reach + 64) if reach else longest
             rows = params.rows
-            splits = decode_splits(rows, params.KV, group, max_keys, ctx.sm_count)
+            splits = decode_splits(rows, params.KV, group, max_keys, ctx.sm_count, ops.attention_rows_mma_key_warps(params))
             if splits > 1:
                 n = ops.attention_rows_mma_scratch_floats(params.T, params.H, params.dv, splits)
                 bound = ops.attention_rows_mma_scratch_floats(max(getattr(ctx, "max_rows", 0), rows), params.H, params.dv, MAX_SPLITS)
