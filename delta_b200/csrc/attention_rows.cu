@@ -271,7 +271,7 @@ __global__ void rows_append_unit_kernel(T* __restrict__ src, int src_stride, con
 
 // The same with sixteen-byte accesses: a thread keeps eight neighbouring columns of the token's row in registers from the one load to the
 // one store, a head's threads lie side by side in a warp (dk / 8 of them, a power of two), and a rotated pair's other half comes by a
-// shuffle.  Bound by latency and bytes: 2,048 tokens of 16 + 4 heads of 128 with a norm over all heads 36 -> 19 us.
+// shuffle.  Bound by latency and bytes: 2,048 tokens of 16 + 4 heads of 128 with a norm over all heads 36 -> 17 us.
 template <typename T>
 __global__ void __launch_bounds__(1024)
 rows_append_unit_vec_kernel(T* __restrict__ src, int src_stride, const int* __restrict__ tok_pos, const int* __restrict__ tok_row,
@@ -280,7 +280,7 @@ rows_append_unit_vec_kernel(T* __restrict__ src, int src_stride, const int* __re
                             int row_width, int k_off, int v_off, int unit_norm, float eps, int value_from_key, const float* __restrict__ bias,
                             const float* __restrict__ q_norm, const float* __restrict__ k_norm, float pre_eps, int norm_whole, float temp_coef,
                             int temp_every, int* err) {
-  __shared__ float scratch[34], whole[2];
+  __shared__ float sums[2][32];
   const int t = blockIdx.x, pos = tok_pos[t], b = tok_row[t], col = threadIdx.x * 8;
   if (pos < 0 || (table != nullptr && pos >= table_positions)) {
     if (threadIdx.x == 0) dk_report(err, DK_DEV_BAD_POSITION, t, pos, table_positions);
@@ -304,28 +304,32 @@ rows_append_unit_vec_kernel(T* __restrict__ src, int src_stride, const int* __re
   const int head = in_head ? col / dk : 0, c = in_head ? col - head * dk : 0, lanes = dk / 8;
   T* crow = in_head && is_key && at >= 0 ? cache + (((size_t)page * KV + (head - H)) * ps + off) * row_width : nullptr;
   if (crow != nullptr && value_from_key && c < dv) store8<T>(crow + v_off + c, x);
+  const float* pre_w = is_key ? k_norm : q_norm;
+  const bool normed = pre_w != nullptr && in_head;
+  float w[8];      // (asked for before the sums that it waits with)
+  if (normed) load8<float>(pre_w + (norm_whole ? col - (is_key ? H * dk : 0) : c), w);
   float ss = 0.f;
 #pragma unroll
   for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
-  if (norm_whole) {      // 1 / rms over all of q's columns, and over all of k's
-    const float sq = block_sum(in_head && !is_key ? ss : 0.f, scratch);
-    const float sk = block_sum(in_head && is_key ? ss : 0.f, scratch);
-    if (threadIdx.x == 0) {
-      whole[0] = 1.f / sqrtf(sq / (float)(H * dk) + pre_eps);
-      whole[1] = KV > 0 ? 1.f / sqrtf(sk / (float)(KV * dk) + pre_eps) : 0.f;
-    }
-    __syncthreads();
-  }
   auto head_sum = [&](float v) {
     for (int o = lanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
   };
-  const float* pre_w = is_key ? k_norm : q_norm;
-  const float head_ss = head_sum(ss);
-  if (pre_w != nullptr && in_head) {
-    const float pre = norm_whole ? whole[is_key ? 1 : 0] : 1.f / sqrtf(head_ss / (float)dk + pre_eps);
-    float w[8];
-    load8<float>(pre_w + (norm_whole ? col - (is_key ? H * dk : 0) : c), w);
+  float pre = 0.f;
+  if (norm_whole) {      // 1 / rms over all of q's columns, or over all of k's
+    const float sq = warp_sum(in_head && !is_key ? ss : 0.f), sk = warp_sum(in_head && is_key ? ss : 0.f);
+    if ((threadIdx.x & 31) == 0) {
+      sums[0][threadIdx.x >> 5] = sq;
+      sums[1][threadIdx.x >> 5] = sk;
+    }
+    __syncthreads();
+    float sum = 0.f;
+    for (int i = 0; i < (int)blockDim.x >> 5; ++i) sum += sums[is_key ? 1 : 0][i];
+    pre = 1.f / sqrtf(sum / (float)((is_key ? KV : H) * dk) + pre_eps);
+  } else if (q_norm != nullptr || k_norm != nullptr) {
+    pre = 1.f / sqrtf(head_sum(ss) / (float)dk + pre_eps);
+  }
+  if (normed) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) x[e] = x[e] * pre * w[e];
   }
