@@ -22,6 +22,18 @@ constexpr int STAGES = 4;
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
 
+// x^n for n up to TC, by squaring: 64 bit, off by less than 2^-46 of it before it is rounded to 32.  (pow() takes several times as long,
+// and a block's first products wait for the table.)
+__device__ __forceinline__ float power(double x, int n) {
+  double r = 1.0;
+#pragma unroll
+  for (int b = 1; b <= TC; b *= 2) {
+    if (n & b) r *= x;
+    x *= x;
+  }
+  return (float)r;
+}
+
 // 64 tokens' entries of a head, activated, into rows of D + 4; zeros behind the last token.
 template <typename T, int D>
 __device__ __forceinline__ void load_rows(float* to, const T* src, int stride, int n, int act, const float* pw, int tid) {
@@ -74,7 +86,7 @@ decay_tiles_chunk_kernel(const T* __restrict__ src, int stride, int q_off, int k
   float* K = Q + TC * (DK + 4);
   float* V = K + TC * (DK + 4);      // times lambda^(n-1-s)
   float* pw = V + TC * (DV + 4);
-  if (tid <= TC) pw[tid] = (float)pow(decays[h], (double)tid);
+  if (tid <= TC) pw[tid] = power(decays[h], tid);
   __syncthreads();
   const T* at = src + (size_t)(row_q_start[row] + c0) * stride;
   load_rows<T, DK>(Q, at + q_off + (size_t)h * DK, stride, n, act, nullptr, tid);
@@ -147,7 +159,7 @@ decay_tiles_scan_kernel(float* __restrict__ U, float* __restrict__ state, const 
   const int row = blockIdx.y / H, h = blockIdx.y % H, e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, n_new = row_q_len[row];
   if (e >= per_head || n_new <= 0) return;
   const int chunks = (n_new + TC - 1) / TC;
-  const float full = (float)pow(decays[h], (double)TC), last = (float)pow(decays[h], (double)(n_new - (chunks - 1) * TC));
+  const float full = power(decays[h], TC), last = power(decays[h], n_new - (chunks - 1) * TC);
   float4* st = reinterpret_cast<float4*>(state + ((size_t)row_slot[row] * H + h) * per_head + e);
   float* u = U + ((size_t)chunk_base[row] * H + h) * per_head + e;
   const size_t step = (size_t)H * per_head;
@@ -197,7 +209,7 @@ decay_tiles_out_kernel(const T* __restrict__ src, int stride, int q_off, int v_o
   };
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) fetch(s);
-  if (tid <= TC) pw[tid] = (float)pow(decays[h], (double)tid);
+  if (tid <= TC) pw[tid] = power(decays[h], tid);
   const T* at = src + (size_t)t0 * stride;
   load_rows<T, DK>(Q, at + q_off + (size_t)h * DK, stride, n, act, nullptr, tid);
   load_rows<T, DV>(V, at + v_off + (size_t)h * DV, stride, n, act, nullptr, tid);
