@@ -4,9 +4,8 @@
 reduced-precision matrix mode, no split over K).  bfloat16 activations go
 through the tensor cores.  For large batches (prompt portions) that is the
 library product the reference uses for its ``nn.Linear`` layers
-(DELTA/Engine/DELTA/model.py:369-370, 498-500), measured once per shape against
-the tcgen05 kernel of this package taking the rows in chunks (which has lost on
-every shape measured so far).  For the few rows of a decode
+(DELTA/Engine/DELTA/model.py:369-370, 498-500), or, where the sums stay in 32
+bit, the persistent tcgen05 kernel of this package.  For the few rows of a decode
 step the product is a stream over the weights and four kernels compete: the
 warp-level MMA kernel that loads weights straight into fragments, the persistent
 tcgen05/TMA kernel that cuts the (tile, K step) sequence into one piece per SM,
@@ -25,7 +24,7 @@ import torch
 from ..kernels import ops
 
 SMALL_M = 128          # up to this many rows a product counts as weight streaming
-MANY_M = 4096          # up to this many rows the library's product is measured against the tcgen05 kernel in chunks of rows
+MANY_M = 4096          # up to this many rows 32-bit results of bfloat16 rows come from the persistent tcgen05 kernel
 _BUCKETS = (8, 16, 32, 64, 128, 256, 512, 1024, 2048, 4096)
 _choice: Dict[tuple, str] = {}
 _times: Dict[tuple, Dict[str, float]] = {}
@@ -56,10 +55,12 @@ def _bucket(m: int) -> int:
 def _candidates(m: int, n: int, k: int, swiglu: bool, out_dtype) -> List[str]:
     c = []
     if m > SMALL_M:
-        # prompt portions: the library (what the reference uses) unless the kernel of this package beats it
+        # Prompt portions: the library (what the reference uses).  The persistent tcgen05 kernel ties with it at some sizes (441 us each for
+        # the SwiGLU of 2,048 x 11,008 x 4,096) and measured alone, at a bucket's most rows, it can win; of the row counts below that it
+        # loses up to 15 % of a layer's time, so a measurement there decides nothing.
         if out_dtype == torch.bfloat16:
             c.append("lib")
-        if ops.gemm_tc_many_rows_supported(m, n, k, swiglu):
+        elif ops.gemm_tc_many_rows_supported(m, n, k, swiglu):
             c.append("tcr")
         return c
     if m <= 64 and ops.gemm_small_m_supported(m, n, k, swiglu):
