@@ -21,6 +21,8 @@
 // e^(L_t) k_t.  So
 //   1. delta_chunk: every chunk of every head in parallel: A, B, U, W and the scaled queries and keys;
 //   2. delta_walk:  along a row, chunk after chunk, a slice of the value columns per block: three small products a chunk.
+// Rows of 1,301 and 747 tokens, 16 heads of 128 x 128: chunks 190 -> 85 us, walk 210 -> 170 us (with the changes that the kernels' comments
+// name).  Against 64 bits as before: outputs 1.6e-7 to 2.3e-7 off, states 1.1e-7 to 2.4e-7, weak to strong decays.
 // No exponent is ever positive.  Sums of log decays are kept as two floats, so that a difference of two of them is as good
 // when the sums themselves are large.
 #include "common.cuh"
@@ -144,9 +146,10 @@ constexpr int C = 32;                    // tokens of a chunk
 constexpr int CP = C + 4;                // padded row of a chunk-by-chunk matrix
 constexpr int PREP_THREADS = 288;        // 36 tiles of 4 x 4 token pairs on and below the diagonal, eight lanes each
 constexpr int WALK_THREADS = 256;
-constexpr int WALK_COLS = 16;            // value columns of a block
+constexpr int WALK_COLS = 16;            // value columns of a slice; a block of the walk takes one or two
 constexpr int SHARES = WALK_THREADS / 32;      // the warps share the channels of the first product
 constexpr int WALK_LD = WALK_COLS + 4;
+constexpr int WALK_U = C * WALK_LD + 16;       // floats of a slice's U in shared memory: neighbouring slices meet no bank twice
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LEAST_LOG2 = -1000.f;    // 2^-1000 is zero in 32 bit: a token's log decay is no smaller, so that sums stay finite
 constexpr size_t SMEM_LIMIT = 220 * 1024;
@@ -175,16 +178,21 @@ struct ChunkLayout {
 };
 
 size_t prep_smem(int dk) { return (size_t)(4 * C * prep_ld(dk) + 2 * C * CP + C) * sizeof(float); }
-size_t walk_stage(int dk) { return (size_t)(2 * C * (pad_k(dk) + 4) + C * pad_k(dk) + C * WALK_LD + C * CP + pad_k(dk)) * sizeof(float); }
-size_t walk_smem(int dk, int stages) { return stages * walk_stage(dk) + (size_t)(pad_k(dk) * WALK_LD + SHARES * 2 * C * WALK_LD + C * WALK_LD) * sizeof(float); }
+size_t walk_stage(int dk, int cols) { return (size_t)(2 * C * (pad_k(dk) + 4) + C * pad_k(dk) + cols / WALK_COLS * WALK_U + C * CP + pad_k(dk)) * sizeof(float); }
+size_t walk_smem(int dk, int stages, int cols = WALK_COLS) {
+  return stages * walk_stage(dk, cols) + (size_t)(pad_k(dk) + SHARES * 2 * C + C) * (cols + 4) * sizeof(float);
+}
 
-// grid (most chunks of a row, rows * H).
-template <typename T>
-__global__ void __launch_bounds__(PREP_THREADS, 2)
+// grid (most chunks of a row, rows * H).  Bound by instructions issued, and by how many warps are there to issue them: keys of 64 or 128 are a
+// constant (DK; 0: any size), so that shared memory is read at constant distances instead of addresses that are computed (173 -> 85 us with
+// the third block an SM and the fence in the triangular system); below the diagonal eight exponentials serve sixteen pairs (190 -> 173).
+template <typename T, int DK>
+__global__ void __launch_bounds__(PREP_THREADS, 3)
 delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, const T* __restrict__ b, int b_stride,
                    const float* __restrict__ a, int a_stride, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                    float* __restrict__ work, const int* __restrict__ row_q_start, const int* __restrict__ row_q_len,
-                   const int* __restrict__ chunk_base, int H, int G, int dk, int dv, float q_scale, float guard, int vec) {
+                   const int* __restrict__ chunk_base, int H, int G, int dk_, int dv, float q_scale, float guard, int vec) {
+  const int dk = DK ? DK : dk_;
   extern __shared__ __align__(16) float sm[];
   const int row = blockIdx.y / H, h = blockIdx.y % H, c0 = blockIdx.x * C, n_new = row_q_len[row];
   if (c0 >= n_new) return;
@@ -203,6 +211,7 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
   const float rate = expf(A_log[h]) * LOG2E;
   if (vec) {      // sizes and addresses allow sixteen-byte loads (eight bfloat16 or float entries at a time)
     const int per = dk / 8;
+#pragma unroll 4
     for (int idx = tid; idx < 2 * C * per; idx += PREP_THREADS) {
       const int r = idx / per, i = (idx - r * per) * 8, t = r & (C - 1);
       float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -210,6 +219,7 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
 #pragma unroll
       for (int e = 0; e < 8; e += 2) *reinterpret_cast<float2*>(Q + r * ld + i + e) = make_float2(x[e], x[e + 1]);      // K's rows follow Q's
     }
+#pragma unroll 2
     for (int idx = tid; idx < C * per; idx += PREP_THREADS) {
       const int t = idx / per, i = (idx - t * per) * 8;
       float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, bias[8];
@@ -253,31 +263,54 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
     }
   }
   __syncthreads();
-  {      // A and B: a tile of 4 x 4 pairs (t, s) per eight lanes, which share the channels
+  {      // A and B: a tile of 4 x 4 pairs (t, s) per eight lanes, which share the channels; 28 tiles below the diagonal, then the eight on it
     const int tile = tid >> 3, part = tid & 7;
-    int ti = 0;
-    while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-    const int tj = tile - ti * (ti + 1) / 2;
+    int ti = tile - 28, tj = ti;
     float acc[32];      // [0, 16): A, [16, 32): B
 #pragma unroll
     for (int x = 0; x < 32; ++x) acc[x] = 0.f;
-    for (int i = part; i < dk; i += 8) {
-      float kt[4], qt[4], ht[4], lt[4], kk[4], hs[4], ls[4];
+    if (tile < 28) {
+      // e^(L_t - L_s) = e^(L_t - L_r) e^(L_r - L_s) with r the last of the four tokens s: eight exponentials for sixteen pairs
+      ti = 1;
+      while (ti * (ti + 1) / 2 <= tile) ++ti;
+      tj = tile - ti * (ti - 1) / 2;
+      for (int i = part; i < dk; i += 8) {
+        float kt[4], qt[4], w[4];
+        const int rr = (4 * tj + 3) * ld + i;
+        const float hr = Lh[rr], lr = Ll[rr];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int rt = (4 * ti + x) * ld + i, rs = (4 * tj + x) * ld + i;
-        kt[x] = K[rt]; qt[x] = Q[rt]; ht[x] = Lh[rt]; lt[x] = Ll[rt];
-        kk[x] = K[rs]; hs[x] = Lh[rs]; ls[x] = Ll[rs];
-      }
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          // above the diagonal the exponent would be positive: those pairs are dropped below
-          const float w = exp2f(fminf((ht[x] - hs[y]) + (lt[x] - ls[y]), 0.f)) * kk[y];
-          acc[4 * x + y] = fmaf(kt[x], w, acc[4 * x + y]);
-          acc[16 + 4 * x + y] = fmaf(qt[x], w, acc[16 + 4 * x + y]);
+        for (int x = 0; x < 4; ++x) {
+          const int rt = (4 * ti + x) * ld + i, rs = (4 * tj + x) * ld + i;
+          const float f = exp2f(fminf((Lh[rt] - hr) + (Ll[rt] - lr), 0.f));
+          kt[x] = K[rt] * f;
+          qt[x] = Q[rt] * f;
+          w[x] = x == 3 ? K[rs] : K[rs] * exp2f(fminf((hr - Lh[rs]) + (lr - Ll[rs]), 0.f));
         }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            acc[4 * x + y] = fmaf(kt[x], w[y], acc[4 * x + y]);
+            acc[16 + 4 * x + y] = fmaf(qt[x], w[y], acc[16 + 4 * x + y]);
+          }
+      }
+    } else {
+      for (int i = part; i < dk; i += 8) {
+        float k[4], q[4], h[4], l[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int rt = (4 * ti + x) * ld + i;
+          k[x] = K[rt]; q[x] = Q[rt]; h[x] = Lh[rt]; l[x] = Ll[rt];
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int y = 0; y <= x; ++y) {
+            const float w = x == y ? k[y] : exp2f(fminf((h[x] - h[y]) + (l[x] - l[y]), 0.f)) * k[y];
+            acc[4 * x + y] = fmaf(k[x], w, acc[4 * x + y]);
+            acc[16 + 4 * x + y] = fmaf(q[x], w, acc[16 + 4 * x + y]);
+          }
+      }
     }
     // the eight lanes' sums: each step halves what a lane keeps, so lane `part` ends with four of the 32
 #pragma unroll
@@ -300,17 +333,19 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
   }
   __syncthreads();
   for (int idx = tid; idx < C * C; idx += PREP_THREADS) ws[at.b + (idx >> 5) * CP + (idx & 31)] = B[(idx >> 5) * CP + (idx & 31)];
-  for (int idx = tid; idx < C * kp; idx += PREP_THREADS) {
-    const int t = idx / kp, i = idx - t * kp;
-    float q = 0.f, k = 0.f;
-    if (i < dk) {
-      const int r = t * ld + i, last = (C - 1) * ld + i;
-      q = Q[r] * exp2f(Lh[r] + Ll[r]);
-      k = K[r] * exp2f((Lh[last] - Lh[r]) + (Ll[last] - Ll[r]));
+  for (int t = warp; t < C; t += PREP_THREADS / 32)
+    for (int i = 2 * lane; i < kp; i += 64) {
+      float q[2] = {0.f, 0.f}, k[2] = {0.f, 0.f};
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (i + e < dk) {
+          const int r = t * ld + i + e, last = (C - 1) * ld + i + e;
+          q[e] = Q[r] * exp2f(Lh[r] + Ll[r]);
+          k[e] = K[r] * exp2f((Lh[last] - Lh[r]) + (Ll[last] - Ll[r]));
+        }
+      *reinterpret_cast<float2*>(ws + at.q + t * at.wl + i) = make_float2(q[0], q[1]);
+      *reinterpret_cast<float2*>(ws + at.k + t * kp + i) = make_float2(k[0], k[1]);
     }
-    ws[at.q + t * at.wl + i] = q;
-    ws[at.k + idx] = k;
-  }
   for (int i = tid; i < kp; i += PREP_THREADS) ws[at.d + i] = i < dk ? exp2f(Lh[(C - 1) * ld + i] + Ll[(C - 1) * ld + i]) : 0.f;
   // the triangular system, a thread per column of the right-hand side: U from the values, W from the decayed keys
   for (int c = tid; c < vp + kp; c += PREP_THREADS) {
@@ -319,13 +354,14 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
     if (c < vp) {
       const T* src = qkv + (size_t)t0 * stride + v_off + (size_t)h * dv + c;
 #pragma unroll
-      for (int t = 0; t < C; ++t) r[t] = (t < n && c < dv) ? to_f32<T>(src[(size_t)t * stride]) : 0.f;
+      for (int t = 0; t < C; ++t, src += stride) r[t] = (t < n && c < dv) ? to_f32<T>(*src) : 0.f;
     } else {
 #pragma unroll
       for (int t = 0; t < C; ++t) r[t] = i < dk ? K[t * ld + i] * exp2f(Lh[t * ld + i] + Ll[t * ld + i]) : 0.f;
     }
 #pragma unroll
     for (int s = 0; s < C; ++s) {
+      if (s % 4 == 0) asm volatile("" ::: "memory");      // or the loads of many steps are hoisted and registers spilled for them
       const float x = beta[s] * r[s];
       r[s] = x;
 #pragma unroll
@@ -340,149 +376,182 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
     float* dst = c < vp ? ws + at.u + (c / WALK_COLS) * C * WALK_LD + c % WALK_COLS : ws + at.w + i;
     const int step = c < vp ? WALK_LD : at.wl;
 #pragma unroll
-    for (int t = 0; t < C; ++t) dst[(size_t)t * step] = r[t];
+    for (int t = 0; t < C; ++t, dst += step) *dst = r[t];
   }
 }
 
-// grid (slices of the value columns, rows * H).  STAGES 2: the next chunk's matrices are fetched during this chunk's products.
-template <int STAGES>
-__global__ void __launch_bounds__(WALK_THREADS)
+// grid (slices of COLS value columns, rows * H).  STAGES 2: the next chunk's matrices are fetched during this chunk's products.  Bound by
+// shared memory, of which a sixteen-byte load takes four cycles whatever its lanes share: with 32 columns a thread has sums of 8 x 8 and
+// 8 x 4 (per FMA two thirds of the loads that 8 x 4 and 4 x 4 sums take), and a chunk's common matrices are read by half as many blocks.
+// Slices of 32 where slices of 16 are more than the SMs (one block an SM, so a row's last slices would wait for another row's): 256 slices
+// of 16 take 210 us, 128 of 32 take 170 (178 with the keys' size a variable); 128 of 16, all at once, are the shorter chain.
+template <int STAGES, int COLS, int DK>
+__global__ void __launch_bounds__(WALK_THREADS, 1)
 delta_walk_kernel(const float* __restrict__ work, float* __restrict__ state, float* __restrict__ out, const int* __restrict__ row_slot,
                   const int* __restrict__ row_q_start, const int* __restrict__ row_q_len, const int* __restrict__ chunk_base, int H,
-                  int dk, int dv) {
+                  int dk_, int dv) {
+  const int dk = DK ? DK : dk_;
+  constexpr int LD = COLS + 4, JT = COLS / 4, SLICES = COLS / WALK_COLS, CT = SLICES;
+  constexpr int RI = COLS / 4;            // channels of the state of a thread
+  constexpr int RO = COLS / 16;           // output rows of a thread
+  constexpr int HALF = WALK_THREADS / 2;
   extern __shared__ __align__(16) float sm[];
-  const int row = blockIdx.y / H, h = blockIdx.y % H, j0 = blockIdx.x * WALK_COLS, n_new = row_q_len[row];
+  const int row = blockIdx.y / H, h = blockIdx.y % H, j0 = blockIdx.x * COLS, n_new = row_q_len[row];
   if (n_new <= 0) return;
   const ChunkLayout at(dk, dv);
   const int kp = pad_k(dk), wl = at.wl, tid = threadIdx.x;
-  const int jn = min(WALK_COLS, dv - j0);
-  const int stage_floats = at.common + C * WALK_LD;
+  const int jn = min(COLS, dv - j0);
+  const int stage_floats = at.common + SLICES * WALK_U;
   float* stages = sm;
-  float* S = sm + STAGES * stage_floats;             // [kp][WALK_LD]
-  float* part = S + kp * WALK_LD;                    // [SHARES][2 C][WALK_LD]: the shares of the first product
-  float* O = part + SHARES * 2 * C * WALK_LD;        // [C][WALK_LD]
+  float* S = sm + STAGES * stage_floats;      // [kp][LD]
+  float* part = S + kp * LD;                  // [SHARES][2 C][LD]: the shares of the first product
+  float* O = part + SHARES * 2 * C * LD;      // [C][LD]
   const int chunks = (n_new + C - 1) / C;
   const float* ws0 = work + ((size_t)chunk_base[row] * H + h) * at.size;
   auto fetch = [&](int c) {
     const float* ws = ws0 + (size_t)c * H * at.size;
     float* X = stages + (STAGES == 2 ? (c & 1) : 0) * stage_floats;
     for (int idx = tid; idx < at.common / 4; idx += WALK_THREADS) cp_async_16(smem_u32(X + idx * 4), ws + idx * 4, true);
-    const float* u = ws + at.u + (size_t)blockIdx.x * C * WALK_LD;
-    for (int idx = tid; idx < C * WALK_LD / 4; idx += WALK_THREADS) cp_async_16(smem_u32(X + at.common + idx * 4), u + idx * 4, true);
+    const float* u = ws + at.u + (size_t)blockIdx.x * SLICES * C * WALK_LD;
+#pragma unroll
+    for (int s = 0; s < SLICES; ++s)
+      for (int idx = tid; idx < C * WALK_LD / 4; idx += WALK_THREADS)
+        cp_async_16(smem_u32(X + at.common + s * WALK_U + idx * 4), u + s * C * WALK_LD + idx * 4, true);
     cp_async_commit();
   };
+  auto u_at = [](float* U, int t, int j) { return reinterpret_cast<float4*>(U + j / WALK_COLS * WALK_U + t * WALK_LD + j % WALK_COLS); };
   fetch(0);
   float* st = state + (((size_t)row_slot[row] * H + h) * dv + j0) * dk;
-  for (int idx = tid; idx < kp * WALK_COLS; idx += WALK_THREADS) {
+  for (int idx = tid; idx < kp * COLS; idx += WALK_THREADS) {
     const int j = idx / kp, i = idx - j * kp;
-    S[i * WALK_LD + j] = (i < dk && j < jn) ? st[(size_t)j * dk + i] : 0.f;
+    S[i * LD + j] = (i < dk && j < jn) ? st[(size_t)j * dk + i] : 0.f;
   }
   const int share = tid >> 5, ti = (tid & 31) >> 2, tj = tid & 3;
   for (int c = 0; c < chunks; ++c) {
-    if (STAGES == 2 && c + 1 < chunks) {
-      fetch(c + 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+    cp_async_wait<0>();
+    __syncthreads();      // the chunk is in; everybody has left the one before
+    if (STAGES == 2 && c + 1 < chunks) fetch(c + 1);
     float* X = stages + (STAGES == 2 ? (c & 1) : 0) * stage_floats;
     const float *Kd = X + at.k, *B = X + at.b, *D = X + at.d;
     float* U = X + at.common;
-    {      // [W ; Q] S: a thread takes the rows ti + 8 q and four columns; the warps share the channels
-      float acc[8][4] = {};
+    {      // [W ; Q] S: a thread takes the rows ti + 8 q and 4 CT neighbouring columns; the warps share the channels
+      float acc[8][4 * CT] = {};
+#pragma unroll 2
       for (int i4 = share; i4 < kp / 4; i4 += SHARES) {
-        float4 s[4];
+        float s[4][4 * CT];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) s[q] = *reinterpret_cast<const float4*>(S + (4 * i4 + q) * WALK_LD + 4 * tj);
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int m = 0; m < CT; ++m)
+            *reinterpret_cast<float4*>(&s[e][4 * m]) = *reinterpret_cast<const float4*>(S + (4 * i4 + e) * LD + 4 * (CT * tj + m));
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const float4 x = *reinterpret_cast<const float4*>(X + (ti + 8 * q) * wl + 4 * i4);
           const float xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            acc[q][0] = fmaf(xv[e], s[e].x, acc[q][0]);
-            acc[q][1] = fmaf(xv[e], s[e].y, acc[q][1]);
-            acc[q][2] = fmaf(xv[e], s[e].z, acc[q][2]);
-            acc[q][3] = fmaf(xv[e], s[e].w, acc[q][3]);
-          }
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int m = 0; m < 4 * CT; ++m) acc[q][m] = fmaf(xv[e], s[e][m], acc[q][m]);
         }
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        *reinterpret_cast<float4*>(part + ((size_t)share * 2 * C + ti + 8 * q) * WALK_LD + 4 * tj) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+#pragma unroll
+        for (int m = 0; m < CT; ++m)
+          *reinterpret_cast<float4*>(part + ((size_t)share * 2 * C + ti + 8 * q) * LD + 4 * (CT * tj + m)) =
+              make_float4(acc[q][4 * m], acc[q][4 * m + 1], acc[q][4 * m + 2], acc[q][4 * m + 3]);
     }
     __syncthreads();
-    {
-      const int t = tid >> 2, j = (tid & 3) * 4;
+#pragma unroll
+    for (int idx = tid; idx < 2 * C * JT; idx += WALK_THREADS) {
+      const int t = idx / JT, j = idx % JT * 4;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int q = 0; q < SHARES; ++q) {
-        const float4 w = *reinterpret_cast<const float4*>(part + ((size_t)q * 2 * C + t) * WALK_LD + j);
+        const float4 w = *reinterpret_cast<const float4*>(part + ((size_t)q * 2 * C + t) * LD + j);
         v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
       }
       if (t < C) {
-        float4* u = reinterpret_cast<float4*>(U + t * WALK_LD + j);
+        float4* u = u_at(U, t, j);
         const float4 o = *u;
         *u = make_float4(o.x - v.x, o.y - v.y, o.z - v.z, o.w - v.w);
       } else {
-        *reinterpret_cast<float4*>(O + (t - C) * WALK_LD + j) = v;
+        *reinterpret_cast<float4*>(O + (t - C) * LD + j) = v;
       }
     }
     __syncthreads();
-    if (tid < WALK_THREADS / 2) {      // half of the warps: the state behind the chunk
-      for (int tile = tid; tile < kp; tile += WALK_THREADS / 2) {
-        const int i = (tile >> 2) * 4, j = (tile & 3) * 4;
-        float acc[4][4];
+    if (tid < HALF) {      // half of the warps: the state behind the chunk, RI neighbouring channels by four columns
+      for (int tile = tid; tile / JT * RI < kp; tile += HALF) {
+        const int i = tile / JT * RI, j = tile % JT * 4;
+        const bool whole = CT == 1 || i + 4 < kp;      // (kp is a multiple of four)
+        float acc[RI][4];
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const float4 s = *reinterpret_cast<const float4*>(S + (i + x) * WALK_LD + j);
+        for (int x = 0; x < RI; ++x) {
+          if (x >= 4 && !whole) continue;
+          const float4 s = *reinterpret_cast<const float4*>(S + (i + x) * LD + j);
           const float d = D[i + x];
           acc[x][0] = d * s.x; acc[x][1] = d * s.y; acc[x][2] = d * s.z; acc[x][3] = d * s.w;
         }
-#pragma unroll 8
+#pragma unroll 4
         for (int s = 0; s < C; ++s) {
-          const float4 k = *reinterpret_cast<const float4*>(Kd + s * kp + i);
-          const float4 u = *reinterpret_cast<const float4*>(U + s * WALK_LD + j);
-          const float kx[4] = {k.x, k.y, k.z, k.w};
+          const float4 u = *u_at(U, s, j);
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            acc[x][0] = fmaf(kx[x], u.x, acc[x][0]);
-            acc[x][1] = fmaf(kx[x], u.y, acc[x][1]);
-            acc[x][2] = fmaf(kx[x], u.z, acc[x][2]);
-            acc[x][3] = fmaf(kx[x], u.w, acc[x][3]);
+          for (int m = 0; m < CT; ++m) {
+            const float4 k = *reinterpret_cast<const float4*>(Kd + s * kp + i + (m == 0 || whole ? 4 * m : 0));
+            const float kx[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              acc[4 * m + x][0] = fmaf(kx[x], u.x, acc[4 * m + x][0]);
+              acc[4 * m + x][1] = fmaf(kx[x], u.y, acc[4 * m + x][1]);
+              acc[4 * m + x][2] = fmaf(kx[x], u.z, acc[4 * m + x][2]);
+              acc[4 * m + x][3] = fmaf(kx[x], u.w, acc[4 * m + x][3]);
+            }
           }
         }
 #pragma unroll
-        for (int x = 0; x < 4; ++x) *reinterpret_cast<float4*>(S + (i + x) * WALK_LD + j) = make_float4(acc[x][0], acc[x][1], acc[x][2], acc[x][3]);
+        for (int x = 0; x < RI; ++x)
+          if (x < 4 || whole) *reinterpret_cast<float4*>(S + (i + x) * LD + j) = make_float4(acc[x][0], acc[x][1], acc[x][2], acc[x][3]);
       }
-    } else {      // the other half: the chunk's outputs
-      const int idx = tid - WALK_THREADS / 2, t = idx >> 2, j = (idx & 3) * 4;
-      float4 o = *reinterpret_cast<const float4*>(O + t * WALK_LD + j);
-#pragma unroll 4
-      for (int s4 = 0; s4 < C / 4; ++s4) {
-        const float4 w = *reinterpret_cast<const float4*>(B + t * CP + 4 * s4);
-        const float wv[4] = {w.x, w.y, w.z, w.w};
+    } else {      // the other half: the chunk's outputs, RO neighbouring rows by four columns; B is zero above the diagonal
+      const int idx = tid - HALF, t = idx / JT * RO, j = idx % JT * 4;
+      float o[RO][4];
+#pragma unroll
+      for (int r = 0; r < RO; ++r) *reinterpret_cast<float4*>(o[r]) = *reinterpret_cast<const float4*>(O + (t + r) * LD + j);
+#pragma unroll 2
+      for (int s4 = 0; s4 <= (t + RO - 1) / 4; ++s4) {
+        float w[RO][4];
+#pragma unroll
+        for (int r = 0; r < RO; ++r) *reinterpret_cast<float4*>(w[r]) = *reinterpret_cast<const float4*>(B + (t + r) * CP + 4 * s4);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float4 u = *reinterpret_cast<const float4*>(U + (4 * s4 + e) * WALK_LD + j);
-          o.x = fmaf(wv[e], u.x, o.x); o.y = fmaf(wv[e], u.y, o.y); o.z = fmaf(wv[e], u.z, o.z); o.w = fmaf(wv[e], u.w, o.w);
+          const float4 u = *u_at(U, 4 * s4 + e, j);
+#pragma unroll
+          for (int r = 0; r < RO; ++r) {
+            o[r][0] = fmaf(w[r][e], u.x, o[r][0]);
+            o[r][1] = fmaf(w[r][e], u.y, o[r][1]);
+            o[r][2] = fmaf(w[r][e], u.z, o[r][2]);
+            o[r][3] = fmaf(w[r][e], u.w, o[r][3]);
+          }
         }
       }
-      if (c * C + t < n_new) {
-        float* dst = out + (size_t)(row_q_start[row] + c * C + t) * H * dv + (size_t)h * dv + j0 + j;
-        const float ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (j + e < jn) dst[e] = ov[e];
-      }
+      for (int r = 0; r < RO; ++r)
+        if (c * C + t + r < n_new) {
+          float* dst = out + (size_t)(row_q_start[row] + c * C + t + r) * H * dv + (size_t)h * dv + j0 + j;
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (j + e < jn) dst[e] = o[r][e];
+        }
     }
-    __syncthreads();
-    if (STAGES == 1 && c + 1 < chunks) fetch(c + 1);
+    if (STAGES == 1 && c + 1 < chunks) {
+      __syncthreads();
+      fetch(c + 1);
+    }
   }
+  __syncthreads();
   for (int idx = tid; idx < dk * jn; idx += WALK_THREADS) {
     const int j = idx / dk, i = idx - j * dk;
-    st[(size_t)j * dk + i] = S[i * WALK_LD + j];
+    st[(size_t)j * dk + i] = S[i * LD + j];
   }
 }
 
@@ -549,10 +618,14 @@ extern "C" int dk_delta_rule_chunked(const void* qkv, int stride, int k_off, int
   static bool granted[DK_MAX_DEVICES] = {false};
   const int dev = dk_current_device();
   if (!granted[dev]) {
-    if (cudaFuncSetAttribute(delta_chunk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
-        cudaFuncSetAttribute(delta_chunk_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
-        cudaFuncSetAttribute(delta_walk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
-        cudaFuncSetAttribute(delta_walk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess) {
+    const auto grant = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT); };
+    if (grant(delta_chunk_kernel<float, 0>) != cudaSuccess || grant(delta_chunk_kernel<float, 64>) != cudaSuccess ||
+        grant(delta_chunk_kernel<float, 128>) != cudaSuccess || grant(delta_chunk_kernel<__nv_bfloat16, 0>) != cudaSuccess ||
+        grant(delta_chunk_kernel<__nv_bfloat16, 64>) != cudaSuccess || grant(delta_chunk_kernel<__nv_bfloat16, 128>) != cudaSuccess ||
+        grant(delta_walk_kernel<1, WALK_COLS, 0>) != cudaSuccess || grant(delta_walk_kernel<2, WALK_COLS, 0>) != cudaSuccess ||
+        grant(delta_walk_kernel<2, WALK_COLS, 64>) != cudaSuccess || grant(delta_walk_kernel<2, WALK_COLS, 128>) != cudaSuccess ||
+        grant(delta_walk_kernel<2, 2 * WALK_COLS, 0>) != cudaSuccess || grant(delta_walk_kernel<2, 2 * WALK_COLS, 64>) != cudaSuccess ||
+        grant(delta_walk_kernel<2, 2 * WALK_COLS, 128>) != cudaSuccess) {
       cudaGetLastError();
       DK_REQUIRE(false, "delta_rule_chunked: %zu bytes of shared memory were not granted", SMEM_LIMIT);
     }
@@ -561,18 +634,35 @@ extern "C" int dk_delta_rule_chunked(const void* qkv, int stride, int k_off, int
   const dim3 grid(max_chunks, rows * H);
   const int vec = dk % 8 == 0 && stride % 8 == 0 && k_off % 8 == 0 && a_stride % 4 == 0 && ((uintptr_t)qkv % 16) == 0 && ((uintptr_t)a % 16) == 0 &&
                   ((uintptr_t)dt_bias % 16) == 0;
-  if (dtype == DK_F32)
-    delta_chunk_kernel<float><<<grid, PREP_THREADS, prep_smem(dk), stream>>>((const float*)qkv, stride, k_off, v_off, (const float*)b, b_stride, a, a_stride,
-                                                                             A_log, dt_bias, work, row_q_start, row_q_len, chunk_base, H, G, dk, dv, q_scale, guard, vec);
-  else
-    delta_chunk_kernel<__nv_bfloat16><<<grid, PREP_THREADS, prep_smem(dk), stream>>>((const __nv_bfloat16*)qkv, stride, k_off, v_off, (const __nv_bfloat16*)b,
-                                                                                     b_stride, a, a_stride, A_log, dt_bias, work, row_q_start, row_q_len,
-                                                                                     chunk_base, H, G, dk, dv, q_scale, guard, vec);
+#define CHUNK(T, DK)                                                                                                                        \
+  delta_chunk_kernel<T, DK><<<grid, PREP_THREADS, prep_smem(dk), stream>>>((const T*)qkv, stride, k_off, v_off, (const T*)b, b_stride, a,     \
+                                                                          a_stride, A_log, dt_bias, work, row_q_start, row_q_len, chunk_base, \
+                                                                          H, G, dk, dv, q_scale, guard, vec)
+#define PICK(T)                       \
+  do {                                \
+    if (dk == 128) CHUNK(T, 128);     \
+    else if (dk == 64) CHUNK(T, 64);  \
+    else CHUNK(T, 0);                 \
+  } while (0)
+  if (dtype == DK_F32) PICK(float);
+  else PICK(__nv_bfloat16);
+#undef PICK
+#undef CHUNK
   if (int e = dk_check_launch("delta_rule_chunked")) return e;
-  const dim3 walk((dv + WALK_COLS - 1) / WALK_COLS, rows * H);
-  if (walk_smem(dk, 2) <= SMEM_LIMIT)
-    delta_walk_kernel<2><<<walk, WALK_THREADS, walk_smem(dk, 2), stream>>>(work, state, out, row_slot, row_q_start, row_q_len, chunk_base, H, dk, dv);
-  else
-    delta_walk_kernel<1><<<walk, WALK_THREADS, walk_smem(dk, 1), stream>>>(work, state, out, row_slot, row_q_start, row_q_len, chunk_base, H, dk, dv);
+  const int slices = pad_v(dv) / WALK_COLS;
+#define WALK(ST, COLS, DK)                                                                                                                     \
+  delta_walk_kernel<ST, COLS, DK><<<dim3(slices * WALK_COLS / (COLS), rows * H), WALK_THREADS, walk_smem(dk, ST, COLS), stream>>>(work, state, out, \
+                                                                                     row_slot, row_q_start, row_q_len, chunk_base, H, dk, dv)
+#define PICK(COLS)                       \
+  do {                                   \
+    if (dk == 128) WALK(2, COLS, 128);   \
+    else if (dk == 64) WALK(2, COLS, 64); \
+    else WALK(2, COLS, 0);               \
+  } while (0)
+  if (slices % 2 == 0 && slices * rows * H > dk_sm_count() && walk_smem(dk, 2, 2 * WALK_COLS) <= SMEM_LIMIT) PICK(2 * WALK_COLS);
+  else if (walk_smem(dk, 2) <= SMEM_LIMIT) PICK(WALK_COLS);
+  else WALK(1, WALK_COLS, 0);
+#undef PICK
+#undef WALK
   return dk_check_launch("delta_rule_chunked");
 }

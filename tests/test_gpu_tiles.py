@@ -212,7 +212,7 @@ def test_gemm_rows_tc_pieces(M, N, K, dtype):
 
 
 @pytest.mark.parametrize("scoring, correction, groups", [("softmax", False, None), ("sigmoid", True, (4, 2)), ("softmax_all", True, (4, 2)), ("sigmoid", False, None)])
-@pytest.mark.parametrize("T, rows, E, d", [(128, 17, 16, 64), (201, 20, 20, 2048), (2048, 16, 16, 1024), (130, 72, 64, 96)])
+@pytest.mark.parametrize("T, rows, E, d", [(128, 17, 16, 64), (201, 20, 20, 2048), (2048, 16, 16, 1024), (130, 72, 64, 96), (901, 17, 16, 64), (1003, 72, 64, 96)])
 def test_router_of_many_tokens(T, rows, E, d, scoring, correction, groups):
     """Tiles of 16 tokens and 32 rows, the last ones partly filled; blocks of 32 entries that not every warp has."""
     o = ops()
@@ -308,7 +308,7 @@ def test_experts_stream(T, E, top, F, d, act):
     assert bool(torch.isfinite(got[1][1]).all()) and (got[0][1] - got[1][1]).abs().max() <= 1e-2 * got[0][1].abs().max()
 
 
-@pytest.mark.parametrize("T, rows, E, d", [(1, 17, 16, 2048), (8, 20, 20, 1000), (127, 40, 33, 4096)])
+@pytest.mark.parametrize("T, rows, E, d", [(1, 17, 16, 2048), (8, 20, 20, 1000), (127, 40, 33, 4096), (384, 32, 32, 2056)])
 def test_router_of_few_tokens(T, rows, E, d):
     o = ops()
     torch.manual_seed(T + rows)
@@ -319,3 +319,35 @@ def test_router_of_few_tokens(T, rows, E, d):
     assert (z.double() - ref).norm() < 3e-7 * ref.norm()      # exact products, sums of 32 bit
     val, idx = torch.topk(z[:, :E], 4, dim=-1)
     assert torch.equal(choice.long(), idx) and torch.allclose(weight, torch.softmax(val, -1), atol=1e-6)
+
+
+# slices of 32 value columns once all rows together have more slices of 16 than the chip has SMs; an odd number of slices keeps 16
+@pytest.mark.parametrize("H, dk, dv", [(16, 128, 128), (30, 100, 50), (24, 40, 72)])
+def test_delta_walk_slices(H, dk, dv):
+    """Rows together and one by one: the same bits whatever the slices; both against the kernel that takes the tokens in turn."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(H + dk)
+    rand = lambda *shape: torch.randn(shape, device=DEV, generator=g)      # noqa: E731
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)      # noqa: E731
+    lens, slots = [97, 32, 1], [3, 0, 2]
+    T, C = sum(lens), o.delta_rule_chunk()
+    qkv, b, a = rand(T, 2 * H * dk + H * dv).bfloat16(), rand(T, H).bfloat16(), rand(T, H * dk)
+    A_log, dt_bias, state = rand(H) * 0.5 - 1.0, rand(H * dk), rand(4, H, dv, dk)
+    def run(rows, st, out, turns):
+        args = (qkv, H * dk, 2 * H * dk, b.data_ptr(), H, a, A_log, dt_bias, st, out)
+        where = dict(row_slot=i32([slots[r] for r in rows]), row_q_start=i32([sum(lens[:r]) for r in rows]), row_q_len=i32([lens[r] for r in rows]))
+        sizes = dict(H=H, G=H, dk=dk, dv=dv, q_scale=0.3, guard=1e-6)
+        if turns:
+            return o.delta_rule(*args, **sizes, **where)
+        chunks = [-(-lens[r] // C) for r in rows]
+        work = torch.full((sum(chunks) * H * o.delta_rule_chunk_floats(dk, dv),), float("nan"), device=DEV)
+        o.delta_rule_chunked(*args, work, i32([sum(chunks[:k]) for k in range(len(rows))]), max(chunks), **sizes, **where)
+    results = []
+    for calls, turns in (([[0, 1, 2]], False), ([[0], [1], [2]], False), ([[0, 1, 2]], True)):
+        st, out = state.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
+        for rows in calls:
+            run(rows, st, out, turns)
+        results.append((out, st))
+    for x, y, z in zip(*results):
+        assert torch.equal(x, y)
+        assert (x - z).abs().max() <= 2e-5 * z.abs().max()      # each of the two kernels' own tests allows 1e-5
