@@ -887,16 +887,20 @@ extern "C" int dk_router(const void* x, const void* w, float* logits, int* choic
   while (tpb > 1 && (ROUTER_WARPS / tpb < row_groups) && (long long)T_ * (ROUTER_WARPS / tpb) < 16LL * dk_sm_count()) tpb /= 2;
   const size_t smem = (size_t)tpb * (n_rows + (scored ? E : 0) + groups) * sizeof(float);
   DK_REQUIRE(smem <= 48 * 1024, "router: %d logits a token do not fit the shared memory", n_rows);
-  // from a few blocks of 16 tokens on the tensor cores share every row of W between them (few tokens: more warps a token are worth more)
+  // From six tokens an SM on the tensor cores share every row of W between 16 tokens; below, a token's own warps end sooner.  Rows of 2,048,
+  // W cold: 1,000 tokens, 17 / 64 / 129 rows of W: 22.5 / 38.9 / 70 us against 24.6 / 38.9 / 74; 700 tokens: 21.5 / 38.9 / 70 against 16.4 / 26.6 / 49.
   const size_t mma_smem = ((size_t)ROUTE_TOKENS * (n_rows + (scored ? E : 0) + groups + 32 * ROUTER_WARPS)) * sizeof(float);
-  if (dtype == DK_BF16 && T_ >= 128 && d % 32 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && mma_smem <= 48 * 1024) {
+  if (dtype == DK_BF16 && T_ >= 6 * dk_sm_count() && d % 32 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && mma_smem <= 48 * 1024) {
     router_mma_kernel<<<(T_ + ROUTE_TOKENS - 1) / ROUTE_TOKENS, ROUTER_WARPS * 32, mma_smem, stream>>>(
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, T_, d, n_rows, E, top, correction, route_scale, scored, groups, keep,
         group_top2);
     return dk_check_launch("router");
   }
+  // One round of loads (or two) instead of a warp's share of the rows: only where that is all of W, where a token's entries keep all eight
+  // warps busy, and while a token's block finds an SM soon.  17 rows of 2,048: 64 tokens 12.3 against 16.4 us, 384 tokens 14.3 against 16.4,
+  // 512 equal; 32 rows: 8 tokens 15.5 against 17.4; 48 rows: 21.5 against 17.4.  32 rows of 1,024: 15.4 against 13.1 (17 rows equal).
   const size_t few_smem = ((size_t)n_rows * (1 + ROUTER_WARPS) + (scored ? E : 0) + groups) * sizeof(float);
-  if (dtype == DK_BF16 && T_ < 128 && d % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && few_smem <= 48 * 1024) {
+  if (dtype == DK_BF16 && d >= ROUTER_WARPS * 256 && n_rows <= 2 * FEW_ROWS && T_ <= 384 && d % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && few_smem <= 48 * 1024) {
     router_few_kernel<<<T_, ROUTER_WARPS * 32, few_smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, d, n_rows, E,
                                                                   top, correction, route_scale, scored, groups, keep, group_top2);
     return dk_check_launch("router");

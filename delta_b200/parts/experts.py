@@ -35,7 +35,12 @@ from .feed_forward import ClampedGLU
 
 TC_TILE = 128               # rows of a tile on the tcgen05 path
 STREAM_TOKENS = 32          # up to this many tokens (so many rows an expert at most) the products are a stream over the experts' weights
-TC_ROWS_PER_EXPERT = 96     # from this many rows an expert on average, the products go to the tcgen05 kernel
+# From this many rows an expert on average the products go to the tcgen05 kernel.  A layer of 16 experts of 2,048 x 1,024 (gated / squared
+# relu) with 35 rows an expert takes 128 / 89 us there and 128 / 95 us on the warp-level kernel, with 50 rows 128 / 91 and 150 / 112, with 93
+# rows 132 / 101 and 189 / 132; of 1,024 x 512 with 50 rows 89 / 60 and 77 / 62, with 93 rows 98 / 67 and 91 / 67.
+TC_ROWS_PER_EXPERT = 96
+TC_ROWS_PER_LARGE_EXPERT = 32       # the same where a product has LARGE_EXPERT weights and more
+LARGE_EXPERT = 1 << 21
 
 
 @FEED_FORWARDS.register("experts")
@@ -125,7 +130,8 @@ class Experts(FeedForward):
         # weight_input: a slot's weight goes into the first product (or into the gathered rows), and the sum at the end has none
         row_scale = weight.view(-1) if self.weight_input else None
         # many rows an expert (prompt portions): tiles of 128 rows through the tcgen05 product; else tiles of 64 through warp-level MMA
-        many = (x.dtype == torch.bfloat16 and "products" not in ctx.plain_kernels and slots >= TC_ROWS_PER_EXPERT * E and
+        most = TC_ROWS_PER_LARGE_EXPERT if d * F >= LARGE_EXPERT else TC_ROWS_PER_EXPERT
+        many = (x.dtype == torch.bfloat16 and "products" not in ctx.plain_kernels and slots >= most * E and
                 ops.experts_gemm_tc_supported(F, d, self.gated) and ops.experts_gemm_tc_supported(d, F, False))
         tile = TC_TILE if many else ops.experts_tile_rows()
         capacity = -(-(slots + (tile - 1) * min(E, slots)) // tile) * tile
