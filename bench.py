@@ -735,12 +735,15 @@ def design_workload(args, design: str) -> int:
             "attention_prefill_tc": (0, 4 * 128 * H * (T * (T + 1) // 2) * runs),
         }
 
+        # launchers that do the work of another where their sizes allow
+        same_work = {"decay_attention_tiles": "decay_attention_chunked", "state_space_mma": "state_space_chunked", "attention_rows_wide_tc": "attention_rows_mma"}
+
         def fractions(launchers, table):
             rows = {}
             for name, (calls, ms) in sorted(launchers.items(), key=lambda kv: -kv[1][1]):
                 row = {"calls": calls, "ms": round(ms, 4)}
-                if name in table and ms > 0:
-                    by, fl = table[name]
+                if (name in table or same_work.get(name) in table) and ms > 0:
+                    by, fl = table[name if name in table else same_work[name]]
                     if by:
                         row["gbs"] = round(by / ms / 1e6, 1)
                         row["of_measured_copy"] = round(by / ms / 1e6 / pk["hbm_gbs"], 3)
