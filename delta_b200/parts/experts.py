@@ -37,9 +37,10 @@ TC_TILE = 128               # rows of a tile on the tcgen05 path
 STREAM_TOKENS = 32          # up to this many tokens (so many rows an expert at most) the products are a stream over the experts' weights
 # From this many rows an expert on average the products go to the tcgen05 kernel.  A layer of 16 experts of 2,048 x 1,024 (gated / squared
 # relu) with 35 rows an expert takes 128 / 89 us there and 128 / 95 us on the warp-level kernel, with 50 rows 128 / 91 and 150 / 112, with 93
-# rows 132 / 101 and 189 / 132; of 1,024 x 512 with 50 rows 89 / 60 and 77 / 62, with 93 rows 98 / 67 and 91 / 67.
+# rows 132 / 101 and 189 / 132; of 1,024 x 512 with 50 rows 89 / 60 and 77 / 62, with 93 rows 98 / 67 and 91 / 67.  With fewer than 48 rows
+# the launches decide (one more, and four tensor maps): 130 tokens 92 against 102 us on the device, 105 against 101 a call.
 TC_ROWS_PER_EXPERT = 96
-TC_ROWS_PER_LARGE_EXPERT = 32       # the same where a product has LARGE_EXPERT weights and more
+TC_ROWS_PER_LARGE_EXPERT = 48       # the same where a product has LARGE_EXPERT weights and more
 LARGE_EXPERT = 1 << 21
 
 
