@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(CH) attention_plain_kernel(const DkAttnParams 
           const T* kr = kv + ((((size_t)page * 2 + 0) * KV + g) * ps + off) * hd;
           float d = 0.f;
           for (int i = 0; i < hd; ++i) d = fmaf(qs[i], to_f32<T>(kr[i]), d);
-          s = d * p.scale;
+          s = __fmul_rn(d, p.scale);      // (rounded by itself, as in attention_f32.cu)
           vo = (long long)((((size_t)page * 2 + 1) * KV + g) * ps + off) * hd;
           if (dumping && key < p.dump_stride) dump[key] = s;
         }
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(CH) attention_plain_kernel(const DkAttnParams 
     const float pr = (vo >= 0) ? expf(s - m_new) : 0.f;
     sc[tid] = pr;
     const float psum = block_sum(pr, scratch);
-    l = l * corr + psum;
+    l = fmaf(l, corr, psum);
     m = m_new;
 #pragma unroll
     for (int dd = 0; dd < 2; ++dd) {

@@ -4,8 +4,9 @@ bfloat16 with head size 64 or 128: rows that bring one token go to the split-key
 kernel (at most 16 query heads per key-value head), rows that bring more go to a tiled
 prefill kernel (tcgen05 with 128-query tiles when a row brings at least 32 tokens, else
 warp-level MMA with 64-query tiles); a mixed step launches both, each skipping the other's
-rows.  Everything else (32 bit, other head sizes) goes to the plain kernel, which takes
-every size.
+rows.  32-bit rows that bring enough tokens go to a kernel with tiles of 32 queries.
+Everything else (other head sizes, 32-bit rows of few tokens) goes to the plain kernel,
+which takes every size.
 
 In a replayable step (``ctx.replayable``) nothing is chosen from the step's host data: the
 grid is the one for the longest request the engine allows, and whether pages are looked for
@@ -120,14 +121,32 @@ def _prefill_kernel(ctx, params):
     return ops.attention_prefill if mma else None
 
 
+def tiles_pay(q_lens, starts, heads: int, sm_count: int) -> bool:
+    """Whether the rows of several tokens of a 32-bit step end sooner in the kernel with tiles of 32 queries than in the plain one.  Microseconds,
+    heads of 128 (heads of 64 take 0.7 of either): a pass over 128 keys takes a block of the plain kernel (one token) 16 and a block of tiles 28,
+    and once there are more blocks than run at once an SM needs 10 and 25 for each of its share.  16 heads behind 4,000 keys: 2 and 8 tokens 529
+    and 532 (tiles 800, 858), 16 tokens 794 (862), 31 tokens 1,319 (931), 300 tokens 10,926 (1,433); 300 tokens of a fresh prompt 450 (94)."""
+    longest = plain = tiles = 0.0
+    for n, start in zip(q_lens, starts):
+        if n > 1:
+            longest = max(longest, -(-(start + n) // 128))
+            passes = (start + n / 2) / 128 + 0.5
+            plain += n * passes
+            tiles += -(-n // 32) * passes
+    share = heads / sm_count
+    return max(28 * longest, 25 * tiles * share) < max(16 * longest, 10 * plain * share)
+
+
 def run(ctx, params, group: str) -> None:
     """Runs paged attention with the kernels that fit the batch.  ``group`` names the cache group
     of the layer (its block tables tell whether pages lie in runs)."""
     if plain(ctx):
-        # 32 bit: rows that bring several tokens share tiles of keys, rows of one token stay with the plain kernel whatever stands
-        # beside them, so that a row's sums are the same in every batch.  Chosen pages and score dumps are the plain kernel's.
+        # 32 bit: rows that bring several tokens may share tiles of keys.  Both kernels give a token the same bits, so the choice is one of
+        # time alone.  Chosen pages, score dumps and windows that cut keys off are the plain kernel's.
         if (not ctx.decode_only and "attention" not in ctx.plain_kernels and params.sel_pages is None and params.dump is None
-                and ops.attention_f32_supported(ctx.dtype, params.H, params.KV, params.hd, params.q_stride)):
+                and (not params.window or ctx.max_seq_len <= params.window)
+                and ops.attention_f32_supported(ctx.dtype, params.H, params.KV, params.hd, params.q_stride)
+                and ctx.memo(("32-bit tiles", params.H), lambda: tiles_pay(ctx.host["q_lens"], [r.start_pos for r in ctx.host["rows"]], params.H, ctx.sm_count))):
             if any(n == 1 for n in ctx.host["q_lens"]):
                 params.row_filter = 1
                 ops.attention_plain(params)

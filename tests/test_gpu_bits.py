@@ -1,0 +1,61 @@
+"""What a kernel must not let into a result: how a prompt was cut, what shares its step, what lies beside what it reads; and results at the
+ends of the number range."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, PagedCase, i32, ops
+
+pytestmark = pytest.mark.gpu
+
+
+# ------------------------------------------------------------------ 32-bit attention: one order of the sums, whichever kernel takes a token
+
+@pytest.mark.parametrize("H, KV, hd, ps", [(4, 2, 128, 16), (3, 3, 64, 8), (8, 1, 32, 64), (2, 1, 128, 128)])
+def test_attention_f32_has_the_bits_of_the_plain_kernel(H, KV, hd, ps):
+    """Passes of 128 keys: one key beside a pass' and a tile's ends on either side, one pass and several, portions of one token and of many."""
+    o = ops()
+    case = PagedCase(torch.float32, H, KV, hd, ps, seq_lens=[2, 33, 127, 128, 129, 160, 161, 257, 400, 700], q_lens=[2, 33, 2, 128, 129, 1, 31, 130, 400, 3],
+                     seed=H + hd)
+    out, lse = torch.full((case.T, H * hd), 9.0, device=DEV), torch.empty(case.T, H, device=DEV)
+    want, want_lse = torch.full_like(out, 9.0), torch.empty_like(lse)
+    o.attention_f32(case.params(out, lse=lse), max(case.q_lens))
+    o.attention_plain(case.params(want, lse=want_lse))
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)
+
+
+def test_attention_f32_infinite_scores_have_the_bits_of_the_plain_kernel():
+    """Keys whose score is minus infinity weigh nothing: a whole pass of them, a part of one, and the first pass."""
+    o = ops()
+    case = PagedCase(torch.float32, 2, 1, 64, 16, seq_lens=[420], q_lens=[300], seed=8)
+    q = case.qcat.view(-1, 2, 64)
+    q[:, :, 5] = q[:, :, 5].abs() + 0.1
+    for at in list(range(0, 128)) + list(range(250, 400)):
+        page = int(case.bt[0, at // 16])
+        case.kv[page, 0, 0, at % 16, 5] = -math.inf
+    out, want = torch.empty(300, 128, device=DEV), torch.empty(300, 128, device=DEV)
+    o.attention_f32(case.params(out), 300)
+    o.attention_plain(case.params(want))
+    assert torch.equal(out, want) and bool(torch.isfinite(out[100:]).all())
+
+
+@pytest.mark.parametrize("cuts", [(300,), (299, 1), (1, 299), (31, 269), (33, 129, 138), (128, 128, 44), (2, 1, 297)])
+def test_f32_logits_do_not_depend_on_the_cuts(cuts):
+    """A 32-bit prompt in portions of any lengths, single tokens among them: the bits of the whole prompt's logits."""
+    import helpers
+    from delta_b200.config import EngineConfig
+    from delta_b200.engine.step import ModelRunner, RowInput
+    cfg = helpers.tiny_config("D")
+    tokens = helpers.random_tokens(300, cfg["vocab_size"], 4)
+
+    def logits(parts):
+        runner = ModelRunner(config_json=cfg, seed=3, engine_config=EngineConfig(max_batch=1, max_seq_len=320, dtype="float32"))
+        slot = runner.cache.acquire_slot()
+        runner.cache.grow(slot, 300)
+        at, got = 0, []
+        for n in parts:
+            got.append(runner.step([RowInput(slot, tokens[at:at + n], at, list(range(n)))]).clone())
+            at += n
+        return torch.cat(got)
+    assert torch.equal(logits(cuts), logits((300,)))
