@@ -325,130 +325,126 @@ router_kernel(const T* __restrict__ x, const T* __restrict__ w, float* __restric
          groups, keep, group_top2, choice + (size_t)t * top, weight + (size_t)t * top, lane);
 }
 
-// The same for many tokens in bfloat16: a block takes 16 tokens, a warp every eighth block of 32 entries of d.  Its products are exact and
-// each MMA's sum of 16 of them starts from zero and is added to a float sum by an FMA unit; the warps' sums are added in order.
-// A lane's sixteen bytes of a row of x or W are two fragments of the MMA (in an order of the entries that both operands share), so nothing is
-// staged and all loads of a step of 128 entries are under way at once.  2,048 tokens, 17 rows of 2,048: 29 -> 18 us.
-constexpr int ROUTE_TOKENS = 16;
-constexpr int ROUTE_TILES = 4;      // tiles of eight rows of W at a time
+// The same for many tokens in bfloat16: a warp takes MANY_TOKENS tokens and ROWS rows of W at a time, so that a row's entries are fetched and
+// converted once for all of them; four warps share a token's rows.  A lane's entries of a product and their order, and the lanes' sums, are
+// the general kernel's: a token's logits have the same bits whichever kernel its step goes to.
+constexpr int MANY_TOKENS = 4, MANY_SHARERS = 4;
+constexpr int MANY_BLOCK = ROUTER_WARPS / MANY_SHARERS * MANY_TOKENS;
 
-__global__ void __launch_bounds__(ROUTER_WARPS * 32)
-router_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, float* __restrict__ logits, int* __restrict__ choice,
-                  float* __restrict__ weight, int T_, int d, int n_rows, int E, int top, const float* __restrict__ correction, float route_scale,
-                  int scored, int groups, int keep, int group_top2) {
-  extern __shared__ float zs[];      // [16][n_rows], (scored: [16][E]), (groups: [16][groups]), then the warps' sums [warps][16][32]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, t0 = blockIdx.x * ROUTE_TOKENS;
-  float* score = zs + (size_t)ROUTE_TOKENS * n_rows;
-  float* group = score + (scored ? (size_t)ROUTE_TOKENS * E : 0);
-  float* part = group + (size_t)ROUTE_TOKENS * groups;
-  const __nv_bfloat16* x0 = x + (size_t)min(t0 + g, T_ - 1) * d + t4 * 8;
-  const __nv_bfloat16* x1 = x + (size_t)min(t0 + g + 8, T_ - 1) * d + t4 * 8;
-  for (int r0 = 0; r0 < n_rows; r0 += 8 * ROUTE_TILES) {
-    float acc[ROUTE_TILES][4];
-    const __nv_bfloat16* wr[ROUTE_TILES];
+template <int ROWS>
+__global__ void __launch_bounds__(ROUTER_WARPS * 32, 2)
+router_many_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, float* __restrict__ logits, int* __restrict__ choice,
+                   float* __restrict__ weight, int T_, int d, int n_rows, int E, int top, const float* __restrict__ correction, float route_scale,
+                   int scored, int groups, int keep, int group_top2) {
+  constexpr int STEPS = ROWS <= 5 ? 2 : 1;      // (registers for two blocks an SM)
+  extern __shared__ float zs[];      // [8][n_rows], (scored: [8][E]), (groups: [8][groups])
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t0 = blockIdx.x * MANY_BLOCK, share = warp % MANY_SHARERS;
+  const int local = warp / MANY_SHARERS * MANY_TOKENS;
+  float* score = zs + (size_t)MANY_BLOCK * n_rows;
+  float* group = score + (scored ? (size_t)MANY_BLOCK * E : 0);
+  for (int r0 = share * ROWS; r0 < n_rows; r0 += MANY_SHARERS * ROWS) {
+    float acc[ROWS][MANY_TOKENS];
 #pragma unroll
-    for (int q = 0; q < ROUTE_TILES; ++q) {
-      wr[q] = w + (size_t)min(r0 + 8 * q + g, n_rows - 1) * d + t4 * 8;
+    for (int q = 0; q < ROWS; ++q)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[q][e] = 0.f;
-    }
-#pragma unroll 4
-    for (int k = warp * 32; k < d; k += ROUTER_WARPS * 32) {
-      const uint4 a = *reinterpret_cast<const uint4*>(x0 + k), b = *reinterpret_cast<const uint4*>(x1 + k);
-      const uint32_t a0[4] = {a.x, b.x, a.y, b.y}, a1[4] = {a.z, b.z, a.w, b.w};
+      for (int k = 0; k < MANY_TOKENS; ++k) acc[q][k] = 0.f;
+    for (int c0 = lane * 8; c0 < d; c0 += 256 * STEPS) {
+      uint4 xraw[STEPS][MANY_TOKENS], wraw[STEPS][ROWS];      // (tokens, rows and entries behind the last ones repeat them)
 #pragma unroll
-      for (int q = 0; q < ROUTE_TILES; ++q) {
-        if (r0 + 8 * q >= n_rows) continue;
-        const uint4 v = *reinterpret_cast<const uint4*>(wr[q] + k);
-        float s[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_bf16(s, a0, v.x, v.y);
-        mma_bf16(u, a1, v.z, v.w);
+      for (int s = 0; s < STEPS; ++s) {
+        const int c = min(c0 + s * 256, d - 8);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[q][e] += s[e] + u[e];
+        for (int k = 0; k < MANY_TOKENS; ++k) xraw[s][k] = __ldg(reinterpret_cast<const uint4*>(x + (size_t)min(t0 + local + k, T_ - 1) * d + c));
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) wraw[s][q] = __ldg(reinterpret_cast<const uint4*>(w + (size_t)min(r0 + q, n_rows - 1) * d + c));
+      }
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        if (c0 + s * 256 >= d) continue;
+        float xv[MANY_TOKENS][8];
+#pragma unroll
+        for (int k = 0; k < MANY_TOKENS; ++k) load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&xraw[s][k]), xv[k]);
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) {
+          float wv[8];
+          load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&wraw[s][q]), wv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < MANY_TOKENS; ++k) acc[q][k] = fmaf(xv[k][i], wv[i], acc[q][k]);
+        }
       }
     }
-    __syncthreads();      // the sums of the rows before have been read
 #pragma unroll
-    for (int q = 0; q < ROUTE_TILES; ++q)
+    for (int q = 0; q < ROWS; ++q)
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        *reinterpret_cast<float2*>(part + ((size_t)warp * ROUTE_TOKENS + g + 8 * e) * 32 + 8 * q + 2 * t4) = make_float2(acc[q][2 * e], acc[q][2 * e + 1]);
-    __syncthreads();
-    for (int i = threadIdx.x; i < ROUTE_TOKENS * 32; i += ROUTER_WARPS * 32) {
-      const int t = i / 32, r = r0 + i % 32;
-      if (r < n_rows) {
-        float v = 0.f;
-#pragma unroll
-        for (int q = 0; q < ROUTER_WARPS; ++q) v += part[((size_t)q * ROUTE_TOKENS + t) * 32 + i % 32];
-        zs[(size_t)t * n_rows + r] = v;
-        if (t0 + t < T_) logits[(size_t)(t0 + t) * n_rows + r] = v;
+      for (int k = 0; k < MANY_TOKENS; ++k) {
+        const float v = warp_sum(acc[q][k]);
+        if (lane == 0 && r0 + q < n_rows) {
+          zs[(size_t)(local + k) * n_rows + r0 + q] = v;
+          if (t0 + local + k < T_) logits[(size_t)(t0 + local + k) * n_rows + r0 + q] = v;
+        }
       }
-    }
   }
   __syncthreads();
-  for (int k = warp; k < ROUTE_TOKENS && t0 + k < T_; k += ROUTER_WARPS)
+  for (int k = warp; k < MANY_BLOCK && t0 + k < T_; k += ROUTER_WARPS)
     choose(zs + (size_t)k * n_rows, score + (size_t)k * E, group + (size_t)k * groups, E, top, correction, route_scale, scored, groups, keep, group_top2,
            choice + (size_t)(t0 + k) * top, weight + (size_t)(t0 + k) * top, lane);
 }
 
-// The same for few tokens in bfloat16: a block takes one token, its warps share d, and sixteen rows of W are asked for at once.  Bound by latency:
-// behind a step that streamed its experts' weights W comes from the memory again, so one round of loads instead of eight.  8 tokens, 17
-// rows of 2,048, after 200 MB: 12.2 -> 6.2 us.
-constexpr int FEW_ROWS = 16;
+// The same for few tokens in bfloat16: a block takes one token, a warp ROWS rows of W, with the loads of FEW_STEPS times 256 entries of all of
+// them under way at once.  Again every product is the general kernel's chain of FMAs.
+constexpr int FEW_STEPS = 8;
 
+template <int ROWS>
 __global__ void __launch_bounds__(ROUTER_WARPS * 32)
 router_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, float* __restrict__ logits, int* __restrict__ choice,
                   float* __restrict__ weight, int d, int n_rows, int E, int top, const float* __restrict__ correction, float route_scale, int scored,
                   int groups, int keep, int group_top2) {
-  extern __shared__ float zs[];      // [n_rows], (scored: [E]), (groups: [groups]), then the warps' sums [warps][n_rows]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x;
-  float* score = zs + n_rows;
-  float* group = score + (scored ? E : 0);
-  float* part = group + groups;
-  for (int r0 = 0; r0 < n_rows; r0 += FEW_ROWS) {
-    float acc[FEW_ROWS];
+  extern __shared__ float zs[];      // [n_rows], (scored: [E]), (groups: [groups])
+  const int lane = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * ROWS, t = blockIdx.x;
+  const __nv_bfloat16* xr = x + (size_t)t * d;
+  float acc[ROWS];
 #pragma unroll
-    for (int q = 0; q < FEW_ROWS; ++q) acc[q] = 0.f;
-    for (int c = (warp * 32 + lane) * 8; c < d; c += ROUTER_WARPS * 256) {
-      uint4 raw[FEW_ROWS];      // (rows behind the last one repeat it)
+  for (int q = 0; q < ROWS; ++q) acc[q] = 0.f;
+  if (r0 < n_rows) {
+    for (int c0 = lane * 8; c0 < d; c0 += 256 * FEW_STEPS) {
+      uint4 xraw[FEW_STEPS], wraw[FEW_STEPS][ROWS];      // (what lies behind a row's end repeats its last entries, and is not used)
 #pragma unroll
-      for (int q = 0; q < FEW_ROWS; ++q) raw[q] = __ldg(reinterpret_cast<const uint4*>(w + (size_t)min(r0 + q, n_rows - 1) * d + c));
-      float xv[8], wv[8];
-      load8<__nv_bfloat16>(x + (size_t)t * d + c, xv);
+      for (int s = 0; s < FEW_STEPS; ++s) {
+        const int c = min(c0 + s * 256, d - 8);
+        xraw[s] = *reinterpret_cast<const uint4*>(xr + c);
 #pragma unroll
-      for (int q = 0; q < FEW_ROWS; ++q) {
-        load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&raw[q]), wv);
+        for (int q = 0; q < ROWS; ++q) wraw[s][q] = __ldg(reinterpret_cast<const uint4*>(w + (size_t)min(r0 + q, n_rows - 1) * d + c));
+      }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[q] = fmaf(xv[i], wv[i], acc[q]);
+      for (int s = 0; s < FEW_STEPS; ++s) {
+        if (c0 + s * 256 >= d) continue;
+        float xv[8], wv[8];
+        load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&xraw[s]), xv);
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) {
+          load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&wraw[s][q]), wv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[q] = fmaf(xv[i], wv[i], acc[q]);
+        }
       }
     }
-    // the lanes' sums: each step halves what a lane keeps, so a pair of lanes ends with one row
 #pragma unroll
-    for (int half = FEW_ROWS / 2, bit = 16; half > 0; half >>= 1, bit >>= 1) {
-      const bool upper = (lane & bit) != 0;
-#pragma unroll
-      for (int q = 0; q < FEW_ROWS / 2; ++q)
-        if (q < half) {
-          const float send = upper ? acc[q] : acc[q + half], mine = upper ? acc[q + half] : acc[q];
-          acc[q] = mine + __shfl_xor_sync(0xffffffffu, send, bit);
-        }
+    for (int q = 0; q < ROWS; ++q) {
+      const float v = warp_sum(acc[q]);
+      if (lane == 0 && r0 + q < n_rows) {
+        zs[r0 + q] = v;
+        logits[(size_t)t * n_rows + r0 + q] = v;
+      }
     }
-    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-    if ((lane & 1) == 0 && r0 + lane / 2 < n_rows) part[(size_t)warp * n_rows + r0 + lane / 2] = acc[0];
   }
   __syncthreads();
-  for (int r = threadIdx.x; r < n_rows; r += ROUTER_WARPS * 32) {
-    float v = 0.f;
-#pragma unroll
-    for (int q = 0; q < ROUTER_WARPS; ++q) v += part[(size_t)q * n_rows + r];
-    zs[r] = v;
-    logits[(size_t)t * n_rows + r] = v;
-  }
-  __syncthreads();
-  if (warp == 0)
-    choose(zs, score, group, E, top, correction, route_scale, scored, groups, keep, group_top2, choice + (size_t)t * top, weight + (size_t)t * top, lane);
+  float* score = zs + n_rows;
+  if (threadIdx.x < 32)
+    choose(zs, score, score + (scored ? E : 0), E, top, correction, route_scale, scored, groups, keep, group_top2, choice + (size_t)t * top,
+           weight + (size_t)t * top, lane);
 }
-
 
 // One block.  sorted[p] = slot (token * top + choice) or -1; tile_expert[tile] = expert or -1.
 // HELD: choices that a thread asks for at once (a load behind every atomic would wait for it).
@@ -887,22 +883,32 @@ extern "C" int dk_router(const void* x, const void* w, float* logits, int* choic
   while (tpb > 1 && (ROUTER_WARPS / tpb < row_groups) && (long long)T_ * (ROUTER_WARPS / tpb) < 16LL * dk_sm_count()) tpb /= 2;
   const size_t smem = (size_t)tpb * (n_rows + (scored ? E : 0) + groups) * sizeof(float);
   DK_REQUIRE(smem <= 48 * 1024, "router: %d logits a token do not fit the shared memory", n_rows);
-  // From six tokens an SM on the tensor cores share every row of W between 16 tokens; below, a token's own warps end sooner.  Rows of 2,048,
-  // W cold: 1,000 tokens, 17 / 64 / 129 rows of W: 22.5 / 38.9 / 70 us against 24.6 / 38.9 / 74; 700 tokens: 21.5 / 38.9 / 70 against 16.4 / 26.6 / 49.
-  const size_t mma_smem = ((size_t)ROUTE_TOKENS * (n_rows + (scored ? E : 0) + groups + 32 * ROUTER_WARPS)) * sizeof(float);
-  if (dtype == DK_BF16 && T_ >= 6 * dk_sm_count() && d % 32 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && mma_smem <= 48 * 1024) {
-    router_mma_kernel<<<(T_ + ROUTE_TOKENS - 1) / ROUTE_TOKENS, ROUTER_WARPS * 32, mma_smem, stream>>>(
-        (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, T_, d, n_rows, E, top, correction, route_scale, scored, groups, keep,
-        group_top2);
+  const bool rows_aligned = dtype == DK_BF16 && d % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0;
+  // Two tokens an SM and less, W's rows for eight warps: one round of loads.  More than six an SM: a row of W for four tokens at a time.  Between
+  // them, and for few tokens and many rows, the general kernel.  Rows of 2,048, everything cold, microseconds: 17 rows of W and 8 / 256 / 384
+  // tokens 8.2 / 12.3 / 16.4 against 16.4 each; 32 rows 10.2 / 14.3 / 18.4 against 16.4; 17 / 64 / 129 rows and 888 tokens 16.4 / 34.8 / 69.6
+  // against 17.4 / 26.6 / 49.2, 1,000 tokens 16.4 / 32.8 / 69.6 against 24.6 / 38.9 / 73.7, 2,048 tokens 18.4 / 36.9 / 71.7 against 32.8 / 67.6 / 132.
+  const size_t many_smem = (size_t)MANY_BLOCK * (n_rows + (scored ? E : 0) + groups) * sizeof(float);
+  if (rows_aligned && T_ > 6 * dk_sm_count() && many_smem <= 48 * 1024) {
+#define MANY(ROWS)                                                                                                                               \
+  router_many_kernel<ROWS><<<(T_ + MANY_BLOCK - 1) / MANY_BLOCK, ROUTER_WARPS * 32, many_smem, stream>>>(                                         \
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, T_, d, n_rows, E, top, correction, route_scale, scored, groups, keep, \
+      group_top2)
+    if (n_rows <= 5 * MANY_SHARERS) MANY(5);
+    else MANY(8);
+#undef MANY
     return dk_check_launch("router");
   }
-  // One round of loads (or two) instead of a warp's share of the rows: only where that is all of W, where a token's entries keep all eight
-  // warps busy, and while a token's block finds an SM soon.  17 rows of 2,048: 64 tokens 12.3 against 16.4 us, 384 tokens 14.3 against 16.4,
-  // 512 equal; 32 rows: 8 tokens 15.5 against 17.4; 48 rows: 21.5 against 17.4.  32 rows of 1,024: 15.4 against 13.1 (17 rows equal).
-  const size_t few_smem = ((size_t)n_rows * (1 + ROUTER_WARPS) + (scored ? E : 0) + groups) * sizeof(float);
-  if (dtype == DK_BF16 && d >= ROUTER_WARPS * 256 && n_rows <= 2 * FEW_ROWS && T_ <= 384 && d % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) % 16) == 0 && few_smem <= 48 * 1024) {
-    router_few_kernel<<<T_, ROUTER_WARPS * 32, few_smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, d, n_rows, E,
-                                                                  top, correction, route_scale, scored, groups, keep, group_top2);
+  const size_t few_smem = (size_t)(n_rows + (scored ? E : 0) + groups) * sizeof(float);
+  if (rows_aligned && T_ <= 2 * dk_sm_count() && n_rows <= 4 * ROUTER_WARPS && few_smem <= 48 * 1024) {
+#define FEW(ROWS)                                                                                                                                 \
+  router_few_kernel<ROWS><<<T_, ROUTER_WARPS * 32, few_smem, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, logits, choice, weight, d, \
+                                                                       n_rows, E, top, correction, route_scale, scored, groups, keep, group_top2)
+    if (n_rows <= ROUTER_WARPS) FEW(1);
+    else if (n_rows <= 2 * ROUTER_WARPS) FEW(2);
+    else if (n_rows <= 3 * ROUTER_WARPS) FEW(3);
+    else FEW(4);
+#undef FEW
     return dk_check_launch("router");
   }
   const int blocks = (T_ + tpb - 1) / tpb;

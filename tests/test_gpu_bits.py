@@ -59,3 +59,44 @@ def test_f32_logits_do_not_depend_on_the_cuts(cuts):
             at += n
         return torch.cat(got)
     assert torch.equal(logits(cuts), logits((300,)))
+
+# ------------------------------------------------------------------ the router: a token's logits are the same in every step
+
+@pytest.mark.parametrize("d, rows, E", [(2048, 17, 16), (2048, 32, 32), (1024, 17, 16), (4096, 65, 64), (520, 20, 20), (2048, 129, 128), (99, 7, 6)])
+def test_a_tokens_logits_do_not_depend_on_the_step(d, rows, E):
+    """One token, a decode step, portions on either side of every line between the kernels: the same bits for the same token."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(d + rows)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x = torch.randn(2048, d, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(rows, d, device=DEV, generator=g) * 0.05).bfloat16()
+    cor = torch.rand(E, device=DEV, generator=g) * 0.1
+
+    def run(T, **kw):
+        z, c, wt = torch.empty(T, rows, device=DEV), torch.empty(T, 4, dtype=torch.int32, device=DEV), torch.empty(T, 4, device=DEV)
+        o.router(x[:T], w, E, 4, z, c, wt, **kw)
+        return z, c, wt
+    for kw in (dict(), dict(scoring="sigmoid", correction=cor, scale=2.5, normalize=True)):
+        z, c, wt = run(2048, **kw)
+        for T in (1, 8, 9, 32, 130, 384, 385, 6 * sms - 1, 6 * sms, 1500):
+            zt, ct, wtt = run(T, **kw)
+            assert torch.equal(zt, z[:T]) and torch.equal(ct, c[:T]) and torch.equal(wtt, wt[:T]), T
+    ref = x.double() @ w.double().T
+    assert (z.double() - ref).norm() < 3e-7 * ref.norm()
+
+
+def test_close_router_scores_are_ranked_by_the_stored_logits():
+    """Logits that lie a few units of their last place apart: the choice is the top of what the same call stored, the lowest expert among equals."""
+    o = ops()
+    d, E = 2048, 16
+    g = torch.Generator(device=DEV).manual_seed(5)
+    base = torch.randn(d, device=DEV, generator=g)
+    w = base.bfloat16().repeat(E, 1)
+    w[torch.arange(E, device=DEV), torch.randint(0, d, (E,), device=DEV, generator=g)] += 2.0 ** -6      # one entry of each differs a little
+    w[7] = w[3]
+    for T in (1, 8, 300, 600, 1200):
+        x = torch.randn(T, d, device=DEV, generator=g).bfloat16()
+        z, c, wt = torch.empty(T, E, device=DEV), torch.empty(T, 4, dtype=torch.int32, device=DEV), torch.empty(T, 4, device=DEV)
+        o.router(x, w, E, 4, z, c, wt)
+        want = [[e for _, e in sorted((-v, e) for e, v in enumerate(row))[:4]] for row in z.tolist()]
+        assert c.tolist() == want and torch.equal(z[:, 3], z[:, 7])
