@@ -17,11 +17,13 @@
 // 256 columns.  One prompt of 2,048 tokens, 16 heads, keys of 320 and values of 256: 60 us; warp-level MMA (attention_rows_mma.cu)
 // 275 us.
 //
-// Every wait is bounded; when one gives up the block records it, stores nothing more, frees its tensor memory and returns.
+// Every wait is bounded; when one gives up the block records it, stores nothing more, waits (bounded again) for the copies and products that it
+// has under way, frees its tensor memory and returns.
 #include "common.cuh"
 #include "row_attention_params.h"
 #include "tcgen05_helpers.cuh"
 #include "attention_pieces.cuh"
+#include "ring.cuh"
 
 namespace {
 constexpr int QT = 128, KT = 64, DKP = 320, DVP = 256;
@@ -120,6 +122,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 
   if (warp == 4) {
     const int ppt = KT / p.ps;      // pages of a tile
+    int q_asked = 0;
     for (int round = 0; round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces || !piece_of(p, index, pieces.sorted, listed, w)) continue;
@@ -129,6 +132,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         for (int i = 0; i < BOXES; ++i)      // (columns behind the head's last one meet zeros of the keys)
           tma_load_2d(sm_q + i * Q_BOX, &map_q, w.h * p.q_head_stride + i * 64, w.t0, q_full);
       }
+      ++q_asked;
       const int kvh = w.h / (p.H / p.KV);
       for (int j = 0; j < w.n_tiles; ++j, ++g) {
         const int s = g % STAGES, lp = (w.kt_first + j) * ppt + lane;
@@ -159,10 +163,11 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       if (failed) break;
       ++done;
     }
-    if (failed && lane == 0) {      // nobody may leave while copies of this block are in flight: wait (bounded) for the last ones asked for
-      if (done > 0 || g > 0) mbar_wait(q_full, done & 1);
-      for (int i = 1; i <= STAGES && i <= g; ++i) mbar_wait(k_full + 8 * ((g - i) % STAGES), ((g - i) / STAGES) & 1);
+    if (lane == 0) {      // its copies have arrived
+      ring_drain(q_asked, 1, [&](int, uint32_t parity) { return mbar_wait(q_full, parity); });
+      ring_drain(g, STAGES, [&](int s, uint32_t parity) { return mbar_wait(k_full + 8 * s, parity); });
     }
+    __syncwarp();
   } else if (warp == 5) {
     const bool leader = elect_one();
     const uint32_t idesc = instr_desc_bf16(QT, KT);
@@ -191,6 +196,8 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       ++done;
     }
     if (!ok) failed = 1;
+    if (lane == 0) ring_drain(g, 2, [&](int c, uint32_t parity) { return mbar_wait(s_full + 8 * c, parity); });      // its products are complete
+    __syncwarp();
   } else if (warp == 6) {
     const bool leader = elect_one();
     const uint32_t idesc = instr_desc_bf16(QT, DVP, true);
@@ -219,6 +226,8 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       }
     }
     if (!ok) failed = 1;
+    if (lane == 0) ring_drain(g, 2, [&](int c, uint32_t parity) { return mbar_wait(o_done + 8 * c, parity); });
+    __syncwarp();
   } else if (warp < 4) {
     const int r = tid;      // query = lane of the tensor memory
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16, t_o = tmem + lane_base + COL_O;

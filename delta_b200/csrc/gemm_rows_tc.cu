@@ -12,9 +12,11 @@
 // 2,048 x 22,016 x 4,096: 250 us = 1,480 TFLOP/s with or without the silu gate (one block a tile, its epilogue uncovered, took 404 and 456;
 // the library 218 without the gate); an expert's products of a 2,048-token prompt (16 experts of 1,024, 4 chosen, width 2,048) 157 -> 62 us.
 //
-// Every wait on an mbarrier is bounded: when one gives up, the kernel records it, stores nothing more, frees its tensor memory and returns.
+// Every wait on an mbarrier is bounded: when one gives up, the kernel records it, stores nothing more, waits (bounded again) for the copies and
+// products that it has under way, frees its tensor memory and returns.
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
+#include "ring.cuh"
 
 namespace {
 constexpr int BM = 128;            // rows of x of a piece
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_tc_kernel(const __grid_c
           }
         }
       }
+      ring_drain(step, STAGES, [&](int s, uint32_t parity) { return mbar_wait(full0 + 8 * s, parity); });      // its copies have arrived
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -150,6 +153,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_tc_kernel(const __grid_c
         umma_commit(tfull0 + 8 * b);
         ++piece;
       }
+      // its products are complete (a commit covers all before it, so the last one would do)
+      ring_drain(step, STAGES, [&](int s, uint32_t parity) { return mbar_wait(empty0 + 8 * s, parity); });
     }
   } else {
     const int quarter = warp & 3;      // the lanes of tensor memory that a warp may read
