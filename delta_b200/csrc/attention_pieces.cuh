@@ -38,3 +38,17 @@ __device__ __forceinline__ int list_pieces(PieceList<N>& list, const int* __rest
   __syncthreads();
   return count;
 }
+
+// Rows [from, to) of boxes of 128-byte rows become zeros, by one warp, after their copy has arrived and before an MMA reads them: rows of a tile
+// that no query of the piece sees.  Their weights are zero, but zero times what another request left in a page, or an earlier token that was
+// not finite, need not be.
+__device__ __forceinline__ void clear_rows(uint32_t boxes, int count, int box_bytes, int from, int to) {      // (an address in shared memory)
+  if (from >= to) return;
+#pragma unroll 1
+  for (uint32_t at = boxes; count-- > 0; at += box_bytes)
+#pragma unroll 1
+    for (int i = from * 8 + (int)(threadIdx.x & 31); i < to * 8; i += 32)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(at + i * 16), "r"(0) : "memory");
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");      // ordinary stores, read by the tensor cores
+  __syncwarp();
+}

@@ -13,7 +13,7 @@
 //     the scores it was made from in TMEM (128 columns of float scores are 64 columns of P_hi and 64 of P_lo) and is the A operand
 //     from there, so it costs no shared memory and no copy; the scores of the half's next tile wait for the products with P.
 //   * Pages of a tile that no query of the block sees (before the window or chunk, given back already, or behind the last token)
-//     are replaced by one that is there: their scores are masked, and what is multiplied by the zeros is finite.
+//     are replaced by one that is there: their scores are masked, and the values of keys that nobody sees are cleared before the product.
 //   * Scores may be shaped first (an instance of its own): capped, s <- cap tanh(s / cap), and given a bias by distance and head.  Three
 //     special-function results a score instead of one.  The head's biases lie in shared memory in powers of two, a copy for each half, with
 //     as many entries before the first and behind the last distance as a tile can ask for, so that a score's bias is one load at a
@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  // barriers: q_full, k_full[2], v_full[2], s_full[2], p_full[2], o_done[2], merge, piece_done, bias_full[2]
-  __shared__ __align__(8) unsigned long long bars[1 + 2 + 2 + 2 + 2 + 2 + 1 + 1 + 2];
+  // barriers: q_full, k_full[2], v_full[2], s_full[2], p_full[2], o_done[2], merge, piece_done, bias_full[2], v_edge
+  __shared__ __align__(8) unsigned long long bars[1 + 2 + 2 + 2 + 2 + 2 + 1 + 1 + 2 + 1];
   auto row_stat = [&](int w) { return reinterpret_cast<float2*>(smem + L::OFF_STAT + w * QT * 8); };     // maximum and sum of half w's tiles, per query
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int failed;
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
   const uint32_t bar0 = s2u(&bars[0]);
   const uint32_t q_full = bar0;
   const uint32_t k_full = bar0 + 8, v_full = k_full + 16, s_full = v_full + 16, p_full = s_full + 16, o_done = p_full + 16,
-                 merge_bar = o_done + 16, piece_done = merge_bar + 8, bias_full = piece_done + 8;
+                 merge_bar = o_done + 16, piece_done = merge_bar + 8, bias_full = piece_done + 8, v_edge = bias_full + 16;
   if (tid == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < STAGES; ++s) {
@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       mbar_init(o_done + 8 * w, 1);
       mbar_init(bias_full + 8 * w, HALF_THREADS);
     }
+    mbar_init(v_edge, 1);
     mbar_init(merge_bar, 2 * HALF_THREADS);
     mbar_init(piece_done, 2 * HALF_THREADS);
     failed = 0;
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
     const CUtensorMap* map_run = kind ? &map_v_run : &map_k_run;
     int q_asked = 0;
     int asked0 = 0, asked1 = 0;   // tiles of each parity asked for so far
+    int edges = 0;
     for (int round = 0; round * (int)gridDim.x < n_pieces && !failed; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces) continue;
@@ -269,15 +271,24 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
         bool ok = true;
         if (ord >= 1) ok = mbar_wait(done + 8 * c, (ord - 1) & 1);
         if (!__all_sync(0xffffffffu, ok && !failed)) { failed = 1; break; }
-        if (lane == 0) mbar_expect_tx(full + 8 * c, tile_bytes);
+        // values of keys at a tile's ends that nobody sees: the tile is announced when they are cleared
+        const int from = kind && j == 0 ? row_first_key(p, w.pos0) % KT : 0, to = kind && j == w.n_tiles - 1 ? w.last_pos % KT + 1 : KT;
+        const bool edge = from > 0 || to < KT;
+        const uint32_t bar = edge ? v_edge : full + 8 * c;
+        if (lane == 0) mbar_expect_tx(bar, tile_bytes);
         __syncwarp();
         if (run) {
           if (lane == 0)
-            for (int half = 0; half < halves; ++half)
-              tma_load_4d(sm_dst + c * tile_bytes + half * BOX_BYTES, map_run, half * 64, 0, kvh, first, full + 8 * c);
+            for (int half = 0; half < halves; ++half) tma_load_4d(sm_dst + c * tile_bytes + half * BOX_BYTES, map_run, half * 64, 0, kvh, first, bar);
         } else if (lane < ppt) {
           for (int half = 0; half < halves; ++half)
-            tma_load_2d(sm_dst + c * tile_bytes + half * BOX_BYTES + lane * ps * 128, map_page, half * 64, grow, full + 8 * c);
+            tma_load_2d(sm_dst + c * tile_bytes + half * BOX_BYTES + lane * ps * 128, map_page, half * 64, grow, bar);
+        }
+        if (edge) {
+          if (!__all_sync(0xffffffffu, mbar_wait(v_edge, edges++ & 1))) { failed = 1; break; }
+          clear_rows(sm_dst + c * tile_bytes, halves, BOX_BYTES, 0, from);
+          clear_rows(sm_dst + c * tile_bytes, halves, BOX_BYTES, to, KT);
+          if (lane == 0) mbar_arrive(full + 8 * c);
         }
         if (c) asked1 = ord + 1; else asked0 = ord + 1;
       }
@@ -291,6 +302,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       if (kind == 0 && q_asked > 0) mbar_wait(q_full, (q_asked - 1) & 1);
       if (asked0 > 0) mbar_wait(full, (asked0 - 1) & 1);
       if (asked1 > 0) mbar_wait(full + 8, (asked1 - 1) & 1);
+      if (edges > 0) mbar_wait(v_edge, (edges - 1) & 1);
     }
   } else if (warp == MMA_WARP) {
     // ------------------------------------------- MMA issuer of the scores

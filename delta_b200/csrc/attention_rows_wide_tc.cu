@@ -47,7 +47,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 struct Piece {
-  int row, h, nq, t0, pos0, kt_first, n_tiles, first_page, last_page;
+  int row, h, nq, t0, pos0, first_key, last_key, kt_first, n_tiles, first_page, last_page;
 };
 
 constexpr int LISTED = 256;      // pairs of row and query tile that the list holds
@@ -62,17 +62,18 @@ __device__ __forceinline__ bool piece_of(const DkRowAttnParams& p, int index, co
   w.nq = min(QT, q_len - qt * QT);
   w.t0 = p.row_q_start[w.row] + qt * QT;
   w.pos0 = p.row_pos_start[w.row] + qt * QT;
-  const int lo = row_first_key(p, w.pos0), last = w.pos0 + w.nq - 1;
-  w.kt_first = lo / KT;
-  w.n_tiles = last / KT - w.kt_first + 1;
-  w.first_page = lo / p.ps;
-  w.last_page = last / p.ps;
+  w.first_key = row_first_key(p, w.pos0);
+  w.last_key = w.pos0 + w.nq - 1;
+  w.kt_first = w.first_key / KT;
+  w.n_tiles = w.last_key / KT - w.kt_first + 1;
+  w.first_page = w.first_key / p.ps;
+  w.last_page = w.last_key / p.ps;
   return true;
 }
 
 // Barriers.  Tiles are numbered through all of a block's pieces; tile g has stage g % 3 and scores g % 2.
 struct Bars {
-  unsigned long long q_full, q_empty, k_full[STAGES], k_empty[STAGES], s_full[2], p_full[2], o_done[2];
+  unsigned long long q_full, q_empty, k_edge, k_full[STAGES], k_empty[STAGES], s_full[2], p_full[2], o_done[2];
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -85,11 +86,12 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   __shared__ volatile int failed;
   __shared__ PieceList<LISTED> pieces;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t q_full = s2u(&bars.q_full), q_empty = s2u(&bars.q_empty), k_full = s2u(bars.k_full), k_empty = s2u(bars.k_empty),
+  const uint32_t q_full = s2u(&bars.q_full), q_empty = s2u(&bars.q_empty), k_edge = s2u(&bars.k_edge), k_full = s2u(bars.k_full), k_empty = s2u(bars.k_empty),
                  s_full = s2u(bars.s_full), p_full = s2u(bars.p_full), o_done = s2u(bars.o_done);
   if (tid == 0) {
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
+    mbar_init(k_edge, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(k_full + 8 * s, 1);
       mbar_init(k_empty + 8 * s, 1);
@@ -122,7 +124,7 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 
   if (warp == 4) {
     const int ppt = KT / p.ps;      // pages of a tile
-    int q_asked = 0;
+    int q_asked = 0, edges = 0;
     for (int round = 0; round * (int)gridDim.x < n_pieces; ++round) {
       const int index = piece_index(round);
       if (index >= n_pieces || !piece_of(p, index, pieces.sorted, listed, w)) continue;
@@ -148,9 +150,12 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         const bool run = __all_sync(0xffffffffu, lane >= ppt || (page >= 0 && page == first + lane));
         const uint32_t there = __ballot_sync(0xffffffffu, page >= 0);
         const int other = there != 0 ? __shfl_sync(0xffffffffu, page, __ffs(there) - 1) : 0;
-        if (page < 0) page = other;      // what no query of the piece sees: masked below, and finite
+        if (page < 0) page = other;      // what no query of the piece sees: cleared and masked below
         if (!together(g < STAGES || mbar_wait(k_empty + 8 * s, (g / STAGES - 1) & 1))) { failed = 1; break; }
-        const uint32_t bar = k_full + 8 * s, dst = sm_k + s * STAGE;
+        // a tile with keys at its ends that nobody sees is announced when they are cleared
+        const int from = j == 0 ? w.first_key % KT : 0, to = j == w.n_tiles - 1 ? w.last_key % KT + 1 : KT;
+        const bool edge = from > 0 || to < KT;
+        const uint32_t bar = edge ? k_edge : k_full + 8 * s, dst = sm_k + s * STAGE;
         if (lane == 0) mbar_expect_tx(bar, STAGE);
         __syncwarp();
         if (run) {
@@ -159,12 +164,19 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         } else if (lane < ppt) {
           for (int i = 0; i < BOXES; ++i) tma_load_2d(dst + i * K_BOX + lane * p.ps * 128, &map_k, i * 64, (page * p.KV + kvh) * p.ps, bar);
         }
+        if (edge) {
+          if (!together(mbar_wait(k_edge, edges++ & 1))) { failed = 1; break; }
+          clear_rows(dst, BOXES, K_BOX, 0, from);
+          clear_rows(dst, BOXES, K_BOX, to, KT);
+          if (lane == 0) mbar_arrive(k_full + 8 * s);
+        }
       }
       if (failed) break;
       ++done;
     }
     if (lane == 0) {      // its copies have arrived
       ring_drain(q_asked, 1, [&](int, uint32_t parity) { return mbar_wait(q_full, parity); });
+      ring_drain(edges, 1, [&](int, uint32_t parity) { return mbar_wait(k_edge, parity); });
       ring_drain(g, STAGES, [&](int s, uint32_t parity) { return mbar_wait(k_full + 8 * s, parity); });
     }
     __syncwarp();

@@ -100,3 +100,64 @@ def test_close_router_scores_are_ranked_by_the_stored_logits():
         o.router(x, w, E, 4, z, c, wt)
         want = [[e for _, e in sorted((-v, e) for e, v in enumerate(row))[:4]] for row in z.tolist()]
         assert c.tolist() == want and torch.equal(z[:, 3], z[:, 7])
+# ------------------------------------------------------------------ tcgen05 attention over rows: what nobody sees
+
+class RowsCase:
+    """Prompt portions over a paged cache of rows (the value behind its key, or the key's front part).  Every row of the cache that no query of
+    the step sees is NaN: what another request left in its pages, and the tokens before a window."""
+
+    def __init__(self, H, KV, dk, dv, latent, lens, before, ps, window=0, chunk=0, shaped=False, seed=0, rest=math.nan):
+        g = torch.Generator().manual_seed(seed)
+        self.H, self.dk, self.dv, self.lens = H, dk, dv, lens
+        width = dk if latent else dk + dv
+        pages = [-(-(b + n) // ps) for b, n in zip(before, lens)]
+        bt = torch.full((len(lens), max(pages)), -1, dtype=torch.int32)
+        order = torch.randperm(sum(pages) + 2, generator=g).to(torch.int32)
+        cache = torch.full((sum(pages) + 2, KV, ps, width), rest).bfloat16()
+        for r, (b, n) in enumerate(zip(before, lens)):
+            bt[r, :pages[r]] = order[sum(pages[:r]):sum(pages[:r + 1])]
+            low = max(0, b - window + 1) if window else 0
+            low = max(low, b // chunk * chunk) if chunk else low
+            for at in range(low, b + n):
+                cache[bt[r, at // ps], :, at % ps] = torch.randn(KV, width, generator=g).bfloat16()
+        T = sum(lens)
+        self.q = torch.randn(T, H * dk, generator=g).bfloat16().to(DEV)
+        self.cache = cache.to(DEV)
+        self.kw = dict(q_stride=H * dk, q_head_stride=dk, H=H, KV=KV, dk=dk, dv=dv, ps=ps, row_width=width, k_off=0, v_off=0 if latent else dk, scale=0.1,
+                       window=window, chunk=chunk, block_table=bt.to(DEV), tok_row=i32([r for r, n in enumerate(lens) for _ in range(n)]),
+                       tok_pos=i32([b + j for b, n in zip(before, lens) for j in range(n)]), row_q_start=i32([sum(lens[:r]) for r in range(len(lens))]),
+                       row_q_len=i32(lens), row_pos_start=i32(before))
+        if shaped:
+            self.kw.update(softcap=20.0, dist_bias=torch.randn(H, 101, generator=g).to(DEV))
+
+    def run(self, kernel, dtype=torch.bfloat16, q=None):
+        o = ops()
+        q = (self.q if q is None else q).to(dtype)
+        out = torch.full((sum(self.lens), self.H * self.dv), 7.0, dtype=dtype, device=DEV)
+        err = o.new_error_record(DEV)
+        params = o.row_attn_params(q=q, cache=self.cache.to(dtype), out=out, err=err, **self.kw)
+        if kernel == "plain":
+            o.attention_rows_plain(params)
+        else:
+            assert getattr(o, kernel + "_supported")(params)
+            getattr(o, kernel)(params, max(self.lens))
+        o.raise_if_error(err)
+        return out
+
+
+ROWS_KERNELS = [("attention_rows_wide", (4, 1, 320, 256), True, False), ("attention_rows_wide", (3, 1, 136, 72), True, False),
+                ("attention_rows_tc", (4, 2, 128, 128), False, True), ("attention_rows_tc", (4, 2, 72, 104), False, True),
+                ("attention_rows_tc", (2, 1, 128, 64), False, False)]
+
+
+@pytest.mark.parametrize("kernel, shape, latent, shaped", ROWS_KERNELS)
+@pytest.mark.parametrize("window, chunk", [(0, 0), (33, 0), (150, 0), (0, 100)])
+def test_what_lies_in_rows_that_nobody_sees_does_not_matter(kernel, shape, latent, shaped, window, chunk):
+    """A weight of zero times NaN is NaN: the rows behind a portion's last token (one to many of its last tile) and before its first key must
+    not meet the product with the values."""
+    args = (*shape, latent, [130, 64, 300, 127], [0, 201, 500, 257], 16, window, chunk, shaped)
+    case, clean = RowsCase(*args), RowsCase(*args, rest=0.0)
+    got, want = case.run(kernel), clean.run("plain", torch.float32)
+    assert bool(torch.isfinite(got).all()) and torch.equal(got, clean.run(kernel))
+    # weights to 16 bits, one rounding of the output to bfloat16
+    assert (got.double() - want.double()).abs().max() < 2.0 ** -8 * want.abs().max()
