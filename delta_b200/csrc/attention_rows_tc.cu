@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
         if (!__all_sync(0xffffffffu, ok && !failed)) { failed = 1; break; }
         if (lane == 0) {
           mbar_expect_tx(q_full, (uint32_t)L::Q_BYTES);
-          for (int half = 0; half < L::K_HALVES; ++half)      // (columns behind the head's last one meet zeros of the keys)
-            tma_load_2d(sm_q + half * BOX_BYTES, &map_q, w.h * p.q_head_stride + half * 64, w.t0, q_full);   // rows past the last token are zeros
+          for (int half = 0; half < L::K_HALVES; ++half)      // columns past the head's last one and rows past the last token are zeros
+            tma_load_4d(sm_q + half * BOX_BYTES, &map_q, half * 64, w.h, 0, w.t0, q_full);
         }
         q_asked = n_done + 1;
       }
@@ -590,7 +590,7 @@ int launch_as(const DkRowAttnParams& p, int max_q_len, cudaStream_t stream) {
   CUtensorMap map_q, map_k, map_k_run, map_v, map_v_run;
   const long long rows = (long long)p.num_pages * p.KV * p.ps;
   DK_REQUIRE(rows < (1ll << 31), "attention_rows_tc: the cache of one layer has too many rows for a tensor map coordinate");
-  DK_REQUIRE(make_tensor_map_bf16(&map_q, p.q, p.T, (p.H - 1) * p.q_head_stride + p.dk, p.q_stride, QT),
+  DK_REQUIRE(make_tensor_map_of_heads(&map_q, p.q, p.T, p.H, p.dk, p.q_stride, p.q_head_stride, QT),
              "attention_rows_tc: cannot encode the tensor map of the queries");
   // the cache as rows, and as [page][head][offset][columns]: a run of pages of one head in one box; once from the key's first
   // column on and once from the value's, each as wide as the key or value

@@ -131,8 +131,8 @@ attention_rows_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       if (!together(done == 0 || mbar_wait(q_empty, (done - 1) & 1))) { failed = 1; break; }
       if (lane == 0) {
         mbar_expect_tx(q_full, BOXES * Q_BOX);
-        for (int i = 0; i < BOXES; ++i)      // (columns behind the head's last one meet zeros of the keys)
-          tma_load_2d(sm_q + i * Q_BOX, &map_q, w.h * p.q_head_stride + i * 64, w.t0, q_full);
+        for (int i = 0; i < BOXES; ++i)      // (columns behind the head's last one are zeros)
+          tma_load_4d(sm_q + i * Q_BOX, &map_q, i * 64, w.h, 0, w.t0, q_full);
       }
       ++q_asked;
       const int kvh = w.h / (p.H / p.KV);
@@ -385,7 +385,7 @@ extern "C" int dk_attention_rows_wide(const DkRowAttnParams* pp, int max_q_len, 
                                          (unsigned long long)p.KV * p.ps * p.row_width * 2};
   const unsigned long long dims[4] = {(unsigned long long)p.dk, (unsigned long long)p.ps, (unsigned long long)p.KV, (unsigned long long)p.num_pages};
   const __nv_bfloat16* base = reinterpret_cast<const __nv_bfloat16*>(p.cache) + p.k_off;
-  DK_REQUIRE(make_tensor_map_bf16(&map_q, p.q, p.T, (p.H - 1) * p.q_head_stride + p.dk, p.q_stride, QT) &&
+  DK_REQUIRE(make_tensor_map_of_heads(&map_q, p.q, p.T, p.H, p.dk, p.q_stride, p.q_head_stride, QT) &&
                  make_tensor_map_bf16(&map_k, base, rows, p.dk, p.row_width, p.ps) &&
                  make_tensor_map_bf16_4d(&map_k_run, base, dims, strides, p.ps, KT / p.ps),
              "attention_rows_wide: cannot encode a tensor map");

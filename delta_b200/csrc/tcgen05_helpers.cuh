@@ -204,6 +204,14 @@ static inline bool make_tensor_map_bf16_4d(CUtensorMap* m, const void* base, con
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The heads of rows: [tokens][1][heads][cols], tokens ``stride`` and heads ``head_stride`` elements apart; boxes of [box_rows tokens x 64
+// columns] of one head (coordinates: column, head, 0, token), zeros past its last column
+static inline bool make_tensor_map_of_heads(CUtensorMap* m, const void* base, int tokens, int heads, int cols, int stride, int head_stride, int box_rows) {
+  const unsigned long long dims[4] = {(unsigned long long)cols, (unsigned long long)heads, 1ull, (unsigned long long)tokens};
+  const unsigned long long strides[3] = {2ull * head_stride, 2ull * head_stride * heads, 2ull * stride};
+  return make_tensor_map_bf16_4d(m, base, dims, strides, 1, box_rows);
+}
+
 // 2-D bfloat16 tensor [rows, cols] with leading size ld: boxes of [box_rows x 64], 128-byte swizzle,
 // zeros where a box reaches past the tensor
 static inline bool make_tensor_map_bf16(CUtensorMap* m, const void* base, long long rows, int cols, long long ld, int box_rows) {

@@ -161,3 +161,15 @@ def test_what_lies_in_rows_that_nobody_sees_does_not_matter(kernel, shape, laten
     assert bool(torch.isfinite(got).all()) and torch.equal(got, clean.run(kernel))
     # weights to 16 bits, one rounding of the output to bfloat16
     assert (got.double() - want.double()).abs().max() < 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("kernel, shape, latent, shaped", [k for k in ROWS_KERNELS if k[1][2] % 64])
+def test_a_heads_queries_do_not_reach_its_neighbour(kernel, shape, latent, shaped):
+    """Heads whose size is no multiple of a box of 64 columns: infinite queries of one head leave the others' bits alone."""
+    case = RowsCase(*shape, latent, [130, 70], [0, 100], 16, 0, 0, shaped)
+    clean = case.run(kernel).view(200, shape[0], shape[3])
+    q = case.q.clone()
+    q.view(200, shape[0], shape[2])[50:90, 1] = math.inf
+    got = case.run(kernel, q=q).view(200, shape[0], shape[3])
+    others = [h for h in range(shape[0]) if h != 1]
+    assert torch.equal(got[:, others], clean[:, others]) and torch.equal(got[:50, 1], clean[:50, 1]) and torch.equal(got[90:, 1], clean[90:, 1])
