@@ -1,20 +1,16 @@
 // Up to 16 rows through one small matrix per head,  C_b[M, N] = A_b[M, K] W_b[N, K]^T  for bfloat16, in one launch: a decode step's
-// way into the latent space and out of it (latent attention), or through the blocks of a recurrence's gates.
+// way into the latent space and out of it (latent attention).
 //
 // Bound by latency: W is a megabyte or two.  A warp takes 16 rows of one W_b and all of K; lane (g, t) of the MMA layout loads 16
 // bytes of rows g and g + 8 of W and of row g of A at the same k, which are two fragments of 16 k each (in an order of k that both
-// operands share), so every load of four k blocks is under way before the first product.  8 rows, 16 heads of 256 x 128: 15.2 -> 3.1 us
+// operands share), so every load of four k blocks is under way before the first product.  Every MMA starts from zero and its sum of 16 exact
+// products is added by an FADD: an MMA that adds to its accumulator cuts the sum off instead of rounding it.  8 rows, 16 heads of 256 x 128: 15.2 -> 3.1 us
 // (the FMA product in tiles of 64 x 64).
 #include "common.cuh"
+#include "mma_helpers.cuh"
 
 namespace {
 constexpr int WARPS = 4;
-
-__device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 template <int MT>      // tiles of 8 rows of A
 __global__ void __launch_bounds__(WARPS * 32) gemm_heads_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W,
@@ -50,8 +46,9 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_heads_kernel(const __nv_bfloa
     for (int s = 0; s < 4; ++s)
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
-        mma(acc[i], a[s].x, b[s].x, a[s].y, b[s].y, x[i][s].x, x[i][s].y);
-        mma(acc[i], a[s].z, b[s].z, a[s].w, b[s].w, x[i][s].z, x[i][s].w);
+        const uint32_t f0[4] = {a[s].x, b[s].x, a[s].y, b[s].y}, f1[4] = {a[s].z, b[s].z, a[s].w, b[s].w};
+        mma_add(acc[i], f0, x[i][s].x, x[i][s].y);
+        mma_add(acc[i], f1, x[i][s].z, x[i][s].w);
       }
   }
 #pragma unroll

@@ -24,6 +24,14 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// c += a b with the sum rounded to nearest: an MMA cuts off what it adds to its third operand, so the products start from zero and an FADD
+// adds them.
+__device__ __forceinline__ void mma_add(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float d[4] = {0.f, 0.f, 0.f, 0.f};
+  mma_bf16(d, a, b0, b1);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) c[e] += d[e];
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

@@ -32,14 +32,6 @@ constexpr double LEAST_LOG2 = -1000.0;   // 2^-1000 is zero in 32 bit: a token's
 constexpr int HEAD_FLOATS = 5 * TC;     // per (chunk, head): dt, the sums of log2 decays as two floats, e^(L_last - L_s) dt_s and e^(L_t)
 constexpr int GROUP_FLOATS = TC * TC;   // per (chunk, group): C_t . B_s
 
-// c += a b, rounded to nearest
-__device__ __forceinline__ void mma_add(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  float d[4] = {0.f, 0.f, 0.f, 0.f};
-  mma_bf16(d, a, b0, b1);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) c[e] += d[e];
-}
-
 __device__ __forceinline__ double softplus_ss(double x) { return x > 40.0 ? x : log1p(exp(x)); }
 
 // grid (most chunks of a row, rows * G)

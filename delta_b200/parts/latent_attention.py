@@ -51,7 +51,7 @@ def heads_product(ctx, a, a_off, lda, sa, w, n, k, c, c_off, ldc, sc, heads):
         ops.count_library("library batched product")
         return
     a_at, w_at = a.data_ptr() + a_off * es, w.data_ptr()
-    if a.dtype == torch.bfloat16 and "products" not in ctx.plain_kernels and w.is_contiguous() and ops.gemm_heads_supported(T, k, lda, sa, n * k, a_at, w_at):
+    if a.dtype == c.dtype == torch.bfloat16 and "products" not in ctx.plain_kernels and w.is_contiguous() and ops.gemm_heads_supported(T, k, lda, sa, n * k, a_at, w_at):
         ops.gemm_heads(a_at, w_at, c.data_ptr() + c_off * es, T, n, k, lda, ldc, heads, sa, n * k, sc)      # a decode step's few rows
         return
     ops.gemm_nt_plain_batched(a.data_ptr() + a_off * es, w.data_ptr(), c.data_ptr() + c_off * es, T, n, k, lda, k, ldc, heads,

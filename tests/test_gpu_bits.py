@@ -173,3 +173,26 @@ def test_a_heads_queries_do_not_reach_its_neighbour(kernel, shape, latent, shape
     got = case.run(kernel, q=q).view(200, shape[0], shape[3])
     others = [h for h in range(shape[0]) if h != 1]
     assert torch.equal(got[:, others], clean[:, others]) and torch.equal(got[:50, 1], clean[:50, 1]) and torch.equal(got[90:, 1], clean[90:, 1])
+
+
+# ------------------------------------------------------------------ sums rounded to nearest; the ends of the number range
+
+@pytest.mark.parametrize("M", [1, 9, 16])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_gemm_heads_rounds_its_sums_to_nearest(M, sign):
+    """A sum that begins between two bfloat16 numbers and grows by three quarters of its last place with every 16 entries: rounded to nearest at
+    every step it passes the middle, cut off at every step it stays there and goes to the even neighbour."""
+    o = ops()
+    K, N = 256, 16
+    a, w = torch.zeros(M, K, device=DEV), torch.ones(N, K, device=DEV)
+    a[:, 0] = sign
+    a[:, 1] = sign * 2.0 ** -8
+    for block in range(1, K // 32):      # (the kernel's MMAs take the first and the second half of every eight entries)
+        a[:, 32 * block] = sign * 1.5 * 2.0 ** -24
+        a[:, 32 * block + 4] = sign * 1.5 * 2.0 ** -24
+    a, w = a.bfloat16(), w.bfloat16()
+    c = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    o.gemm_heads(a.data_ptr(), w.data_ptr(), c.data_ptr(), M, N, K, K, N, 1, M * K, N * K, M * N)
+    exact = a.double() @ w.double().T
+    assert bool((exact.abs() > 1.0 + 2.0 ** -8).all())
+    assert torch.equal(c, torch.full_like(c, sign * (1.0 + 2.0 ** -7)))
