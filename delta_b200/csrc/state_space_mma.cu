@@ -13,8 +13,10 @@
 //      they fetch (cp.async, three buffers) and make what does not depend on the state, M x + D x.
 // An MMA rounds the sum it adds to towards zero: the high parts' products therefore start from zero and are added by FMA units, which
 // round to nearest; decays and step sizes come from 64-bit functions.  Bound by the chain along a row (64 heads fill 128 blocks, one an SM).  One row of 2,048 tokens, 64 heads of 64 x 128:
-// chunks 16 us and walk 136 us; the 32-bit kernels, in chunks of 32, 27 and 310 us.  Against 64 bits the outputs are 8e-8 off, the states
-// 5e-8 to 1e-7 (the 32-bit kernels: 1e-7 and 7e-8 to 1e-7; with decays near one 5e-7 against 1.2e-7).
+// chunks 16 us and walk 137 us; the 32-bit kernels, in chunks of 32, 27 and 310 us.  Errors against 64 bits (2-norm, 200 to 1,500 tokens) of
+// outputs and states, in units of 1e-8: decays near one 10 to 13 and 9 to 13 here, 25 to 62 and 25 to 74 in the 32-bit kernels; mixed decays 9.4
+// to 10.1 and 6.0 to 7.6 here, 7.8 to 10.0 and 4.8 to 11.6 there; strong ones 6.7 to 8.2 and 3.7 to 4.9 here, 6.6 to 8.3 and 4.4 to 4.7 there.
+// An infinite state entry stays in its channel; an infinite C, B or x meets zero parts of the other operand and may give a NaN.
 #include "common.cuh"
 #include "mma_helpers.cuh"
 #include "split_bf16.cuh"

@@ -196,3 +196,45 @@ def test_gemm_heads_rounds_its_sums_to_nearest(M, sign):
     exact = a.double() @ w.double().T
     assert bool((exact.abs() > 1.0 + 2.0 ** -8).all())
     assert torch.equal(c, torch.full_like(c, sign * (1.0 + 2.0 ** -7)))
+
+
+@pytest.mark.parametrize("value", [math.inf, -math.inf, 3.4e38, -3.4e38, 3.39e38])
+def test_state_space_mma_keeps_infinite_and_large_states(value):
+    """A state entry that is infinite, or finite and above bfloat16's largest number: it stays in its channel, and the outputs are what 64 bits give."""
+    from test_gpu_tiles import ssd_inputs, ssd_reference
+    o = ops()
+    H, G, N, P, lens = 4, 2, 128, 64, [130]
+    xbc, dtraw, A_log, dt_bias, D, state = (t.to(DEV) for t in ssd_inputs(H, G, N, P, lens, [0], 3, "weak"))
+    C = xbc[:, H * P + G * N:]
+    C.copy_(torch.where(C.abs() < 2.0 ** -3, torch.full_like(C, 0.5), C) * 2.0 ** -10)      # no zeros, and outputs in range
+    state[0, 1, 5, 77] = value
+    st, out = state.clone(), torch.empty(130, H * P, device=DEV)
+    counts = -(-130 // o.state_space_mma_chunk())
+    work = torch.empty(counts * o.state_space_mma_floats(H, G), device=DEV)
+    o.state_space_mma(xbc, dtraw.data_ptr(), H + 3, A_log, dt_bias, D, st, out, work, i32([0]), counts, counts, H=H, G=G, N=N, P=P, row_slot=i32([0]),
+                      row_q_start=i32([0]), row_q_len=i32([130]))
+    y, S = ssd_reference(xbc, dtraw, A_log, dt_bias, D, state[0].double(), H, G, N, P)
+    y, S, out, st = y.view(130, H * P), S, out.double(), st[0].double()
+    inf = torch.isinf(y)
+    assert torch.equal(torch.isinf(out), inf) and torch.equal(out[inf], y[inf]) and not bool(torch.isnan(out).any())
+    assert bool(((out - y)[~inf].abs() <= 1e-6 * y[~inf].abs().clamp(min=1.0)).all() if math.isinf(value) else ((out - y).abs() <= 1e-5 * y.abs().clamp(min=1.0)).all())
+    inf = torch.isinf(S)
+    assert torch.equal(torch.isinf(st), inf) and torch.equal(st[inf], S[inf]) and bool(((st - S)[~inf].abs() <= 1e-5 * S[~inf].abs().clamp(min=1.0)).all())
+
+
+@pytest.mark.parametrize("decays", ["weak", "mixed", "strong"])
+@pytest.mark.parametrize("H, G, N, P", [(4, 2, 128, 64), (3, 1, 64, 32)])
+def test_state_space_mma_loses_no_part_of_its_operands(H, G, N, P, decays):
+    """Several chunks against 64 bits in the 2-norm: sums of 32 bit leave about 1e-7; without the lowest part of an operand it would be 2^-17 and
+    with two parts rounded together 2^-20."""
+    from test_gpu_tiles import ssd_inputs, ssd_reference
+    o = ops()
+    n = 700
+    xbc, dtraw, A_log, dt_bias, D, state = (t.to(DEV) for t in ssd_inputs(H, G, N, P, [n], [0], N, decays))
+    st, out = state.clone(), torch.empty(n, H * P, device=DEV)
+    chunks = -(-n // o.state_space_mma_chunk())
+    work = torch.empty(chunks * o.state_space_mma_floats(H, G), device=DEV)
+    o.state_space_mma(xbc, dtraw.data_ptr(), H + 3, A_log, dt_bias, D, st, out, work, i32([0]), chunks, chunks, H=H, G=G, N=N, P=P, row_slot=i32([0]),
+                      row_q_start=i32([0]), row_q_len=i32([n]))
+    y, S = ssd_reference(xbc, dtraw, A_log, dt_bias, D, state[0].double(), H, G, N, P)
+    assert (out.double() - y.view(n, H * P)).norm() < 3e-7 * y.norm() and (st[0].double() - S).norm() < 3e-7 * S.norm()
