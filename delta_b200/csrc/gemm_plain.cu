@@ -235,7 +235,6 @@ int launch_f32(const float* A, const float* W, float* C, int M, int N, int K, in
     }
   }
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-  DK_REQUIRE(grid.y <= 65535, "gemm: M=%d is too large for this kernel", M);
   kernel<<<grid, (BM / TM) * (BN / TN), SMEM, stream>>>(A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc);
   return 0;
 }
@@ -244,7 +243,6 @@ template <typename TI, typename TO>
 int launch(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
            long long sc, cudaStream_t stream) {
   const dim3 grid((N + 63) / 64, (M + 31) / 32, batch);
-  DK_REQUIRE(grid.y <= 65535, "gemm: M=%d is too large for this kernel", M);
   const uintptr_t vec = 4 * sizeof(TI);      // rows of four entries as one vector, where every row and product begins on one's boundary
   const bool aligned = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && sa % 4 == 0 && sw % 4 == 0 && (uintptr_t)A % vec == 0 && (uintptr_t)W % vec == 0;
   if constexpr (sizeof(TI) == 4) {
@@ -270,12 +268,21 @@ int launch(const void* A, const void* W, void* C, int M, int N, int K, int lda, 
 
 int launch_any(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
                long long sc, int in_dtype, int out_dtype, cudaStream_t stream) {
-#define LAUNCH(TI, TO) launch<TI, TO>(A, W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream)
-  if (in_dtype == DK_F32 && out_dtype == DK_F32) return LAUNCH(float, float);
-  if (in_dtype == DK_BF16 && out_dtype == DK_BF16) return LAUNCH(__nv_bfloat16, __nv_bfloat16);
-  if (in_dtype == DK_BF16 && out_dtype == DK_F32) return LAUNCH(__nv_bfloat16, float);
+  DK_REQUIRE((M + 63LL) / 64 <= 65535, "gemm: M=%d is too large for this kernel", M);
+  DK_REQUIRE(in_dtype == DK_F32 ? out_dtype == DK_F32 : in_dtype == DK_BF16 && (out_dtype == DK_BF16 || out_dtype == DK_F32),
+             "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
+  constexpr int MOST = 65535 * 32;      // rows that tiles of 32 can number: more of them go in two launches
+  for (int m = 0; m < M; m += MOST) {
+    const int rows = min(M - m, MOST);
+#define LAUNCH(TI, TO) \
+  launch<TI, TO>((const TI*)A + (size_t)m * lda, W, (TO*)C + (size_t)m * ldc, rows, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream)
+    int rc;
+    if (in_dtype == DK_F32) rc = LAUNCH(float, float);
+    else if (out_dtype == DK_BF16) rc = LAUNCH(__nv_bfloat16, __nv_bfloat16);
+    else rc = LAUNCH(__nv_bfloat16, float);
 #undef LAUNCH
-  DK_REQUIRE(false, "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
+    if (rc) return rc;
+  }
   return 0;
 }
 }  // namespace

@@ -238,3 +238,19 @@ def test_state_space_mma_loses_no_part_of_its_operands(H, G, N, P, decays):
                       row_q_start=i32([0]), row_q_len=i32([n]))
     y, S = ssd_reference(xbc, dtraw, A_log, dt_bias, D, state[0].double(), H, G, N, P)
     assert (out.double() - y.view(n, H * P)).norm() < 3e-7 * y.norm() and (st[0].double() - S).norm() < 3e-7 * S.norm()
+
+
+@pytest.mark.parametrize("M", [65535 * 32 + 1, 65535 * 64])
+@pytest.mark.parametrize("dtype, K", [(torch.float32, 4), (torch.float32, 3), (torch.bfloat16, 4)])
+def test_gemm_plain_takes_millions_of_rows(M, dtype, K):
+    """The most rows that tiles of 64 can number, one more than tiles of 32 can; one row more than that is refused."""
+    o = ops()
+    a = torch.randint(-3, 4, (M, K), device=DEV).to(dtype)
+    w = torch.randint(-3, 4, (2, K), device=DEV).to(dtype)
+    out = torch.empty(M, 2, device=DEV)
+    o.gemm_nt_plain(a, w, out)
+    assert torch.equal(out, (a.float()[:, None, :] * w.float()[None]).sum(-1))
+    if M == 65535 * 64:
+        a, out = torch.zeros(M + 1, K, dtype=dtype, device=DEV), torch.empty(M + 1, 2, device=DEV)
+        with pytest.raises(o.KernelError, match="too large"):
+            o.gemm_nt_plain(a, w, out)
