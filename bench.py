@@ -500,6 +500,10 @@ def roletar_workload(args) -> int:
     return design_workload(args, "roletar")
 
 
+# launchers that do the work of another where their sizes allow
+SAME_WORK = {"decay_attention_tiles": "decay_attention_chunked", "state_space_mma": "state_space_chunked", "attention_rows_wide": "attention_rows_mma"}
+
+
 def design_workload(args, design: str) -> int:
     """Prefill (one prompt of 2,048 tokens in one step) and decode (batch 8 at context 2,048) of a design (Roletar, Pibalorn, Mufalix, Mevulix, Vazunex, Burolorn) beside the
     Yi architecture at equal width and layer count (Mufalix also beside Pibalorn, the closest design; Mevulix beside Pibalorn and Roletar;
@@ -690,13 +694,13 @@ def design_workload(args, design: str) -> int:
                 "latent_prepare": ((H * 192 + 320 + 320 + H * 64) * 2 * T * n_lat, 0),      # counted as in the Roletar table: the whole query row
                 "rows_append_unit": (((2 * H + 4 * G) * n_own + 2 * H * (n_att - n_own)) * 128 * 2 * T, 0),
                 "glu_clamped": (3 * (Fd * n_dense + F * n_moe) * 2 * T, 0),
-                "experts_scale_rows": ((1 + top) * d * 2 * T * n_moe, 0),
                 "experts_gather": (2 * top * d * 2 * T * n_moe, 0),
                 "experts_combine": ((top * d * 4 + 2 * d * 2) * T * n_moe, 0),
                 "experts_gemm_tc": (0, 2 * T * top * 3 * d * F * n_moe),
                 "library batched product": (0, 2 * T * H * (128 * 256 + 256 * 128) * n_lat),
                 "gemm_nt_plain_batched": (0, 2 * T * H * (128 * 256 + 256 * 128) * n_lat),
-                "attention_rows_mma": (0, 2 * H * (320 + 256) * pairs * n_lat + 4 * 128 * H * pairs * n_att),
+                "attention_rows_mma": (0, 2 * H * (320 + 256) * pairs * n_lat),
+                "attention_rows_tc": (0, 4 * 128 * H * pairs * n_att),
             }
         if design == "mevulix":
             work = mevulix_work()
@@ -735,15 +739,12 @@ def design_workload(args, design: str) -> int:
             "attention_prefill_tc": (0, 4 * 128 * H * (T * (T + 1) // 2) * runs),
         }
 
-        # launchers that do the work of another where their sizes allow
-        same_work = {"decay_attention_tiles": "decay_attention_chunked", "state_space_mma": "state_space_chunked", "attention_rows_wide_tc": "attention_rows_mma"}
-
         def fractions(launchers, table):
             rows = {}
             for name, (calls, ms) in sorted(launchers.items(), key=lambda kv: -kv[1][1]):
                 row = {"calls": calls, "ms": round(ms, 4)}
-                if (name in table or same_work.get(name) in table) and ms > 0:
-                    by, fl = table[name if name in table else same_work[name]]
+                if (name in table or SAME_WORK.get(name) in table) and ms > 0:
+                    by, fl = table[name if name in table else SAME_WORK[name]]
                     if by:
                         row["gbs"] = round(by / ms / 1e6, 1)
                         row["of_measured_copy"] = round(by / ms / 1e6 / pk["hbm_gbs"], 3)
