@@ -254,3 +254,89 @@ def test_gemm_plain_takes_millions_of_rows(M, dtype, K):
         a, out = torch.zeros(M + 1, K, dtype=dtype, device=DEV), torch.empty(M + 1, 2, device=DEV)
         with pytest.raises(o.KernelError, match="too large"):
             o.gemm_nt_plain(a, w, out)
+
+
+# ------------------------------------------------------------------ single tokens whose key tiles are shared by four warps; lists of pieces at their ends
+
+@pytest.mark.parametrize("shape", [(16, 1, 320, 256), (5, 1, 272, 160), (12, 2, 192, 144)])
+@pytest.mark.parametrize("splits", [1, 2, 7])
+@pytest.mark.parametrize("shaped, window", [(False, 0), (True, 0), (False, 50)])
+def test_key_warps_of_single_tokens(shape, splits, shaped, window):
+    """Four warps take tiles of 32 keys in turn and meet under one maximum: fewer keys than a tile, tiles for some warps only, one key beside a
+    round of all four, more splits than tiles; the largest score with any of the warps."""
+    o = ops()
+    H, KV, dk, dv = shape
+    before = [0, 19, 31, 32, 95, 127, 128, 129, 700, 1100]
+    case = RowsCase(H, KV, dk, dv, True, [1] * len(before), before, 16, window, 0, shaped, seed=dk + splits)
+    for r, b in enumerate(before):      # a key that stands out, in another warp's tile for every row
+        at = max(b - 37 * r, max(0, b - window + 1) if window else 0)
+        page = int(case.kw["block_table"][r, at // 16])
+        case.cache[page, :, at % 16, :8] += 6.0
+    sink, gate = torch.randn(H, device=DEV), torch.randn(len(before), H, device=DEV).bfloat16()
+
+    def run(dtype):
+        q, cache = case.q.to(dtype), case.cache.to(dtype)
+        g = gate.to(dtype)
+        out = torch.full((len(before), H * dv), 7.0, dtype=dtype, device=DEV)
+        p = o.row_attn_params(q=q, cache=cache, out=out, sink=sink, gate_ptr=g.data_ptr(), gate_stride=H, **case.kw)
+        if dtype == torch.float32:
+            o.attention_rows_plain(p)
+        else:
+            assert o.attention_rows_mma_key_warps(p) == 4
+            n = o.attention_rows_mma_scratch_floats(p.T, H, dv, splits)
+            scratch = torch.full((max(n, 1),), math.nan, device=DEV)
+            o.attention_rows_mma(p, H // KV, splits, scratch if splits > 1 else None)
+        torch.cuda.synchronize()
+        return out.double()
+    got, want = run(torch.bfloat16), run(torch.float32)
+    # weights to 16 bits, one rounding of the output to bfloat16 (2^-9 of it)
+    assert bool(torch.isfinite(got).all()) and (got - want).abs().max() < 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("rows, n", [(256, 2), (257, 2), (128, 129), (511, 1), (512, 2), (600, 3)])
+@pytest.mark.parametrize("kernel, shape, latent", [("attention_rows_tc", (2, 1, 64, 64), False), ("attention_rows_wide", (2, 1, 136, 64), True)])
+def test_rows_pieces_at_the_ends_of_their_list(kernel, shape, latent, rows, n):
+    """As many pairs of row and query tile as the list holds, one more, and more rows than its entries can name: the old numbering takes over."""
+    lens = [n] * rows
+    lens[rows // 2], lens[rows - 1] = 140 if n == 3 else n, 1 if n == 2 else n
+    case = RowsCase(*shape, latent, lens, [(7 * r) % 50 for r in range(rows)], 8, seed=rows)
+    got, want = case.run(kernel).double(), case.run("plain", torch.float32).double()
+    assert (got - want).abs().max() < 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("rows, n, window", [(64, 33, 0), (65, 33, 0), (32, 200, 40), (511, 2, 0), (520, 2, 0), (7, 1100, 0)])
+def test_prefill_pieces_at_the_ends_of_their_list(rows, n, window):
+    o = ops()
+    q_lens = [n if r % 5 else max(1, n - 1) for r in range(rows)]
+    case = PagedCase(torch.bfloat16, 2, 1, 64, 16, seq_lens=[q + (11 * r) % 60 for r, q in enumerate(q_lens)], q_lens=q_lens, seed=rows)
+    out, want = torch.empty(case.T, 128, dtype=torch.bfloat16, device=DEV), torch.empty(case.T, 128, dtype=torch.bfloat16, device=DEV)
+    o.attention_prefill_tc(case.params(out, window=window), max(q_lens))
+    o.attention_plain(case.params(want, window=window))
+    # both round their output to bfloat16; the weights of the one have 16 bits
+    assert (out.double() - want.double()).abs().max() < 2.0 ** -7 * want.double().abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("C, stride, with_bias, silu", [(8, 8, True, True), (1032, 1040, False, True), (264, 264, True, False)])
+def test_convolution_over_tiles_of_eight_tokens(C, stride, with_bias, silu, taps, dtype):
+    """Rows that begin and end inside a tile of eight tokens, several in one tile, shorter than the taps; a last tile of one token."""
+    o = ops()
+    lens, slots = [1, 2, 3, 9, 8, 1, 1, 7, 17], [4, 2, 7, 0, 1, 3, 5, 6, 8]
+    g = torch.Generator().manual_seed(C + taps)
+    T = sum(lens)
+    x = torch.randn(T, stride, generator=g).to(dtype)
+    w, b = torch.randn(C, taps, generator=g), torch.randn(C, generator=g) if with_bias else None
+    state = torch.randn(10, taps - 1, C, generator=g)
+    st, out = state.to(DEV), torch.full((T, C), 9.0, dtype=dtype, device=DEV)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    o.conv_silu(x.to(DEV), stride, w.to(DEV), b.to(DEV) if with_bias else None, st, out, tok_row=i32([r for r, n in enumerate(lens) for _ in range(n)]),
+                row_slot=i32(slots), row_q_start=i32(starts), row_q_len=i32(lens), silu=silu)
+    for r, n in enumerate(lens):
+        seq = torch.cat([state[slots[r]].double(), x[starts[r]:starts[r] + n, :C].double()])
+        want = sum(w[:, j].double() * seq[j:j + n] for j in range(taps)) + (b.double() if with_bias else 0.0)
+        want = torch.nn.functional.silu(want) if silu else want
+        # up to five products of 32 bit, and the one rounding of the output
+        assert bool(((out[starts[r]:starts[r] + n].double().cpu() - want).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2e-6) * want.abs() + 5e-6).all()), r
+        assert torch.equal(st[slots[r]].cpu(), seq[-(taps - 1):].float())
+    assert torch.equal(st[9].cpu(), state[9])
