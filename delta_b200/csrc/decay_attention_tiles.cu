@@ -8,7 +8,7 @@
 //   3. out:    every chunk in parallel: one product [q | A] [S ; v] of 64 rows, the first part's sums multiplied by lambda^(t+1) in between.
 // 32-bit FMA throughout, powers from the 64-bit decay, never divided by.  Bound by the FMA units and shared memory: a thread holds
 // 8 x 8 sums of U, or 8 x 4 of an output, in registers and reads shared memory sixteen bytes at a time; S comes by cp.async, 16 rows a
-// stage.  One row of 2,048 tokens, 16 heads of 128 x 128: chunk 63, scan 12, out 75 us
+// stage.  At 128 x 128 the output kernel's 118 KB leave an SM one block of eight warps (its registers would allow two).  One row of 2,048 tokens, 16 heads of 128 x 128: chunk 63, scan 12, out 75 us
 // (outputs of 8 x 8 sums in blocks of 128 threads: the layer 283 instead of 236 us); the kernels with chunks of 32 and 4 x 4 sums a
 // thread 50, 27 and 160 us.  Against 64 bits: outputs 2.0e-7 off as before, states 1.0e-7 (1.5e-7).
 #include "common.cuh"
