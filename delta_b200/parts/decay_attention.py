@@ -8,7 +8,7 @@ A request's state is S [H, dk, dv] in 32 bit, zero at its start, one per run of 
 the request's earlier steps left, so a prompt may be cut anywhere.  The four projections are one product; the
 recurrence, its decays and the norm are 32 bit whatever the compute type.  Steps of single tokens stream the state through
 registers once; short portions run one block per (row, head) over the row's chunks in turn; long portions run their chunks in parallel (``csrc/decay_attention.cu``;
-heads of 64 or 128 entries in chunks of 64 tokens, ``csrc/decay_attention_tiles.cu``).
+heads of 64 or 128 entries in chunks of 64 tokens where those are enough blocks, ``csrc/decay_attention_tiles.cu``).
 """
 from __future__ import annotations
 
@@ -21,6 +21,13 @@ from .chunks import chunk_layout
 
 STATE = "decay_attention"
 PARALLEL_FROM = 65      # portions of at least this many tokens run their chunks in parallel
+
+
+def tiles_pay(q_lens, chunk: int, heads: int, sm_count: int) -> bool:
+    """Whether chunks of 64 tokens give the device enough blocks (one a chunk and head): a block works twice as long as one of the kernels with
+    chunks of 32.  The layer of 8 heads (16 heads), microseconds, chunks of 64 against 32: 65 tokens, 16 (32) blocks, 69 against 60 (77, 68);
+    257 tokens, 40 (80) blocks, 71 against 61 (81, 81); 500 tokens, 64 (128) blocks, 76 against 72 (88, 116); eight rows of 65 76 against 107."""
+    return 2 * heads * sum(-(-n // chunk) for n in q_lens) >= sm_count
 
 
 @MIXERS.register("decay_attention")
@@ -60,8 +67,9 @@ class DecayAttention(Mixer):
         rows = dict(row_slot=ctx.row_slot, row_q_start=ctx.row_q_start, row_q_len=ctx.row_q_len)
         portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
         # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
-        if portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk):
-            chunk = ops.decay_attention_tiles_chunk()
+        chunk = ops.decay_attention_tiles_chunk()
+        if (portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk)
+                and tiles_pay(ctx.host["q_lens"], chunk, H, ctx.sm_count)):
             base, total, most = chunk_layout(ctx, chunk)
             per = H * ops.decay_attention_tiles_floats(dk, dv)
             bound = (-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per

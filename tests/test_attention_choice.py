@@ -1,4 +1,4 @@
-"""Which kernel takes the rows of several tokens of a 32-bit step."""
+"""Which kernel takes a step's portions, where two of them could."""
 import pytest
 
 
@@ -10,3 +10,10 @@ def test_few_tokens_behind_a_long_context_stay_with_the_plain_kernel(q_lens, sta
     """A block of tiles walks all keys of its 32 queries alone: it pays once there are more single-token blocks than the device runs at once."""
     from delta_b200.parts.attention_kernels import tiles_pay
     assert tiles_pay(q_lens, starts, heads, 148) is tiles
+
+
+@pytest.mark.parametrize("q_lens, heads, tiles", [([65], 8, False), ([65], 16, False), ([129], 16, False), ([257], 8, False), ([257], 16, True), ([500], 8, False),
+                                                  ([500], 16, True), ([65] * 8, 8, True), ([2048], 2, False), ([2048], 16, True)])
+def test_linear_attention_takes_long_chunks_where_they_fill_the_device(q_lens, heads, tiles):
+    from delta_b200.parts.decay_attention import tiles_pay
+    assert tiles_pay(q_lens, 64, heads, 148) is tiles
