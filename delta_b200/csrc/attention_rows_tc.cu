@@ -24,11 +24,13 @@
 //   warps 8, 9  producers, one for keys and one for values
 //   warp 10     issues the score products, warp 11 the products with the values
 //
-// Every wait is bounded; when one gives up the block records it, stores nothing more, frees its tensor memory and returns.
+// Every wait is bounded; when one gives up the block records it, stores nothing more, waits (bounded again) for the copies and products that it
+// has under way, frees its tensor memory and returns.
 #include "common.cuh"
 #include "row_attention_params.h"
 #include "tcgen05_helpers.cuh"
 #include "attention_pieces.cuh"
+#include "ring.cuh"
 
 namespace {
 constexpr int QT = 128;            // queries per block (rows of both MMAs)
@@ -297,13 +299,13 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       had1 += w.n_tiles / 2;
       ++n_done;
     }
-    if (failed && lane == 0) {
-      // nobody may leave while copies of this block are in flight: wait (bounded) for the last ones asked for
-      if (kind == 0 && q_asked > 0) mbar_wait(q_full, (q_asked - 1) & 1);
-      if (asked0 > 0) mbar_wait(full, (asked0 - 1) & 1);
-      if (asked1 > 0) mbar_wait(full + 8, (asked1 - 1) & 1);
-      if (edges > 0) mbar_wait(v_edge, (edges - 1) & 1);
+    if (lane == 0) {      // its copies have arrived
+      if (kind == 0) ring_drain(q_asked, 1, [&](int, uint32_t parity) { return mbar_wait(q_full, parity); });
+      ring_drain(asked0, 1, [&](int, uint32_t parity) { return mbar_wait(full, parity); });
+      ring_drain(asked1, 1, [&](int, uint32_t parity) { return mbar_wait(full + 8, parity); });
+      ring_drain(edges, 1, [&](int, uint32_t parity) { return mbar_wait(v_edge, parity); });
     }
+    __syncwarp();
   } else if (warp == MMA_WARP) {
     // ------------------------------------------- MMA issuer of the scores
     // The whole warp runs the loop, so that descriptors and addresses stay warp-uniform; one
@@ -322,7 +324,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
       ok = wait_all(q_full, n_done & 1);
-      for (int j = 0; ok && j < w.n_tiles; ++j) {
+      int j = 0;
+      for (; ok && j < w.n_tiles; ++j) {
         const int c = j & 1, ord = (c ? had1 : had0) + j / 2;
         if (ord >= 1 && !wait_all(o_done + 8 * c, (ord - 1) & 1)) { ok = false; break; }
         if (!wait_all(k_full + 8 * c, ord & 1)) { ok = false; break; }
@@ -338,11 +341,16 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
         }
         __syncwarp();
       }
-      had0 += (w.n_tiles + 1) / 2;
-      had1 += w.n_tiles / 2;
+      had0 += (j + 1) / 2;
+      had1 += j / 2;
       ++n_done;
     }
     if (!ok) failed = 1;
+    if (lane == 0) {      // its products are complete
+      ring_drain(had0, 1, [&](int, uint32_t parity) { return mbar_wait(s_full, parity); });
+      ring_drain(had1, 1, [&](int, uint32_t parity) { return mbar_wait(s_full + 8, parity); });
+    }
+    __syncwarp();
   } else if (warp == MMA_WARP + 1) {
     // ------------------------------------------ MMA issuer of P V
     const bool leader = elect_one();
@@ -356,7 +364,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
       if (index >= n_pieces) continue;
       const Piece w = piece_of(p, index, row_lo, n_rows, pieces.sorted, listed);
       if (!w.valid) continue;
-      for (int j = 0; ok && j < w.n_tiles; ++j) {
+      int j = 0;
+      for (; ok && j < w.n_tiles; ++j) {
         const int c = j & 1, ord = (c ? had1 : had0) + j / 2;
         if (!wait_all(v_full + 8 * c, ord & 1) || !wait_all(p_full + 8 * c, ord & 1)) { ok = false; break; }
         tc_fence_after();
@@ -373,11 +382,16 @@ __global__ void __launch_bounds__(THREADS, 1) attention_rows_tc_kernel(const __g
         }
         __syncwarp();
       }
-      had0 += (w.n_tiles + 1) / 2;
-      had1 += w.n_tiles / 2;
+      had0 += (j + 1) / 2;
+      had1 += j / 2;
       ++n_done;
     }
     if (!ok) failed = 1;
+    if (lane == 0) {
+      ring_drain(had0, 1, [&](int, uint32_t parity) { return mbar_wait(o_done, parity); });
+      ring_drain(had1, 1, [&](int, uint32_t parity) { return mbar_wait(o_done + 8, parity); });
+    }
+    __syncwarp();
   }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;\n");

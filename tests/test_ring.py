@@ -50,8 +50,13 @@ def test_ring_drain_leaves_nothing_under_way(tmp_path):
 
 
 # (kernel file, the calls that belong to the warp that copies, to the warps that multiply)
+TWO_STAGES = ["s_full,", r"s_full \+ 8", "o_done,", r"o_done \+ 8"]
+
+
 @pytest.mark.parametrize("name, copies, products", [("gemm_rows_tc.cu", ["full0"], ["empty0"]),
-                                                    ("attention_rows_wide_tc.cu", ["q_full", "k_full"], ["s_full", "o_done"])])
+                                                    ("attention_rows_wide_tc.cu", ["q_full", "k_edge", "k_full"], ["s_full", "o_done"]),
+                                                    ("attention_rows_tc.cu", ["q_full", "full,", r"full \+ 8", "v_edge"], TWO_STAGES),
+                                                    ("attention_prefill_tc.cu", ["q_full", "full,", r"full \+ 8"], TWO_STAGES)])
 def test_persistent_kernels_wait_for_what_they_started(name, copies, products):
     """Each warp that starts copies or products waits for their barriers on every way out: the calls stand behind its loop, under no condition
     on success, before the block's last barrier."""
