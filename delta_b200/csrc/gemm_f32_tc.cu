@@ -1,0 +1,504 @@
+// 32-bit product  C[M,N] = A[M,K] * W[N,K]^T  on the fifth-generation tensor cores, with no fewer bits than 32-bit sums have.
+//
+// A 32-bit number is three bfloat16 parts exactly (eight bits of the mantissa each, cut off), x = x1 + x2 + x3, and products of parts are
+// exact in 32 bit.  Of the nine products of parts six are made; the three left out are below 2^-24 of a term.  A tensor core cuts off what
+// it adds to its accumulator, so a sum stays there for 64 entries of K only, the small products before the large: every chunk of 64 begins
+// at zero and is added to 32-bit sums in registers, rounded to nearest.  The order of a sum depends on nothing but W's sizes: a token's result
+// has the same bits whatever shares its step.  Against 64 bits (2-norm, normal operands) sums of 2,048 / 5,504 products are 1.6e-7 / 1.5e-7
+// off, chains of fused multiply-adds (gemm_plain.cu) 8.1e-7 / 1.3e-6.
+//   1. split_rows: the tokens' rows as three bfloat16 arrays, and which rows are out of the parts' reach;
+//   2. the product: W's rows are the M side (128 lanes), tokens the N side of the tiles.  One persistent block per SM:
+//      warp 0       fetches W (32 bit, TMA, 128-byte swizzle), warp 2 the tokens' parts (a box each, a ring of its own),
+//      warps 4-7    turn W into parts: a thread holds a row, and its parts go straight into tensor memory as an MMA's first operand, so that the
+//                   shared memory's bandwidth is left to the tokens' parts,
+//      warp 1       issues 24 products a chunk into one of two accumulators,
+//      warps 8-15   add finished chunks to the sums in registers and store them;
+//   3. add_segments, where K is cut into segments (W of few tiles): their sums in order.
+// Rows with infinite or NaN entries, or whose largest entry is outside 2^-40 .. 2^60 (parts or their products would leave the exponent's
+// range), are found on the way, and their results are summed by FMA over k instead.
+// Bound by the products' issue: a chunk takes about 1,500 cycles for up to 120 tokens (24 MMAs, each waited for by what converts the chunk after
+// next), 12 a token above.  Everything cold, microseconds, against the tiles of gemm_plain.cu: 300 x 2,048 x 2,048 107 -> 40, 300 x 11,008 x 2,048
+// 317 -> 126, 300 x 2,048 x 5,504 274 -> 66, 300 x 32,000 x 2,048 930 -> 240, 2,048 x 22,016 x 4,096 7,590 -> 2,020 (183 TFLOP/s); one row: 44 -> 28,
+// 76 -> 66, 106 -> 40, 137 -> 120, and 207 -> 220 with 22,016 x 4,096 (172 tiles in two rounds).
+//
+// Every wait on an mbarrier is bounded: when one gives up, the kernel records it, stores nothing more, waits (bounded again) for the copies and
+// products that it has under way, frees its tensor memory and returns.
+#include "common.cuh"
+#include "tcgen05_helpers.cuh"
+#include "ring.cuh"
+
+namespace {
+constexpr int BM = 128;                 // rows of W of a piece
+constexpr int KC = 64;                  // entries of K of a chunk
+constexpr int THREADS = 512;
+constexpr int W_STAGE = BM * KC * 4;
+constexpr int MAX_W = 6, MAX_X = 12;
+constexpr int SMEM_ROOM = 222 * 1024;
+constexpr int TMEM_COLS = 512;
+constexpr int A_COLS = 3 * KC / 2;      // tensor memory of a chunk of W in parts
+constexpr int MOST_ROWS = 16384;        // of A in a launch
+constexpr long long MOST_PARTIAL = 32ll << 20;      // floats of the segments' sums
+
+// The largest magnitude's bits: zero is in reach, infinities and NaNs are not.
+__device__ __forceinline__ bool out_of_reach(uint32_t largest) { return largest != 0 && (largest < (127u - 40u) << 23 || largest >= (127u + 60u) << 23); }
+
+__device__ __forceinline__ void parts_of(float x, float y, uint32_t& high, uint32_t& middle, uint32_t& low) {
+  const uint32_t bx = __float_as_uint(x), by = __float_as_uint(y);
+  high = __byte_perm(bx, by, 0x7632);
+  const float rx = x - __uint_as_float(bx & 0xffff0000u), ry = y - __uint_as_float(by & 0xffff0000u);
+  const uint32_t cx = __float_as_uint(rx), cy = __float_as_uint(ry);
+  middle = __byte_perm(cx, cy, 0x7632);
+  low = __byte_perm(__float_as_uint(rx - __uint_as_float(cx & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(cy & 0xffff0000u)), 0x7632);
+}
+
+// grid (rows): parts [3][M][K] and a row's flag.  w_largest (or null): N numbers that begin at zero.
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, int lda, __nv_bfloat16* __restrict__ parts, int* __restrict__ flags,
+                                                         uint32_t* __restrict__ w_largest, int M, int N, int K, int ldp, int vec) {
+  if (w_largest != nullptr)
+    for (int n = blockIdx.x * 256 + threadIdx.x; n < N; n += gridDim.x * 256) w_largest[n] = 0;
+  __shared__ uint32_t most[8];
+  const int m = blockIdx.x, tid = threadIdx.x;
+  const float* row = A + (size_t)m * lda;
+  const size_t plane = (size_t)M * ldp;
+  __nv_bfloat16* to = parts + (size_t)m * ldp;
+  uint32_t largest = 0;
+  for (int k = tid * 4; k < K; k += 1024) {      // K is a multiple of 4
+    float4 v;
+    if (vec) v = *reinterpret_cast<const float4*>(row + k);
+    else v = make_float4(row[k], row[k + 1], row[k + 2], row[k + 3]);
+    uint2 h, m2, l;
+    parts_of(v.x, v.y, h.x, m2.x, l.x);
+    parts_of(v.z, v.w, h.y, m2.y, l.y);
+    *reinterpret_cast<uint2*>(to + k) = h;
+    *reinterpret_cast<uint2*>(to + plane + k) = m2;
+    *reinterpret_cast<uint2*>(to + 2 * plane + k) = l;
+    const uint32_t a = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
+    const uint32_t b = max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu);
+    largest = max(largest, max(a, b));
+  }
+  largest = __reduce_max_sync(0xffffffffu, largest);
+  if ((tid & 31) == 0) most[tid >> 5] = largest;
+  __syncthreads();
+  if (tid == 0) {
+    for (int i = 1; i < 8; ++i) largest = max(largest, most[i]);
+    flags[m] = out_of_reach(largest);
+  }
+}
+
+template <int BN>
+struct Sizes {
+  static constexpr int X_STAGE = BN * KC * 2;
+  static constexpr int WS = BN <= 32 ? 6 : BN <= 64 ? 4 : 3;
+  static constexpr int XS = (SMEM_ROOM - WS * W_STAGE) / X_STAGE < MAX_X ? (SMEM_ROOM - WS * W_STAGE) / X_STAGE : MAX_X;
+  static constexpr int SMEM = WS * W_STAGE + XS * X_STAGE + 1024;
+  static_assert(XS >= 6, "two chunks of parts");
+  static constexpr int D_COLS = (BN + 31) / 32 * 32;
+  static_assert(2 * D_COLS + 2 * A_COLS <= TMEM_COLS, "two accumulators beside two chunks of W");
+};
+
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+}
+
+struct F32Args {
+  const float* A;
+  const float* W;
+  float* C;
+  const int* flags;      // rows of A out of reach
+  float* partial;        // [segments][M][N] where K is cut into segments, else null
+  uint32_t* w_largest;   // [N], with segments: the largest magnitude of a row of W
+  int* err;
+  int M, N, K, lda, ldw, ldc, tok_tiles, items;
+  int segments, per;     // chunks of K of a segment
+};
+
+// Piece number `item`: token tiles fastest, so that a tile of W comes from memory once; then K's segments, then W's tiles.
+struct Piece {
+  int m0, n0, segment, first, chunks;
+  __device__ __forceinline__ Piece(const F32Args& a, int item, int bn) {
+    const int rest = item / a.tok_tiles;
+    m0 = (item - rest * a.tok_tiles) * bn;
+    segment = rest % a.segments;
+    n0 = rest / a.segments * BM;
+    first = segment * a.per;
+    chunks = min(a.per, (a.K + KC - 1) / KC - first);
+  }
+};
+
+// The plain kernel's sum.
+__device__ __noinline__ float fma_sum(const float* x, const float* w, int K) {
+  float v = 0.f;
+  for (int k = 0; k < K; ++k) v = fmaf(x[k], w[k], v);
+  return v;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                                                                 const F32Args a) {
+  constexpr int WS = Sizes<BN>::WS, XS = Sizes<BN>::XS, X_STAGE = Sizes<BN>::X_STAGE, D_COLS = Sizes<BN>::D_COLS, NC = BN / 2;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* xs = smem + WS * W_STAGE;
+  __shared__ __align__(8) unsigned long long bars[2 * MAX_W + 2 * MAX_X + 8];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int failed;
+  __shared__ int w_flags[2][BM];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t wfull = s2u(&bars[0]), wempty = s2u(&bars[MAX_W]), xfull = s2u(&bars[2 * MAX_W]), xempty = s2u(&bars[2 * MAX_W + MAX_X]);
+  const uint32_t afull = s2u(&bars[2 * MAX_W + 2 * MAX_X]), done = afull + 16, dempty = afull + 32, flagged = afull + 48;
+  if (tid == 0) {
+    for (int s = 0; s < WS; ++s) {
+      mbar_init(wfull + 8 * s, 1);
+      mbar_init(wempty + 8 * s, 4);
+    }
+    for (int s = 0; s < XS; ++s) {
+      mbar_init(xfull + 8 * s, 1);
+      mbar_init(xempty + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(afull + 8 * b, 4);
+      mbar_init(done + 8 * b, 1);
+      mbar_init(dempty + 8 * b, 8);
+      mbar_init(flagged + 8 * b, 4);
+    }
+    failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc(s2u(&tmem_base_slot), TMEM_COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot, tmem_a = tmem_base + 2 * D_COLS;
+  volatile int* gave_up = &failed;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int c = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+        const Piece p(a, item, BN);
+        for (int k = p.first; k < p.first + p.chunks; ++k, ++c) {
+          const int s = ring_slot(c, WS);
+          if (c >= WS && !mbar_wait(wempty + 8 * s, ring_parity(c - WS, WS))) {
+            *gave_up = 1;
+            ok = false;
+            break;
+          }
+          const uint32_t to = s2u(smem + (size_t)s * W_STAGE), bar = wfull + 8 * s;
+          mbar_expect_tx(bar, W_STAGE);
+          tma_load_2d(to, &map_w, k * KC, p.n0, bar);      // rows past N and entries past K are zeros
+          tma_load_2d(to + W_STAGE / 2, &map_w, k * KC + KC / 2, p.n0, bar);
+        }
+      }
+      ring_drain(c, WS, [&](int s, uint32_t parity) { return mbar_wait(wfull + 8 * s, parity); });
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      int c = 0;      // parts asked for: the third, the second, the first of every chunk
+      bool ok = true;
+      for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+        const Piece piece(a, item, BN);
+        for (int k = piece.first; k < piece.first + piece.chunks && ok; ++k)
+          for (int p = 2; p >= 0; --p, ++c) {
+            const int s = ring_slot(c, XS);
+            if (c >= XS && !mbar_wait(xempty + 8 * s, ring_parity(c - XS, XS))) {
+              *gave_up = 1;
+              ok = false;
+              break;
+            }
+            const uint32_t bar = xfull + 8 * s;
+            mbar_expect_tx(bar, X_STAGE);
+            tma_load_2d(s2u(xs + (size_t)s * X_STAGE), &map_x, k * KC, p * a.M + piece.m0, bar);      // (rows past M: another part's, of no token's column)
+          }
+      }
+      ring_drain(c, XS, [&](int s, uint32_t parity) { return mbar_wait(xfull + 8 * s, parity); });
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = instr_desc_bf16(BM, BN);
+    int c = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
+      const Piece p(a, item, BN);
+      for (int k = 0; k < p.chunks; ++k, ++c) {
+        const int b = c & 1, x = 3 * c;
+        bool there = true;      // a lane waits for each of what a chunk needs: one after the other the waits took as long as the products
+        if (lane == 0) there = c < 2 || mbar_wait(dempty + 8 * b, ring_parity(c - 2, 2));
+        else if (lane == 1) there = mbar_wait(afull + 8 * b, ring_parity(c, 2));
+        else if (lane < 5) there = mbar_wait(xfull + 8 * ring_slot(x + lane - 2, XS), ring_parity(x + lane - 2, XS));
+        if (__any_sync(0xffffffffu, !there)) {
+          *gave_up = 1;
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (lane == 0) {
+          const uint32_t wa = tmem_a + b * A_COLS, d = tmem_base + b * D_COLS;
+#pragma unroll
+          for (int q = 2; q >= 0; --q) {      // the tokens' part q with W's parts 2 - q .. 0, the smallest first
+            const int s = ring_slot(x + 2 - q, XS);
+            const uint64_t db = smem_desc_k_major(s2u(xs + (size_t)s * X_STAGE));
+#pragma unroll
+            for (int r = 2 - q; r >= 0; --r)
+#pragma unroll
+              for (int i = 0; i < KC / 16; ++i)
+                umma_a_tmem(d, wa + r * (KC / 2) + i * 8, db + (uint64_t)(i * 2), idesc, (q == 2 && i == 0) ? 0u : 1u);
+            umma_commit(xempty + 8 * s);
+          }
+          umma_commit(done + 8 * b);
+        }
+        __syncwarp();
+      }
+    }
+    if (lane == 0) ring_drain(3 * c, XS, [&](int s, uint32_t parity) { return mbar_wait(xempty + 8 * s, parity); });      // its products are complete
+  } else if (warp >= 4 && warp < 8) {
+    const int row = tid & 127;
+    int c = 0, piece = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x, ++piece) {
+      const Piece p(a, item, BN);
+      uint32_t largest = 0;
+      for (int k = 0; k < p.chunks; ++k, ++c) {
+        const int s = ring_slot(c, WS), b = c & 1;
+        const bool there = mbar_wait(wfull + 8 * s, ring_parity(c, WS)) && (c < 2 || mbar_wait(done + 8 * b, ring_parity(c - 2, 2))) && *gave_up == 0;
+        if (__any_sync(0xffffffffu, !there)) {      // the whole warp leaves, or none of it
+          *gave_up = 1;
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const unsigned char* from = smem + (size_t)s * W_STAGE + row * 128;
+        const uint32_t to = tmem_a + b * A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t h[16], m[16], l[16];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(from + half * (W_STAGE / 2) + ((j ^ (row & 7)) << 4));
+            parts_of(v.x, v.y, h[2 * j], m[2 * j], l[2 * j]);
+            parts_of(v.z, v.w, h[2 * j + 1], m[2 * j + 1], l[2 * j + 1]);
+            largest = max(largest, max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
+                                       max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu)));
+          }
+          tmem_st16(to + half * 16, h);
+          tmem_st16(to + KC / 2 + half * 16, m);
+          tmem_st16(to + KC + half * 16, l);
+        }
+        if (k + 1 == p.chunks) {
+          if (a.partial == nullptr) w_flags[piece & 1][row] = out_of_reach(largest);
+          else if (p.n0 + row < a.N) atomicMax(a.w_largest + p.n0 + row, largest);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(wempty + 8 * s);
+          mbar_arrive(afull + 8 * b);
+          if (k + 1 == p.chunks && a.partial == nullptr) mbar_arrive(flagged + 8 * (piece & 1));
+        }
+      }
+    }
+  } else if (warp >= 8) {
+    const int quarter = warp & 3, half = (warp - 8) >> 2;
+    const int row = quarter * 32 + lane;
+    int c = 0, piece = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x, ++piece) {
+      const Piece p(a, item, BN);
+      const int n = p.n0 + row, m0 = p.m0 + half * NC;
+      float sum[NC];
+#pragma unroll
+      for (int j = 0; j < NC; ++j) sum[j] = 0.f;
+      for (int k = 0; k < p.chunks; ++k, ++c) {
+        const int b = c & 1;
+        const bool there = mbar_wait(done + 8 * b, ring_parity(c, 2)) && *gave_up == 0;
+        if (__any_sync(0xffffffffu, !there)) {
+          *gave_up = 1;
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t at = tmem_base + b * D_COLS + half * NC + ((uint32_t)(quarter * 32) << 16);
+        constexpr int G = NC % 40 == 0 ? 40 : NC % 32 == 0 ? 32 : NC;      // columns on their way at a time
+#pragma unroll
+        for (int g = 0; g < NC; g += G) {
+          float v[G];
+#pragma unroll
+          for (int j = 0; j < G; j += 8) tmem_ld8_nowait(at + g + j, v + j);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < G; ++j) sum[g + j] += v[j];
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dempty + 8 * b);
+      }
+      const bool there = ok && (a.partial != nullptr || mbar_wait(flagged + 8 * (piece & 1), ring_parity(piece, 2)));      // (eight chunks and more a piece)
+      if (__any_sync(0xffffffffu, !there)) {
+        *gave_up = 1;
+        break;
+      }
+      float* to = a.partial != nullptr ? a.partial + (size_t)p.segment * a.M * a.N : a.C;
+      const int ld = a.partial != nullptr ? a.N : a.ldc;
+#pragma unroll
+      for (int j = 0; j < NC; ++j)
+        if (n < a.N && m0 + j < a.M) to[(size_t)(m0 + j) * ld + n] = sum[j];
+      if (a.partial != nullptr) continue;
+      const bool own = w_flags[piece & 1][row] != 0;
+      bool odd = own;
+      for (int j = lane; j < NC; j += 32) odd |= m0 + j < a.M && a.flags[m0 + j] != 0;
+      if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll 1
+        for (int j = 0; j < NC; ++j)
+          if (n < a.N && m0 + j < a.M && (own || a.flags[m0 + j] != 0))
+            a.C[(size_t)(m0 + j) * a.ldc + n] = fma_sum(a.A + (size_t)(m0 + j) * a.lda, a.W + (size_t)n * a.ldw, a.K);
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (failed && tid == 0) dk_report(a.err, DK_DEV_TIMEOUT, blockIdx.x, 0, a.per);
+  if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// The segments' sums, added in their order.
+__global__ void __launch_bounds__(256) add_segments_kernel(const F32Args a) {
+  const long long total = (long long)a.M * a.N;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+    const int m = (int)(i / a.N), n = (int)(i - (long long)m * a.N);
+    float v = a.partial[i];
+#pragma unroll 4
+    for (int s = 1; s < a.segments; ++s) v += a.partial[i + s * total];
+    if (out_of_reach(a.w_largest[n]) || a.flags[m] != 0) v = fma_sum(a.A + (size_t)m * a.lda, a.W + (size_t)n * a.ldw, a.K);
+    a.C[(size_t)m * a.ldc + n] = v;
+  }
+}
+
+// 2-D tensor [rows, cols] of floats, boxes of [box_rows x 32], 128-byte swizzle, zeros where a box reaches past the tensor
+bool make_tensor_map_f32(CUtensorMap* m, const void* base, long long rows, int cols, long long ld, int box_rows) {
+  TensorMapEncodeFn fn = tensor_map_encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN>
+int launch(F32Args a, const __nv_bfloat16* parts, int ldp, const CUtensorMap& map_w, cudaStream_t stream) {
+  static bool granted[DK_MAX_DEVICES] = {false};
+  bool& ok = granted[dk_current_device()];
+  if (!ok) {
+    DK_REQUIRE(cudaFuncSetAttribute(gemm_f32_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes<BN>::SMEM) == cudaSuccess,
+               "gemm_f32_tc: %d bytes of shared memory were refused", Sizes<BN>::SMEM);
+    ok = true;
+  }
+  CUtensorMap map_x;
+  DK_REQUIRE(make_tensor_map_bf16(&map_x, parts, 3ll * a.M, a.K, ldp, BN), "gemm_f32_tc: cannot encode the tensor map of the parts");
+  a.tok_tiles = (a.M + BN - 1) / BN;
+  const long long items = (long long)a.tok_tiles * a.segments * ((a.N + BM - 1) / BM);
+  DK_REQUIRE(items < (1ll << 30), "gemm_f32_tc: too many pieces");
+  a.items = (int)items;
+  gemm_f32_tc_kernel<BN><<<min(a.items, dk_sm_count()), THREADS, Sizes<BN>::SMEM, stream>>>(map_w, map_x, a);
+  return 0;
+}
+// How K is cut: by W's sizes alone, so that a token's sum has one order whatever the step.  A matrix of few tiles would leave most SMs idle
+// (2,048 rows are 16 tiles); with segments of four chunks and more its tiles fill SPREAD of them, and their sums are added by a kernel of their own.
+constexpr int SPREAD = 148, LEAST_CHUNKS = 4;
+struct Cut {
+  int segments, per;
+  Cut(int N, int K) {
+    const int chunks = (K + KC - 1) / KC;
+    const long long tiles = (N + BM - 1) / BM;
+    per = chunks;
+    if (tiles <= SPREAD / 2) per = (int)max((long long)LEAST_CHUNKS, (chunks * tiles + SPREAD - 1) / SPREAD);
+    segments = (chunks + per - 1) / per;
+  }
+};
+// Rows of A that one launch takes: they bound the working memory.
+int slab_rows(int N, int segments) {
+  if (segments == 1) return MOST_ROWS;
+  const long long rows = MOST_PARTIAL / ((long long)segments * N) / 32 * 32;
+  return (int)min((long long)MOST_ROWS, max(32ll, rows));
+}
+}  // namespace
+
+// Whether a product with W [N, K] takes this way: a rule on W alone, so that a token's sums are made in one order whatever the step.
+extern "C" int dk_gemm_f32_tc_supported(const void* W, int N, int K) {
+  // Shorter sums are as fast or faster by FMA: 1,024 x 1,024 25.6 against 24.6 us for one row and 27.6 against 43 for 300; 256 x 512 23.6 against 16.4.
+  return K >= (N >= 4096 ? 512 : 1024) && K <= (1 << 20) && K % 4 == 0 && N > 0 && N <= (1 << 24) && (uintptr_t)W % 16 == 0;
+}
+
+// Kilobytes of working memory for M rows, and the launches that they take.
+extern "C" int dk_gemm_f32_tc_plan(int M, int N, int K, int* kilobytes, int* launches) {
+  DK_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32_tc: bad sizes M=%d N=%d K=%d", M, N, K);
+  const Cut cut(N, K);
+  const int slab = slab_rows(N, cut.segments);
+  const long long rows = min(M, slab), ldp = (K + 7) / 8 * 8;
+  long long bytes = 6 * rows * ldp + 4 * rows + 16;
+  if (cut.segments > 1) bytes += 4ll * N + 16 + 4ll * cut.segments * rows * N;
+  *kilobytes = (int)((bytes + 1023) / 1024);
+  *launches = (M + slab - 1) / slab * (cut.segments > 1 ? 3 : 2);
+  return 0;
+}
+
+extern "C" int dk_gemm_f32_tc(const void* A, const void* W, void* C, void* work, int M, int N, int K, int lda, int ldw, int ldc, int* err,
+                              cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  DK_REQUIRE(M > 0 && dk_gemm_f32_tc_supported(W, N, K), "gemm_f32_tc: sizes not taken: M=%d N=%d K=%d", M, N, K);
+  DK_REQUIRE(lda >= K && ldw >= K && ldc >= N && ldw % 4 == 0, "gemm_f32_tc: leading sizes %d %d %d are not taken", lda, ldw, ldc);
+  DK_REQUIRE(work != nullptr && (uintptr_t)work % 16 == 0, "gemm_f32_tc: working memory must start on a 16-byte boundary");
+  const int ldp = (K + 7) / 8 * 8, sms = dk_sm_count();
+  const Cut cut(N, K);
+  const int slab = slab_rows(N, cut.segments);
+  CUtensorMap map_w;
+  DK_REQUIRE(make_tensor_map_f32(&map_w, W, N, K, ldw, BM), "gemm_f32_tc: cannot encode the tensor map of W");
+  for (int m = 0; m < M; m += slab) {
+    F32Args a = {};
+    a.M = min(slab, M - m);
+    a.A = (const float*)A + (size_t)m * lda;
+    a.W = (const float*)W;
+    a.C = (float*)C + (size_t)m * ldc;
+    a.N = N; a.K = K; a.lda = lda; a.ldw = ldw; a.ldc = ldc;
+    a.segments = cut.segments; a.per = cut.per;
+    a.err = err;
+    auto* parts = (__nv_bfloat16*)work;
+    int* flags = (int*)(parts + 3ll * a.M * ldp);
+    a.flags = flags;
+    if (cut.segments > 1) {
+      a.w_largest = (uint32_t*)(flags + (a.M + 3) / 4 * 4);
+      a.partial = (float*)(a.w_largest + (N + 3) / 4 * 4);
+    }
+    split_rows_kernel<<<a.M, 256, 0, stream>>>(a.A, lda, parts, flags, a.w_largest, a.M, N, K, ldp, (uintptr_t)a.A % 16 == 0 && lda % 4 == 0);
+    // Tokens of a piece: a chunk takes 12 cycles a token on the tensor cores, and about 1,500 whatever their number (24 products' issue, W's
+    // way into parts).  Least rounds of pieces times that.
+    const int sizes[] = {160, 128, 96, 64, 48, 32, 16};
+    int best = 0;
+    long long least = 0;
+    for (int bn : sizes) {
+      const long long items = (long long)((a.M + bn - 1) / bn) * cut.segments * ((N + BM - 1) / BM), cost = (items + sms - 1) / sms * max(12 * bn, 1500);
+      if (best == 0 || cost < least) { best = bn; least = cost; }
+    }
+    int rc = 0;
+    switch (best) {
+      case 160: rc = launch<160>(a, parts, ldp, map_w, stream); break;
+      case 128: rc = launch<128>(a, parts, ldp, map_w, stream); break;
+      case 96: rc = launch<96>(a, parts, ldp, map_w, stream); break;
+      case 64: rc = launch<64>(a, parts, ldp, map_w, stream); break;
+      case 48: rc = launch<48>(a, parts, ldp, map_w, stream); break;
+      case 32: rc = launch<32>(a, parts, ldp, map_w, stream); break;
+      default: rc = launch<16>(a, parts, ldp, map_w, stream);
+    }
+    if (rc) return rc;
+    if (cut.segments > 1) {
+      const long long blocks = ((long long)a.M * N + 255) / 256;
+      add_segments_kernel<<<(int)min(blocks, 16ll * sms), 256, 0, stream>>>(a);
+    }
+  }
+  return dk_check_launch("gemm_f32_tc");
+}

@@ -1,8 +1,9 @@
 // Plain matrix product  C[M,N] = A[M,K] * W[N,K]^T  on the FMA units, float
 // accumulation, no reduced-precision matrix mode and no split over K: the sum of
 // one output element runs over k in the same order whatever M is, so a token's
-// result does not depend on what shares its batch.  This is the product of the
-// 32-bit path and the plain twin of the tensor-core products.
+// result does not depend on what shares its batch.  This is the plain twin of the
+// tensor-core products, and the 32-bit path's product where sums are short (long
+// ones: gemm_f32_tc.cu).
 //
 // Two kernels.  32-bit operands whose rows begin on 16-byte boundaries: tiles come by cp.async, three to four stages ahead, and stay as
 // they lie (rows of 16 entries, 20 apart, so that eight neighbouring rows' 16-byte reads meet no bank twice); a thread keeps TM x TN

@@ -75,6 +75,9 @@ _SIGNATURES = {
     "dk_silu_mul": [P, P, I, I, I, P],
     "dk_rope_append": [P, P, P, P, I, P, I, P, I, I, I, I, I, I, I, I, P, P],
     "dk_gemm_nt_plain": [P, P, P, I, I, I, I, I, I, I, I, P],
+    "dk_gemm_f32_tc_supported": [P, I, I],
+    "dk_gemm_f32_tc_plan": [I, I, I, C.POINTER(I), C.POINTER(I)],
+    "dk_gemm_f32_tc": [P, P, P, P, I, I, I, I, I, I, P, P],
     "dk_attention_f32_supported": [I, I, I, I, I],
     "dk_attention_f32": [C.POINTER(AttnParams), I, P],
     "dk_attention_plain": [C.POINTER(AttnParams), P],

@@ -174,6 +174,36 @@ def gemm_nt_plain(a, w, out):
     return out
 
 
+_f32_plans = {}      # (rows, N, K) -> bytes of working memory, launches
+
+
+def gemm_f32_tc_supported(w) -> bool:
+    """Whether products with this 32-bit ``w`` [N, K] may go to ``gemm_f32_tc``: nothing but ``w`` decides."""
+    return w.dtype == torch.float32 and w.is_contiguous() and bool(_l.load().dk_gemm_f32_tc_supported(_ptr(w, "w"), w.shape[0], w.shape[1]))
+
+
+def gemm_f32_tc(a, w, out, err=None):
+    """out[M,N] = a[M,K] @ w[N,K]^T of 32-bit operands, exactly split into bfloat16 parts for the tensor cores: no operand or sum of fewer bits."""
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K or tuple(out.shape) != (M, N) or not (a.dtype == w.dtype == out.dtype == torch.float32):
+        raise KernelError(f"gemm: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)} or dtypes do not fit")
+    if M == 0 or N == 0:
+        return out
+    lib = _l.load()
+    plan = _f32_plans.get((M, N, K))
+    if plan is None:
+        kb, launches = C.c_int(), C.c_int()
+        _l.check(lib.dk_gemm_f32_tc_plan(M, N, K, C.byref(kb), C.byref(launches)), "gemm_f32_tc", 0)
+        if len(_f32_plans) >= 4096:
+            _f32_plans.clear()
+        plan = _f32_plans[(M, N, K)] = (kb.value * 1024, launches.value)
+    work = torch.empty(plan[0], dtype=torch.uint8, device=a.device)
+    _l.check(lib.dk_gemm_f32_tc(_ptr(a, "a"), _ptr(w, "w"), _ptr(out, "out"), _ptr(work, "work"), M, N, K, K, K, N,
+                                _ptr(err, "err", torch.int32), _stream()), "gemm_f32_tc", plan[1])
+    return out
+
+
 def attn_step_params(*, tok_row, tok_pos, row_slot=None, row_flags=None, row_q_start=None, row_q_len=None, row_pos_start=None,
                      err=None) -> AttnParams:
     """The part of the attention kernels' parameters that is the same for every layer of a step (the step's

@@ -1,7 +1,8 @@
 """Matrix products  y = x W^T  of the parts.
 
-32-bit activations go through the plain FMA kernel (true 32 bit: no
-reduced-precision matrix mode, no split over K).  bfloat16 activations go
+32-bit activations keep 32-bit operands and sums: they go to the tensor cores in
+three exact bfloat16 parts, or, for short sums, through the plain FMA kernel; which
+one is decided by the weights alone, and neither splits K by the number of rows.  bfloat16 activations go
 through the tensor cores.  For large batches (prompt portions) that is the
 library product the reference uses for its ``nn.Linear`` layers
 (DELTA/Engine/DELTA/model.py:369-370, 498-500), or, where the sums stay in 32
@@ -216,7 +217,9 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, out_dtype=None) -> torch.Tenso
     T, N = x.shape[0], w.shape[0]
     if x.dtype == torch.float32 or ("products" in ctx.plain_kernels):
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
-        if T:
+        if T and out_dtype == torch.float32 and "products" not in ctx.plain_kernels and ops.gemm_f32_tc_supported(w):
+            ops.gemm_f32_tc(x, w, out, err=ctx.err)
+        elif T:
             ops.gemm_nt_plain(x, w, out)
         return out
     if 0 < T <= MANY_M:

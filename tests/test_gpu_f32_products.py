@@ -1,0 +1,79 @@
+"""32-bit products by tensor cores: tiles' and chunks' ends, the same bits whatever shares a step, numbers that the parts do not reach."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def run(a, w):
+    o = ops()
+    assert o.gemm_f32_tc_supported(w)
+    out = torch.full((a.shape[0] + 1, w.shape[0]), 7.0, device=DEV)
+    err = o.new_error_record(DEV)
+    o.gemm_f32_tc(a, w, out[:-1], err=err)
+    o.raise_if_error(err)
+    assert bool((out[-1] == 7.0).all())
+    return out[:-1]
+
+
+# token tiles of 16 to 160, K beside a chunk of 64 and in segments of 4 to 10 chunks, fewer and more rows of W than a tile, more pieces than SMs,
+# more rows than a launch takes
+@pytest.mark.parametrize("M, N, K", [(1, 128, 1024), (16, 127, 1028), (17, 1, 1100), (33, 300, 2044), (49, 2049, 1080), (129, 4096, 4100), (161, 8200, 516),
+                                     (300, 2560, 2048), (319, 11008, 512), (700, 9700, 1028), (16385, 40, 1024)])
+def test_gemm_f32_tc(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    a, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(N, K, device=DEV, generator=g) * 0.05
+    out = run(a, w)
+    ref = a.double() @ w.double().T
+    # parts and products left out: 2^-24 of a term; cut-off sums of a chunk and the rounded sum of K / 64 of them: (24 + K / 64) 2^-24 of the magnitudes bounds it by far
+    bound = (26 + K // 64) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    plain = torch.empty(M, N, device=DEV)
+    ops().gemm_nt_plain(a, w, plain)
+    assert (out.double() - ref).norm() <= (plain.double() - ref).norm()      # nearer than the chain of fused multiply-adds
+    for m in (1, 2, 31, 100, 160, 299):
+        if m < M:
+            assert torch.equal(run(a[M - m:], w), out[M - m:]), m
+
+
+@pytest.mark.parametrize("N", [300, 9500])      # K in segments, and as a whole
+def test_gemm_f32_tc_numbers_out_of_the_parts_reach(N):
+    """Infinite, NaN, very large and very small entries: the sums of the plain kernel for the rows that hold them, the others untouched."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    a, w = torch.randn(70, 1024, device=DEV, generator=g), torch.randn(N, 1024, device=DEV, generator=g)
+    want = run(a, w)
+    rows, cols = {3: math.inf, 9: -math.inf, 20: math.nan, 41: 3e38, 69: 1.5 * 2.0 ** 60}, {0: math.inf, 130: -3.3e38, 131: math.nan, 299: 2.0 ** 100}
+    b, v = a.clone(), w.clone()
+    for r, x in rows.items():
+        b[r, (7 * r) % 1024] = x
+    for r, x in cols.items():
+        v[r, (5 * r) % 1024] = x
+    b[50] *= 2.0 ** -60
+    b[51] *= 2.0 ** -120
+    b[52] = 0.0
+    v[200] *= 2.0 ** -100
+    v[201] = 0.0
+    out, plain = run(b, v), torch.empty(70, N, device=DEV)
+    ops().gemm_nt_plain(b, v, plain)
+    odd_r, odd_c = list(rows) + [50, 51], list(cols) + [200]
+    same = lambda x, y: torch.equal(torch.nan_to_num(x, nan=1.0), torch.nan_to_num(y, nan=1.0)) and torch.equal(x.isnan(), y.isnan())      # noqa: E731
+    assert same(out[odd_r], plain[odd_r]) and same(out[:, odd_c], plain[:, odd_c])
+    rest_r = [r for r in range(70) if r not in odd_r + [52]]
+    rest_c = [c for c in range(N) if c not in odd_c + [201]]
+    assert torch.equal(out[rest_r][:, rest_c], want[rest_r][:, rest_c])
+    assert bool((out[52][rest_c] == 0).all()) and bool((out[rest_r][:, 201] == 0).all())
+
+
+def test_gemm_f32_tc_refuses_what_it_does_not_take():
+    o = ops()
+    ok = torch.empty(8, 1024, device=DEV)
+    assert o.gemm_f32_tc_supported(ok)
+    for w in (torch.empty(8, 1020, device=DEV), torch.empty(8, 1026, device=DEV), torch.empty(8, 1024, device=DEV).bfloat16(), torch.empty(8193, device=DEV)[1:].view(8, 1024),
+              torch.empty(1024, 8, device=DEV).T):
+        assert not o.gemm_f32_tc_supported(w)
+    with pytest.raises(o.KernelError):
+        o.gemm_f32_tc(torch.empty(2, 1020, device=DEV), ok, torch.empty(2, 8, device=DEV))
