@@ -6,11 +6,14 @@
 // 128-byte swizzle); two accumulators in tensor memory take turns, so that a piece's epilogue runs under the next one's products:
 //   warp 0      asks for the boxes,
 //   warp 1      issues the products and owns the tensor memory,
-//   warps 2-5   epilogue: a thread holds one row of the tile, so a row's outputs leave as they are contiguous in memory, through no
-//               shared memory; gated activations find gate and up columns in one accumulator (half of the tile each).
+//   warps 2-9   epilogue: a warp takes 32 rows and half of the columns, 16 at a time; a thread holds one row of the tile, and 16 x 32 values
+//               are turned in shared memory, so that a store reaches four or eight rows in whole sectors and not 32; gated activations find gate and
+//               up columns in one accumulator (half of the tile each).
 // Bound by the shared memory's bandwidth: 48 KB a step are written and read once more by the tensor core, 96 bytes a cycle each.
 // 2,048 x 22,016 x 4,096: 250 us = 1,480 TFLOP/s with or without the silu gate (one block a tile, its epilogue uncovered, took 404 and 456;
-// the library 218 without the gate); an expert's products of a 2,048-token prompt (16 experts of 1,024, 4 chosen, width 2,048) 157 -> 62 us.
+// the library 218 without the gate); an expert's products of a 2,048-token prompt (16 experts of 1,024, 4 chosen, width 2,048) 157 -> 62 us, and
+// 64 -> 52 (two of them on average, the second with 67 MB of 32-bit results) since eight warps write instead of four, in rows that lanes share.
+// (Rows gathered by the copies themselves, tile::gather4, in place of a kernel of 13 us before the first product: that product 55 -> 170 us.)
 //
 // Every wait on an mbarrier is bounded: when one gives up, the kernel records it, stores nothing more, waits (bounded again) for the copies and
 // products that it has under way, frees its tensor memory and returns.
@@ -21,7 +24,11 @@
 namespace {
 constexpr int BM = 128;            // rows of x of a piece
 constexpr int KSTEP = 64;          // entries of K of a box: one 128-byte swizzle row
-constexpr int THREADS = 192;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = (2 + EPI_WARPS) * 32;
+constexpr int EPI_COLS = 16;       // columns that a warp turns at a time
+constexpr int EPI_LD = EPI_COLS + 4;
+constexpr int EPI_BYTES = 32 * EPI_LD * 4;      // of shared memory a warp
 constexpr int MAX_STAGES = 7;
 
 enum Epilogue { PLAIN = 0, GLU = 1, RELU_SQUARED = 2, SILU = 3 };
@@ -42,8 +49,9 @@ struct RowsArgs {
 template <int BN>
 struct Sizes {
   static constexpr int STAGE = (BM + BN) * KSTEP * 2;
-  static constexpr int STAGES = (224 * 1024) / STAGE < MAX_STAGES ? (224 * 1024) / STAGE : MAX_STAGES;
-  static constexpr int SMEM = STAGES * STAGE + 1024;
+  static constexpr int ROOM = 224 * 1024 - EPI_WARPS * EPI_BYTES;
+  static constexpr int STAGES = ROOM / STAGE < MAX_STAGES ? ROOM / STAGE : MAX_STAGES;
+  static constexpr int SMEM = STAGES * STAGE + EPI_WARPS * EPI_BYTES + 1024;
 };
 
 template <int BN>
@@ -64,7 +72,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_tc_kernel(const __grid_c
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, 4);
+      mbar_init(tempty0 + 8 * b, EPI_WARPS);
     }
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -157,14 +165,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_tc_kernel(const __grid_c
       ring_drain(step, STAGES, [&](int s, uint32_t parity) { return mbar_wait(empty0 + 8 * s, parity); });
     }
   } else {
-    const int quarter = warp & 3;      // the lanes of tensor memory that a warp may read
+    const int quarter = warp & 3, half = (warp - 2) >> 2;      // the lanes of tensor memory that a warp may read, and its half of the columns
+    float* turn = reinterpret_cast<float*>(smem + (size_t)STAGES * STAGE + (size_t)(warp - 2) * EPI_BYTES);
     int piece = 0;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       int rt, ct, w_row;
       if (!place(item, rt, ct, w_row)) continue;
       const int b = piece & 1;
       const int r = rt * BM + quarter * 32 + lane;
-      long long out_row = r < a.M ? (a.row_map != nullptr ? a.row_map[r] : r) : -1;
+      const int out_row = r < a.M ? (a.row_map != nullptr ? a.row_map[r] : r) : -1;
       const bool there = mbar_wait(tfull0 + 8 * b, (piece >> 1) & 1) && *gave_up == 0;
       if (__any_sync(0xffffffffu, !there)) {      // the whole warp leaves, or none of it
         *gave_up = 1;
@@ -173,36 +182,50 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_rows_tc_kernel(const __grid_c
       tc_fence_after();
       const uint32_t acc = tmem_base + b * BN + ((uint32_t)(quarter * 32) << 16);
       const int n0 = ct * cols;
-      for (int c = 0; c < cols; c += 32) {
+      for (int c = half * (cols / 2); c < (half + 1) * (cols / 2); c += EPI_COLS) {
         if (n0 + c >= a.N) break;
-        float y[32], u[32];
-        tmem_ld32_nowait(acc + c, y);
-        if (gated) tmem_ld32_nowait(acc + BN / 2 + c, u);
-        tmem_wait_ld();
+        float y[EPI_COLS], u[EPI_COLS];
+        tmem_ld16(acc + c, y);
+        if (gated) tmem_ld16(acc + BN / 2 + c, u);
         if (a.epilogue == GLU) {      // both products rounded to bfloat16 first, as separate products would be
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
+          for (int i = 0; i < EPI_COLS; ++i)
             y[i] = dk_glu_value(__bfloat162float(__float2bfloat16_rn(y[i])), __bfloat162float(__float2bfloat16_rn(u[i])), a.limit, a.alpha, a.shift);
         } else if (a.epilogue == SILU) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) y[i] = y[i] / (1.f + expf(-y[i])) * u[i];
+          for (int i = 0; i < EPI_COLS; ++i) y[i] = y[i] / (1.f + expf(-y[i])) * u[i];
         } else if (a.epilogue == RELU_SQUARED) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < EPI_COLS; ++i) {
             const float v = fmaxf(__bfloat162float(__float2bfloat16_rn(y[i])), 0.f);
             y[i] = v * v;
           }
         }
+        // a thread holds a row; through shared memory, so that neighbouring lanes store neighbouring pieces of a row
+        __syncwarp();
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {      // N is a multiple of 8: a group of eight is in or out as a whole
-          const int n = n0 + c + 8 * g;
-          if (out_row >= 0 && n < a.N) {
-            const float v[8] = {y[8 * g], y[8 * g + 1], y[8 * g + 2], y[8 * g + 3], y[8 * g + 4], y[8 * g + 5], y[8 * g + 6], y[8 * g + 7]};
-            if (a.out_f32) store8<float>((float*)a.out + (size_t)out_row * a.ldc + n, v);
-            else store8<__nv_bfloat16>((__nv_bfloat16*)a.out + (size_t)out_row * a.ldc + n, v);
+        for (int g = 0; g < EPI_COLS / 4; ++g)
+          *reinterpret_cast<float4*>(turn + lane * EPI_LD + 4 * g) = make_float4(y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3]);
+        __syncwarp();
+        if (a.out_f32) {      // four lanes a row, eight rows at a time
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int row = i * 8 + (lane >> 2), n = n0 + c + (lane & 3) * 4;
+            const int to = __shfl_sync(0xffffffffu, out_row, row);
+            const float4 v = *reinterpret_cast<const float4*>(turn + row * EPI_LD + (lane & 3) * 4);
+            if (to >= 0 && n < a.N) *reinterpret_cast<float4*>((float*)a.out + (size_t)to * a.ldc + n) = v;      // N is a multiple of 8
+          }
+        } else {      // two lanes a row
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int row = i * 16 + (lane >> 1), n = n0 + c + (lane & 1) * 8;
+            const int to = __shfl_sync(0xffffffffu, out_row, row);
+            const float4 p = *reinterpret_cast<const float4*>(turn + row * EPI_LD + (lane & 1) * 8);
+            const float4 q = *reinterpret_cast<const float4*>(turn + row * EPI_LD + (lane & 1) * 8 + 4);
+            const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+            if (to >= 0 && n < a.N) store8<__nv_bfloat16>((__nv_bfloat16*)a.out + (size_t)to * a.ldc + n, v);
           }
         }
-        __syncwarp();      // (tensor memory is read by whole warps)
       }
       tc_fence_before();
       __syncwarp();

@@ -84,3 +84,20 @@ def test_shaped_portions(dk, dv, cap, far):
     want = got[torch.float32]
     # weights to 16 bits, one rounding of the output to bfloat16 (2^-9 of it); values are about one
     assert (got[torch.bfloat16] - want).abs().max() < 2.0 ** -8 * want.abs().max()
+
+
+# the persistent product's epilogue: columns that end beside a warp's 16 and its half of the tile, rows beside a tile's 128, every kind of result
+@pytest.mark.parametrize("M, N", [(129, 8), (129, 136), (257, 264), (200, 392), (385, 520), (1300, 2056)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_rows_product_writes_its_columns_and_no_others(M, N, out_dtype):
+    from delta_b200.kernels import ops as o
+    g = torch.Generator(device="cuda:0").manual_seed(M + N)
+    x, w = torch.randn(M, 192, device="cuda:0", generator=g).bfloat16(), torch.randn(N, 192, device="cuda:0", generator=g).bfloat16()
+    room = torch.full((M + 2, N), 5.0, dtype=out_dtype, device="cuda:0")
+    err = o.new_error_record("cuda:0")
+    o.gemm_tc(x, w, room[1:M + 1], err=err)
+    o.raise_if_error(err)
+    ref = x.double() @ w.double().T
+    # 192 exact products summed in 32 bit; a bfloat16 result is rounded once more
+    bound = 192 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + (2.0 ** -8 * ref.abs() if out_dtype == torch.bfloat16 else 0)
+    assert bool(((room[1:M + 1].double() - ref).abs() <= bound).all()) and bool((room[0] == 5).all()) and bool((room[M + 1] == 5).all())
