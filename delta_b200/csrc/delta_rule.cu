@@ -26,7 +26,8 @@
 // No exponent is ever positive.  Sums of log decays are kept as two floats, so that a difference of two of them is as good
 // when the sums themselves are large.
 #include "common.cuh"
-#include "mma_helpers.cuh"
+#include "tcgen05_helpers.cuh"
+#include "ring.cuh"
 
 namespace {
 
@@ -384,18 +385,21 @@ delta_chunk_kernel(const T* __restrict__ qkv, int stride, int k_off, int v_off, 
 // shared memory, of which a sixteen-byte load takes four cycles whatever its lanes share: with 32 columns a thread has sums of 8 x 8 and
 // 8 x 4 (per FMA two thirds of the loads that 8 x 4 and 4 x 4 sums take), and a chunk's common matrices are read by half as many blocks.
 // Slices of 32 where slices of 16 are more than the SMs (one block an SM, so a row's last slices would wait for another row's): 256 slices
-// of 16 take 210 us, 128 of 32 take 170 (178 with the keys' size a variable); 128 of 16, all at once, are the shorter chain.
+// of 16 take 210 us, 128 of 32 take 165 (178 with the keys' size a variable; 170 while 256 threads fetched by cp.async what three bulk copies
+// bring now); 128 of 16, all at once, are the shorter chain.
 template <int STAGES, int COLS, int DK>
 __global__ void __launch_bounds__(WALK_THREADS, 1)
 delta_walk_kernel(const float* __restrict__ work, float* __restrict__ state, float* __restrict__ out, const int* __restrict__ row_slot,
                   const int* __restrict__ row_q_start, const int* __restrict__ row_q_len, const int* __restrict__ chunk_base, int H,
-                  int dk_, int dv) {
+                  int dk_, int dv, int* __restrict__ err) {
   const int dk = DK ? DK : dk_;
   constexpr int LD = COLS + 4, JT = COLS / 4, SLICES = COLS / WALK_COLS, CT = SLICES;
   constexpr int RI = COLS / 4;            // channels of the state of a thread
   constexpr int RO = COLS / 16;           // output rows of a thread
   constexpr int HALF = WALK_THREADS / 2;
   extern __shared__ __align__(16) float sm[];
+  __shared__ __align__(8) unsigned long long bars[STAGES];
+  __shared__ int failed;
   const int row = blockIdx.y / H, h = blockIdx.y % H, j0 = blockIdx.x * COLS, n_new = row_q_len[row];
   if (n_new <= 0) return;
   const ChunkLayout at(dk, dv);
@@ -408,16 +412,26 @@ delta_walk_kernel(const float* __restrict__ work, float* __restrict__ state, flo
   float* O = part + SHARES * 2 * C * LD;      // [C][LD]
   const int chunks = (n_new + C - 1) / C;
   const float* ws0 = work + ((size_t)chunk_base[row] * H + h) * at.size;
+  const uint32_t full0 = s2u(&bars[0]);
+  volatile int* gave_up = &failed;
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) mbar_init(full0 + 8 * s, 1);
+    failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  fence_async_smem();
+  __syncthreads();
+  // A chunk's matrices lie as the products want them: one piece, and one for each slice's U.
   auto fetch = [&](int c) {
+    if (tid != 0) return;
     const float* ws = ws0 + (size_t)c * H * at.size;
     float* X = stages + (STAGES == 2 ? (c & 1) : 0) * stage_floats;
-    for (int idx = tid; idx < at.common / 4; idx += WALK_THREADS) cp_async_16(smem_u32(X + idx * 4), ws + idx * 4, true);
-    const float* u = ws + at.u + (size_t)blockIdx.x * SLICES * C * WALK_LD;
+    const uint32_t bar = full0 + 8 * ring_slot(c, STAGES);
+    mbar_expect_tx(bar, (uint32_t)(at.common + SLICES * C * WALK_LD) * 4);
+    bulk_load(s2u(X), ws, (uint32_t)at.common * 4, bar);
 #pragma unroll
     for (int s = 0; s < SLICES; ++s)
-      for (int idx = tid; idx < C * WALK_LD / 4; idx += WALK_THREADS)
-        cp_async_16(smem_u32(X + at.common + s * WALK_U + idx * 4), u + s * C * WALK_LD + idx * 4, true);
-    cp_async_commit();
+      bulk_load(s2u(X + at.common + s * WALK_U), ws + at.u + (size_t)(blockIdx.x * SLICES + s) * C * WALK_LD, C * WALK_LD * 4, bar);
   };
   auto u_at = [](float* U, int t, int j) { return reinterpret_cast<float4*>(U + j / WALK_COLS * WALK_U + t * WALK_LD + j % WALK_COLS); };
   fetch(0);
@@ -428,8 +442,11 @@ delta_walk_kernel(const float* __restrict__ work, float* __restrict__ state, flo
   }
   const int share = tid >> 5, ti = (tid & 31) >> 2, tj = tid & 3;
   for (int c = 0; c < chunks; ++c) {
-    cp_async_wait<0>();
-    __syncthreads();      // the chunk is in; everybody has left the one before
+    // the chunk is in (a wait that gives up lets the rest run through, on whatever is there); everybody has left the one before, and what it wrote
+    // into its stage comes before what is fetched there
+    if (*gave_up == 0 && !mbar_wait(full0 + 8 * ring_slot(c, STAGES), ring_parity(c, STAGES))) *gave_up = 1;
+    fence_async_smem();
+    __syncthreads();
     if (STAGES == 2 && c + 1 < chunks) fetch(c + 1);
     float* X = stages + (STAGES == 2 ? (c & 1) : 0) * stage_floats;
     const float *Kd = X + at.k, *B = X + at.b, *D = X + at.d;
@@ -544,11 +561,14 @@ delta_walk_kernel(const float* __restrict__ work, float* __restrict__ state, flo
         }
     }
     if (STAGES == 1 && c + 1 < chunks) {
+      fence_async_smem();
       __syncthreads();
       fetch(c + 1);
     }
   }
+  if (tid == 0) ring_drain(chunks, STAGES, [&](int s, uint32_t parity) { return mbar_wait(full0 + 8 * s, parity); });
   __syncthreads();
+  if (failed && tid == 0) dk_report(err, DK_DEV_TIMEOUT, blockIdx.x, blockIdx.y, chunks);
   for (int idx = tid; idx < dk * jn; idx += WALK_THREADS) {
     const int j = idx / dk, i = idx - j * dk;
     st[(size_t)j * dk + i] = S[i * LD + j];
@@ -609,7 +629,7 @@ extern "C" int dk_delta_rule_chunked(const void* qkv, int stride, int k_off, int
                                      int a_stride, const float* A_log, const float* dt_bias, float* state, float* out, float* work,
                                      const int* row_slot, const int* row_q_start, const int* row_q_len, const int* chunk_base, int rows,
                                      int max_chunks, int H, int G, int dk, int dv, float q_scale, float guard, int dtype,
-                                     cudaStream_t stream) {
+                                     int* err, cudaStream_t stream) {
   if (rows == 0 || max_chunks == 0) return 0;
   if (int e = check_sizes("delta_rule_chunked", rows, H, G, dk, dv)) return e;
   DK_REQUIRE(max_chunks > 0 && dk_delta_rule_chunked_supported(dk, dv), "delta_rule_chunked: heads of %d x %d do not fit the shared memory", dk, dv);
@@ -652,7 +672,7 @@ extern "C" int dk_delta_rule_chunked(const void* qkv, int stride, int k_off, int
   const int slices = pad_v(dv) / WALK_COLS;
 #define WALK(ST, COLS, DK)                                                                                                                     \
   delta_walk_kernel<ST, COLS, DK><<<dim3(slices * WALK_COLS / (COLS), rows * H), WALK_THREADS, walk_smem(dk, ST, COLS), stream>>>(work, state, out, \
-                                                                                     row_slot, row_q_start, row_q_len, chunk_base, H, dk, dv)
+                                                                                     row_slot, row_q_start, row_q_len, chunk_base, H, dk, dv, err)
 #define PICK(COLS)                       \
   do {                                   \
     if (dk == 128) WALK(2, COLS, 128);   \

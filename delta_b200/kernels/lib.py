@@ -135,7 +135,7 @@ _SIGNATURES = {
     "dk_delta_rule_chunk": [],
     "dk_delta_rule_chunked_supported": [I, I],
     "dk_delta_rule_chunk_floats": [I, I],
-    "dk_delta_rule_chunked": [P, I, I, I, P, I, P, I, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, F, I, P],
+    "dk_delta_rule_chunked": [P, I, I, I, P, I, P, I, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, F, I, P, P],
     "dk_state_space_max_state": [],
     "dk_state_space": [P, I, P, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "dk_state_space_chunk": [],
@@ -144,7 +144,7 @@ _SIGNATURES = {
     "dk_state_space_mma_chunk": [],
     "dk_state_space_mma_supported": [I, I, I],
     "dk_state_space_mma_floats": [I, I],
-    "dk_state_space_mma": [P, I, P, I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+    "dk_state_space_mma": [P, I, P, I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
     "dk_state_space_chunked": [P, I, P, I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
     "dk_glu_clamped": [P, P, L, I, F, F, F, F, I, P],
     "dk_table_gate": [P, P, P, L, L, I, P, I, I, F, F, I, P, P],

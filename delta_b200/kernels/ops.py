@@ -1140,7 +1140,7 @@ def delta_rule_chunk_floats(dk, dv) -> int:
 
 
 def delta_rule_chunked(qkv, k_off, v_off, b_ptr, b_stride, a, A_log, dt_bias, state, out, work, chunk_base, max_chunks, *, H, G, dk, dv,
-                       q_scale, guard, row_slot, row_q_start, row_q_len):
+                       q_scale, guard, row_slot, row_q_start, row_q_len, err=None):
     """``delta_rule`` for long portions (two kernels: every chunk alone, then the states along each row).  ``chunk_base`` [rows] int32:
     the chunks of all rows before each row; ``max_chunks``: the most chunks of a row; ``work`` float32 with
     (all chunks) * H * ``delta_rule_chunk_floats`` entries."""
@@ -1151,7 +1151,7 @@ def delta_rule_chunked(qkv, k_off, v_off, b_ptr, b_stride, a, A_log, dt_bias, st
         _ptr(dt_bias, "dt_bias", f32), _ptr(state, "state", f32), _ptr(out, "out", f32), _ptr(work, "work", f32),
         _ptr(row_slot, "row_slot", i32), _ptr(row_q_start, "row_q_start", i32), _ptr(row_q_len, "row_q_len", i32),
         _ptr(chunk_base, "chunk_base", i32), row_slot.shape[0], int(max_chunks), H, G, dk, dv, float(q_scale), float(guard),
-        dtype_code(qkv.dtype), _stream()), "delta_rule_chunked", 2)
+        dtype_code(qkv.dtype), _ptr(err, "err", i32), _stream()), "delta_rule_chunked", 2)
     return out
 
 
@@ -1214,7 +1214,7 @@ def state_space_mma_floats(H, G) -> int:
 
 
 def state_space_mma(xbc, dt_ptr, dt_stride, A_log, dt_bias, D, state, out, work, chunk_base, total_chunks, max_chunks, *, H, G, N, P,
-                        row_slot, row_q_start, row_q_len):
+                        row_slot, row_q_start, row_q_len, err=None):
     """``state_space_chunked`` for bfloat16 portions on the tensor cores, in chunks of ``state_space_mma_chunk`` tokens; ``work`` float32 with
     total_chunks * ``state_space_mma_floats`` entries."""
     if xbc.dtype != torch.bfloat16:
@@ -1224,8 +1224,8 @@ def state_space_mma(xbc, dt_ptr, dt_stride, A_log, dt_bias, D, state, out, work,
     _l.check(_l.load().dk_state_space_mma(
         _ptr(xbc, "xbc"), xbc.shape[1], dt_ptr, int(dt_stride), _ptr(A_log, "A_log", f32), _ptr(dt_bias, "dt_bias", f32), _ptr(D, "D", f32),
         _ptr(state, "state", f32), _ptr(out, "out", f32), _ptr(work, "work", f32), _ptr(row_slot, "row_slot", i32),
-        _ptr(row_q_start, "row_q_start", i32), _ptr(row_q_len, "row_q_len", i32), _ptr(chunk_base, "chunk_base", i32), row_slot.shape[0],
-        int(total_chunks), int(max_chunks), H, G, N, P, _stream()), "state_space_mma", 2)
+        _ptr(row_q_start, "row_q_start", i32), _ptr(row_q_len, "row_q_len", i32), _ptr(chunk_base, "chunk_base", i32), xbc.shape[0],
+        row_slot.shape[0], int(total_chunks), int(max_chunks), H, G, N, P, _ptr(err, "err", i32), _stream()), "state_space_mma", 3)
     return out
 
 

@@ -99,7 +99,7 @@ class ChannelDelta(Mixer):
             per = H * ops.delta_rule_chunk_floats(dk, dv)
             bound = (-(-ctx.max_step_tokens // ops.delta_rule_chunk()) + ctx.max_rows) * per
             work = ctx.scratch("channel_delta.chunks", (total * per,), torch.float32, bound=(bound,))
-            ops.delta_rule_chunked(*args, work, base, most, **sizes, **rows)
+            ops.delta_rule_chunked(*args, work, base, most, err=ctx.err, **sizes, **rows)
         else:
             if ctx.decode_only:
                 rows["row_q_len"] = None

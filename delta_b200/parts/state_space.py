@@ -86,7 +86,7 @@ class StateSpace(Mixer):
             per = ops.state_space_mma_floats(H, G)
             bound = (-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per
             work = ctx.scratch("state_space.chunks", (total * per,), torch.float32, bound=(bound,))
-            ops.state_space_mma(*args, work, base, total, most, **sizes, **rows)
+            ops.state_space_mma(*args, work, base, total, most, err=ctx.err, **sizes, **rows)
         elif portions and ops.state_space_chunked_supported(N, P, x.dtype):
             base, total, most = chunk_layout(ctx, ops.state_space_chunk())
             per = ops.state_space_chunk_floats(H, G)

@@ -240,6 +240,30 @@ def test_state_space_mma_loses_no_part_of_its_operands(H, G, N, P, decays):
     assert (out.double() - y.view(n, H * P)).norm() < 3e-7 * y.norm() and (st[0].double() - S).norm() < 3e-7 * S.norm()
 
 
+@pytest.mark.parametrize("n", [1, 63, 65, 130])
+@pytest.mark.parametrize("H, G, N, P", [(4, 2, 128, 64), (3, 1, 64, 32)])
+def test_state_space_mma_the_next_rows_tokens_stay_out(H, G, N, P, n):
+    """What lies behind a row's last token is another request's: not a number there leaves the row's outputs and state as they are."""
+    from test_gpu_tiles import ssd_inputs
+    o = ops()
+    xbc, dtraw, A_log, dt_bias, D, state = (t.to(DEV) for t in ssd_inputs(H, G, N, P, [n, 70], [0, 1], 5, "mixed"))
+
+    def run(xbc, dtraw):
+        st, out = state.clone(), torch.zeros(n + 70, H * P, device=DEV)
+        counts = [-(-n // o.state_space_mma_chunk()), 2]
+        work = torch.empty(sum(counts) * o.state_space_mma_floats(H, G), device=DEV)
+        err = o.new_error_record(DEV)
+        o.state_space_mma(xbc, dtraw.data_ptr(), H + 3, A_log, dt_bias, D, st, out, work, i32([0, counts[0]]), sum(counts), max(counts), H=H, G=G, N=N, P=P,
+                          row_slot=i32([0, 1]), row_q_start=i32([0, n]), row_q_len=i32([n, 70]), err=err)
+        o.raise_if_error(err)
+        return out[:n], st[0]
+    out, st = run(xbc, dtraw)
+    xbc, dtraw = xbc.clone(), dtraw.clone()
+    xbc[n:], dtraw[n:] = math.nan, math.nan
+    got, got_st = run(xbc, dtraw)
+    assert torch.equal(got, out) and torch.equal(got_st, st) and bool(torch.isfinite(out).all())
+
+
 @pytest.mark.parametrize("M", [65535 * 32 + 1, 65535 * 64])
 @pytest.mark.parametrize("dtype, K", [(torch.float32, 4), (torch.float32, 3), (torch.bfloat16, 4)])
 def test_gemm_plain_takes_millions_of_rows(M, dtype, K):
