@@ -157,10 +157,11 @@ class ModelRunner:
                 raise ValueError("a row of a step needs at least one token")
             if not self.cache.is_live(r.slot):
                 raise ValueError(f"slot {r.slot} is not live")
-            for w in r.want:
-                if not (0 <= w < n):
+            if len(r.want):
+                if not (0 <= min(r.want) and max(r.want) < n):
+                    w = next(w for w in r.want if not 0 <= w < n)
                     raise ValueError(f"wanted place {w} lies outside the row's {n} tokens")
-                wants.append(off + w)
+                wants += [off + w for w in r.want]
             q_start.append(off)
             off += n
             end = r.start_pos + n
@@ -191,12 +192,11 @@ class ModelRunner:
         if wants:
             temp, top_p, pos, seed = [], [], [], []
             for r in rows:
-                sp = r.sampling
-                for w in r.want:
-                    temp.append(sp.temperature if sp else 0.0)
-                    top_p.append(sp.top_p if sp else 1.0)
-                    seed.append((sp.seed if sp else 0) & 0xFFFFFFFFFFFFFFFF)
-                    pos.append(r.start_pos + w + 1)     # the position the new token will take
+                sp, k, first = r.sampling, len(r.want), r.start_pos + 1
+                temp += [sp.temperature if sp else 0.0] * k
+                top_p += [sp.top_p if sp else 1.0] * k
+                seed += [(sp.seed if sp else 0) & 0xFFFFFFFFFFFFFFFF] * k
+                pos += [first + w for w in r.want]     # the position the new token will take
             put("samp_temp", np.asarray(temp, dtype=np.float32).view(np.int32))
             put("samp_top_p", np.asarray(top_p, dtype=np.float32).view(np.int32))
             put("samp_pos", pos)

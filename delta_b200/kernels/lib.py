@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import threading
 
+from . import native_calls
 from .build import build
 
 _lock = threading.Lock()
@@ -193,6 +194,8 @@ def load():
             fn = getattr(lib, name)
             fn.restype = I
             fn.argtypes = args
+        for name, fn in (native_calls.load(lib, path, _SIGNATURES) or {}).items():
+            setattr(lib, name, fn)
         _lib = lib
     return _lib
 
@@ -201,9 +204,10 @@ def declare(name: str, argtypes: list) -> None:
     """Adds a launcher's signature (used by kernel files that come later)."""
     _SIGNATURES[name] = argtypes
     if _lib is not None:
-        fn = getattr(_lib, name)
+        fn = _lib[name]
         fn.restype = I
         fn.argtypes = argtypes
+        setattr(_lib, name, fn)
 
 
 LAUNCHES = [0]
