@@ -501,7 +501,8 @@ def roletar_workload(args) -> int:
 
 
 # launchers that do the work of another where their sizes allow
-SAME_WORK = {"decay_attention_tiles": "decay_attention_chunked", "state_space_mma": "state_space_chunked", "attention_rows_wide": "attention_rows_mma"}
+SAME_WORK = {"decay_attention_tiles": "decay_attention_chunked", "decay_attention_tc": "decay_attention_chunked", "state_space_mma": "state_space_chunked",
+             "attention_rows_wide": "attention_rows_mma"}
 
 
 def design_workload(args, design: str) -> int:

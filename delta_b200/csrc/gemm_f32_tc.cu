@@ -96,12 +96,6 @@ struct Sizes {
   static_assert(2 * D_COLS + 2 * A_COLS <= TMEM_COLS, "two accumulators beside two chunks of W");
 };
 
-__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, float* v) {
-  uint32_t* r = reinterpret_cast<uint32_t*>(v);
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
-}
-
 struct F32Args {
   const float* A;
   const float* W;

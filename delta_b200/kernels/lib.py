@@ -116,6 +116,9 @@ _SIGNATURES = {
     "dk_decay_attention_tiles_supported": [I, I, I, I, I, I],
     "dk_decay_attention_tiles_floats": [I, I],
     "dk_decay_attention_tiles": [P, I, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+    "dk_decay_attention_tc_chunk": [],
+    "dk_decay_attention_tc_supported": [I, I, I, I, I, I],
+    "dk_decay_attention_tc": [P, I, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, P, P],
     "dk_decay_attention_chunked": [P, I, I, I, I, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "dk_decay_attention_step_supported": [I, I],
     "dk_decay_attention_step": [P, I, I, I, I, I, P, P, P, P, P, I, I, I, I, I, P],

@@ -947,6 +947,29 @@ def decay_attention_tiles(src, q_off, k_off, v_off, decays, state, out, work, ch
     return out
 
 
+def decay_attention_tc_chunk() -> int:
+    return int(_l.load().dk_decay_attention_tc_chunk())
+
+
+def decay_attention_tc_supported(dk, dv, stride, q_off, k_off, v_off, dtype) -> bool:
+    return dtype == torch.bfloat16 and bool(_l.load().dk_decay_attention_tc_supported(int(dk), int(dv), int(stride), int(q_off), int(k_off), int(v_off)))
+
+
+def decay_attention_tc(src, q_off, k_off, v_off, decays, state, out, work, chunk_base, max_chunks, *, H, dk, dv, row_slot, row_q_start, row_q_len,
+                       silu=True, err=None):
+    """``decay_attention_chunked`` for bfloat16 heads of 128 x 128 on the tcgen05 tensor cores, in chunks of ``decay_attention_tc_chunk`` tokens;
+    ``work`` float32 with room for (all chunks) x H x dk x dv."""
+    if tuple(state.shape[1:]) != (H, dk, dv) or not decay_attention_tc_supported(dk, dv, src.shape[1], q_off, k_off, v_off, src.dtype):
+        raise KernelError(f"decay_attention_tc: rows {tuple(src.shape)} of {src.dtype} and a state {tuple(state.shape)} are not taken")
+    i32 = torch.int32
+    _l.check(_l.load().dk_decay_attention_tc(
+        _ptr(src, "src"), src.shape[1], int(q_off), int(k_off), int(v_off), int(bool(silu)), _ptr(decays, "decays", torch.float64),
+        _ptr(state, "state", torch.float32), _ptr(out, "out", torch.float32), _ptr(work, "work", torch.float32),
+        _ptr(row_slot, "row_slot", i32), _ptr(row_q_start, "row_q_start", i32), _ptr(row_q_len, "row_q_len", i32),
+        _ptr(chunk_base, "chunk_base", i32), row_slot.shape[0], int(max_chunks), H, _ptr(err, "err", i32), _stream()), "decay_attention_tc", 3)
+    return out
+
+
 def gated_rms_norm(o, gate_ptr, gate_stride, weight, out, eps, group=None, gate_first=False, gate_dtype=None):
     """out = o / sqrt(mean(o^2) + eps) * weight * sigmoid(gate) per token; ``o`` float32 [T, n]; the gate's n values of a token
     lie at ``gate_ptr`` + t * ``gate_stride`` elements of the type of ``out``.  ``group``: the mean is taken over every ``group``

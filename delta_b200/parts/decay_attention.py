@@ -67,8 +67,17 @@ class DecayAttention(Mixer):
         rows = dict(row_slot=ctx.row_slot, row_q_start=ctx.row_q_start, row_q_len=ctx.row_q_len)
         portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
         # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
-        chunk = ops.decay_attention_tiles_chunk()
-        if (portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk)
+        chunk, long = ops.decay_attention_tiles_chunk(), ops.decay_attention_tc_chunk()
+        # heads of 128 x 128 in bfloat16 go to the tensor cores whatever their number: 8 heads of 65 / 400 / 2,048 tokens 42 / 42 / 50 us, by FMA in
+        # chunks of 32 40 / 50 / 138 and of 64 48 / 52 / 85; 32 heads of 130 / 700 / 2,048 tokens 44 / 77 / 177 against 73 / 175 / 515 and 50 / 118 / 310
+        if portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype):
+            base, total, most = chunk_layout(ctx, long)
+            per = H * dk * dv
+            work = ctx.scratch("decay_attention.long_chunks", (total * per,), torch.float32,
+                               bound=((-(-ctx.max_step_tokens // long) + ctx.max_rows) * per,))
+            ops.decay_attention_tc(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, most, H=H, dk=dk, dv=dv, silu=True,
+                                   err=ctx.err, **rows)
+        elif (portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk)
                 and tiles_pay(ctx.host["q_lens"], chunk, H, ctx.sm_count)):
             base, total, most = chunk_layout(ctx, chunk)
             per = H * ops.decay_attention_tiles_floats(dk, dv)

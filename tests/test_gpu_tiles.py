@@ -351,3 +351,57 @@ def test_delta_walk_slices(H, dk, dv):
     for x, y, z in zip(*results):
         assert torch.equal(x, y)
         assert (x - z).abs().max() <= 2e-5 * z.abs().max()      # each of the two kernels' own tests allows 1e-5
+
+
+def decay_tc(o, src, state, decays, rows, lens, H):
+    counts = [-(-n // o.decay_attention_tc_chunk()) for n in lens]
+    base = torch.tensor([sum(counts[:i]) for i in range(len(counts))], dtype=torch.int32, device=DEV)
+    work = torch.full((sum(counts) * H * 128 * 128,), float("nan"), device=DEV)
+    out = torch.full((sum(lens) + 1, H * 128), 7.0, device=DEV)
+    err = o.new_error_record(DEV)
+    o.decay_attention_tc(src, 0, H * 128, 2 * H * 128, decays, state, out, work, base, max(counts), H=H, dk=128, dv=128, err=err, **rows)
+    o.raise_if_error(err)
+    assert bool((out[-1] == 7.0).all())
+    return out[:-1]
+
+
+@pytest.mark.parametrize("decays", [[0.999, 0.02, 0.7], [0.9995, 0.97, 0.99]])
+def test_decay_attention_tc(decays):
+    """Chunks of 128: rows of one token, beside a chunk's end on either side, of more chunks than the scan has under way; a slot of no row."""
+    o = ops()
+    H, lens, slots = 3, [1, 127, 128, 129, 700], [2, 0, 4, 1, 5]
+    src, state, dec, rows = decay_case(lens, slots, H, 128, 128, torch.bfloat16, decays, 3)
+    st = state.clone()
+    assert o.decay_attention_tc_supported(128, 128, src.shape[1], 0, H * 128, 2 * H * 128, src.dtype)
+    out = decay_tc(o, src, st, dec, rows, lens, H)
+    at = 0
+    for r, n in enumerate(lens):
+        y, S = decay_reference(src[at:at + n], state[slots[r]].double(), dec, H, 128, 128)
+        # three activations of 2^-23 at most each, and sums of 128 terms that are cut off at eight places
+        assert (out[at:at + n].double() - y.reshape(n, -1)).norm() < 5e-7 * y.norm(), r
+        assert (st[slots[r]].double() - S).norm() < 5e-7 * S.norm(), r
+        at += n
+    assert torch.equal(st[3], state[3]) and torch.equal(st[6], state[6])
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "state", "small"])
+def test_decay_attention_tc_numbers_out_of_the_parts_reach(what):
+    """Infinite entries, and rows of very small ones: the chunk that holds them is summed by FMA, and nothing before an infinite token sees it."""
+    o = ops()
+    H, lens, slots = 2, [300], [1]
+    src, state, dec, rows = decay_case(lens, slots, H, 128, 128, torch.bfloat16, [0.99, 0.9], 4)
+    if what == "state":
+        state[1, 0, 3, 5] = float("inf")
+    elif what == "small":
+        src[140, :256] = 1e-35
+    else:
+        src[140, {"q": 0, "k": 256, "v": 512}[what] + 7] = float("inf")
+    st, ref = state.clone(), state.clone()
+    out = decay_tc(o, src, st, dec, rows, lens, H)
+    want = decay_tiles(o, src, ref, dec, rows, lens, H, 128, 128)
+    assert torch.equal(out[:140].isfinite(), want[:140].isfinite())
+    if what in "qkv":
+        assert bool(out[:140].isfinite().all()) and not bool(out[140].isfinite().all()) and bool(out[140:, 128:].isfinite().all())
+    for a, b in ((out, want), (st, ref)):
+        both = a.isfinite() & b.isfinite()
+        assert (a[both] - b[both]).norm() < 1e-6 * b[both].norm()
