@@ -27,16 +27,7 @@ constexpr int BOX = TC * 128, PART = 2 * BOX;      // bytes: 128 rows of 64 entr
 constexpr int TURN_LD = 36;
 constexpr int TMEM_COLS = 512, COL_A = 0, COL_D = 192;      // the first operand's parts, and two accumulators; or four accumulators
 
-// z / (1 + e^-z).  The reciprocal of a quarter of 1 + e^-z (which is finite whenever e^-z is) by an estimate and one step of Newton's iteration: rounded
-// to nearest but for the last unit, without the branches of a division, behind which a warp's next entries wait (with one, 55 cycles of a
-// scheduler an entry and a third of the kernel's time).
-__device__ __forceinline__ float silu(float z) {
-  const float e = expf(-z), d = fmaf(0.25f, e, 0.25f);
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  r = fmaf(r, fmaf(-d, r, 1.f), r);
-  return e == INFINITY ? z * 0.f : 0.25f * z * r;
-}
+__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
 
 // x^n for n up to TC, by squaring: 64 bit, off by less than 2^-45 of it before it is rounded to 32.
 __device__ __forceinline__ float power(double x, int n) {
