@@ -62,32 +62,52 @@ __global__ void conv_state_kernel(const T* __restrict__ xin, int in_stride, floa
     if (j < taps - 1) st[(size_t)j * C + c] = v[j];
 }
 
-// The same for 2 to 4 taps, C a multiple of 8 and 16-byte aligned rows: a thread takes eight channels of CONV_TOKENS tokens that
-// follow one another and keeps the window of inputs in registers, so every input is read once per tile.  Bound by latency: the tile's
-// inputs, taps and rows are all asked for before the first product.  2,048 tokens of 6,144 channels,
-// bfloat16, four taps: 53 -> 27 us (50 MB).
-// grid (ceil(tokens / CONV_TOKENS), ceil(C / 8 / blockDim))
-constexpr int CONV_TOKENS = 8;
+// The same for 2 to 4 taps, C a multiple of 8 and 16-byte aligned rows: a thread takes four channels of CONV_TOKENS tokens that
+// follow one another and keeps the window of inputs in registers, so every input is read once per tile.  Bound by instructions: the tile's
+// inputs, taps and rows are all asked for before the first product, and four channels a thread leave room for 32 warps an SM to issue them (eight, as it
+// was: 122 registers, 16 warps that had nothing to issue in half of the cycles).  2,048 tokens of 6,144 channels, bfloat16, four taps: 27.5 -> 20.2 us, 2,048 of 4,352 24.5 -> 16.7 (50 and 36 MB).
+// grid (ceil(tokens / CONV_TOKENS), ceil(C / 4 / blockDim))
+constexpr int CONV_TOKENS = 8, CONV_CHANNELS = 4;
 
-// Eight neighbouring entries as they lie in memory.
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
+  const uint2 a = *reinterpret_cast<const uint2*>(p);
+  v[0] = __uint_as_float(a.x << 16); v[1] = __uint_as_float(a.x & 0xffff0000u);
+  v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xffff0000u);
+}
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+// Four neighbouring entries as they lie in memory.
 template <typename T>
-struct Eight {
-  uint4 v[sizeof(T) / 2];
+struct Four {
+  uint2 v[sizeof(T) / 2];
   __device__ __forceinline__ void get(const T* p) {
-#pragma unroll
-    for (int i = 0; i < (int)sizeof(T) / 2; ++i) v[i] = reinterpret_cast<const uint4*>(p)[i];
+    if constexpr (sizeof(T) == 4) {
+      const uint4 a = *reinterpret_cast<const uint4*>(p);
+      v[0] = make_uint2(a.x, a.y);
+      v[1] = make_uint2(a.z, a.w);
+    } else {
+      v[0] = *reinterpret_cast<const uint2*>(p);
+    }
   }
-  __device__ __forceinline__ void floats(float (&x)[8]) const { load8<T>(reinterpret_cast<const T*>(v), x); }
+  __device__ __forceinline__ void floats(float (&x)[4]) const { load4(reinterpret_cast<const T*>(v), x); }
 };
 
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) conv_silu_vec_kernel(const T* __restrict__ xin, int in_stride, const float* __restrict__ w, const float* __restrict__ bias,
                                      const float* __restrict__ conv_state, T* __restrict__ out, const int* __restrict__ tok_row,
                                      const int* __restrict__ row_slot, const int* __restrict__ row_q_start, int tokens, int C, int act) {
-  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  constexpr int E = CONV_CHANNELS;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * E;
   if (c >= C) return;
   const int t_from = blockIdx.x * CONV_TOKENS, n = min(CONV_TOKENS, tokens - t_from);
-  Eight<T> raw[CONV_TOKENS];
+  Four<T> raw[CONV_TOKENS];
   int rows[CONV_TOKENS];
 #pragma unroll
   for (int i = 0; i < CONV_TOKENS; ++i) {
@@ -95,14 +115,14 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(const T* __restrict_
     raw[i].get(xin + (size_t)t * in_stride + c);
     rows[i] = tok_row[t];
   }
-  float wv[8 * TAPS], b[8], win[TAPS - 1][8];      // wv[e TAPS + j]: a channel's taps side by side, as they lie
+  float wv[E * TAPS], b[E], win[TAPS - 1][E];      // wv[e TAPS + j]: a channel's taps side by side, as they lie
 #pragma unroll
-  for (int e = 0; e < 2 * TAPS; ++e) *reinterpret_cast<float4*>(wv + 4 * e) = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + 4 * e);
+  for (int e = 0; e < TAPS; ++e) *reinterpret_cast<float4*>(wv + 4 * e) = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + 4 * e);
   if (bias != nullptr) {
-    load8<float>(bias + c, b);
+    load4(bias + c, b);
   } else {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) b[e] = 0.f;
+    for (int e = 0; e < E; ++e) b[e] = 0.f;
   }
   int row = -1;
 #pragma unroll
@@ -115,14 +135,14 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(const T* __restrict_
 #pragma unroll
       for (int j = 0; j < TAPS - 1; ++j) {
         const int k = t_from + i - q0 - (TAPS - 1) + j;
-        if (k >= 0) load8<T>(xin + (size_t)(q0 + k) * in_stride + c, win[j]);
-        else load8<float>(st + (size_t)(TAPS - 1 + k) * C + c, win[j]);
+        if (k >= 0) load4(xin + (size_t)(q0 + k) * in_stride + c, win[j]);
+        else load4(st + (size_t)(TAPS - 1 + k) * C + c, win[j]);
       }
     }
-    float x[8], o[8];
+    float x[E], o[E];
     raw[i].floats(x);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < E; ++e) {
       float acc = b[e];
 #pragma unroll
       for (int j = 0; j < TAPS - 1; ++j) acc = fmaf(wv[e * TAPS + j], win[j][e], acc);
@@ -132,7 +152,7 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(const T* __restrict_
       for (int j = 0; j + 1 < TAPS - 1; ++j) win[j][e] = win[j + 1][e];
       win[TAPS - 2][e] = x[e];
     }
-    store8<T>(out + (size_t)(t_from + i) * C + c, o);
+    store4(out + (size_t)(t_from + i) * C + c, o);
   }
 }
 
@@ -336,7 +356,7 @@ extern "C" int dk_conv_silu(const void* xin, int in_stride, const float* w, cons
   }
   if (taps >= 2 && taps <= 4 && in_bias == nullptr && C % 8 == 0 && in_stride % 8 == 0 && ((uintptr_t)xin % 16) == 0 && ((uintptr_t)out % 16) == 0 &&
       (((uintptr_t)conv_state | (uintptr_t)w | (uintptr_t)bias) % 16) == 0) {
-    const dim3 gv((T_ + CONV_TOKENS - 1) / CONV_TOKENS, (C / 8 + 127) / 128);
+    const dim3 gv((T_ + CONV_TOKENS - 1) / CONV_TOKENS, (C / CONV_CHANNELS + 127) / 128);
 #define VEC(T, TAPS)                                                                                                              \
   conv_silu_vec_kernel<T, TAPS><<<gv, 128, 0, stream>>>((const T*)xin, in_stride, w, bias, conv_state, (T*)out, tok_row, row_slot, row_q_start, \
                                                         T_, C, act)
