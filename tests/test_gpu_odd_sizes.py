@@ -48,3 +48,24 @@ def test_odd_sizes(tmp_path, name, dtype):
     steps, ends = helpers.mixed(lengths, [n // 2 for n in lengths], seed=8)
     res = helpers.run_schedule(r, toks, steps, ends)
     compare(res, refs, lengths, dtype, f"{name}: mixed")
+
+
+@pytest.mark.parametrize("group, groups", [(8, 1), (8, 40), (120, 3), (128, 1), (128, 17), (136, 3), (256, 5)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gate_first", [False, True])
+def test_gated_norm_of_groups_by_half_a_warp(group, groups, dtype, gate_first):
+    """Groups up to and beside 128 entries, odd numbers of them (half of a warp has none in the last round), more than a block takes at once."""
+    from delta_b200.kernels import ops as o
+    g = torch.Generator(device="cuda:0").manual_seed(group + groups)
+    n, T = group * groups, 5
+    x, w = torch.randn(T, n, device="cuda:0", generator=g), torch.rand(n, device="cuda:0", generator=g) + 0.5
+    gate = torch.randn(T, n, device="cuda:0", generator=g).to(dtype)
+    out = torch.full((T, n), 9.0, dtype=dtype, device="cuda:0")
+    o.gated_rms_norm(x, gate.data_ptr(), n, w, out, 1e-5, group=group, gate_first=gate_first, gate_dtype=dtype)
+    z, y = gate.double(), x.double()
+    if gate_first:
+        y = y * torch.nn.functional.silu(z)
+    y = y.view(T, groups, group)
+    want = (y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)).view(T, n) * w.double() * (1.0 if gate_first else torch.sigmoid(z))
+    # a handful of 32-bit roundings and a mean of up to 256 squares; bfloat16 rounds once more
+    assert bool(((out.double() - want).abs() <= (2.0 ** -19 + (2.0 ** -8 if dtype == torch.bfloat16 else 0)) * want.abs() + 1e-30).all())
