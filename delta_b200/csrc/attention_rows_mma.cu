@@ -17,12 +17,16 @@
 #include "common.cuh"
 #include "row_attention_params.h"
 #include "mma_helpers.cuh"
+#include "tcgen05_helpers.cuh"
+#include "ring.cuh"
 
 namespace {
 constexpr int PSTAGES = 2;
 constexpr float LOG2E = 1.4426950408889634f;
 
 __host__ __device__ inline int pad128(int bytes) { return (bytes + 127) / 128 * 128; }
+// Rows that bulk copies leave as they lie: an odd number of 16-byte pieces apart, so that eight neighbouring rows' pieces meet no bank twice.
+__host__ __device__ inline int odd_pieces(int bytes) { return (bytes / 16 | 1) * 16; }
 
 // tanh(t) = 1 - 2 / (1 + e^(2t)) through the exponential and reciprocal units, without a branch: exact at both ends (e^(2t) of 0
 // or infinity), absolute error about 3e-7 elsewhere, which a score made of bfloat16 queries and keys does not see.
@@ -38,8 +42,9 @@ __device__ __forceinline__ float tanh_by_exp(float t) {
 // SHAPED: scores are capped and take biases by distance (an instance of its own, so that the others keep their registers).
 // KW > 1 (with one warp and one tile of query rows): that many warps take the key tiles in turn, each with stages, sums and a maximum of its own, and
 // are merged in shared memory at the end.  For single tokens with wide rows, whose tiles leave an SM room for four warps: more of them
-// per block mean fewer splits to merge.  8 tokens, 16 heads, keys of 320, values of 256, 2,048 keys:
-// 19 -> 13 us, the merge behind it 5.9 -> 4.4.
+// per block mean fewer splits to merge.  Rows come by bulk copies, a lane a key: a tile of 32 is 20 KB, whose 16-byte copies took four warps 8,400 of
+// the kernel's 21,600 cycles to ask for.  8 tokens, 16 heads, keys of 320, values of 256, 2,048 keys:
+// 19 -> 13 -> 9.4 us, the merge behind it 5.9 -> 4.4.
 template <int WARPS, int KT, int DVMAX, int RM, bool SHAPED, int KW>
 __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(const DkRowAttnParams p, float* __restrict__ part) {
   static_assert(KW == 1 || (WARPS == 1 && RM == 1), "key tiles are shared out over warps for one tile of query rows");
@@ -55,7 +60,11 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
   const int tid = threadIdx.x, warp = KW > 1 ? 0 : tid >> 5, kw = KW > 1 ? tid >> 5 : 0, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int dk = p.dk, dv = p.dv, ps = p.ps;
   const int KB = dk / 16;
-  const int ROWS = pad128(p.row_width * 2), QS = pad128(dk * 2);   // bytes between rows of a key tile / of the query tile
+  constexpr bool BULK = KW > 1;
+  const int ROWS = BULK ? odd_pieces(p.row_width * 2) : pad128(p.row_width * 2), QS = BULK ? odd_pieces(dk * 2) : pad128(dk * 2);   // bytes between rows of a key tile / of the query tile
+  const auto place = [](int piece, int r) { return (BULK ? piece : piece ^ (r & 7)) * 16; };      // of a row's 16-byte piece
+  __shared__ __align__(8) unsigned long long bars[BULK ? KW * PSTAGES + 1 : 1];      // BULK: a warp's stages are in; the queries are
+  const uint32_t stage_bar = s2u(&bars[0]) + kw * PSTAGES * 8, query_bar = s2u(&bars[0]) + KW * PSTAGES * 8;
   const int CPR = p.row_width / 8;                                  // 16-byte chunks of a cached row
   unsigned char* q_smem = smem;
   unsigned char* kv_smem = smem + QT * QS + (size_t)kw * PSTAGES * KT * ROWS;
@@ -71,6 +80,21 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
   const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(p.q);
 
   // the tile's query rows into shared memory
+  if constexpr (BULK) {
+    if (tid == 0) {
+      for (int i = 0; i < KW * PSTAGES + 1; ++i) mbar_init(s2u(&bars[i]), 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (kw == 0) {
+      if (lane == 0) mbar_expect_tx(query_bar, (uint32_t)(QT * dk * 2));
+      __syncwarp();
+      if (lane < QT) {
+        const int m = m0 + min(lane, nrows - 1);
+        bulk_load(s2u(q_smem + lane * QS), q + (size_t)(q_start + m / G) * p.q_stride + (size_t)(g * G + m % G) * p.q_head_stride, (uint32_t)(dk * 2), query_bar);
+      }
+    }
+  } else
   for (int c = tid; c < QT * (dk / 8); c += THREADS) {
     const int r = c / (dk / 8), part_c = c % (dk / 8);
     const int m = m0 + min(r, nrows - 1);
@@ -93,6 +117,17 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
         const int page = lp < p.max_pages ? p.block_table[(size_t)row * p.max_pages + lp] : -1;
         if (page < 0 || page >= p.num_pages) dk_report(p.err, DK_DEV_BAD_PAGE, q_start, lp, page);
         else at = ((page * p.KV + g) << ps_shift) + (key & (ps - 1));
+      }
+      if constexpr (BULK) {      // a row a lane; zeros for keys that are not there
+        const uint32_t there = __ballot_sync(0xffffffffu, at >= 0);
+        unsigned char* trow = dst + lane * ROWS;
+        if (at < 0)
+          for (int c = 0; c < CPR; ++c) *reinterpret_cast<uint4*>(trow + c * 16) = make_uint4(0, 0, 0, 0);
+        fence_async_smem();      // (what was written to the stage comes before what is copied there)
+        if (lane == 0) mbar_expect_tx(stage_bar + 8 * stage, (uint32_t)(__popc(there) * p.row_width * 2));
+        __syncwarp();
+        if (at >= 0) bulk_load(s2u(trow), cache + (size_t)at * p.row_width, (uint32_t)(p.row_width * 2), stage_bar + 8 * stage);
+        continue;
       }
 #pragma unroll 4
       for (int t = warp * tpi; t < 32; t += WARPS * tpi) {
@@ -137,18 +172,21 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
   const int warp_lo = row_first_key(p, warp_first_pos);
   const int kc0 = p.k_off / 8, vc0 = p.v_off / 8;
 
+  bool arrived = true;      // BULK: no wait has given up
   if (kt_a + kw < kt_b) load_tile(kt_a + kw, 0);
-  cp_async_commit();
-  if (KW > 1) {      // everybody's queries
-    cp_async_wait<0>();
-    __syncthreads();
-  }
+  if constexpr (BULK) arrived = mbar_wait(query_bar, 0);
+  else cp_async_commit();
   for (int kt = kt_a + kw; kt < kt_b; kt += KW) {
-    if (kt + KW < kt_b) load_tile(kt + KW, ((kt - kt_a) / KW + 1) % PSTAGES);
-    cp_async_commit();
-    cp_async_wait<1>();
-    if (KW > 1) __syncwarp();
-    else __syncthreads();
+    const int round = (kt - kt_a) / KW;
+    if (kt + KW < kt_b) load_tile(kt + KW, (round + 1) % PSTAGES);
+    if constexpr (BULK) {
+      arrived = arrived && mbar_wait(stage_bar + 8 * ring_slot(round, PSTAGES), ring_parity(round, PSTAGES));
+      __syncwarp();
+    } else {
+      cp_async_commit();
+      cp_async_wait<1>();
+      __syncthreads();
+    }
     const uint32_t kbase = smem_u32(kv_smem + (size_t)(((kt - kt_a) / KW) % PSTAGES) * KT * ROWS);
     const uint32_t qbase = smem_u32(q_smem);
     const int kt0 = kt * KT;
@@ -164,9 +202,9 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
 #pragma unroll
         for (int rm = 0; rm < RM; ++rm) {
           const int r = warp * WR + rm * 16 + (lane & 15);
-          ldmatrix_x4(qa[rm][0], qa[rm][1], qa[rm][2], qa[rm][3], qbase + r * QS + (((2 * kb + (lane >> 4)) ^ (r & 7)) * 16));
+          ldmatrix_x4(qa[rm][0], qa[rm][1], qa[rm][2], qa[rm][3], qbase + r * QS + place(2 * kb + (lane >> 4), r));
           if (kb + 1 < KB)
-            ldmatrix_x4(qb[rm][0], qb[rm][1], qb[rm][2], qb[rm][3], qbase + r * QS + (((2 * kb + 2 + (lane >> 4)) ^ (r & 7)) * 16));
+            ldmatrix_x4(qb[rm][0], qb[rm][1], qb[rm][2], qb[rm][3], qbase + r * QS + place(2 * kb + 2 + (lane >> 4), r));
         }
 #pragma unroll
         for (int j = 0; j < KT / 8; ++j) {
@@ -174,7 +212,7 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
           uint32_t b0, b1, b2, b3;
           // (an odd count of 16-element blocks: the second pair of the last load repeats the first and is not used)
           const int cj = kc0 + 2 * kb + (kb + 1 < KB ? (lane >> 3) : ((lane >> 3) & 1));
-          ldmatrix_x4(b0, b1, b2, b3, kbase + tok * ROWS + ((cj ^ (tok & 7)) * 16));
+          ldmatrix_x4(b0, b1, b2, b3, kbase + tok * ROWS + place(cj, tok));
 #pragma unroll
           for (int rm = 0; rm < RM; ++rm) {
             mma_bf16(s[rm][j], qa[rm], b0, b1);
@@ -265,18 +303,18 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
         }
         const int tok = kb2 * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
 #pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-          if (n * 8 < dv) {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(b0, b1, b2, b3, kbase + tok * ROWS + (((vc0 + n + (lane >> 4)) ^ (tok & 7)) * 16));
+        for (int n = 0; n < NT; n += 4) {      // (four accumulators in turn, so that no MMA waits for the one before it; dv is a multiple of 16)
+          uint32_t b[2][4];
 #pragma unroll
-            for (int rm = 0; rm < RM; ++rm) {
-              mma_bf16(o[rm][n], hi[rm], b0, b1);
-              mma_bf16(o[rm][n + 1], hi[rm], b2, b3);
-              mma_bf16(o[rm][n], lo[rm], b0, b1);
-              mma_bf16(o[rm][n + 1], lo[rm], b2, b3);
-            }
-          }
+          for (int i = 0; i < 2; ++i)
+            if ((n + 2 * i) * 8 < dv) ldmatrix_x4_trans(b[i][0], b[i][1], b[i][2], b[i][3], kbase + tok * ROWS + place(vc0 + n + 2 * i + (lane >> 4), tok));
+#pragma unroll
+          for (int rm = 0; rm < RM; ++rm)
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if ((n + i / 2 * 2) * 8 < dv) mma_bf16(o[rm][n + i], part ? lo[rm] : hi[rm], b[i / 2][i % 2 * 2], b[i / 2][i % 2 * 2 + 1]);
         }
       }
     }
@@ -286,6 +324,12 @@ __global__ void __launch_bounds__(WARPS * KW * 32) attention_rows_mma_kernel(con
   cp_async_wait<0>();
 
   if constexpr (KW > 1) {
+    if (!arrived) {      // its copies may still be under way: it waits for them once more before it goes on with whatever is there
+      if (lane == 0) dk_report(p.err, DK_DEV_TIMEOUT, blockIdx.y, blockIdx.z, kw);
+      const int rounds = kt_b > kt_a + kw ? (kt_b - kt_a - kw + KW - 1) / KW : 0;
+      mbar_wait(query_bar, 0);
+      ring_drain(rounds, PSTAGES, [&](int i, uint32_t parity) { return mbar_wait(stage_bar + 8 * i, parity); });
+    }
     // The warps' sums meet under the largest maximum: each leaves its own, scaled, where its stages were, and everybody adds.
     __shared__ float stat[2][KW][16];
     float* mine = reinterpret_cast<float*>(kv_smem);
@@ -442,7 +486,8 @@ __global__ void attention_rows_merge_kernel(const DkRowAttnParams p, const float
 template <int WARPS, int KT, int DVMAX, int RM, bool SHAPED, int KW = 1>
 int launch_as(const DkRowAttnParams& p, int max_m, int splits, float* part, cudaStream_t stream) {
   const int m_tiles = (max_m + 16 * WARPS * RM - 1) / (16 * WARPS * RM);
-  const size_t smem = (size_t)16 * WARPS * RM * pad128(p.dk * 2) + (size_t)KW * PSTAGES * KT * pad128(p.row_width * 2);
+  const size_t smem = KW > 1 ? (size_t)16 * odd_pieces(p.dk * 2) + (size_t)KW * PSTAGES * KT * odd_pieces(p.row_width * 2)
+                             : (size_t)16 * WARPS * RM * pad128(p.dk * 2) + (size_t)PSTAGES * KT * pad128(p.row_width * 2);
   if (smem > 220 * 1024) {
     dk_set_error("attention_rows_mma: rows of %d elements need more shared memory than a block has", p.row_width);
     return DK_ERR_ARG;
@@ -487,7 +532,7 @@ extern "C" long long dk_attention_rows_mma_scratch_floats(int T, int H, int dv, 
 
 // Warps of a block that share the key tiles (of 32) of a single token's group of up to 16 heads.
 extern "C" int dk_attention_rows_mma_key_warps(int dv, int row_width, int dk) {
-  return dv > 128 && (size_t)16 * pad128(dk * 2) + (size_t)4 * PSTAGES * 32 * pad128(row_width * 2) <= 200 * 1024 ? 4 : 1;
+  return dv > 128 && (size_t)16 * odd_pieces(dk * 2) + (size_t)4 * PSTAGES * 32 * odd_pieces(row_width * 2) <= 200 * 1024 ? 4 : 1;
 }
 
 // max_m: the most query rows (tokens * heads of a group) any batch row brings among those the filter lets through.
