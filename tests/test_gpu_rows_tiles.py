@@ -101,3 +101,45 @@ def test_rows_product_writes_its_columns_and_no_others(M, N, out_dtype):
     # 192 exact products summed in 32 bit; a bfloat16 result is rounded once more
     bound = 192 * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + (2.0 ** -8 * ref.abs() if out_dtype == torch.bfloat16 else 0)
     assert bool(((room[1:M + 1].double() - ref).abs() <= bound).all()) and bool((room[0] == 5).all()) and bool((room[M + 1] == 5).all())
+
+
+@pytest.mark.parametrize("H, dq, dr, R, rot, interleaved", [(16, 128, 64, 256, 64, False), (1, 8, 16, 8, 16, False), (5, 16, 24, 264, 16, True), (3, 64, 32, 512, 16, False),
+                                                            (2, 8, 8, 520, 8, True), (4, 24, 16, 72, 8, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("apart", [False, True])
+def test_latent_prepare_of_eight_entries_at_a_time(H, dq, dr, R, rot, interleaved, dtype, apart):
+    """Latents below, at and above a warp's 256 and 512 entries (above: the general kernel), rotated parts that end inside the part, halves that are no whole
+    number of eight (the general kernel), latents in rows of their own; tokens in pages out of order."""
+    from delta_b200.kernels import ops as o
+    g = torch.Generator().manual_seed(R + dr)
+    T, ps, width = 19, 4, R + dr
+    rows = torch.randn(T, H * (dq + dr) + (0 if apart else width), generator=g).to(dtype).to(DEV)
+    low = torch.randn(T, width + 8, generator=g).to(dtype).to(DEV) if apart else None
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    bt = torch.randperm(5, generator=g).to(torch.int32).view(1, 5).to(DEV)
+    angle = torch.arange(32, dtype=torch.float64)[:, None] * 100.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / rot)
+    table = torch.stack([angle.cos(), angle.sin()], dim=-1).float().contiguous().to(DEV)
+    w = (torch.rand(R, generator=g) + 0.5).to(DEV)
+    cache = torch.full((6, 1, ps, width), 5.0, dtype=dtype, device=DEV)
+    qabs = torch.full((T, H, width), 7.0, dtype=dtype, device=DEV)
+    err = o.new_error_record(DEV)
+    kw = dict(low=low, low_offset=8) if apart else {}
+    o.latent_prepare(rows, pos, torch.zeros(T, dtype=torch.int32, device=DEV), bt, cache, qabs, norm_weight=w, eps=1e-5, H=H, dq=dq, dr=dr, R=R, ps=ps, table=table,
+                     rot_dims=rot, interleaved=interleaved, err=err, **kw)
+    o.raise_if_error(err)
+    lat = (low[:, 8:] if apart else rows[:, H * (dq + dr):]).double()
+
+    def turned(x):
+        x = x.clone()
+        c, s = table[:T, :, 0].double()[:, None], table[:T, :, 1].double()[:, None]
+        a, b = (slice(0, rot, 2), slice(1, rot, 2)) if interleaved else (slice(0, rot // 2), slice(rot // 2, rot))
+        u, v = x[..., a].clone(), x[..., b].clone()
+        x[..., a], x[..., b] = u * c - v * s, v * c + u * s
+        return x
+    q = turned(rows[:, :H * (dq + dr)].double().view(T, H, dq + dr)[..., dq:])
+    k = turned(lat[:, None, R:])[:, 0]
+    c = lat[:, :R] / torch.sqrt((lat[:, :R] ** 2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    got = torch.stack([cache[bt[0, t // ps].item(), 0, t % ps] for t in range(T)]).double()
+    tol = dict(atol=1e-2, rtol=2.0 ** -8) if dtype == torch.bfloat16 else dict(atol=2e-6, rtol=2e-6)      # one rounding of the result, a few of 32 bit
+    assert torch.allclose(got, torch.cat([c, k], dim=1), **tol) and torch.allclose(qabs[..., R:].double(), q, **tol)
+    assert bool((qabs[..., :R] == 7).all()) and bool((cache[5] == 5).all())
