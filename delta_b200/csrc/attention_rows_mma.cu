@@ -477,7 +477,7 @@ __global__ void attention_rows_merge_kernel(const DkRowAttnParams p, const float
   __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + ((size_t)t * p.H + head) * dv;
   for (int d = threadIdx.x; d < dv; d += blockDim.x) {
     float a = 0.f;
-#pragma unroll 8
+#pragma unroll 16
     for (int s = 0; s < splits; ++s) a = fmaf(src[(size_t)s * (dv + 2) + d], factor[s], a);
     orow[d] = __float2bfloat16_rn(a * inv_sum);
   }
@@ -572,6 +572,6 @@ extern "C" int dk_attention_rows_mma(const DkRowAttnParams* pp, int max_m, int s
   }
   if (e != 0 || splits == 1) return e;
   DK_REQUIRE(p.H <= 65535, "attention_rows_mma: too many heads");
-  attention_rows_merge_kernel<<<dim3(p.T, p.H), 128, 0, stream>>>(p, part, splits);
+  attention_rows_merge_kernel<<<dim3(p.T, p.H), p.dv > 128 ? 256 : 128, 0, stream>>>(p, part, splits);
   return dk_check_launch("attention_rows_merge");
 }
