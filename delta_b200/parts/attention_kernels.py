@@ -122,10 +122,12 @@ def _prefill_kernel(ctx, params):
 
 
 def tiles_pay(q_lens, starts, heads: int, sm_count: int) -> bool:
-    """Whether the rows of several tokens of a 32-bit step end sooner in the kernel with tiles of 32 queries than in the plain one.  Microseconds,
-    heads of 128 (heads of 64 take 0.7 of either): a pass over 128 keys takes a block of the plain kernel (one token) 16 and a block of tiles 28,
-    and once there are more blocks than run at once an SM needs 10 and 25 for each of its share.  16 heads behind 4,000 keys: 2 and 8 tokens 529
-    and 532 (tiles 800, 858), 16 tokens 794 (862), 31 tokens 1,319 (931), 300 tokens 10,926 (1,433); 300 tokens of a fresh prompt 450 (94)."""
+    """Whether the rows of several tokens of a 32-bit step go to the kernel with tiles rather than to the plain one.  The line was drawn for tiles of
+    32 queries, in microseconds, heads of 128: a pass over 128 keys took a block of the plain kernel (one token) 16 and a block of tiles 28, and
+    once there were more blocks than run at once an SM needed 10 and 25 for each of its share.  With tiles of 16 and a fetching warp every case
+    measured where it says tiles is further ahead (16 heads, plain and tiles: 31 tokens behind 4,000 keys 1,249 and 457, 300 tokens 10,926 and
+    828, 300 tokens of a fresh prompt 446 and 50), and where it says plain the two are closer (2, 8, 16 tokens behind 4,000 keys 527 and 420, 529
+    and 443, 779 and 454; 16 tokens of a fresh prompt 13 and 10): there it errs to the plain kernel, which gives the same bits."""
     longest = plain = tiles = 0.0
     for n, start in zip(q_lens, starts):
         if n > 1:

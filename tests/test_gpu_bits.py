@@ -25,6 +25,18 @@ def test_attention_f32_has_the_bits_of_the_plain_kernel(H, KV, hd, ps):
     assert torch.equal(out, want) and torch.equal(lse, want_lse)
 
 
+@pytest.mark.parametrize("q_len", [2, 15, 16, 17, 31, 48, 49])
+def test_attention_f32_tiles_of_16_queries_have_the_bits_of_the_plain_kernel(q_len):
+    """A query beside a tile's end on either side, behind no key, one key, nearly a tile of keys and several passes of them."""
+    o = ops()
+    starts = [0, 1, 31, 300, 500]
+    case = PagedCase(torch.float32, 5, 5, 64, 8, seq_lens=[s + q_len for s in starts], q_lens=[q_len] * 5, seed=q_len)
+    out, want = torch.full((case.T, 5 * 64), 9.0, device=DEV), torch.full((case.T, 5 * 64), 9.0, device=DEV)
+    o.attention_f32(case.params(out), q_len)
+    o.attention_plain(case.params(want))
+    assert torch.equal(out, want)
+
+
 def test_attention_f32_infinite_scores_have_the_bits_of_the_plain_kernel():
     """Keys whose score is minus infinity weigh nothing: a whole pass of them, a part of one, and the first pass."""
     o = ops()
