@@ -724,23 +724,36 @@ experts_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16
 // side by side (csrc/gemm_rows_tc.cu).  K is a multiple of 8.
 // row_scale (or null): rows[p] = row_scale[sorted[p]] * x[sorted[p] / top], rounded once: a choice's weight multiplies what its
 // expert reads.
+// Bound by the bytes written and by the chain from a place to its row: a block takes four neighbouring places, so that four rows are under way
+// at once.  8,192 rows of 2,048 entries among their padding: 12.7 -> 8.6 us against a row a block.
+constexpr int GATHER_ROWS = 4;
+
 __global__ void experts_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ sorted, int top,
-                                      __nv_bfloat16* __restrict__ rows, int K, const float* __restrict__ row_scale) {
-  const int p = blockIdx.x;
-  const int s = sorted[p];
-  const uint4* src = s < 0 ? nullptr : reinterpret_cast<const uint4*>(x + (size_t)(s / top) * K);
-  uint4* dst = reinterpret_cast<uint4*>(rows + (size_t)p * K);
-  if (src == nullptr || row_scale == nullptr) {
-    for (int c = threadIdx.x; c < K / 8; c += blockDim.x) dst[c] = src ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  const float w = row_scale[s];
-  for (int c = threadIdx.x; c < K / 8; c += blockDim.x) {
-    float v[8];
-    load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(src + c), v);
+                                      __nv_bfloat16* __restrict__ rows, int K, const float* __restrict__ row_scale, int capacity) {
+  const int p0 = blockIdx.x * GATHER_ROWS;
+  int from[GATHER_ROWS];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] *= w;
-    store8<__nv_bfloat16>(reinterpret_cast<__nv_bfloat16*>(dst + c), v);
+  for (int q = 0; q < GATHER_ROWS; ++q) from[q] = p0 + q < capacity ? sorted[p0 + q] : -1;
+  float w[GATHER_ROWS];
+#pragma unroll
+  for (int q = 0; q < GATHER_ROWS; ++q) w[q] = row_scale != nullptr && from[q] >= 0 ? row_scale[from[q]] : 1.f;
+  for (int c = threadIdx.x; c < K / 8; c += blockDim.x) {
+    uint4 v[GATHER_ROWS];
+#pragma unroll
+    for (int q = 0; q < GATHER_ROWS; ++q)
+      v[q] = from[q] >= 0 ? reinterpret_cast<const uint4*>(x + (size_t)(from[q] / top) * K)[c] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int q = 0; q < GATHER_ROWS; ++q) {
+      if (p0 + q >= capacity) break;
+      if (row_scale != nullptr && from[q] >= 0) {
+        float u[8];
+        load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&v[q]), u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) u[e] *= w[q];
+        store8<__nv_bfloat16>(reinterpret_cast<__nv_bfloat16*>(&v[q]), u);
+      }
+      reinterpret_cast<uint4*>(rows + (size_t)(p0 + q) * K)[c] = v[q];
+    }
   }
 }
 
@@ -988,7 +1001,8 @@ extern "C" int dk_experts_gather(const void* x, const int* sorted, int top, void
   if (capacity == 0) return 0;
   DK_REQUIRE(capacity > 0 && K > 0 && K % 8 == 0 && top > 0 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)rows % 16) == 0,
              "experts_gather: bad arguments capacity=%d K=%d top=%d", capacity, K, top);
-  experts_gather_kernel<<<capacity, K >= 2048 ? 256 : 128, 0, stream>>>((const __nv_bfloat16*)x, sorted, top, (__nv_bfloat16*)rows, K, row_scale);
+  experts_gather_kernel<<<(capacity + GATHER_ROWS - 1) / GATHER_ROWS, K >= 2048 ? 256 : 128, 0, stream>>>(
+      (const __nv_bfloat16*)x, sorted, top, (__nv_bfloat16*)rows, K, row_scale, capacity);
   return dk_check_launch("experts_gather");
 }
 

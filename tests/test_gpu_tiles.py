@@ -405,3 +405,24 @@ def test_decay_attention_tc_numbers_out_of_the_parts_reach(what):
     for a, b in ((out, want), (st, ref)):
         both = a.isfinite() & b.isfinite()
         assert (a[both] - b[both]).norm() < 1e-6 * b[both].norm()
+
+
+@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("capacity, K, top", [(1, 8, 1), (3, 1032, 2), (4, 2048, 4), (5, 2056, 3), (9, 4096, 8), (130, 24, 4)])
+def test_experts_gather_places_beside_a_block(capacity, K, top, scaled):
+    """Four places a block: one place, a block's worth, one more, the last block not full; empty places among them and behind them."""
+    o = ops()
+    torch.manual_seed(capacity + K)
+    tokens = (capacity + top - 1) // top + 1
+    x = torch.randn(tokens, K, device=DEV).bfloat16()
+    places = torch.randint(-1, tokens * top, (capacity,), device=DEV, dtype=torch.int32)
+    places[-1] = -1 if capacity > 1 else tokens * top - 1
+    scale = torch.rand(tokens * top, device=DEV) if scaled else None
+    rows = torch.full((capacity + 1, K), 3.0, dtype=torch.bfloat16, device=DEV)
+    o.experts_gather(x, places, top, rows[:capacity], row_scale=scale)
+    at = places.long().clamp(min=0)
+    want = x[at // top]
+    if scaled:
+        want = (want.float() * scale[at][:, None]).bfloat16()      # one product, rounded once
+    want[places < 0] = 0
+    assert torch.equal(rows[:capacity], want) and bool((rows[capacity] == 3.0).all())
