@@ -1,9 +1,9 @@
 """The library's launchers as functions of a CPython module, for the host's time in steps that are not replayed.
 
 A launcher takes up to thirty numbers and addresses, which ``ctypes`` turns over one by one: 3.8 us for 22 of them, half of what a small launch
-costs the host.  From the signatures a C file is written that does the same with the interpreter's own calls (0.5 us), and compiled beside the
-library.  It holds no kernel: it calls the library's functions by address, without the interpreter's lock as ``ctypes`` does.  Where no C compiler or
-no ``Python.h`` is there, the launchers are called through ``ctypes``.
+costs the host.  From the signatures a C file is written that does the same with the interpreter's own calls (0.2 us), and compiled beside the
+library.  It holds no kernel: it calls the library's functions by address, without the interpreter's lock as ``ctypes`` does.  Where it cannot be
+compiled or loaded, a warning says why and the launchers are called through ``ctypes``.
 """
 from __future__ import annotations
 
@@ -12,9 +12,11 @@ import hashlib
 import importlib.machinery
 import importlib.util
 import os
+import shlex
 import shutil
 import subprocess
 import sysconfig
+import warnings
 from pathlib import Path
 from typing import Dict, Optional
 
@@ -67,35 +69,44 @@ def _source(signatures: Dict[str, list]) -> str:
     return "\n".join(out) + "\n"
 
 
-def _compile(source: str, to: Path) -> bool:
-    cc, include = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc"), sysconfig.get_paths()["include"]
-    if not cc or not (Path(include) / "Python.h").is_file():
-        return False
+def _compile(source: str, to: Path) -> str:
+    """An empty text, or why there is no module."""
+    include = sysconfig.get_paths()["include"]
+    cc = shlex.split(os.environ.get("CC") or "") or [c for c in (shutil.which("gcc"), shutil.which("cc")) if c][:1]      # (CC may bring arguments)
+    if not cc:
+        return "there is no C compiler"
+    if not (Path(include) / "Python.h").is_file():
+        return f"there is no Python.h in {include}"
     c, tmp = to.with_suffix(f".{os.getpid()}.c"), to.with_suffix(f".{os.getpid()}.tmp")
     try:
         c.write_text(source)
-        r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, str(c), "-o", str(tmp), "-ldl"], capture_output=True, text=True)
+        r = subprocess.run([*cc, "-O2", "-shared", "-fPIC", "-I", include, str(c), "-o", str(tmp), "-ldl"], capture_output=True, text=True)
         if r.returncode != 0:
-            return False
+            return f"{shlex.join(cc)} ended with {r.returncode}: {r.stderr.strip()[-500:]}"
         os.replace(tmp, to)
-        return True
-    except OSError:
-        return False
+        return ""
+    except OSError as e:
+        return str(e)
     finally:
         c.unlink(missing_ok=True)
         tmp.unlink(missing_ok=True)
 
 
 def load(library: C.CDLL, path: Path, signatures: Dict[str, list]) -> Optional[dict]:
-    """{launcher: function} for those of ``signatures`` that take numbers and addresses only; None where the module cannot be built."""
+    """{launcher: function} for those of ``signatures`` that take numbers and addresses only; None, with a warning, where there is no module."""
     plain = {name: args for name, args in signatures.items() if all(a in _TYPES for a in args)}
     source = _source(plain)
     so = Path(path).parent / ("dk_calls_" + hashlib.sha256((source + sysconfig.get_config_var("EXT_SUFFIX")).encode()).hexdigest()[:16]
                               + sysconfig.get_config_var("EXT_SUFFIX"))
-    if not so.is_file() and not _compile(source, so):
-        return None
-    loader = importlib.machinery.ExtensionFileLoader("dk_calls", str(so))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("dk_calls", str(so), loader=loader))
-    loader.exec_module(module)
-    module.connect(library._handle)
-    return {name: getattr(module, name) for name in plain}
+    why = "" if so.is_file() else _compile(source, so)
+    if not why:
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("dk_calls", str(so))
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("dk_calls", str(so), loader=loader))
+            loader.exec_module(module)
+            module.connect(library._handle)
+            return {name: getattr(module, name) for name in plain}
+        except ImportError as e:
+            why = str(e)
+    warnings.warn(f"the launchers are called through ctypes, which costs the host about 4 us a launch: {why}", RuntimeWarning, stacklevel=2)
+    return None

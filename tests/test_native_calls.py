@@ -45,3 +45,35 @@ def test_wrong_arguments_are_errors(both):
 def test_launchers_with_structures_stay_with_ctypes(both):
     _, calls = both
     assert "dk_attention_plain" not in calls and lib.load().dk_attention_plain.argtypes is not None
+
+
+@pytest.fixture
+def apart(tmp_path):
+    """The library with a folder of its own for the module."""
+    path = tmp_path / "lib.so"
+    path.symlink_to(lib.build())
+    return C.CDLL(str(path)), path, {k: lib._SIGNATURES[k] for k in ("dk_gemm_tc_supported", "dk_softcap")}
+
+
+def test_a_compiler_with_arguments(apart, monkeypatch, recwarn):
+    monkeypatch.setenv("CC", "gcc -pipe")
+    calls = native_calls.load(*apart)
+    assert calls is not None and calls["dk_gemm_tc_supported"](128, 4096, 4096, 1) and not recwarn
+
+
+@pytest.mark.parametrize("cc, why", [("/bin/false -pipe", "false -pipe ended with"), ("/nowhere/cc", "nowhere/cc")])
+def test_a_compiler_that_fails_is_told(apart, monkeypatch, cc, why):
+    monkeypatch.setenv("CC", cc)
+    with pytest.warns(RuntimeWarning, match=f"through ctypes.*{why}"):
+        assert native_calls.load(*apart) is None
+
+
+def test_a_module_that_does_not_load_is_told(apart, tmp_path):
+    plain, path, signatures = apart
+    assert native_calls.load(plain, path, signatures) is not None
+    (so,) = path.parent.glob("dk_calls_*.so")
+    other = tmp_path / "other"
+    other.mkdir()
+    (other / so.name).write_bytes(b"no module")
+    with pytest.warns(RuntimeWarning, match="through ctypes"):
+        assert native_calls.load(plain, other / "lib.so", signatures) is None
