@@ -466,19 +466,30 @@ __global__ void latent_prepare_vec_kernel(const T* __restrict__ src, int src_str
     return;
   }
   if (threadIdx.x < 32) {
-    float x[2][8];
-    float ss = 0.f;
+    float x[2][8], ss[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int c = (threadIdx.x + 32 * k) * 8;
       if (c < R) {
         load8<T>(low + c, x[k]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) ss = fmaf(x[k][e], x[k][e], ss);
+        for (int e = 0; e < 8; ++e) ss[e] = fmaf(x[k][e], x[k][e], ss[e]);
       }
     }
     const long long at = cache != nullptr ? row_slot_of(block_table, max_pages, num_pages, b, pos, ps, t, err) : -1;
-    const float inv = 1.f / sqrtf(warp_sum(ss) / (float)R + eps);
+    // The sum of the squares in the order of the block of 256 threads above, one entry (and the one 256 behind it) each, so that a row has the same
+    // bits from either kernel: 32 neighbouring entries 16, 8, 4, 2 and 1 apart, then those sums 4, 2 and 1 apart.
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], o);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < o; ++e) ss[e] += ss[e + o];
+#pragma unroll
+    for (int o = 16; o > 2; o >>= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+    const float inv = 1.f / sqrtf(ss[0] / (float)R + eps);
     if (at < 0) return;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -507,8 +518,8 @@ __global__ void latent_prepare_vec_kernel(const T* __restrict__ src, int src_str
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
           const float u = x[e], v = x[e + 1];
-          x[e] = u * f[e] - v * f[e + 1];
-          x[e + 1] = v * f[e] + u * f[e + 1];
+          x[e] = fmaf(u, f[e], -__fmul_rn(v, f[e + 1]));      // (rounded as the kernel above has it)
+          x[e + 1] = fmaf(v, f[e], __fmul_rn(u, f[e + 1]));
         }
       } else {
         const bool first = i < half;

@@ -143,3 +143,25 @@ def test_latent_prepare_of_eight_entries_at_a_time(H, dq, dr, R, rot, interleave
     tol = dict(atol=1e-2, rtol=2.0 ** -8) if dtype == torch.bfloat16 else dict(atol=2e-6, rtol=2e-6)      # one rounding of the result, a few of 32 bit
     assert torch.allclose(got, torch.cat([c, k], dim=1), **tol) and torch.allclose(qabs[..., R:].double(), q, **tol)
     assert bool((qabs[..., :R] == 7).all()) and bool((cache[5] == 5).all())
+
+
+@pytest.mark.parametrize("H, dq, dr, R, rot, interleaved", [(16, 128, 64, 256, 64, False), (2, 8, 16, 8, 16, False), (3, 16, 24, 264, 16, True), (2, 64, 32, 512, 16, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_latent_prepare_has_the_same_bits_from_either_kernel(H, dq, dr, R, rot, interleaved, dtype):
+    """Latents that begin on a boundary of eight entries (eight at a time) and beside it (one at a time): norms and rotated parts are the same numbers."""
+    from delta_b200.kernels import ops as o
+    g = torch.Generator().manual_seed(R)
+    T, ps, width = 300, 16, R + dr
+    rows, lat = torch.randn(T, H * (dq + dr), generator=g).to(dtype).to(DEV), torch.randn(T, width, generator=g).to(dtype).to(DEV)
+    angle = torch.arange(T, dtype=torch.float64)[:, None] * 100.0 ** (-2.0 * torch.arange(rot // 2, dtype=torch.float64) / rot)
+    table = torch.stack([angle.cos(), angle.sin()], dim=-1).float().contiguous().to(DEV)
+    w, bt = (torch.rand(R, generator=g) + 0.5).to(DEV), torch.arange(19, dtype=torch.int32, device=DEV).view(1, 19)
+    got = []
+    for off in (8, 3):
+        low = torch.zeros(T, width + 8, dtype=dtype, device=DEV)
+        low[:, off:off + width] = lat
+        cache, qabs = torch.zeros((19, 1, ps, width), dtype=dtype, device=DEV), torch.zeros((T, H, width), dtype=dtype, device=DEV)
+        o.latent_prepare(rows, torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV), bt, cache, qabs, norm_weight=w, eps=1e-5,
+                         H=H, dq=dq, dr=dr, R=R, ps=ps, table=table, rot_dims=rot, interleaved=interleaved, low=low, low_offset=off)
+        got.append((cache, qabs))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
