@@ -3,8 +3,8 @@
 // The rows of an expert are a tile of the sorted slots (experts.cu), nearly empty when a step brings few tokens.  As in gemm_small_m.cu a block owns
 // 16 rows of an expert's matrix (and the 16 up rows that belong to its gate rows), its warps share K in chunks of 32 entries, and
 // weights and activations go from memory into MMA fragments with sixteen-byte loads under a permutation of k that both share; the warps'
-// sums are added in shared memory in a fixed order.  Bound by the memory: 8 tokens, 16 experts of 1,024, 4 chosen, width 2,048: 28
-// and 15 us for the two products (188 MB); in tiles of 64 rows through shared memory (experts.cu) 38 and 21 us.
+// sums are added in shared memory in a fixed order.  Bound by the memory: 8 tokens, 16 experts of 1,024, 4 chosen, width 2,048: 24.7
+// and 13.4 us for the two products (188 MB); in tiles of 64 rows through shared memory (experts.cu) 38 and 21 us.
 #include "common.cuh"
 #include "mma_helpers.cuh"
 
@@ -18,11 +18,18 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {      // weights: rea
 }
 
 // MODE 1: gated, rows gathered from the tokens; 2: relu squared, gathered; 0: rows in sorted order, the result in 32 bit to the slots.
-// Up to eight rows: held to 64 registers (a few spilled), so that an SM has 32 warps and not 24 of these streams, and 1,024 blocks go in two rounds and not
-// three.  16 experts of 2 x 1,024 x 2,048 and 2,048 x 1,024, 8 tokens: 28.1 -> 24.7 and 15.2 -> 13.4 us (5.4 and 5.0 TB/s); 48 registers with fewer
-// loads under way 29.8 and 14.9.
+// Blocks that an SM shall have room for (0: as the compiler has it, 71 to 130 registers).  Up to eight rows: held to 64 registers (a few spilled), so that an SM
+// has 32 warps and not 24 of these streams, and 1,024 blocks go in two rounds and not three: 16 experts of 2 x 1,024 x 2,048 and 2,048 x 1,024, 8 tokens:
+// 28.1 -> 24.7 and 15.2 -> 13.4 us (5.4 and 5.0 TB/s); 48 registers with fewer loads under way 29.8 and 14.9.  But gated products of K <= 1,024 in blocks of four
+// warps lose by it (the layer at width 1,024, 8 tokens: 34.6 -> 35.6 us).  The first product of relu squared gains for 17 and more rows by more loads under way,
+// 106 registers and 16 warps: the layer with 24 tokens, width 2,048 and 1,024: 68.1 -> 61.2 and 32.1 -> 29.5.  The others of nine and more rows lose by more registers: relu
+// squared, 16 tokens, 45.3 -> 51.4 and 26.6 -> 28.2; gated ones, whose 146 and 158 leave room for 12 warps and not 16, 74.1 -> 86.7 at 16 tokens and
+// 92.4 -> 100.6 at 24, width 2,048; results in 32 bit for 17 and more rows, behind gated ones, 91.0 -> 95.5 at 24.
+constexpr int least_blocks(int mode, int mt, int warps) {
+  return mt == 1 && !(mode == 1 && warps == 4) ? 32 / warps : mt == 4 && mode == 2 ? 16 / warps : 0;
+}
 template <int MODE, int MT, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, MT == 1 ? 32 / WARPS : 1)
+__global__ void __launch_bounds__(WARPS * 32, least_blocks(MODE, MT, WARPS))
 experts_stream_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W, void* __restrict__ out, const int* __restrict__ sorted,
                       const int* __restrict__ tile_expert, int top, int N, int K, float limit, float alpha, float shift,
                       const float* __restrict__ row_scale) {
