@@ -19,12 +19,14 @@
 // (2-norm, 700 and 1,000 tokens): outputs 1.3e-7, states 0.8e-7 off, 1.9e-7 and 1.0e-7 there (with parts cut off instead of rounded 2.2e-7 and 1.3e-7).
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
+#include "ring.cuh"
 
 namespace {
 constexpr int TC = 128, D = 128;
 constexpr int WARPS = 16, THREADS = (WARPS + 1) * 32;
 constexpr int BOX = TC * 128, PART = 2 * BOX;      // bytes: 128 rows of 64 entries; an operand's part
 constexpr int TURN_LD = 36;
+constexpr int PRODUCTS = 3;      // of a block, at most
 constexpr int TMEM_COLS = 512, COL_A = 0, COL_D = 192;      // the first operand's parts, and two accumulators; or four accumulators
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
@@ -161,13 +163,13 @@ __device__ __forceinline__ uint64_t across(uint32_t parts, int p, int s) { retur
 struct Shared {
   float pw[TC + 4];
   uint32_t largest[TC];      // of a row of queries
-  unsigned long long done;
+  unsigned long long done[PRODUCTS];      // a product's operands have been read and its sums are there
   uint32_t tmem_base_slot;
   int failed;
 };
 __device__ __forceinline__ void begin(Shared& sh, int warp, int tid, double decay) {
   if (tid == 0) {
-    mbar_init(s2u(&sh.done), 1);
+    for (int p = 0; p < PRODUCTS; ++p) mbar_init(s2u(&sh.done[p]), 1);
     sh.failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -186,20 +188,29 @@ __device__ __forceinline__ bool row_out_of_reach(Shared& sh, const float (&x)[32
   atomicMax(&sh.largest[r], m);
   return too_large(m);
 }
-// `products` were issued; they are complete before the block leaves
-__device__ __forceinline__ void end(Shared& sh, int warp, int lane, int products, int* err) {
-  if (warp == WARPS && lane == 0 && products > 0) mbar_wait(s2u(&sh.done), (products - 1) & 1);
+// `issued`: products that the caller's thread has issued; each is complete before the block leaves, whatever became of the waits for it
+__device__ __forceinline__ void end(Shared& sh, int warp, int lane, int issued, int* err) {
+  if (warp == WARPS && lane == 0) ring_drain(issued, PRODUCTS, [&](int p, uint32_t parity) { return mbar_wait(s2u(&sh.done[p]), parity); });
   __syncwarp();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (sh.failed && threadIdx.x == 0) dk_report(err, DK_DEV_TIMEOUT, blockIdx.x, blockIdx.y, products);
+  if (sh.failed && threadIdx.x == 0) dk_report(err, DK_DEV_TIMEOUT, blockIdx.x, blockIdx.y, 0);
   if (warp == WARPS) tmem_dealloc(sh.tmem_base_slot, TMEM_COLS);
+}
+// The next product, unless a wait has given up (what it would read may not be there, and nobody waits for it).
+template <typename Issue>
+__device__ __forceinline__ void issue_next(Shared& sh, int lane, int& issued, Issue&& product) {
+  if (lane == 0 && *(volatile int*)&sh.failed == 0) {
+    product();
+    umma_commit(s2u(&sh.done[issued++]));
+  }
+  __syncwarp();
 }
 // Number `p` (0, 1, ..) of a block's products is complete.
 __device__ __forceinline__ void wait_product(Shared& sh, int p) {
   volatile int* gave_up = &sh.failed;
-  if (*gave_up == 0 && !mbar_wait(s2u(&sh.done), p & 1)) *gave_up = 1;
+  if (*gave_up == 0 && !mbar_wait(s2u(&sh.done[p]), 0)) *gave_up = 1;
   tc_fence_after();
 }
 // A warp's 32 rows of 32 floats as they lie in memory, neighbouring lanes at neighbouring places: f(row, column, float4)
@@ -270,7 +281,7 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
   const int r = (warp & 3) * 32 + lane, group = (warp >> 2) & 3;
   const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   const bool converts = warp < WARPS;
-  const uint32_t done = s2u(&sh.done), r0 = s2u(R0), r1 = s2u(R1);
+  const uint32_t r0 = s2u(R0), r1 = s2u(R1);
   float x[32], k[32];
   uint4 raw[4];
   bool odd = false;
@@ -295,16 +306,13 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
   odd |= tid < TC && too_small(sh.largest[tid]);
   odd = __syncthreads_or(odd) != 0;
   tc_fence_after();
-  int products = 0;
-  if (!odd) {
-    if (warp == WARPS && lane == 0) {      // q . k
+  int issued = 0;
+  const bool scored = !odd;
+  if (scored && warp == WARPS)
+    issue_next(sh, lane, issued, [&]() {      // q . k
       const uint32_t idesc = instr_desc_bf16(TC, TC);
       issue<2>([&](int q, int a, int b, int s, uint32_t add) { umma_a_tmem(tmem + COL_D + q * D, tmem + COL_A + a * 64 + s * 8, along(r1, b, s), idesc, add); });
-      umma_commit(done);
-    }
-    __syncwarp();
-    products = 1;
-  }
+    });
   bool odd_v = false;
   if (converts) {      // meanwhile
     activate(x, raw, act);
@@ -313,10 +321,10 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
   }
   odd |= __syncthreads_or(odd_v) != 0;
   if (odd) {
-    if (products) wait_product(sh, 0);      // before its operands are overwritten
+    if (scored) wait_product(sh, 0);      // before its operands are overwritten
     __syncthreads();
     chunk_by_fma(reinterpret_cast<float*>(smem), at + q_off, at + k_off, at + v_off, stride, act, n, sh.pw, Uc, oc, H * D);
-    end(sh, warp, lane, products, err);
+    end(sh, warp, lane, issued, err);
     return;
   }
   if (converts) {
@@ -329,12 +337,10 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
   __syncthreads();
   tc_fence_after();
   if (warp == WARPS) {
-    if (lane == 0) {      // the contribution to the state: keys' entries by values' entries, both operands read transposed
+    issue_next(sh, lane, issued, [&]() {      // the contribution to the state: keys' entries by values' entries, both operands read transposed
       const uint32_t idesc = instr_desc_bf16(TC, D, true) | 1u << 15;
       issue<4>([&](int q, int a, int b, int s, uint32_t add) { umma(tmem + q * D, across(r1, a, s), across(r0, b, s), idesc, add); });
-      umma_commit(done);
-    }
-    __syncwarp();
+    });
   } else {
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
@@ -353,12 +359,10 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
   __syncthreads();
   tc_fence_after();
   if (warp == WARPS) {
-    if (lane == 0) {      // A v
+    issue_next(sh, lane, issued, [&]() {      // A v
       const uint32_t idesc = instr_desc_bf16(TC, D, true);
       issue<2>([&](int q, int a, int b, int s, uint32_t add) { umma_a_tmem(tmem + COL_D + q * D, tmem + COL_A + a * 64 + s * 8, across(r0, b, s), idesc, add); });
-      umma_commit(done);
-    }
-    __syncwarp();
+    });
   } else {
     float* turn = reinterpret_cast<float*>(R1) + warp * 32 * TURN_LD;      // (the keys have been read)
     float* to = Uc + (size_t)((warp & 3) * 32) * D + group * 32;
@@ -371,7 +375,7 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
       if (t < n) *reinterpret_cast<float4*>(o + (size_t)t * H * D + c) = v;
     });
   }
-  end(sh, warp, lane, 3, err);
+  end(sh, warp, lane, issued, err);
 }
 
 // grid (dk dv / 4 / 128, rows * H): four neighbouring entries a thread, four chunks' under way
@@ -425,7 +429,8 @@ decay_tc_out_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_off
   float* oc = out + ((size_t)t0 * H + h) * D;
   const int r = (warp & 3) * 32 + lane, group = (warp >> 2) & 3;
   const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  const uint32_t done = s2u(&sh.done), sp = s2u(Sp);
+  const uint32_t sp = s2u(Sp);
+  int issued = 0;
   float x[32];
   bool odd = false;
   if (warp < WARPS) {
@@ -461,17 +466,15 @@ decay_tc_out_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_off
       }
       oc[(size_t)t * H * D + c] = fmaf(sum, sh.pw[t + 1], oc[(size_t)t * H * D + c]);
     }
-    end(sh, warp, lane, 0, err);
+    end(sh, warp, lane, issued, err);
     return;
   }
   tc_fence_after();
   if (warp == WARPS) {
-    if (lane == 0) {
+    issue_next(sh, lane, issued, [&]() {
       const uint32_t idesc = instr_desc_bf16(TC, D, true);
       issue<2>([&](int q, int a, int b, int s, uint32_t add) { umma_a_tmem(tmem + COL_D + q * D, tmem + COL_A + a * 64 + s * 8, across(sp, b, s), idesc, add); });
-      umma_commit(done);
-    }
-    __syncwarp();
+    });
   } else {
     wait_product(sh, 0);
     read_product<2>(lanes + COL_D, group, x);
@@ -488,7 +491,7 @@ decay_tc_out_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_off
       }
     });
   }
-  end(sh, warp, lane, 1, err);
+  end(sh, warp, lane, issued, err);
 }
 constexpr int CHUNK_SMEM = 6 * PART + 1024, OUT_SMEM = 3 * PART + 1024;
 static_assert(3 * TC * D * 4 <= 6 * PART && WARPS * 32 * TURN_LD * 4 <= 3 * PART, "what else the parts' memory is used for");

@@ -68,3 +68,23 @@ def test_persistent_kernels_wait_for_what_they_started(name, copies, products):
         line = body[body.rindex("\n", 0, calls[0]):calls[0]]
         assert "failed" not in line and "gave_up" not in line and "ok" not in line.split("//")[0], line
         assert body.rindex("__syncthreads") > calls[0]
+
+
+def test_linear_attention_waits_for_each_product_it_issued():
+    """Up to three products, each with a barrier that completes once: none is issued after a wait has given up, and the thread that issued them waits for every one
+    of them before the block leaves.  (One barrier for all three was waited for by its parity: the first product's end passed for the third's.)"""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "decay_attention_tc.cu").read_text())
+    most = int(re.search(r"constexpr int PRODUCTS = (\d+);", text).group(1))
+    assert "done[PRODUCTS]" in text and re.search(r"for \(int p = 0; p < PRODUCTS; \+\+p\) mbar_init\(s2u\(&sh\.done\[p\]\), 1\)", text)
+    assert len(re.findall(r"umma_commit\(", text)) == 1      # of issue_next, which counts what it issued
+    body = text[text.index("void issue_next"):]
+    body = body[:body.index("\n}")]
+    assert "failed == 0" in body and "umma_commit(s2u(&sh.done[issued++]))" in body
+    for kernel in text.split("__global__")[1:]:
+        assert len(re.findall(r"issue_next\(sh, lane, issued,", kernel)) <= most
+        assert len(re.findall(r"\bumma(?:_a_tmem)?\(", kernel)) == len(re.findall(r"issue_next\(", kernel))
+        assert all(m == "issued" for m in re.findall(r"\bend\(sh, warp, lane, (\w+), err\)", kernel))
+    end = text[text.index("void end("):]
+    end = end[:end.index("\n}")]
+    drain = re.search(r"ring_drain\(issued, PRODUCTS, [^;]*mbar_wait\(s2u\(&sh\.done\[p\]\), parity\)", end)
+    assert drain and "failed" not in end[:drain.start()] and drain.end() < end.index("__syncthreads") < end.index("tmem_dealloc")
