@@ -15,7 +15,8 @@
 //      warps 8-15   add finished chunks to the sums in registers and store them;
 //   3. add_segments, where K is cut into segments (W of few tiles): their sums in order.
 // Rows with infinite or NaN entries, or whose largest entry is outside 2^-40 .. 2^60 (parts or their products would leave the exponent's
-// range), are found on the way, and their results are summed by FMA over k instead.
+// range), are found on the way, and their results are summed by FMA over k instead, a tile at a time, when nothing waits any more: by the product's own
+// blocks behind their pieces, or by add_segments.
 // Bound by the products' issue: a chunk takes about 1,500 cycles for up to 120 tokens (24 MMAs, each waited for by what converts the chunk after
 // next), 12 a token above.  Everything cold, microseconds, against the tiles of gemm_plain.cu: 300 x 2,048 x 2,048 107 -> 40, 300 x 11,008 x 2,048
 // 317 -> 126, 300 x 2,048 x 5,504 274 -> 66, 300 x 32,000 x 2,048 930 -> 240, 2,048 x 22,016 x 4,096 7,590 -> 2,020 (183 TFLOP/s); one row: 44 -> 28,
@@ -24,6 +25,7 @@
 // Every wait on an mbarrier is bounded: when one gives up, the kernel records it, stores nothing more, waits (bounded again) for the copies and
 // products that it has under way, frees its tensor memory and returns.
 #include "common.cuh"
+#include "mma_helpers.cuh"
 #include "tcgen05_helpers.cuh"
 #include "ring.cuh"
 
@@ -51,11 +53,10 @@ __device__ __forceinline__ void parts_of(float x, float y, uint32_t& high, uint3
   low = __byte_perm(__float_as_uint(rx - __uint_as_float(cx & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(cy & 0xffff0000u)), 0x7632);
 }
 
-// grid (rows): parts [3][M][K] and a row's flag.  w_largest (or null): N numbers that begin at zero.
+// grid (rows): parts [3][M][K] and a row's flag; the flags of W's rows, and the one behind them, begin at zero.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, int lda, __nv_bfloat16* __restrict__ parts, int* __restrict__ flags,
-                                                         uint32_t* __restrict__ w_largest, int M, int N, int K, int ldp, int vec) {
-  if (w_largest != nullptr)
-    for (int n = blockIdx.x * 256 + threadIdx.x; n < N; n += gridDim.x * 256) w_largest[n] = 0;
+                                                         int* __restrict__ w_flags, int M, int N, int K, int ldp, int vec) {
+  for (int n = blockIdx.x * 256 + threadIdx.x; n <= N; n += gridDim.x * 256) w_flags[n] = 0;
   __shared__ uint32_t most[8];
   const int m = blockIdx.x, tid = threadIdx.x;
   const float* row = A + (size_t)m * lda;
@@ -102,9 +103,10 @@ struct F32Args {
   float* C;
   const int* flags;      // rows of A out of reach
   float* partial;        // [segments][M][N] where K is cut into segments, else null
-  uint32_t* w_largest;   // [N], with segments: the largest magnitude of a row of W
+  int* w_flags;          // [N + 1]: rows of W out of reach; the last, with segments: some row of A or W is
   int* err;
   int M, N, K, lda, ldw, ldc, tok_tiles, items;
+  int vec;               // rows of A begin on 16-byte boundaries
   int segments, per;     // chunks of K of a segment
 };
 
@@ -121,12 +123,102 @@ struct Piece {
   }
 };
 
-// The plain kernel's sum.
-__device__ __noinline__ float fma_sum(const float* x, const float* w, int K) {
-  float v = 0.f;
-  for (int k = 0; k < K; ++k) v = fmaf(x[k], w[k], v);
-  return v;
+// Results out of the parts' reach, for `most` tokens from m0 on and 128 rows of W from n0 on: the rows of A that need it, by the rows of W, every sum in the
+// plain kernel's order over k.  A thread has EACH tokens by four rows of W; both come by cp.async, STAGES - 1 steps of K ahead.  Bound by the reads of
+// shared memory (four cycles a sixteen-byte load, whatever its lanes share).
+// 300 rows with a NaN each by 2,048 x 2,048 and 9,600 x 1,024: 201 and 364 us in all (gemm_plain.cu alone 106 and 186); one by 12,000 x 2,048 169 (74).
+constexpr int FMA_K = 16, FMA_LD = FMA_K + 4;
+template <int T, int EACH, int STAGES>
+struct FmaTile {
+  static constexpr int AT_ONCE = T / 32 * EACH;
+  float w[STAGES][BM][FMA_LD], x[STAGES][AT_ONCE][FMA_LD];
+  int rows[160], count;
+};
+template <int T, int EACH, int STAGES>
+__device__ __forceinline__ void fma_tile(FmaTile<T, EACH, STAGES>& sm, const F32Args& a, int m0, int most, int n0) {
+  constexpr int AT_ONCE = FmaTile<T, EACH, STAGES>::AT_ONCE, V = FMA_K / 4, LX = AT_ONCE * V;
+  static_assert(LX <= T, "a vector a thread");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = tid % V * 4;
+  int w_odd = 0;      // of the thread's rows of W
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (n0 + lane + 32 * j < a.N) w_odd |= (*(volatile const int*)(a.w_flags + n0 + lane + 32 * j) != 0) << j;
+  const bool all = __syncthreads_or(w_odd) != 0;
+  if (warp == 0) {
+    int count = 0;
+    for (int j0 = 0; j0 < most; j0 += 32) {
+      const int j = j0 + lane;
+      const bool mine = j < most && m0 + j < a.M && (all || a.flags[m0 + j] != 0);
+      const uint32_t them = __ballot_sync(0xffffffffu, mine);
+      if (mine) sm.rows[count + __popc(them & ((1u << lane) - 1u))] = m0 + j;
+      count += __popc(them);
+    }
+    if (lane == 0) sm.count = count;
+  }
+  __syncthreads();
+  const int count = sm.count, steps = (a.K + FMA_K - 1) / FMA_K;
+  for (int p0 = 0; p0 < count; p0 += AT_ONCE) {
+    const bool has_x = tid < LX && p0 + tid / V < count;
+    const float* xrow = a.A + (size_t)(has_x ? sm.rows[p0 + tid / V] : 0) * a.lda + c;
+    auto fetch = [&](int s) {
+      const int k0 = s * FMA_K;
+      if (s < steps) {
+        for (int v = tid; v < BM * V; v += T) {      // (T is a multiple of V)
+          const int r = v / V;
+          const bool in = n0 + r < a.N && k0 + c < a.K;
+          cp_async_16(s2u(&sm.w[s % STAGES][r][c]), in ? a.W + (size_t)(n0 + r) * a.ldw + k0 + c : a.W, in);
+        }
+        if (tid < LX) {
+          const bool in = has_x && k0 + c < a.K;
+          float* to = &sm.x[s % STAGES][tid / V][c];
+          if (a.vec) cp_async_16(s2u(to), in ? xrow + k0 : a.W, in);
+          else
+            for (int i = 0; i < 4; ++i) to[i] = in ? xrow[k0 + i] : 0.f;
+        }
+      }
+      cp_async_commit();
+    };
+    float acc[EACH][4];
+#pragma unroll
+    for (int i = 0; i < EACH; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const bool some = p0 + warp * EACH < count;
+    for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+    for (int s = 0; s < steps; ++s) {
+      cp_async_wait<STAGES - 2>();
+      __syncthreads();      // step s is in, and everybody has left the one whose place is taken next
+      fetch(s + STAGES - 1);
+      if (!some) continue;
+      const float *w = sm.w[s % STAGES][lane], *x = sm.x[s % STAGES][warp * EACH];
+#pragma unroll
+      for (int k = 0; k < FMA_K; k += 4) {
+        float4 b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(w + j * 32 * FMA_LD + k);
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+          const float4 v = *reinterpret_cast<const float4*>(x + i * FMA_LD + k);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(v.w, b[j].w, fmaf(v.z, b[j].z, fmaf(v.y, b[j].y, fmaf(v.x, b[j].x, acc[i][j]))));
+        }
+      }
+    }
+    cp_async_wait<0>();
+    __syncthreads();      // (the stages are the next tokens')
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int r = p0 + warp * EACH + i;
+      if (r >= count) continue;
+      const int m = sm.rows[r], x_odd = a.flags[m];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (n0 + lane + 32 * j < a.N && (x_odd != 0 || (w_odd >> j & 1) != 0)) a.C[(size_t)m * a.ldc + n0 + lane + 32 * j] = acc[i][j];
+    }
+  }
+  __syncthreads();      // (the list is another tile's next)
 }
+using OwnTile = FmaTile<THREADS, 8, 4>;
 
 template <int BN>
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -135,13 +227,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* xs = smem + WS * W_STAGE;
-  __shared__ __align__(8) unsigned long long bars[2 * MAX_W + 2 * MAX_X + 8];
+  __shared__ __align__(8) unsigned long long bars[2 * MAX_W + 2 * MAX_X + 6];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ int failed;
-  __shared__ int w_flags[2][BM];
+  __shared__ int failed, odd;      // odd: some row of the block's pieces is out of reach
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t wfull = s2u(&bars[0]), wempty = s2u(&bars[MAX_W]), xfull = s2u(&bars[2 * MAX_W]), xempty = s2u(&bars[2 * MAX_W + MAX_X]);
-  const uint32_t afull = s2u(&bars[2 * MAX_W + 2 * MAX_X]), done = afull + 16, dempty = afull + 32, flagged = afull + 48;
+  const uint32_t afull = s2u(&bars[2 * MAX_W + 2 * MAX_X]), done = afull + 16, dempty = afull + 32;
   if (tid == 0) {
     for (int s = 0; s < WS; ++s) {
       mbar_init(wfull + 8 * s, 1);
@@ -155,9 +246,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
       mbar_init(afull + 8 * b, 4);
       mbar_init(done + 8 * b, 1);
       mbar_init(dempty + 8 * b, 8);
-      mbar_init(flagged + 8 * b, 4);
     }
-    failed = 0;
+    failed = odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 1) tmem_alloc(s2u(&tmem_base_slot), TMEM_COLS);
@@ -248,9 +338,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
     if (lane == 0) ring_drain(3 * c, XS, [&](int s, uint32_t parity) { return mbar_wait(xempty + 8 * s, parity); });      // its products are complete
   } else if (warp >= 4 && warp < 8) {
     const int row = tid & 127;
-    int c = 0, piece = 0;
+    int c = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x, ++piece) {
+    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const Piece p(a, item, BN);
       uint32_t largest = 0;
       for (int k = 0; k < p.chunks; ++k, ++c) {
@@ -279,9 +369,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
           tmem_st16(to + KC / 2 + half * 16, m);
           tmem_st16(to + KC + half * 16, l);
         }
-        if (k + 1 == p.chunks) {
-          if (a.partial == nullptr) w_flags[piece & 1][row] = out_of_reach(largest);
-          else if (p.n0 + row < a.N) atomicMax(a.w_largest + p.n0 + row, largest);
+        if (k + 1 == p.chunks && out_of_reach(largest) && p.n0 + row < a.N) {
+          a.w_flags[p.n0 + row] = 1;
+          odd = 1;
         }
         tmem_wait_st();
         tc_fence_before();
@@ -289,16 +379,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         if (lane == 0) {
           mbar_arrive(wempty + 8 * s);
           mbar_arrive(afull + 8 * b);
-          if (k + 1 == p.chunks && a.partial == nullptr) mbar_arrive(flagged + 8 * (piece & 1));
         }
       }
     }
   } else if (warp >= 8) {
     const int quarter = warp & 3, half = (warp - 8) >> 2;
     const int row = quarter * 32 + lane;
-    int c = 0, piece = 0;
+    int c = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x, ++piece) {
+    for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const Piece p(a, item, BN);
       const int n = p.n0 + row, m0 = p.m0 + half * NC;
       float sum[NC];
@@ -328,27 +417,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         __syncwarp();
         if (lane == 0) mbar_arrive(dempty + 8 * b);
       }
-      const bool there = ok && (a.partial != nullptr || mbar_wait(flagged + 8 * (piece & 1), ring_parity(piece, 2)));      // (eight chunks and more a piece)
-      if (__any_sync(0xffffffffu, !there)) {
-        *gave_up = 1;
-        break;
-      }
+      if (!ok) break;
       float* to = a.partial != nullptr ? a.partial + (size_t)p.segment * a.M * a.N : a.C;
       const int ld = a.partial != nullptr ? a.N : a.ldc;
 #pragma unroll
       for (int j = 0; j < NC; ++j)
         if (n < a.N && m0 + j < a.M) to[(size_t)(m0 + j) * ld + n] = sum[j];
-      if (a.partial != nullptr) continue;
-      const bool own = w_flags[piece & 1][row] != 0;
-      bool odd = own;
-      for (int j = lane; j < NC; j += 32) odd |= m0 + j < a.M && a.flags[m0 + j] != 0;
-      if (__any_sync(0xffffffffu, odd)) {
-#pragma unroll 1
-        for (int j = 0; j < NC; ++j)
-          if (n < a.N && m0 + j < a.M && (own || a.flags[m0 + j] != 0))
-            a.C[(size_t)(m0 + j) * a.ldc + n] = fma_sum(a.A + (size_t)(m0 + j) * a.lda, a.W + (size_t)n * a.ldw, a.K);
-      }
     }
+  } else if (warp == 3) {      // looks for tokens out of reach meanwhile
+    bool mine = false;
+    for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+      const Piece p(a, item, BN);
+      for (int j = lane; j < BN; j += 32) mine |= p.m0 + j < a.M && a.flags[p.m0 + j] != 0;
+    }
+    if (mine) odd = 1;
   }
   __syncwarp();
   tc_fence_before();
@@ -356,19 +438,32 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
   tc_fence_after();
   if (failed && tid == 0) dk_report(a.err, DK_DEV_TIMEOUT, blockIdx.x, 0, a.per);
   if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (!odd || failed) return;
+  if (a.partial != nullptr) {
+    if (tid == 0) a.w_flags[a.N] = 1;
+    return;
+  }
+  for (int item = blockIdx.x; item < a.items; item += gridDim.x) {      // (with no copy and no product under way, and nobody waiting)
+    const Piece p(a, item, BN);
+    fma_tile(*reinterpret_cast<OwnTile*>(smem), a, p.m0, BN, p.n0);
+  }
 }
 
 // The segments' sums, added in their order.
-__global__ void __launch_bounds__(256) add_segments_kernel(const F32Args a) {
+__global__ void __launch_bounds__(256, 8) add_segments_kernel(const F32Args a) {      // (32 registers: the sums wait for memory)
+  using Tile = FmaTile<256, 2, 2>;
+  __shared__ __align__(16) Tile sm;
   const long long total = (long long)a.M * a.N;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
     const int m = (int)(i / a.N), n = (int)(i - (long long)m * a.N);
     float v = a.partial[i];
 #pragma unroll 4
     for (int s = 1; s < a.segments; ++s) v += a.partial[i + s * total];
-    if (out_of_reach(a.w_largest[n]) || a.flags[m] != 0) v = fma_sum(a.A + (size_t)m * a.lda, a.W + (size_t)n * a.ldw, a.K);
-    a.C[(size_t)m * a.ldc + n] = v;
+    if (a.w_flags[n] == 0 && a.flags[m] == 0) a.C[(size_t)m * a.ldc + n] = v;
   }
+  if (a.w_flags[a.N] == 0) return;
+  const int across = (a.N + BM - 1) / BM, down = (a.M + Tile::AT_ONCE - 1) / Tile::AT_ONCE;
+  for (int t = blockIdx.x; t < across * down; t += gridDim.x) fma_tile(sm, a, t / across * Tile::AT_ONCE, Tile::AT_ONCE, t % across * BM);
 }
 
 // 2-D tensor [rows, cols] of floats, boxes of [box_rows x 32], 128-byte swizzle, zeros where a box reaches past the tensor
@@ -397,6 +492,7 @@ int launch(F32Args a, const __nv_bfloat16* parts, int ldp, const CUtensorMap& ma
   a.tok_tiles = (a.M + BN - 1) / BN;
   const long long items = (long long)a.tok_tiles * a.segments * ((a.N + BM - 1) / BM);
   DK_REQUIRE(items < (1ll << 30), "gemm_f32_tc: too many pieces");
+  static_assert(sizeof(OwnTile) <= Sizes<BN>::SMEM - 1024 && BN <= 160, "the rows out of reach take the stages' place");
   a.items = (int)items;
   gemm_f32_tc_kernel<BN><<<min(a.items, dk_sm_count()), THREADS, Sizes<BN>::SMEM, stream>>>(map_w, map_x, a);
   return 0;
@@ -434,8 +530,8 @@ extern "C" int dk_gemm_f32_tc_plan(int M, int N, int K, int* kilobytes, int* lau
   const Cut cut(N, K);
   const int slab = slab_rows(N, cut.segments);
   const long long rows = min(M, slab), ldp = (K + 7) / 8 * 8;
-  long long bytes = 6 * rows * ldp + 4 * rows + 16;
-  if (cut.segments > 1) bytes += 4ll * N + 16 + 4ll * cut.segments * rows * N;
+  long long bytes = 6 * rows * ldp + 4 * rows + 16 + 4ll * N + 32;
+  if (cut.segments > 1) bytes += 4ll * cut.segments * rows * N;
   *kilobytes = (int)((bytes + 1023) / 1024);
   *launches = (M + slab - 1) / slab * (cut.segments > 1 ? 3 : 2);
   return 0;
@@ -464,11 +560,10 @@ extern "C" int dk_gemm_f32_tc(const void* A, const void* W, void* C, void* work,
     auto* parts = (__nv_bfloat16*)work;
     int* flags = (int*)(parts + 3ll * a.M * ldp);
     a.flags = flags;
-    if (cut.segments > 1) {
-      a.w_largest = (uint32_t*)(flags + (a.M + 3) / 4 * 4);
-      a.partial = (float*)(a.w_largest + (N + 3) / 4 * 4);
-    }
-    split_rows_kernel<<<a.M, 256, 0, stream>>>(a.A, lda, parts, flags, a.w_largest, a.M, N, K, ldp, (uintptr_t)a.A % 16 == 0 && lda % 4 == 0);
+    a.w_flags = flags + (a.M + 3) / 4 * 4;
+    if (cut.segments > 1) a.partial = (float*)(a.w_flags + N / 4 * 4 + 4);
+    a.vec = (uintptr_t)a.A % 16 == 0 && lda % 4 == 0;
+    split_rows_kernel<<<a.M, 256, 0, stream>>>(a.A, lda, parts, flags, a.w_flags, a.M, N, K, ldp, a.vec);
     // Tokens of a piece: a chunk takes 12 cycles a token on the tensor cores, and about 1,500 whatever their number (24 products' issue, W's
     // way into parts).  Least rounds of pieces times that.
     const int sizes[] = {160, 128, 96, 64, 48, 32, 16};

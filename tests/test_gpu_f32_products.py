@@ -77,3 +77,32 @@ def test_gemm_f32_tc_refuses_what_it_does_not_take():
         assert not o.gemm_f32_tc_supported(w)
     with pytest.raises(o.KernelError):
         o.gemm_f32_tc(torch.empty(2, 1020, device=DEV), ok, torch.empty(2, 8, device=DEV))
+
+
+@pytest.mark.parametrize("M, N, K", [(300, 2048, 2048), (300, 9600, 1024), (1, 12000, 2048), (161, 9500, 1028)])
+def test_gemm_f32_tc_rows_out_of_reach_take_about_the_plain_kernels_time(M, N, K):
+    """A prompt of rows that hold a NaN, and one whose weights do: the plain kernel's bits, without every output being summed by a thread of its own."""
+    g = torch.Generator(device=DEV).manual_seed(4)
+    a, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(N, K, device=DEV, generator=g)
+    a[:, 5] = math.nan
+    a[M // 2, 5] = 2.0 ** 80
+    w[N - 1, 3] = math.inf
+    out, plain = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    o = ops()
+
+    def took(f):
+        f()
+        best = math.inf
+        for _ in range(5):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            f()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+    t, p = took(lambda: o.gemm_f32_tc(a, w, out)), took(lambda: o.gemm_nt_plain(a, w, plain))
+    assert torch.equal(torch.nan_to_num(out, nan=1.0), torch.nan_to_num(plain, nan=1.0)) and torch.equal(out.isnan(), plain.isnan())
+    assert bool(out[M // 2, :N - 1].isfinite().all())
+    print(f"{M} x {N} x {K}: {t * 1e3:.0f} us, plain {p * 1e3:.0f}")
+    assert t < 4 * p + 0.2      # (a thread an output reads a row of W of its own, 4 bytes at a time: tens of times the plain kernel's time)
