@@ -1,26 +1,29 @@
-// 32-bit product  C[M,N] = A[M,K] * W[N,K]^T  on the fifth-generation tensor cores, with no fewer bits than 32-bit sums have.
+// 32-bit product  C[M,N] = A[M,K] * W[N,K]^T  on the fifth-generation tensor cores, operands in three exact bfloat16 parts.
 //
-// A 32-bit number is three bfloat16 parts exactly (eight bits of the mantissa each, cut off), x = x1 + x2 + x3, and products of parts are
-// exact in 32 bit.  Of the nine products of parts six are made; the three left out are below 2^-24 of a term.  A tensor core cuts off what
-// it adds to its accumulator, so a sum stays there for 64 entries of K only, the small products before the large: every chunk of 64 begins
-// at zero and is added to 32-bit sums in registers, rounded to nearest.  The order of a sum depends on nothing but W's sizes: a token's result
-// has the same bits whatever shares its step.  Against 64 bits (2-norm, normal operands) sums of 2,048 / 5,504 products are 1.6e-7 / 1.5e-7
-// off, chains of fused multiply-adds (gemm_plain.cu) 8.1e-7 / 1.3e-6.
+// A 32-bit number is three bfloat16 parts exactly (each what the parts before it leave, rounded to nearest), x = x1 + x2 + x3, and products of parts
+// are exact in 32 bit.  Of the nine products of parts six are made; the three left out are at most 2^-24 of a term together, of either sign, 2^-26.5 in
+// the mean square (a multiply-add's rounding: 2^-24.3).  A tensor core cuts off what it adds to its accumulator, so the high parts' products, of which a sum
+// of 24 bits holds nearly all, have one of their own, which begins at zero every 64 entries of K; the other five, 2^-8 of those, are kept together for
+// KEEP chunks.  Either is added to 32-bit sums in registers, rounded to nearest.  The order of a sum depends on nothing but W's sizes: a token's result
+// has the same bits whatever shares its step.  Errors against 64 bits (2-norm), and those of chains of fused multiply-adds (gemm_plain.cu): normal operands,
+// K of 1,024 to 11,008, 1.0e-7 to 1.5e-7 and 5.7e-7 to 18.8e-7; rows that one or four entries dominate 1.3e-7 to 1.7e-7 and 5.8e-7 to 18.5e-7; operands of one
+// sign 0.5e-7 to 1.0e-7 and 4.4e-7 to 16.1e-7; rows of four entries 0.44e-7 to 0.47e-7 and 0.40e-7 to 0.41e-7; a single product is off by 2^-23 of it at most.
 //   1. split_rows: the tokens' rows as three bfloat16 arrays, and which rows are out of the parts' reach;
 //   2. the product: W's rows are the M side (128 lanes), tokens the N side of the tiles.  One persistent block per SM:
 //      warp 0       fetches W (32 bit, TMA, 128-byte swizzle), warp 2 the tokens' parts (a box each, a ring of its own),
-//      warps 4-7    turn W into parts: a thread holds a row, and its parts go straight into tensor memory as an MMA's first operand, so that the
+//      warps 4-11   turn W into parts: a thread holds half of a row, and its parts go straight into tensor memory as an MMA's first operand, so that the
 //                   shared memory's bandwidth is left to the tokens' parts,
-//      warp 1       issues 24 products a chunk into one of two accumulators,
-//      warps 8-15   add finished chunks to the sums in registers and store them;
+//      warp 1       issues 24 products a chunk, four of them the high parts',
+//      warps 12-19  add finished chunks to the sums in registers and store them;
 //   3. add_segments, where K is cut into segments (W of few tiles): their sums in order.
-// Rows with infinite or NaN entries, or whose largest entry is outside 2^-40 .. 2^60 (parts or their products would leave the exponent's
-// range), are found on the way, and their results are summed by FMA over k instead, a tile at a time, when nothing waits any more: by the product's own
-// blocks behind their pieces, or by add_segments.
-// Bound by the products' issue: a chunk takes about 1,500 cycles for up to 120 tokens (24 MMAs, each waited for by what converts the chunk after
-// next), 12 a token above.  Everything cold, microseconds, against the tiles of gemm_plain.cu: 300 x 2,048 x 2,048 107 -> 40, 300 x 11,008 x 2,048
-// 317 -> 126, 300 x 2,048 x 5,504 274 -> 66, 300 x 32,000 x 2,048 930 -> 240, 2,048 x 22,016 x 4,096 7,590 -> 2,020 (183 TFLOP/s); one row: 44 -> 28,
-// 76 -> 66, 106 -> 40, 137 -> 120, and 207 -> 220 with 22,016 x 4,096 (172 tiles in two rounds).
+// Rows with infinite or NaN entries, or whose largest entry is outside 2^-40 .. 2^29, are found on the way, and their results are summed by FMA over k
+// instead, a tile at a time, when nothing waits any more: by the product's own blocks behind their pieces, or by add_segments.
+// A chunk takes about 1,650 cycles for few tokens, the converting warps' own time, and 2,500 for 160 of them: 24 products, and one chunk in four waits for
+// sums that are being read.  Parts that are rounded cost half as much again as parts that are cut off, so eight warps make them and not four; a product's
+// operands reach it from one elected thread in 50 to 80 cycles (in a branch for lane 0 in 100, which bound everything), and one wait stands for all that
+// a chunk needs.  Everything cold, microseconds, against the tiles of gemm_plain.cu: 300 x 2,048 x 2,048 107 -> 40, 300 x 11,008 x 2,048 317 -> 97,
+// 300 x 2,048 x 5,504 274 -> 63, 300 x 32,000 x 2,048 930 -> 212, 2,048 x 22,016 x 4,096 7,590 -> 1,690 (218 TFLOP/s); one row: 44 -> 24, 76 -> 46,
+// 107 -> 34, 139 -> 83, and 203 -> 138 with 22,016 x 4,096.
 //
 // Every wait on an mbarrier is bounded: when one gives up, the kernel records it, stores nothing more, waits (bounded again) for the copies and
 // products that it has under way, frees its tensor memory and returns.
@@ -32,25 +35,35 @@
 namespace {
 constexpr int BM = 128;                 // rows of W of a piece
 constexpr int KC = 64;                  // entries of K of a chunk
-constexpr int THREADS = 512;
+constexpr int THREADS = 640, CONVERT = 4, STORE = 12;      // the first warp that turns W into parts, that adds up and stores
 constexpr int W_STAGE = BM * KC * 4;
 constexpr int MAX_W = 6, MAX_X = 12;
 constexpr int SMEM_ROOM = 222 * 1024;
 constexpr int TMEM_COLS = 512;
+constexpr int KEEP = 4;                 // chunks for which the products of other parts than the high ones stay in tensor memory
 constexpr int A_COLS = 3 * KC / 2;      // tensor memory of a chunk of W in parts
 constexpr int MOST_ROWS = 16384;        // of A in a launch
 constexpr long long MOST_PARTIAL = 32ll << 20;      // floats of the segments' sums
 
-// The largest magnitude's bits: zero is in reach, infinities and NaNs are not.
-__device__ __forceinline__ bool out_of_reach(uint32_t largest) { return largest != 0 && (largest < (127u - 40u) << 23 || largest >= (127u + 60u) << 23); }
+// A row is in reach of the parts if its largest entry is zero or lies in 2^-40 .. 2^29.  Operands are multiplied by 2^24 first (the results by
+// 2^-48): the last part of the smallest entry is still a normal bfloat16 number, and 2^20 products of two numbers in reach stay below the exponent's
+// range.
+constexpr float SCALE = 16777216.f, UNSCALE = 1.f / 16777216.f / 16777216.f;
+__device__ __forceinline__ bool out_of_reach(uint32_t largest) { return largest != 0 && (largest < (127u - 40u) << 23 || largest >= (127u + 29u) << 23); }
 
+// Two numbers' parts, each rounded to nearest: what a part leaves fits the two after it, and the products that are left out have either sign.
+__device__ __forceinline__ uint32_t nearest(float x, float y) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 __device__ __forceinline__ void parts_of(float x, float y, uint32_t& high, uint32_t& middle, uint32_t& low) {
-  const uint32_t bx = __float_as_uint(x), by = __float_as_uint(y);
-  high = __byte_perm(bx, by, 0x7632);
-  const float rx = x - __uint_as_float(bx & 0xffff0000u), ry = y - __uint_as_float(by & 0xffff0000u);
-  const uint32_t cx = __float_as_uint(rx), cy = __float_as_uint(ry);
-  middle = __byte_perm(cx, cy, 0x7632);
-  low = __byte_perm(__float_as_uint(rx - __uint_as_float(cx & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(cy & 0xffff0000u)), 0x7632);
+  x *= SCALE;
+  y *= SCALE;
+  high = nearest(x, y);
+  x -= __uint_as_float(high << 16);
+  y -= __uint_as_float(high & 0xffff0000u);
+  middle = nearest(x, y);
+  low = nearest(x - __uint_as_float(middle << 16), y - __uint_as_float(middle & 0xffff0000u));
 }
 
 // grid (rows): parts [3][M][K] and a row's flag; the flags of W's rows, and the one behind them, begin at zero.
@@ -94,7 +107,9 @@ struct Sizes {
   static constexpr int SMEM = WS * W_STAGE + XS * X_STAGE + 1024;
   static_assert(XS >= 6, "two chunks of parts");
   static constexpr int D_COLS = (BN + 31) / 32 * 32;
-  static_assert(2 * D_COLS + 2 * A_COLS <= TMEM_COLS, "two accumulators beside two chunks of W");
+  // Accumulators of the products of high parts, and of the others: two of either, as far as there is room beside two chunks of W.
+  static constexpr int HIGH = 3 * D_COLS + 2 * A_COLS <= TMEM_COLS ? 2 : 1, REST = 4 * D_COLS + 2 * A_COLS <= TMEM_COLS ? 2 : 1;
+  static_assert((HIGH + REST) * D_COLS + 2 * A_COLS <= TMEM_COLS, "accumulators beside two chunks of W");
 };
 
 struct F32Args {
@@ -126,7 +141,7 @@ struct Piece {
 // Results out of the parts' reach, for `most` tokens from m0 on and 128 rows of W from n0 on: the rows of A that need it, by the rows of W, every sum in the
 // plain kernel's order over k.  A thread has EACH tokens by four rows of W; both come by cp.async, STAGES - 1 steps of K ahead.  Bound by the reads of
 // shared memory (four cycles a sixteen-byte load, whatever its lanes share).
-// 300 rows with a NaN each by 2,048 x 2,048 and 9,600 x 1,024: 201 and 364 us in all (gemm_plain.cu alone 106 and 186); one by 12,000 x 2,048 169 (74).
+// 300 rows with a NaN each by 2,048 x 2,048 and 9,600 x 1,024: 227 and 323 us in all (gemm_plain.cu alone 105 and 186); one by 12,000 x 2,048 146 (75).
 constexpr int FMA_K = 16, FMA_LD = FMA_K + 4;
 template <int T, int EACH, int STAGES>
 struct FmaTile {
@@ -218,34 +233,38 @@ __device__ __forceinline__ void fma_tile(FmaTile<T, EACH, STAGES>& sm, const F32
   }
   __syncthreads();      // (the list is another tile's next)
 }
-using OwnTile = FmaTile<THREADS, 8, 4>;
+using OwnTile = FmaTile<THREADS, 7, 4>;
 
 template <int BN>
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                                                                  const F32Args a) {
   constexpr int WS = Sizes<BN>::WS, XS = Sizes<BN>::XS, X_STAGE = Sizes<BN>::X_STAGE, D_COLS = Sizes<BN>::D_COLS, NC = BN / 2;
+  constexpr int HIGH = Sizes<BN>::HIGH, REST = Sizes<BN>::REST;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* xs = smem + WS * W_STAGE;
-  __shared__ __align__(8) unsigned long long bars[2 * MAX_W + 2 * MAX_X + 6];
+  __shared__ __align__(8) unsigned long long bars[2 * MAX_W + 2 * MAX_X + 10];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int failed, odd;      // odd: some row of the block's pieces is out of reach
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t wfull = s2u(&bars[0]), wempty = s2u(&bars[MAX_W]), xfull = s2u(&bars[2 * MAX_W]), xempty = s2u(&bars[2 * MAX_W + MAX_X]);
   const uint32_t afull = s2u(&bars[2 * MAX_W + 2 * MAX_X]), done = afull + 16, dempty = afull + 32;
+  const uint32_t rdone = afull + 48, rempty = afull + 64;      // the rest's sums are complete; have been read
   if (tid == 0) {
     for (int s = 0; s < WS; ++s) {
       mbar_init(wfull + 8 * s, 1);
-      mbar_init(wempty + 8 * s, 4);
+      mbar_init(wempty + 8 * s, STORE - CONVERT);
     }
     for (int s = 0; s < XS; ++s) {
       mbar_init(xfull + 8 * s, 1);
       mbar_init(xempty + 8 * s, 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(afull + 8 * b, 4);
+      mbar_init(afull + 8 * b, STORE - CONVERT);
       mbar_init(done + 8 * b, 1);
       mbar_init(dempty + 8 * b, 8);
+      mbar_init(rdone + 8 * b, 1);
+      mbar_init(rempty + 8 * b, 8);
     }
     failed = odd = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -254,7 +273,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot, tmem_a = tmem_base + 2 * D_COLS;
+  const uint32_t tmem_base = tmem_base_slot, tmem_rest = tmem_base + HIGH * D_COLS, tmem_a = tmem_rest + REST * D_COLS;
   volatile int* gave_up = &failed;
 
   if (warp == 0) {
@@ -301,43 +320,65 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
     }
   } else if (warp == 1) {
     const uint32_t idesc = instr_desc_bf16(BM, BN);
-    int c = 0;
+    int c = 0, rest = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const Piece p(a, item, BN);
       for (int k = 0; k < p.chunks; ++k, ++c) {
-        const int b = c & 1, x = 3 * c;
-        bool there = true;      // a lane waits for each of what a chunk needs: one after the other the waits took as long as the products
-        if (lane == 0) there = c < 2 || mbar_wait(dempty + 8 * b, ring_parity(c - 2, 2));
-        else if (lane == 1) there = mbar_wait(afull + 8 * b, ring_parity(c, 2));
-        else if (lane < 5) there = mbar_wait(xfull + 8 * ring_slot(x + lane - 2, XS), ring_parity(x + lane - 2, XS));
+        const int b = c & 1, x = 3 * c, first = k % KEEP == 0;
+        // a lane waits for each of what a chunk needs, all at once: in a branch of its own for each the waits took 870 cycles
+        const int part = x + min(max(lane - 2, 0), 2);
+        uint32_t bar = xfull + 8 * ring_slot(part, XS), parity = ring_parity(part, XS);
+        if (lane == 0 && first && rest >= REST) bar = rempty + 8 * ((rest - REST) & 1), parity = ring_parity(rest - REST, 2);
+        if (lane == 1) bar = afull + 8 * b, parity = ring_parity(c, 2);
+        bool there = mbar_wait(bar, parity);
         if (__any_sync(0xffffffffu, !there)) {
           *gave_up = 1;
           ok = false;
           break;
         }
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t wa = tmem_a + b * A_COLS, d = tmem_base + b * D_COLS;
+        const uint32_t wa = tmem_a + b * A_COLS, xlast = xempty + 8 * ring_slot(x + 2, XS);
+        const auto multiply = [&](uint32_t d, int q, int r, bool add) {      // the tokens' part q with W's part r
+          const uint64_t db = smem_desc_k_major(s2u(xs + (size_t)ring_slot(x + 2 - q, XS) * X_STAGE));
 #pragma unroll
-          for (int q = 2; q >= 0; --q) {      // the tokens' part q with W's parts 2 - q .. 0, the smallest first
-            const int s = ring_slot(x + 2 - q, XS);
-            const uint64_t db = smem_desc_k_major(s2u(xs + (size_t)s * X_STAGE));
-#pragma unroll
-            for (int r = 2 - q; r >= 0; --r)
-#pragma unroll
-              for (int i = 0; i < KC / 16; ++i)
-                umma_a_tmem(d, wa + r * (KC / 2) + i * 8, db + (uint64_t)(i * 2), idesc, (q == 2 && i == 0) ? 0u : 1u);
-            umma_commit(xempty + 8 * s);
-          }
-          umma_commit(done + 8 * b);
+          for (int i = 0; i < KC / 16; ++i) umma_a_tmem(d, wa + r * (KC / 2) + i * 8, db + (uint64_t)(i * 2), idesc, (add || i > 0) ? 1u : 0u);
+        };
+        if (elect_one()) {      // the smallest products first
+          const uint32_t d = tmem_rest + rest % REST * D_COLS;
+          multiply(d, 2, 0, !first);
+          umma_commit(xempty + 8 * ring_slot(x, XS));
+          multiply(d, 1, 1, true);
+          multiply(d, 1, 0, true);
+          umma_commit(xempty + 8 * ring_slot(x + 1, XS));
+          multiply(d, 0, 2, true);
+          multiply(d, 0, 1, true);
         }
         __syncwarp();
+        if (k % KEEP == KEEP - 1 || k + 1 == p.chunks) {
+          if (elect_one()) umma_commit(rdone + 8 * (rest & 1));
+          ++rest;
+        }
+        there = c < HIGH || mbar_wait(dempty + 8 * ((c - HIGH) & 1), ring_parity(c - HIGH, 2));
+        const bool go = !__any_sync(0xffffffffu, !there);
+        tc_fence_after();
+        if (elect_one()) {
+          if (go) multiply(tmem_base + c % HIGH * D_COLS, 0, 0, false);
+          umma_commit(xlast);
+          if (go) umma_commit(done + 8 * b);
+        }
+        __syncwarp();
+        if (!go) {
+          *gave_up = 1;
+          ok = false;
+          ++c;
+          break;
+        }
       }
     }
     if (lane == 0) ring_drain(3 * c, XS, [&](int s, uint32_t parity) { return mbar_wait(xempty + 8 * s, parity); });      // its products are complete
-  } else if (warp >= 4 && warp < 8) {
-    const int row = tid & 127;
+  } else if (warp >= CONVERT && warp < STORE) {
+    const int row = tid & 127, half = (warp - CONVERT) >> 2;      // 32 of a row's 64 entries
     int c = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
@@ -354,22 +395,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         tc_fence_after();
         const unsigned char* from = smem + (size_t)s * W_STAGE + row * 128;
         const uint32_t to = tmem_a + b * A_COLS + ((uint32_t)((warp & 3) * 32) << 16);
+        uint32_t h[16], m[16], l[16];
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t h[16], m[16], l[16];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 v = *reinterpret_cast<const float4*>(from + half * (W_STAGE / 2) + ((j ^ (row & 7)) << 4));
-            parts_of(v.x, v.y, h[2 * j], m[2 * j], l[2 * j]);
-            parts_of(v.z, v.w, h[2 * j + 1], m[2 * j + 1], l[2 * j + 1]);
-            largest = max(largest, max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
-                                       max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu)));
-          }
-          tmem_st16(to + half * 16, h);
-          tmem_st16(to + KC / 2 + half * 16, m);
-          tmem_st16(to + KC + half * 16, l);
+        for (int j = 0; j < 8; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(from + half * (W_STAGE / 2) + ((j ^ (row & 7)) << 4));
+          parts_of(v.x, v.y, h[2 * j], m[2 * j], l[2 * j]);
+          parts_of(v.z, v.w, h[2 * j + 1], m[2 * j + 1], l[2 * j + 1]);
+          largest = max(largest, max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
+                                     max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu)));
         }
-        if (k + 1 == p.chunks && out_of_reach(largest) && p.n0 + row < a.N) {
+        tmem_st16(to + half * 16, h);
+        tmem_st16(to + KC / 2 + half * 16, m);
+        tmem_st16(to + KC + half * 16, l);
+        if (k + 1 == p.chunks && out_of_reach(largest) && p.n0 + row < a.N) {      // (what the thread saw of the row: half of the piece's K)
           a.w_flags[p.n0 + row] = 1;
           odd = 1;
         }
@@ -382,10 +420,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         }
       }
     }
-  } else if (warp >= 8) {
-    const int quarter = warp & 3, half = (warp - 8) >> 2;
+  } else if (warp >= STORE) {
+    const int quarter = warp & 3, half = (warp - STORE) >> 2;
     const int row = quarter * 32 + lane;
-    int c = 0;
+    int c = 0, rest = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
       const Piece p(a, item, BN);
@@ -394,35 +432,43 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
 #pragma unroll
       for (int j = 0; j < NC; ++j) sum[j] = 0.f;
       for (int k = 0; k < p.chunks; ++k, ++c) {
-        const int b = c & 1;
-        const bool there = mbar_wait(done + 8 * b, ring_parity(c, 2)) && *gave_up == 0;
-        if (__any_sync(0xffffffffu, !there)) {
-          *gave_up = 1;
-          ok = false;
-          break;
+        const bool all = k % KEEP == KEEP - 1 || k + 1 == p.chunks;      // the rest is complete, too
+#pragma unroll 1
+        for (int high = all ? 0 : 1; high < 2; ++high) {
+          const int use = high ? c : rest++;
+          const bool there = mbar_wait((high ? done : rdone) + 8 * (use & 1), ring_parity(use, 2)) && *gave_up == 0;
+          if (__any_sync(0xffffffffu, !there)) {
+            *gave_up = 1;
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t at = (high ? tmem_base + use % HIGH * D_COLS : tmem_rest + use % REST * D_COLS) + half * NC + ((uint32_t)(quarter * 32) << 16);
+          constexpr int G = NC > 64 ? 8 : NC > 48 ? 16 : 32;      // columns on their way at a time: as many as there are registers for
+#pragma unroll
+          for (int g = 0; g < NC; g += G) {
+            float v[G];
+#pragma unroll
+            for (int j = 0; j < G; j += 8)
+              if (g + j < NC) tmem_ld8_nowait(at + g + j, v + j);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < G; ++j)
+              if (g + j < NC) sum[g + j] += v[j];
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive((high ? dempty : rempty) + 8 * (use & 1));
         }
-        tc_fence_after();
-        const uint32_t at = tmem_base + b * D_COLS + half * NC + ((uint32_t)(quarter * 32) << 16);
-        constexpr int G = NC % 40 == 0 ? 40 : NC % 32 == 0 ? 32 : NC;      // columns on their way at a time
-#pragma unroll
-        for (int g = 0; g < NC; g += G) {
-          float v[G];
-#pragma unroll
-          for (int j = 0; j < G; j += 8) tmem_ld8_nowait(at + g + j, v + j);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < G; ++j) sum[g + j] += v[j];
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(dempty + 8 * b);
+        if (!ok) break;
       }
       if (!ok) break;
       float* to = a.partial != nullptr ? a.partial + (size_t)p.segment * a.M * a.N : a.C;
       const int ld = a.partial != nullptr ? a.N : a.ldc;
+      const float unscale = a.partial != nullptr ? 1.f : UNSCALE;
 #pragma unroll
       for (int j = 0; j < NC; ++j)
-        if (n < a.N && m0 + j < a.M) to[(size_t)(m0 + j) * ld + n] = sum[j];
+        if (n < a.N && m0 + j < a.M) to[(size_t)(m0 + j) * ld + n] = sum[j] * unscale;
     }
   } else if (warp == 3) {      // looks for tokens out of reach meanwhile
     bool mine = false;
@@ -459,7 +505,7 @@ __global__ void __launch_bounds__(256, 8) add_segments_kernel(const F32Args a) {
     float v = a.partial[i];
 #pragma unroll 4
     for (int s = 1; s < a.segments; ++s) v += a.partial[i + s * total];
-    if (a.w_flags[n] == 0 && a.flags[m] == 0) a.C[(size_t)m * a.ldc + n] = v;
+    if (a.w_flags[n] == 0 && a.flags[m] == 0) a.C[(size_t)m * a.ldc + n] = v * UNSCALE;
   }
   if (a.w_flags[a.N] == 0) return;
   const int across = (a.N + BM - 1) / BM, down = (a.M + Tile::AT_ONCE - 1) / Tile::AT_ONCE;
@@ -564,20 +610,23 @@ extern "C" int dk_gemm_f32_tc(const void* A, const void* W, void* C, void* work,
     if (cut.segments > 1) a.partial = (float*)(a.w_flags + N / 4 * 4 + 4);
     a.vec = (uintptr_t)a.A % 16 == 0 && lda % 4 == 0;
     split_rows_kernel<<<a.M, 256, 0, stream>>>(a.A, lda, parts, flags, a.w_flags, a.M, N, K, ldp, a.vec);
-    // Tokens of a piece: a chunk takes 12 cycles a token on the tensor cores, and about 1,500 whatever their number (24 products' issue, W's
-    // way into parts).  Least rounds of pieces times that.
-    const int sizes[] = {160, 128, 96, 64, 48, 32, 16};
+    // Tokens of a piece: a chunk takes 12 cycles a token on the tensor cores, and about 2,000 whatever their number (W's way into parts, 24 products'
+    // issue).  Least rounds of pieces times that, and the fewest tokens that give it: more stages of W beside them.
+    const int sizes[] = {160, 144, 128, 112, 96, 80, 64, 48, 32, 16};
     int best = 0;
     long long least = 0;
     for (int bn : sizes) {
-      const long long items = (long long)((a.M + bn - 1) / bn) * cut.segments * ((N + BM - 1) / BM), cost = (items + sms - 1) / sms * max(12 * bn, 1500);
-      if (best == 0 || cost < least) { best = bn; least = cost; }
+      const long long items = (long long)((a.M + bn - 1) / bn) * cut.segments * ((N + BM - 1) / BM), cost = (items + sms - 1) / sms * max(12 * bn, 2000);
+      if (best == 0 || cost <= least) { best = bn; least = cost; }
     }
     int rc = 0;
     switch (best) {
       case 160: rc = launch<160>(a, parts, ldp, map_w, stream); break;
+      case 144: rc = launch<144>(a, parts, ldp, map_w, stream); break;
       case 128: rc = launch<128>(a, parts, ldp, map_w, stream); break;
+      case 112: rc = launch<112>(a, parts, ldp, map_w, stream); break;
       case 96: rc = launch<96>(a, parts, ldp, map_w, stream); break;
+      case 80: rc = launch<80>(a, parts, ldp, map_w, stream); break;
       case 64: rc = launch<64>(a, parts, ldp, map_w, stream); break;
       case 48: rc = launch<48>(a, parts, ldp, map_w, stream); break;
       case 32: rc = launch<32>(a, parts, ldp, map_w, stream); break;

@@ -106,3 +106,71 @@ def test_gemm_f32_tc_rows_out_of_reach_take_about_the_plain_kernels_time(M, N, K
     assert bool(out[M // 2, :N - 1].isfinite().all())
     print(f"{M} x {N} x {K}: {t * 1e3:.0f} us, plain {p * 1e3:.0f}")
     assert t < 4 * p + 0.2      # (a thread an output reads a row of W of its own, 4 bytes at a time: tens of times the plain kernel's time)
+
+
+def one(bits):
+    return torch.tensor([bits], dtype=torch.int32).view(torch.float32).item()
+
+
+@pytest.mark.parametrize("N", [300, 9500])
+def test_gemm_f32_tc_a_single_product_is_rounded_once(N):
+    """Rows of one entry: the products left out are below 2^-24 of it, and the sum of those that are made is rounded once."""
+    g = torch.Generator(device=DEV).manual_seed(2)
+    K, M = 1024, 40
+    at = torch.randint(0, K, (M,), device=DEV, generator=g)
+    a = torch.zeros(M, K, device=DEV)
+    a[torch.arange(M), at] = torch.randn(M, device=DEV, generator=g)
+    w = torch.randn(N, K, device=DEV, generator=g)
+    a[7, at[7]] = w[0] = one(0x3f80ffff)      # parts that are cut off leave 2^-7 and 2^-15 behind the first two
+    out = run(a, w)
+    ref = a.double() @ w.double().T
+    assert bool(((out.double() - ref).abs() <= 2.0 ** -23 * ref.abs()).all())
+
+
+@pytest.mark.parametrize("kind", ["one large entry", "four large entries", "few entries", "positive", "one sign a row"])
+@pytest.mark.parametrize("N, K", [(600, 2048), (9600, 1024), (4100, 11008)])
+def test_gemm_f32_tc_is_no_further_off_than_multiply_adds(kind, N, K):
+    """Rows that a few entries dominate, and operands of one sign, where errors of one sign would add up: 2-norm and mean of the error against 64 bits."""
+    g = torch.Generator(device=DEV).manual_seed(K)
+    M = 64
+    a, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(N, K, device=DEV, generator=g) * 0.05
+    far = torch.rand(M, K, device=DEV, generator=g)
+    if kind == "one large entry":
+        a.scatter_(1, far.topk(1).indices, 3000.0)
+    elif kind == "four large entries":
+        a.mul_(torch.where(far >= far.topk(4).values[:, -1:], 1000.0, 1.0))
+    elif kind == "few entries":
+        a.mul_(far >= far.topk(4).values[:, -1:])
+    elif kind == "positive":
+        a, w = far + 1.0, torch.rand(N, K, device=DEV, generator=g) + 1.0
+    else:
+        a, w = a.abs() * torch.where(torch.arange(M, device=DEV) % 2 == 0, 1.0, -1.0)[:, None], w.abs()
+    out, plain = run(a, w), torch.empty(M, N, device=DEV)
+    ops().gemm_nt_plain(a, w, plain)
+    ref = a.double() @ w.double().T
+    e, p = (out.double() - ref) / ref.norm(), (plain.double() - ref) / ref.norm()
+    mean = ((out.double() - ref) / ref).mean()
+    print(f"{kind} {N} x {K}: {e.norm():.3g} against {p.norm():.3g}, mean {mean:.3g}")
+    # What is left out of a term is up to 2^-24 of it, 2^-26.5 in the mean square, beside its rounding of 2^-24.3: 2.3 % of the error where a row is hardly more
+    # than a term.  Four terms are four roundings either way, here of a term's high parts' sum and there of a sum's: a quarter for that.
+    assert e.norm() <= (1.25 if kind == "few entries" else 1.03) * p.norm()
+    if kind in ("positive", "one sign a row"):
+        # the relative error's mean: a chunk's sum is cut off after each of its four steps, at a quarter, half, three quarters and all of it, by half of 2^-23 on average
+        # where its terms have more bits than the sum has room for
+        assert mean.abs() <= 2.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("N", [300, 9500])
+def test_gemm_f32_tc_small_entries_keep_their_bits(N):
+    """Entries far below their row's largest, which the weights do not read: down to 2^-126 they have all of their 24 bits."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    K, M = 1024, 33
+    a, w = torch.randn(M, K, device=DEV, generator=g), torch.zeros(N, K, device=DEV)
+    col = torch.randint(0, K, (N,), device=DEV, generator=g)
+    w[torch.arange(N), col] = 1.0 + torch.rand(N, device=DEV, generator=g)
+    small = torch.rand(M, K, device=DEV, generator=g) < 0.5
+    a[small] *= 2.0 ** -118
+    out = run(a, w)
+    ref = a.double() @ w.double().T
+    held = ref.abs() >= 2.0 ** -124      # (a result below has fewer than 24 bits itself)
+    assert bool(((out.double() - ref).abs() <= 2.0 ** -23 * ref.abs())[held].all()) and held.sum() > held.numel() // 2
