@@ -43,7 +43,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int KEEP = 4;                 // chunks for which the products of other parts than the high ones stay in tensor memory
 constexpr int A_COLS = 3 * KC / 2;      // tensor memory of a chunk of W in parts
 constexpr int MOST_ROWS = 16384;        // of A in a launch
-constexpr long long MOST_PARTIAL = 32ll << 20;      // floats of the segments' sums
+constexpr long long MOST_PARTS = 48ll << 20, MOST_PARTIAL = 64ll << 20;      // bytes of the tokens' parts and of the segments' sums
 
 // A row is in reach of the parts if its largest entry is zero or lies in 2^-40 .. 2^29.  Operands are multiplied by 2^24 first (the results by
 // 2^-48): the last part of the smallest entry is still a normal bfloat16 number, and 2^20 products of two numbers in reach stay below the exponent's
@@ -556,11 +556,12 @@ struct Cut {
     segments = (chunks + per - 1) / per;
   }
 };
-// Rows of A that one launch takes: they bound the working memory.
-int slab_rows(int N, int segments) {
-  if (segments == 1) return MOST_ROWS;
-  const long long rows = MOST_PARTIAL / ((long long)segments * N) / 32 * 32;
-  return (int)min((long long)MOST_ROWS, max(32ll, rows));
+// Rows of A that one launch takes: they bound the working memory to 113 MB and 4 bytes a row of W.  Every launch reads W
+// anew: 2,048 rows by 2,048 x 5,504 are three, 345 us in all, of which W's 45 MB take 7 each.
+int slab_rows(int N, int K, int segments) {
+  long long rows = min((long long)MOST_ROWS, MOST_PARTS / (6ll * ((K + 7) / 8 * 8)));
+  if (segments > 1) rows = min(rows, MOST_PARTIAL / (4ll * segments * N));
+  return (int)max(32ll, rows / 32 * 32);
 }
 }  // namespace
 
@@ -574,7 +575,7 @@ extern "C" int dk_gemm_f32_tc_supported(const void* W, int N, int K) {
 extern "C" int dk_gemm_f32_tc_plan(int M, int N, int K, int* kilobytes, int* launches) {
   DK_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32_tc: bad sizes M=%d N=%d K=%d", M, N, K);
   const Cut cut(N, K);
-  const int slab = slab_rows(N, cut.segments);
+  const int slab = slab_rows(N, K, cut.segments);
   const long long rows = min(M, slab), ldp = (K + 7) / 8 * 8;
   long long bytes = 6 * rows * ldp + 4 * rows + 16 + 4ll * N + 32;
   if (cut.segments > 1) bytes += 4ll * cut.segments * rows * N;
@@ -591,7 +592,7 @@ extern "C" int dk_gemm_f32_tc(const void* A, const void* W, void* C, void* work,
   DK_REQUIRE(work != nullptr && (uintptr_t)work % 16 == 0, "gemm_f32_tc: working memory must start on a 16-byte boundary");
   const int ldp = (K + 7) / 8 * 8, sms = dk_sm_count();
   const Cut cut(N, K);
-  const int slab = slab_rows(N, cut.segments);
+  const int slab = slab_rows(N, K, cut.segments);
   CUtensorMap map_w;
   DK_REQUIRE(make_tensor_map_f32(&map_w, W, N, K, ldw, BM), "gemm_f32_tc: cannot encode the tensor map of W");
   for (int m = 0; m < M; m += slab) {

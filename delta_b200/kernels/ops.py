@@ -182,25 +182,38 @@ def gemm_f32_tc_supported(w) -> bool:
     return w.dtype == torch.float32 and w.is_contiguous() and bool(_l.load().dk_gemm_f32_tc_supported(_ptr(w, "w"), w.shape[0], w.shape[1]))
 
 
-def gemm_f32_tc(a, w, out, err=None):
-    """out[M,N] = a[M,K] @ w[N,K]^T of 32-bit operands, exactly split into bfloat16 parts for the tensor cores: no operand or sum of fewer bits."""
+def _f32_plan(M, N, K):
+    plan = _f32_plans.get((M, N, K))
+    if plan is None:
+        kb, launches = C.c_int(), C.c_int()
+        _l.check(_l.load().dk_gemm_f32_tc_plan(M, N, K, C.byref(kb), C.byref(launches)), "gemm_f32_tc", 0)
+        if len(_f32_plans) >= 4096:
+            _f32_plans.clear()
+        plan = _f32_plans[(M, N, K)] = (kb.value * 1024, launches.value)
+    return plan
+
+
+def gemm_f32_tc_bytes(M, N, K) -> int:
+    """Bytes of working memory of a product of ``M`` rows: no more for more rows than one launch takes."""
+    return _f32_plan(M, N, K)[0]
+
+
+def gemm_f32_tc(a, w, out, err=None, work=None):
+    """out[M,N] = a[M,K] @ w[N,K]^T of 32-bit operands, exactly split into bfloat16 parts for the tensor cores.
+    ``work``: at least ``gemm_f32_tc_bytes`` of uint8 (allocated here when None)."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or tuple(out.shape) != (M, N) or not (a.dtype == w.dtype == out.dtype == torch.float32):
         raise KernelError(f"gemm: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)} or dtypes do not fit")
     if M == 0 or N == 0:
         return out
-    lib = _l.load()
-    plan = _f32_plans.get((M, N, K))
-    if plan is None:
-        kb, launches = C.c_int(), C.c_int()
-        _l.check(lib.dk_gemm_f32_tc_plan(M, N, K, C.byref(kb), C.byref(launches)), "gemm_f32_tc", 0)
-        if len(_f32_plans) >= 4096:
-            _f32_plans.clear()
-        plan = _f32_plans[(M, N, K)] = (kb.value * 1024, launches.value)
-    work = torch.empty(plan[0], dtype=torch.uint8, device=a.device)
-    _l.check(lib.dk_gemm_f32_tc(_ptr(a, "a"), _ptr(w, "w"), _ptr(out, "out"), _ptr(work, "work"), M, N, K, K, K, N,
-                                _ptr(err, "err", torch.int32), _stream()), "gemm_f32_tc", plan[1])
+    need, launches = _f32_plan(M, N, K)
+    if work is None:
+        work = torch.empty(need, dtype=torch.uint8, device=a.device)
+    elif work.numel() < need:
+        raise KernelError(f"gemm_f32_tc: {work.numel()} bytes of working memory are given, {need} are needed")
+    _l.check(_l.load().dk_gemm_f32_tc(_ptr(a, "a"), _ptr(w, "w"), _ptr(out, "out"), _ptr(work, "work", torch.uint8), M, N, K, K, K, N,
+                                      _ptr(err, "err", torch.int32), _stream()), "gemm_f32_tc", launches)
     return out
 
 

@@ -211,6 +211,24 @@ def swiglu_linear(ctx, x: torch.Tensor, w_gate_up: torch.Tensor):
     return out
 
 
+_f32_sizes: Dict[tuple, int] = {}      # (rows, most rows of a step, N, K) -> bytes
+
+
+def _f32_work(ctx, rows: int, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """The step's working memory for a 32-bit product: one buffer for all of them, in powers of two, so that what wider products leave behind is no more
+    than the last one.  (None for a context without a pool: the product allocates its own.)"""
+    scratch = getattr(ctx, "scratch", None)
+    if scratch is None:
+        return None
+    key = (rows, ctx.max_step_tokens, *w.shape)
+    size = _f32_sizes.get(key)
+    if size is None:
+        if len(_f32_sizes) >= 4096:
+            _f32_sizes.clear()
+        size = _f32_sizes[key] = 1 << (max(ops.gemm_f32_tc_bytes(m, *w.shape) for m in (rows, max(rows, ctx.max_step_tokens))) - 1).bit_length()
+    return scratch("linear.f32", (size,), torch.uint8)
+
+
 def linear(ctx, x: torch.Tensor, w: torch.Tensor, out_dtype=None) -> torch.Tensor:
     """x [T, K], w [N, K] -> [T, N] in ``out_dtype`` (the type of x by default)."""
     out_dtype = out_dtype or x.dtype
@@ -218,7 +236,7 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, out_dtype=None) -> torch.Tenso
     if x.dtype == torch.float32 or ("products" in ctx.plain_kernels):
         out = torch.empty((T, N), dtype=out_dtype, device=x.device)
         if T and out_dtype == torch.float32 and "products" not in ctx.plain_kernels and ops.gemm_f32_tc_supported(w):
-            ops.gemm_f32_tc(x, w, out, err=ctx.err)
+            ops.gemm_f32_tc(x, w, out, err=ctx.err, work=_f32_work(ctx, T, w))
         elif T:
             ops.gemm_nt_plain(x, w, out)
         return out

@@ -174,3 +174,23 @@ def test_gemm_f32_tc_small_entries_keep_their_bits(N):
     ref = a.double() @ w.double().T
     held = ref.abs() >= 2.0 ** -124      # (a result below has fewer than 24 bits itself)
     assert bool(((out.double() - ref).abs() <= 2.0 ** -23 * ref.abs())[held].all()) and held.sum() > held.numel() // 2
+
+
+def test_gemm_f32_tc_takes_its_memory_from_the_steps_pool():
+    """One buffer for all products of a model's steps, made at the first step for the longest one."""
+    from delta_b200.config import EngineConfig
+    from delta_b200.engine.step import ModelRunner, RowInput
+    config = dict(architectures=["YiForCausalLM"], model_type="llama", hidden_size=1024, num_hidden_layers=1, num_attention_heads=8, num_key_value_heads=2,
+                  intermediate_size=2816, vocab_size=8000, rms_norm_eps=1e-5, rope_theta=5e6, max_position_embeddings=512)
+    r = ModelRunner(config_json=config, seed=0, engine_config=EngineConfig(max_batch=2, max_seq_len=256, page_size=16, dtype="float32"))
+    slot = r.cache.acquire_slot()
+    r.cache.grow(slot, 256)
+    r.step([RowInput(slot, list(range(5)), 0, [4])])
+    buf = r._scratch["linear.f32"]
+    assert buf.numel() >= ops().gemm_f32_tc_bytes(5, 8000, 1024)
+    r.step([RowInput(slot, list(range(200)), 5, [199])])
+    r.step([RowInput(slot, list(range(20)), 205, [0])])
+    assert r._scratch["linear.f32"].data_ptr() == buf.data_ptr()
+    with pytest.raises(ops().KernelError, match="working memory"):
+        ops().gemm_f32_tc(torch.empty(2, 1024, device=DEV), torch.empty(8, 1024, device=DEV), torch.empty(2, 8, device=DEV),
+                          work=torch.empty(1024, dtype=torch.uint8, device=DEV))

@@ -77,3 +77,16 @@ def test_a_module_that_does_not_load_is_told(apart, tmp_path):
     (other / so.name).write_bytes(b"no module")
     with pytest.warns(RuntimeWarning, match="through ctypes"):
         assert native_calls.load(plain, other / "lib.so", signatures) is None
+
+
+@pytest.mark.parametrize("N, K", [(2048, 2048), (2048, 5504), (2048, 11008), (4096, 11008), (9472, 4096), (11008, 2048), (22016, 4096), (64000, 4096), (128, 1024)])
+def test_the_working_memory_of_32_bit_products_is_bounded(N, K):
+    """Prompts of any length: 128 MB and no more, and short ones in one pass over the weights."""
+    def plan(M):
+        kb, launches = C.c_int(), C.c_int()
+        assert lib.load().dk_gemm_f32_tc_plan(M, N, K, C.byref(kb), C.byref(launches)) == 0
+        return kb.value / 1024, launches.value
+    few = plan(1)[1]
+    assert plan(256)[1] == few
+    for M in (1, 300, 2048, 16384, 1 << 20):
+        assert plan(M)[0] <= 128
