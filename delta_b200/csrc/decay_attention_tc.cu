@@ -6,17 +6,18 @@
 //   2. scan:   S_c = lambda^n S_(c-1) + U_c along a row, element by element; the state BEFORE chunk c takes the place of U_c, the last one
 //              goes to the request's slot;
 //   3. out:    every chunk in parallel: what the state before it adds to its outputs.
-// Activated queries, keys and values, A and S are 32 bit.  They enter the products as three bfloat16 parts each, which give the number
-// exactly, and six of the nine products of parts are made; those left out are below 2^-25 of a term.  A tensor core cuts off
-// what it adds to its accumulator: a sum stays there for 64 of its 128 terms (32 in U), the small products before the large, and halves (quarters) are
-// added in 32 bit.  Powers come from the 64-bit decay, never divided by.  A chunk with infinite, NaN, very large or (a whole row of them) very small
-// numbers is summed by FMA instead.
+// Activated queries, keys and values, A and S are 32 bit.  They enter the products times 2^24 as three bfloat16 parts each, which give the number
+// exactly, and six of the nine products of parts are made; those left out are at most 2^-24 of a term together, of either sign.  A tensor core cuts off what
+// it adds to its accumulator: a sum stays there for 64 of its 128 terms (32 in U), the small products before the large, and halves (quarters) are
+// added in 32 bit.  Powers come from the 64-bit decay, never divided by.  A chunk with infinite, NaN or very large numbers is summed by FMA instead.
 //
 // A block has 16 warps that turn numbers into parts and one that issues products.  Queries and A go to tensor memory as the first operand: with both
 // operands in shared memory, 192 KB of it here, a product takes twice as long (its reads come at 64 bytes a cycle), as U's does.  Every wait is bounded; one that gives up is reported, the rest runs through.
 // Bound by turning numbers into parts (and activating them) between three products that wait for one another, one block an SM.  One row of 2,048
 // tokens, 16 heads: chunk 53 (two rounds of 128 blocks and more), scan 8, out 24 us; the FMA kernels in chunks of 64 63, 12 and 75.  Against 64 bits
-// (2-norm, 700 and 1,000 tokens): outputs 1.3e-7, states 0.8e-7 off, 1.9e-7 and 1.0e-7 there (with parts cut off instead of rounded 2.2e-7 and 1.3e-7).
+// (2-norm, 389 tokens): outputs 1.3e-7, states 0.6e-7 off, 2.0e-7 and 1.3e-7 there; rows that one entry dominates 1.8e-7 and 0.9e-7 (2.7e-7, 1.7e-7), operands
+// of one sign 1.1e-7 and 0.5e-7 (2.0e-7, 1.1e-7), queries and keys of 2^-57 1.4e-7 and 0.9e-7 (2.7e-7, 1.8e-7); with parts cut off instead of rounded, normal
+// operands, 2.2e-7 and 1.3e-7.
 #include "common.cuh"
 #include "tcgen05_helpers.cuh"
 #include "ring.cuh"
@@ -42,8 +43,17 @@ __device__ __forceinline__ float power(double x, int n) {
   return (float)r;
 }
 
-__device__ __forceinline__ bool too_large(uint32_t largest) { return largest >= (127u + 60u) << 23; }      // infinities and NaNs too
-__device__ __forceinline__ bool too_small(uint32_t largest) { return largest != 0 && largest < (127u - 90u) << 23; }
+// Operands are in reach of the parts below 2^20 (queries, keys, values) and 2^50 (the state).  They are multiplied by 2^24 first, and so is A = q . k
+// before it is an operand: the last part of the smallest number is still a normal bfloat16 number, and no product leaves the exponent's range.
+constexpr float SCALE = 16777216.f, UNSCALE = 1.f / 16777216.f / 16777216.f;
+constexpr int REACH = 20, STATE_REACH = 50;
+template <int EXPONENT>
+__device__ __forceinline__ bool out_of_reach(const float (&x)[32]) {      // infinities and NaNs too
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) m = max(m, __float_as_uint(x[i]) & 0x7fffffffu);
+  return m >= (127u + EXPONENT) << 23;
+}
 
 // Two numbers' parts, each rounded to nearest: what is left behind a part fits the two after it, so the three give the number, and the products
 // that are left out have either sign (with parts cut off they would all add to the error).
@@ -79,28 +89,11 @@ __device__ __forceinline__ void activate(float (&x)[32], const uint4 (&raw)[4], 
     }
   }
 }
-// Whether an entry is out of the parts' reach; `rows_too`: or all of a row's are very small.
-__device__ __forceinline__ bool out_of_reach(const float (&x)[32], bool rows_too, int lane) {
-  bool odd = false;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) m = max(m, __float_as_uint(x[8 * i + e]) & 0x7fffffffu);
-    if (rows_too) {      // the largest of the row, which half of the warp holds
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-      odd |= too_small(m);
-    }
-    odd |= too_large(m);
-  }
-  return odd;
-}
-// Rows times factor(row) as parts in shared memory: [row][entry], boxes of 64 entries with the 128-byte swizzle.
+// Rows times factor(row) times 2^24 as parts in shared memory: [row][entry], boxes of 64 entries with the 128-byte swizzle.
 template <typename F>
 __device__ __forceinline__ void parts_to_shared(unsigned char* to, int row, int piece, const float* x, F&& f) {
   unsigned char* at = to + (piece >> 3) * BOX + row * 128 + (((piece & 7) ^ (row & 7)) << 4);
-  const float w = f(row);
+  const float w = f(row) * SCALE;
   uint4 p[3];
   parts_of(x[0] * w, x[1] * w, p[0].x, p[1].x, p[2].x);
   parts_of(x[2] * w, x[3] * w, p[0].y, p[1].y, p[2].y);
@@ -115,21 +108,21 @@ __device__ __forceinline__ void rows_to_shared(unsigned char* to, const float (&
   for (int i = 0; i < 4; ++i) parts_to_shared(to, row_of(tid, i), tid & 15, x + 8 * i, f);
 }
 __device__ __forceinline__ float as_it_is(int) { return 1.f; }
-// 32 entries of a row as an MMA's first operand in tensor memory: a row a lane
-__device__ __forceinline__ void parts_to_tmem(uint32_t lanes, int group, const float (&x)[32]) {
+// 32 entries of a row times `scale` as an MMA's first operand in tensor memory: a row a lane
+__device__ __forceinline__ void parts_to_tmem(uint32_t lanes, int group, const float (&x)[32], float scale) {
 #pragma unroll
   for (int g = 0; g < 32; g += 16) {
     uint32_t h[8], m[8], l[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) parts_of(x[g + 2 * i], x[g + 2 * i + 1], h[i], m[i], l[i]);
+    for (int i = 0; i < 8; ++i) parts_of(x[g + 2 * i] * scale, x[g + 2 * i + 1] * scale, h[i], m[i], l[i]);
     tmem_st8(lanes + COL_A + group * 16 + g / 2, h);
     tmem_st8(lanes + COL_A + 64 + group * 16 + g / 2, m);
     tmem_st8(lanes + COL_A + 128 + group * 16 + g / 2, l);
   }
 }
-// 32 columns of a product: the sums of its SPLIT accumulators, 128 columns apart, added
+// 32 columns of a product: the sums of its SPLIT accumulators, 128 columns apart, added, times `unscale`
 template <int SPLIT>
-__device__ __forceinline__ void read_product(uint32_t at, int group, float (&x)[32]) {
+__device__ __forceinline__ void read_product(uint32_t at, int group, float (&x)[32], float unscale) {
 #pragma unroll
   for (int c = 0; c < 32; c += 8) {
     float y[SPLIT][8];
@@ -138,8 +131,8 @@ __device__ __forceinline__ void read_product(uint32_t at, int group, float (&x)[
     tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      if constexpr (SPLIT == 2) x[c + i] = y[0][i] + y[1][i];
-      else x[c + i] = (y[0][i] + y[1][i]) + (y[2][i] + y[3][i]);
+      if constexpr (SPLIT == 2) x[c + i] = (y[0][i] + y[1][i]) * unscale;
+      else x[c + i] = ((y[0][i] + y[1][i]) + (y[2][i] + y[3][i])) * unscale;
     }
   }
 }
@@ -162,7 +155,6 @@ __device__ __forceinline__ uint64_t across(uint32_t parts, int p, int s) { retur
 
 struct Shared {
   float pw[TC + 4];
-  uint32_t largest[TC];      // of a row of queries
   unsigned long long done[PRODUCTS];      // a product's operands have been read and its sums are there
   uint32_t tmem_base_slot;
   int failed;
@@ -173,22 +165,13 @@ __device__ __forceinline__ void begin(Shared& sh, int warp, int tid, double deca
     sh.failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (tid < TC) sh.largest[tid] = 0;
   if (tid <= TC) sh.pw[tid] = power(decay, tid);
   if (warp == WARPS) tmem_alloc(s2u(&sh.tmem_base_slot), TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
 }
-// The same of a thread's 32 entries of row r, whose largest is looked at when all have been here.
-__device__ __forceinline__ bool row_out_of_reach(Shared& sh, const float (&x)[32], int r) {
-  uint32_t m = 0;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) m = max(m, __float_as_uint(x[i]) & 0x7fffffffu);
-  atomicMax(&sh.largest[r], m);
-  return too_large(m);
-}
-// `issued`: products that the caller's thread has issued; each is complete before the block leaves, whatever became of the waits for it
+// `issued`: products that the caller's warp has issued; each is complete before the block leaves, whatever became of the waits for it
 __device__ __forceinline__ void end(Shared& sh, int warp, int lane, int issued, int* err) {
   if (warp == WARPS && lane == 0) ring_drain(issued, PRODUCTS, [&](int p, uint32_t parity) { return mbar_wait(s2u(&sh.done[p]), parity); });
   __syncwarp();
@@ -198,12 +181,16 @@ __device__ __forceinline__ void end(Shared& sh, int warp, int lane, int issued, 
   if (sh.failed && threadIdx.x == 0) dk_report(err, DK_DEV_TIMEOUT, blockIdx.x, blockIdx.y, 0);
   if (warp == WARPS) tmem_dealloc(sh.tmem_base_slot, TMEM_COLS);
 }
-// The next product, unless a wait has given up (what it would read may not be there, and nobody waits for it).
+// The next product, unless a wait has given up (what it would read may not be there, and nobody waits for it).  By an elected thread: in a branch for lane 0
+// an MMA took 100 cycles to issue.
 template <typename Issue>
-__device__ __forceinline__ void issue_next(Shared& sh, int lane, int& issued, Issue&& product) {
-  if (lane == 0 && *(volatile int*)&sh.failed == 0) {
-    product();
-    umma_commit(s2u(&sh.done[issued++]));
+__device__ __forceinline__ void issue_next(Shared& sh, int& issued, Issue&& product) {
+  if (__all_sync(0xffffffffu, *(volatile int*)&sh.failed == 0)) {
+    if (elect_one()) {
+      product();
+      umma_commit(s2u(&sh.done[issued]));
+    }
+    ++issued;
   }
   __syncwarp();
 }
@@ -292,31 +279,29 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
     for (int i = 0; i < 4; ++i) first[i] = r < n ? *reinterpret_cast<const uint4*>(mine + 8 * i) : make_uint4(0, 0, 0, 0);
     fetch_rows(raw, at + k_off, stride, n, tid);
     activate(x, first, act);
-    odd = row_out_of_reach(sh, x, r);
-    parts_to_tmem(lanes, group, x);
+    odd = out_of_reach<REACH>(x);
+    parts_to_tmem(lanes, group, x, SCALE);
     activate(k, raw, act);
     fetch_rows(raw, at + v_off, stride, n, tid);
-    odd |= out_of_reach(k, true, lane);
+    odd |= out_of_reach<REACH>(k);
     rows_to_shared(R1, k, tid, as_it_is);
     tmem_wait_st();
     fence_async_smem();
     tc_fence_before();
   }
-  __syncthreads();
-  odd |= tid < TC && too_small(sh.largest[tid]);
   odd = __syncthreads_or(odd) != 0;
   tc_fence_after();
   int issued = 0;
   const bool scored = !odd;
   if (scored && warp == WARPS)
-    issue_next(sh, lane, issued, [&]() {      // q . k
+    issue_next(sh, issued, [&]() {      // q . k
       const uint32_t idesc = instr_desc_bf16(TC, TC);
       issue<2>([&](int q, int a, int b, int s, uint32_t add) { umma_a_tmem(tmem + COL_D + q * D, tmem + COL_A + a * 64 + s * 8, along(r1, b, s), idesc, add); });
     });
   bool odd_v = false;
   if (converts) {      // meanwhile
     activate(x, raw, act);
-    odd_v = out_of_reach(x, false, lane);
+    odd_v = out_of_reach<REACH>(x);
     rows_to_shared(R0, x, tid, as_it_is);
   }
   odd |= __syncthreads_or(odd_v) != 0;
@@ -330,14 +315,14 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
   if (converts) {
     wait_product(sh, 0);
     rows_to_shared(R1, k, tid, [&](int s) { return s < n ? sh.pw[n - 1 - s] : 0.f; });
-    read_product<2>(lanes + COL_D, group, x);
+    read_product<2>(lanes + COL_D, group, x, 1.f / SCALE);      // (A is an operand: times 2^24)
     fence_async_smem();
     tc_fence_before();
   }
   __syncthreads();
   tc_fence_after();
   if (warp == WARPS) {
-    issue_next(sh, lane, issued, [&]() {      // the contribution to the state: keys' entries by values' entries, both operands read transposed
+    issue_next(sh, issued, [&]() {      // the contribution to the state: keys' entries by values' entries, both operands read transposed
       const uint32_t idesc = instr_desc_bf16(TC, D, true) | 1u << 15;
       issue<4>([&](int q, int a, int b, int s, uint32_t add) { umma(tmem + q * D, across(r1, a, s), across(r0, b, s), idesc, add); });
     });
@@ -348,18 +333,18 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
       x[j] = s <= r ? x[j] * sh.pw[r - s] : 0.f;
     }
     wait_product(sh, 1);
-    read_product<4>(lanes, group, k);
+    read_product<4>(lanes, group, k, UNSCALE);
     tc_fence_before();
     asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");      // A takes columns of what was read
     tc_fence_after();
-    parts_to_tmem(lanes, group, x);
+    parts_to_tmem(lanes, group, x, 1.f);
     tmem_wait_st();
     tc_fence_before();
   }
   __syncthreads();
   tc_fence_after();
   if (warp == WARPS) {
-    issue_next(sh, lane, issued, [&]() {      // A v
+    issue_next(sh, issued, [&]() {      // A v
       const uint32_t idesc = instr_desc_bf16(TC, D, true);
       issue<2>([&](int q, int a, int b, int s, uint32_t add) { umma_a_tmem(tmem + COL_D + q * D, tmem + COL_A + a * 64 + s * 8, across(r0, b, s), idesc, add); });
     });
@@ -368,7 +353,7 @@ decay_tc_chunk_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_o
     float* to = Uc + (size_t)((warp & 3) * 32) * D + group * 32;
     turned(turn, k, lane, [&](int i, int c, float4 v) { *reinterpret_cast<float4*>(to + (size_t)i * D + c) = v; });
     wait_product(sh, 2);
-    read_product<2>(lanes + COL_D, group, x);
+    read_product<2>(lanes + COL_D, group, x, UNSCALE);
     float* o = oc + group * 32;
     turned(turn, x, lane, [&](int i, int c, float4 v) {
       const int t = (warp & 3) * 32 + i;
@@ -445,17 +430,15 @@ decay_tc_out_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_off
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[8 * i + e] = v[e];
     }
-    odd = out_of_reach(x, false, lane);
+    odd = out_of_reach<STATE_REACH>(x);
     rows_to_shared(Sp, x, tid, as_it_is);
     activate(x, raw, act);
-    odd |= row_out_of_reach(sh, x, r);
-    parts_to_tmem(lanes, group, x);
+    odd |= out_of_reach<REACH>(x);
+    parts_to_tmem(lanes, group, x, SCALE);
     tmem_wait_st();
     fence_async_smem();
     tc_fence_before();
   }
-  __syncthreads();
-  odd |= tid < TC && too_small(sh.largest[tid]);
   if (__syncthreads_or(odd)) {
     for (int i = tid; i < n * D; i += THREADS) {
       const int t = i / D, c = i % D;
@@ -471,13 +454,13 @@ decay_tc_out_kernel(const __nv_bfloat16* __restrict__ src, int stride, int q_off
   }
   tc_fence_after();
   if (warp == WARPS) {
-    issue_next(sh, lane, issued, [&]() {
+    issue_next(sh, issued, [&]() {
       const uint32_t idesc = instr_desc_bf16(TC, D, true);
       issue<2>([&](int q, int a, int b, int s, uint32_t add) { umma_a_tmem(tmem + COL_D + q * D, tmem + COL_A + a * 64 + s * 8, across(sp, b, s), idesc, add); });
     });
   } else {
     wait_product(sh, 0);
-    read_product<2>(lanes + COL_D, group, x);
+    read_product<2>(lanes + COL_D, group, x, UNSCALE);
     const float w = sh.pw[r + 1];
 #pragma unroll
     for (int i = 0; i < 32; ++i) x[i] *= w;

@@ -426,3 +426,36 @@ def test_experts_gather_places_beside_a_block(capacity, K, top, scaled):
         want = (want.float() * scale[at][:, None]).bfloat16()      # one product, rounded once
     want[places < 0] = 0
     assert torch.equal(rows[:capacity], want) and bool((rows[capacity] == 3.0).all())
+
+
+@pytest.mark.parametrize("kind", ["normal", "one large entry", "one entry", "positive", "small", "small state"])
+def test_decay_attention_tc_is_no_further_off_than_multiply_adds(kind):
+    """Rows that one entry dominates, operands of one sign, numbers whose products come near the smallest exponents: errors against 64 bits, beside the kernel that
+    sums by FMA in chunks of 64."""
+    o = ops()
+    H, lens, slots = 2, [389], [1]
+    src, state, dec, rows = decay_case(lens, slots, H, 128, 128, torch.bfloat16, [0.999, 0.97], 8)
+    g = torch.Generator(device=DEV).manual_seed(9)
+    n, C = lens[0], H * 128
+    far = torch.rand(n, 2 * H, 128, device=DEV, generator=g)
+    if kind == "one large entry":
+        src[:, :2 * C] = torch.where(far == far.amax(-1, keepdim=True), 1000.0, src[:, :2 * C].view(n, 2 * H, 128).float()).view(n, -1).bfloat16()
+    elif kind == "one entry":
+        src[:, :2 * C] *= (far == far.amax(-1, keepdim=True)).view(n, -1)
+        src[:, 2 * C:3 * C] *= 8.0
+    elif kind == "positive":
+        src[:, :3 * C] = src[:, :3 * C].abs() + 1.0
+    elif kind == "small":
+        src[:, :2 * C] *= 2.0 ** -57
+        state.zero_()
+    elif kind == "small state":
+        src[:, C:2 * C] *= 2.0 ** -118
+        state *= 2.0 ** -118
+    want, S = decay_reference(src, state[1].double(), dec, H, 128, 128)
+    want = want.reshape(n, -1)
+    st, ref = state.clone(), state.clone()
+    out, fma = decay_tc(o, src, st, dec, rows, lens, H), decay_tiles(o, src, ref, dec, rows, lens, H, 128, 128)
+    e, p, es, ps = ((a.double() - b).norm() / b.norm() for a, b in ((out, want), (fma, want), (st[1], S), (ref[1], S)))
+    print(f"{kind}: outputs {e:.3g} against {p:.3g}, states {es:.3g} against {ps:.3g}")
+    # two activations rounded alike on either side; products left out of a term: 2^-24 of it at most
+    assert e <= max(1.05 * p, 1e-7) and es <= max(1.05 * ps, 1e-7)
