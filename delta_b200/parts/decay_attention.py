@@ -8,7 +8,8 @@ A request's state is S [H, dk, dv] in 32 bit, zero at its start, one per run of 
 the request's earlier steps left, so a prompt may be cut anywhere.  The four projections are one product; the
 recurrence, its decays and the norm are 32 bit whatever the compute type.  Steps of single tokens stream the state through
 registers once; short portions run one block per (row, head) over the row's chunks in turn; long portions run their chunks in parallel (``csrc/decay_attention.cu``;
-heads of 64 or 128 entries in chunks of 64 tokens where those are enough blocks, ``csrc/decay_attention_tiles.cu``).
+heads of 64 or 128 entries in chunks of 64 tokens where those are enough blocks, ``csrc/decay_attention_tiles.cu``; heads of 128 x 128 in chunks of 128 on the
+tensor cores where those are full enough, ``csrc/decay_attention_tc.cu``).
 """
 from __future__ import annotations
 
@@ -28,6 +29,18 @@ def tiles_pay(q_lens, chunk: int, heads: int, sm_count: int) -> bool:
     chunks of 32.  The layer of 8 heads (16 heads), microseconds, chunks of 64 against 32: 65 tokens, 16 (32) blocks, 69 against 60 (77, 68);
     257 tokens, 40 (80) blocks, 71 against 61 (81, 81); 500 tokens, 64 (128) blocks, 76 against 72 (88, 116); eight rows of 65 76 against 107."""
     return 2 * heads * sum(-(-n // chunk) for n in q_lens) >= sm_count
+
+
+def tensor_cores_pay(q_lens, chunk: int, heads: int, sm_count: int) -> bool:
+    """Whether a step's portions (heads of 128 x 128, bfloat16) go to the tcgen05 kernels with chunks of 128 tokens or to the FMA kernels in chunks of 64
+    and 32.  A block of the former holds an SM alone, full chunk or single token: about 47 us for every time that the SMs have one each.  The others' time
+    follows tokens and chunks of 64.  Everything cold, microseconds, tcgen05 and the better of the others.  16 heads: 65 tokens 64, 46; 300 58, 56; 1,000 63, 87; eight rows of
+    65 73, 87; four of 500 108, 163; 20 of 100 165, 200; beside a portion of 65 tokens 8 / 16 / 32 single ones 73 / 120 / 220, 67 / 77 / 110; 2,000 beside 32
+    single ones 382, 304; 300 beside 16 of 20 159, 103.  8 heads: 1,000 tokens 63, 60; eight rows of 65 67, 56; 16 of them 73, 87.  32 heads: 300 tokens 61, 83; 15 rows of
+    130 343, 380; 512 tokens beside 8 single ones 169, 134."""
+    blocks = heads * sum(-(-n // chunk) for n in q_lens)
+    halves = heads * sum(-(-n // (chunk // 2)) for n in q_lens)
+    return 20 + 47 * -(-blocks // sm_count) <= 40 + (0.27 * heads * sum(q_lens) + 21 * halves) / sm_count
 
 
 @MIXERS.register("decay_attention")
@@ -68,9 +81,8 @@ class DecayAttention(Mixer):
         portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
         # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
         chunk, long = ops.decay_attention_tiles_chunk(), ops.decay_attention_tc_chunk()
-        # heads of 128 x 128 in bfloat16 go to the tensor cores whatever their number: 8 heads of 65 / 400 / 2,048 tokens 42 / 42 / 50 us, by FMA in
-        # chunks of 32 40 / 50 / 138 and of 64 48 / 52 / 85; 32 heads of 130 / 700 / 2,048 tokens 44 / 77 / 177 against 73 / 175 / 515 and 50 / 118 / 310
-        if portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype):
+        if (portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype)
+                and tensor_cores_pay(ctx.host["q_lens"], long, H, ctx.sm_count)):
             base, total, most = chunk_layout(ctx, long)
             per = H * dk * dv
             work = ctx.scratch("decay_attention.long_chunks", (total * per,), torch.float32,

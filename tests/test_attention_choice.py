@@ -17,3 +17,13 @@ def test_few_tokens_behind_a_long_context_stay_with_the_plain_kernel(q_lens, sta
 def test_linear_attention_takes_long_chunks_where_they_fill_the_device(q_lens, heads, tiles):
     from delta_b200.parts.decay_attention import tiles_pay
     assert tiles_pay(q_lens, 64, heads, 148) is tiles
+
+
+@pytest.mark.parametrize("q_lens, heads, tc", [
+    ([65], 8, False), ([65], 16, False), ([300], 32, True), ([1000], 16, True), ([2048], 16, True), ([65] * 8, 16, True), ([65] * 16, 8, True), ([500] * 4, 16, True),
+    ([100] * 20, 16, True), ([130] * 15, 32, True), ([65] + [1] * 16, 16, False), ([65] + [1] * 32, 32, False), ([512] + [1] * 8, 16, False),
+    ([512] + [1] * 32, 8, False), ([2000] + [1] * 32, 16, False), ([300] + [20] * 16, 16, False), ([2000, 20], 16, True)])
+def test_linear_attention_leaves_the_tensor_cores_where_their_chunks_would_be_empty(q_lens, heads, tc):
+    """A portion beside single tokens, each of which would be a chunk of 128 that holds an SM; short prompts, whose few chunks end sooner in smaller ones."""
+    from delta_b200.parts.decay_attention import tensor_cores_pay
+    assert tensor_cores_pay(q_lens, 128, heads, 148) is tc

@@ -386,7 +386,7 @@ def test_decay_attention_tc(decays):
 
 @pytest.mark.parametrize("what", ["q", "k", "v", "state", "small"])
 def test_decay_attention_tc_numbers_out_of_the_parts_reach(what):
-    """Infinite entries, and rows of very small ones: the chunk that holds them is summed by FMA, and nothing before an infinite token sees it."""
+    """Infinite entries: the chunk that holds them is summed by FMA, and nothing before an infinite token sees it; rows of very small ones."""
     o = ops()
     H, lens, slots = 2, [300], [1]
     src, state, dec, rows = decay_case(lens, slots, H, 128, 128, torch.bfloat16, [0.99, 0.9], 4)
