@@ -72,6 +72,13 @@ class DecayAttention(Mixer):
     def run_state_specs(self):
         return {STATE: StateSpec((self.heads, self.dk, self.dv), torch.float32, 0.0)}
 
+    def _chunks(self, ctx, floats: int):
+        """Working memory for a step's chunks: one buffer, whichever of the three forms a step takes."""
+        dk, dv = self.dk, self.dv
+        most = max((-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per for chunk, per in (
+            (ops.decay_attention_chunk(), dk * dv), (ops.decay_attention_tiles_chunk(), ops.decay_attention_tiles_floats(dk, dv)), (ops.decay_attention_tc_chunk(), dk * dv)))
+        return ctx.scratch("decay_attention.chunks", (floats,), torch.float32, bound=(most * self.heads,))
+
     def forward(self, ctx, x, cache):
         H, dk, dv = self.heads, self.dk, self.dv
         T = x.shape[0]
@@ -84,17 +91,13 @@ class DecayAttention(Mixer):
         if (portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype)
                 and tensor_cores_pay(ctx.host["q_lens"], long, H, ctx.sm_count)):
             base, total, most = chunk_layout(ctx, long)
-            per = H * dk * dv
-            work = ctx.scratch("decay_attention.long_chunks", (total * per,), torch.float32,
-                               bound=((-(-ctx.max_step_tokens // long) + ctx.max_rows) * per,))
+            work = self._chunks(ctx, total * H * dk * dv)
             ops.decay_attention_tc(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, most, H=H, dk=dk, dv=dv, silu=True,
                                    err=ctx.err, **rows)
         elif (portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk)
                 and tiles_pay(ctx.host["q_lens"], chunk, H, ctx.sm_count)):
             base, total, most = chunk_layout(ctx, chunk)
-            per = H * ops.decay_attention_tiles_floats(dk, dv)
-            bound = (-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per
-            work = ctx.scratch("decay_attention.chunks", (total * per,), torch.float32, bound=(bound,))
+            work = self._chunks(ctx, total * H * ops.decay_attention_tiles_floats(dk, dv))
             ops.decay_attention_tiles(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, total, most, H=H, dk=dk,
                                       dv=dv, silu=True, **rows)
         elif portions and ops.decay_attention_chunked_supported(dk, dv):
@@ -105,8 +108,7 @@ class DecayAttention(Mixer):
                 base = [sum(counts[:i]) for i in range(len(counts))]
                 return torch.tensor(base, dtype=torch.int32).to(x.device, non_blocking=True), sum(counts), max(counts)
             base, total, most = ctx.memo(("decay_attention chunks", chunk), layout)
-            bound = (-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * H * dk * dv
-            work = ctx.scratch("decay_attention.chunks", (total * H * dk * dv,), torch.float32, bound=(bound,))
+            work = self._chunks(ctx, total * H * dk * dv)
             ops.decay_attention_chunked(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, most, H=H, dk=dk,
                                         dv=dv, silu=True, **rows)
         elif ctx.decode_only and ops.decay_attention_step_supported(dk, dv):

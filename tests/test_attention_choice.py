@@ -27,3 +27,27 @@ def test_linear_attention_leaves_the_tensor_cores_where_their_chunks_would_be_em
     """A portion beside single tokens, each of which would be a chunk of 128 that holds an SM; short prompts, whose few chunks end sooner in smaller ones."""
     from delta_b200.parts.decay_attention import tensor_cores_pay
     assert tensor_cores_pay(q_lens, 128, heads, 148) is tc
+
+
+def test_linear_attentions_forms_share_their_working_memory(monkeypatch):
+    """Steps of full chunks, of chunks that would be nearly empty and of few tokens, in any order: one buffer, as large as any of them asks for at the engine's limits."""
+    from types import SimpleNamespace
+    import torch
+    from delta_b200.engine.context import StepContext
+    from delta_b200.parts import decay_attention as part
+    H, taken, steps = 16, [], [[2000] + [1] * 32, [2048], [65], [300, 300]]
+    for name in ("decay_attention_tc", "decay_attention_tiles", "decay_attention_chunked"):
+        monkeypatch.setattr(part.ops, name, lambda *a, name=name, **kw: taken.append(name))
+    monkeypatch.setattr(part.ops, "gated_rms_norm", lambda *a, **kw: None)
+    monkeypatch.setattr(part.linear, "linear", lambda ctx, x, w: torch.empty((x.shape[0], w), dtype=torch.bfloat16))
+    mixer = part.DecayAttention("", 2048, H, 128, 128, [0.9] * H, 1e-5)
+    mixer.w_in, mixer.w_o = 4 * H * 128, 2048
+    for order in (steps, steps[::-1]):
+        pool = {}
+        for q_lens in order:
+            ctx = SimpleNamespace(_scratch_pool=pool, device="cpu", host=dict(q_lens=q_lens), max_step_tokens=2048, max_rows=33, sm_count=148, replayable=False, decode_only=False,
+                                  max_q_len=max(q_lens), err=None, row_slot=None, row_q_start=None, row_q_len=None, memo=lambda key, make: make())
+            ctx.scratch = lambda *a, ctx=ctx, **kw: StepContext.scratch(ctx, *a, **kw)
+            mixer.forward(ctx, torch.empty((sum(q_lens), 2048), dtype=torch.bfloat16), SimpleNamespace(state={part.STATE: None}))
+        assert len(pool) == 1 and "__retired__" not in pool
+    assert set(taken) == {"decay_attention_tc", "decay_attention_tiles", "decay_attention_chunked"}
