@@ -21,7 +21,7 @@
 // e^(L_t) k_t.  So
 //   1. delta_chunk: every chunk of every head in parallel: A, B, U, W and the scaled queries and keys;
 //   2. delta_walk:  along a row, chunk after chunk, a slice of the value columns per block: three small products a chunk.
-// Rows of 1,301 and 747 tokens, 16 heads of 128 x 128: chunks 190 -> 85 us, walk 210 -> 170 us (with the changes that the kernels' comments
+// Rows of 1,301 and 747 tokens, 16 heads of 128 x 128: chunks 190 -> 85 us, walk 210 -> 165 us (with the changes that the kernels' comments
 // name).  Against 64 bits as before: outputs 1.6e-7 to 2.3e-7 off, states 1.1e-7 to 2.4e-7, weak to strong decays.
 // No exponent is ever positive.  Sums of log decays are kept as two floats, so that a difference of two of them is as good
 // when the sums themselves are large.
