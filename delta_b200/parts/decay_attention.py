@@ -33,13 +33,15 @@ def tiles_pay(q_lens, chunk: int, heads: int, sm_count: int) -> bool:
 
 def tensor_cores_pay(q_lens, chunk: int, heads: int, sm_count: int) -> bool:
     """Whether a step's portions (heads of 128 x 128, bfloat16) go to the tcgen05 kernels with chunks of 128 tokens or to the FMA kernels in chunks of 64
-    and 32.  A block of the former holds an SM alone, full chunk or single token: about 47 us for every time that the SMs have one each.  The others' time
-    follows tokens and chunks of 64.  Everything cold, microseconds, tcgen05 and the better of the others.  16 heads: 65 tokens 64, 46; 300 58, 56; 1,000 63, 87; eight rows of
-    65 73, 87; four of 500 108, 163; 20 of 100 165, 200; beside a portion of 65 tokens 8 / 16 / 32 single ones 73 / 120 / 220, 67 / 77 / 110; 2,000 beside 32
-    single ones 382, 304; 300 beside 16 of 20 159, 103.  8 heads: 1,000 tokens 63, 60; eight rows of 65 67, 56; 16 of them 73, 87.  32 heads: 300 tokens 61, 83; 15 rows of
-    130 343, 380; 512 tokens beside 8 single ones 169, 134."""
-    blocks = heads * sum(-(-n // chunk) for n in q_lens)
-    halves = heads * sum(-(-n // (chunk // 2)) for n in q_lens)
+    and 32.  A block of the former holds an SM alone, full chunk or single token.  Where all run at once they are ahead in the layer, with its launches and products
+    beside them (microseconds, tcgen05 and FMA): 8 heads, 65 tokens 103, 109; two rows of 150 99, 106; 65 beside 16 single ones 112, 121; 16 heads, 300 beside
+    four of 20 101, 105.  Then every time that the SMs have one each takes about 47, and the others' time follows tokens and chunks of 64.  The kernels alone, everything cold,
+    16 heads: eight rows of 65 tokens 73, 87; four of 500 108, 163; 20 of 100 165, 200; 65 tokens beside 16 / 32 single ones 120 / 220, 77 / 110; 2,000 beside 32 single ones
+    382, 304; 300 beside 16 of 20 159, 103.  32 heads: 15 rows of 130 343, 380; 512 tokens beside 8 single ones 169, 134."""
+    blocks = heads * sum([-(-n // chunk) for n in q_lens])
+    if blocks <= sm_count:
+        return True
+    halves = heads * sum([-(-n // (chunk // 2)) for n in q_lens])
     return 20 + 47 * -(-blocks // sm_count) <= 40 + (0.27 * heads * sum(q_lens) + 21 * halves) / sm_count
 
 
@@ -55,6 +57,7 @@ class DecayAttention(Mixer):
             raise ValueError(f"{len(self.decays)} decays for {self.heads} heads")
         self.eps = float(eps)
         self.w_in = self.w_o = self.norm_w = self._decays = None
+        self._most = (None, 0)      # the engine's limits, and the most floats that a step's chunks take under them
 
     def tensor_specs(self):
         p, d, H, dk, dv = self.prefix, self.width, self.heads, self.dk, self.dv
@@ -72,12 +75,16 @@ class DecayAttention(Mixer):
     def run_state_specs(self):
         return {STATE: StateSpec((self.heads, self.dk, self.dv), torch.float32, 0.0)}
 
-    def _chunks(self, ctx, floats: int):
-        """Working memory for a step's chunks: one buffer, whichever of the three forms a step takes."""
-        dk, dv = self.dk, self.dv
-        most = max((-(-ctx.max_step_tokens // chunk) + ctx.max_rows) * per for chunk, per in (
-            (ops.decay_attention_chunk(), dk * dv), (ops.decay_attention_tiles_chunk(), ops.decay_attention_tiles_floats(dk, dv)), (ops.decay_attention_tc_chunk(), dk * dv)))
-        return ctx.scratch("decay_attention.chunks", (floats,), torch.float32, bound=(most * self.heads,))
+    def _chunks(self, ctx, floats: int, tensor_cores: bool):
+        """Working memory for a step's chunks: one buffer, whichever of the forms that these heads have a step takes (chunks of 64, and of 128 on the tensor cores
+        or of 32)."""
+        key = (ctx.max_step_tokens, ctx.max_rows, tensor_cores)
+        if self._most[0] != key:      # (the host's time counts in short steps)
+            forms = [(ops.decay_attention_tc_chunk() if tensor_cores else ops.decay_attention_chunk(), self.dk * self.dv)]
+            if ops.decay_attention_tiles_supported(self.dk, self.dv, 8, 0, 0, 0):
+                forms.append((ops.decay_attention_tiles_chunk(), ops.decay_attention_tiles_floats(self.dk, self.dv)))
+            self._most = (key, self.heads * max((-(-key[0] // chunk) + key[1]) * per for chunk, per in forms))
+        return ctx.scratch("decay_attention.chunks", (floats,), torch.float32, bound=(self._most[1],))
 
     def forward(self, ctx, x, cache):
         H, dk, dv = self.heads, self.dk, self.dv
@@ -88,16 +95,16 @@ class DecayAttention(Mixer):
         portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
         # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
         chunk, long = ops.decay_attention_tiles_chunk(), ops.decay_attention_tc_chunk()
-        if (portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype)
-                and tensor_cores_pay(ctx.host["q_lens"], long, H, ctx.sm_count)):
+        tc = portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype)
+        if tc and tensor_cores_pay(ctx.host["q_lens"], long, H, ctx.sm_count):
             base, total, most = chunk_layout(ctx, long)
-            work = self._chunks(ctx, total * H * dk * dv)
+            work = self._chunks(ctx, total * H * dk * dv, tc)
             ops.decay_attention_tc(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, most, H=H, dk=dk, dv=dv, silu=True,
                                    err=ctx.err, **rows)
         elif (portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk)
                 and tiles_pay(ctx.host["q_lens"], chunk, H, ctx.sm_count)):
             base, total, most = chunk_layout(ctx, chunk)
-            work = self._chunks(ctx, total * H * ops.decay_attention_tiles_floats(dk, dv))
+            work = self._chunks(ctx, total * H * ops.decay_attention_tiles_floats(dk, dv), tc)
             ops.decay_attention_tiles(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, total, most, H=H, dk=dk,
                                       dv=dv, silu=True, **rows)
         elif portions and ops.decay_attention_chunked_supported(dk, dv):
@@ -108,7 +115,7 @@ class DecayAttention(Mixer):
                 base = [sum(counts[:i]) for i in range(len(counts))]
                 return torch.tensor(base, dtype=torch.int32).to(x.device, non_blocking=True), sum(counts), max(counts)
             base, total, most = ctx.memo(("decay_attention chunks", chunk), layout)
-            work = self._chunks(ctx, total * H * dk * dv)
+            work = self._chunks(ctx, total * H * dk * dv, tc)
             ops.decay_attention_chunked(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, most, H=H, dk=dk,
                                         dv=dv, silu=True, **rows)
         elif ctx.decode_only and ops.decay_attention_step_supported(dk, dv):

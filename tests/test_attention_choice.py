@@ -20,11 +20,11 @@ def test_linear_attention_takes_long_chunks_where_they_fill_the_device(q_lens, h
 
 
 @pytest.mark.parametrize("q_lens, heads, tc", [
-    ([65], 8, False), ([65], 16, False), ([300], 32, True), ([1000], 16, True), ([2048], 16, True), ([65] * 8, 16, True), ([65] * 16, 8, True), ([500] * 4, 16, True),
+    ([65], 8, True), ([300] + [20] * 4, 16, True), ([65] + [1] * 16, 8, True), ([300], 32, True), ([1000], 16, True), ([2048], 16, True), ([65] * 8, 16, True), ([65] * 16, 8, True), ([500] * 4, 16, True),
     ([100] * 20, 16, True), ([130] * 15, 32, True), ([65] + [1] * 16, 16, False), ([65] + [1] * 32, 32, False), ([512] + [1] * 8, 16, False),
     ([512] + [1] * 32, 8, False), ([2000] + [1] * 32, 16, False), ([300] + [20] * 16, 16, False), ([2000, 20], 16, True)])
 def test_linear_attention_leaves_the_tensor_cores_where_their_chunks_would_be_empty(q_lens, heads, tc):
-    """A portion beside single tokens, each of which would be a chunk of 128 that holds an SM; short prompts, whose few chunks end sooner in smaller ones."""
+    """A portion beside single tokens, each of which would be a chunk of 128 that holds an SM, and more of them than SMs."""
     from delta_b200.parts.decay_attention import tensor_cores_pay
     assert tensor_cores_pay(q_lens, 128, heads, 148) is tc
 
@@ -40,14 +40,14 @@ def test_linear_attentions_forms_share_their_working_memory(monkeypatch):
         monkeypatch.setattr(part.ops, name, lambda *a, name=name, **kw: taken.append(name))
     monkeypatch.setattr(part.ops, "gated_rms_norm", lambda *a, **kw: None)
     monkeypatch.setattr(part.linear, "linear", lambda ctx, x, w: torch.empty((x.shape[0], w), dtype=torch.bfloat16))
-    mixer = part.DecayAttention("", 2048, H, 128, 128, [0.9] * H, 1e-5)
-    mixer.w_in, mixer.w_o = 4 * H * 128, 2048
-    for order in (steps, steps[::-1]):
-        pool = {}
+    for d, order in ((128, steps), (128, steps[::-1]), (64, steps), (64, steps[::-1])):
+        mixer, pool = part.DecayAttention("", 2048, H, d, d, [0.9] * H, 1e-5), {}
+        mixer.w_in, mixer.w_o = 4 * H * d, 2048
         for q_lens in order:
             ctx = SimpleNamespace(_scratch_pool=pool, device="cpu", host=dict(q_lens=q_lens), max_step_tokens=2048, max_rows=33, sm_count=148, replayable=False, decode_only=False,
                                   max_q_len=max(q_lens), err=None, row_slot=None, row_q_start=None, row_q_len=None, memo=lambda key, make: make())
             ctx.scratch = lambda *a, ctx=ctx, **kw: StepContext.scratch(ctx, *a, **kw)
             mixer.forward(ctx, torch.empty((sum(q_lens), 2048), dtype=torch.bfloat16), SimpleNamespace(state={part.STATE: None}))
         assert len(pool) == 1 and "__retired__" not in pool
+        assert len(set(taken[-4:])) == 2
     assert set(taken) == {"decay_attention_tc", "decay_attention_tiles", "decay_attention_chunked"}
