@@ -21,15 +21,16 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {      // weights: rea
 // Blocks that an SM shall have room for (0: as the compiler has it, 71 to 130 registers).  Up to eight rows: held to 64 registers (a few spilled), so that an SM
 // has 32 warps and not 24 of these streams, and 1,024 blocks go in two rounds and not three: 16 experts of 2 x 1,024 x 2,048 and 2,048 x 1,024, 8 tokens:
 // 28.1 -> 24.7 and 15.2 -> 13.4 us (5.4 and 5.0 TB/s); 48 registers with fewer loads under way 29.8 and 14.9.  But gated products of K <= 1,024 in blocks of four
-// warps lose by it (the layer at width 1,024, 8 tokens: 34.6 -> 35.6 us).  The first product of relu squared gains for 17 and more rows by more loads under way,
+// warps lose by it (the layer at width 1,024, 8 tokens: 34.6 -> 35.6 us), and so do results in 32 bit with K <= 512 behind them (SHORT: 34.8 -> 35.4; K = 1,024
+// gains, 60.5 -> 58.4 at width 2,048).  The first product of relu squared gains for 17 and more rows by more loads under way,
 // 106 registers and 16 warps: the layer with 24 tokens, width 2,048 and 1,024: 68.1 -> 61.2 and 32.1 -> 29.5.  The others of nine and more rows lose by more registers: relu
 // squared, 16 tokens, 45.3 -> 51.4 and 26.6 -> 28.2; gated ones, whose 146 and 158 leave room for 12 warps and not 16, 74.1 -> 86.7 at 16 tokens and
 // 92.4 -> 100.6 at 24, width 2,048; results in 32 bit for 17 and more rows, behind gated ones, 91.0 -> 95.5 at 24.
-constexpr int least_blocks(int mode, int mt, int warps) {
-  return mt == 1 && !(mode == 1 && warps == 4) ? 32 / warps : mt == 4 && mode == 2 ? 16 / warps : 0;
+constexpr int least_blocks(int mode, int mt, int warps, bool shorter) {
+  return mt == 1 && !shorter && !(mode == 1 && warps == 4) ? 32 / warps : mt == 4 && mode == 2 ? 16 / warps : 0;
 }
-template <int MODE, int MT, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, least_blocks(MODE, MT, WARPS))
+template <int MODE, int MT, int WARPS, bool SHORT>
+__global__ void __launch_bounds__(WARPS * 32, least_blocks(MODE, MT, WARPS, SHORT))
 experts_stream_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W, void* __restrict__ out, const int* __restrict__ sorted,
                       const int* __restrict__ tile_expert, int top, int N, int K, float limit, float alpha, float shift,
                       const float* __restrict__ row_scale) {
@@ -136,12 +137,13 @@ extern "C" int dk_experts_stream(const void* A, const void* W, void* out, const 
   const dim3 grid((N + 15) / 16, max_tiles);
   const auto *a = (const __nv_bfloat16*)A, *w = (const __nv_bfloat16*)W;
   // four warps a block where a warp of eight would have four chunks of K or fewer
-#define RUN(MODE, MT, WARPS) \
-  experts_stream_kernel<MODE, MT, WARPS><<<grid, WARPS * 32, 0, stream>>>(a, w, out, sorted, tile_expert, top, N, K, limit, alpha, shift, row_scale)
-#define SIZE(MODE, MT)                   \
-  do {                                   \
-    if (K <= 1024) RUN(MODE, MT, 4);     \
-    else RUN(MODE, MT, 8);               \
+#define RUN(MODE, MT, WARPS, SHORT) \
+  experts_stream_kernel<MODE, MT, WARPS, SHORT><<<grid, WARPS * 32, 0, stream>>>(a, w, out, sorted, tile_expert, top, N, K, limit, alpha, shift, row_scale)
+#define SIZE(MODE, MT)                                              \
+  do {                                                              \
+    if (MODE == 0 && MT == 1 && K <= 512) RUN(MODE, MT, 4, MODE == 0 && MT == 1); \
+    else if (K <= 1024) RUN(MODE, MT, 4, false);                    \
+    else RUN(MODE, MT, 8, false);                                   \
   } while (0)
 #define PICK(MODE)                       \
   do {                                   \

@@ -6,9 +6,10 @@ import pytest
 
 from delta_b200.kernels import build
 
-# (0: a result in 32 bit, 1: gated, 2: relu squared; tiles of eight rows; warps a block) -> warps an SM
-ROOM = {(mode, 1, warps): 32 for mode in (0, 1, 2) for warps in (4, 8)} | {(1, 1, 4): 28} | {(mode, 2, warps): 24 for mode in (0, 2) for warps in (4, 8)} \
-    | {(0, 4, warps): 24 for warps in (4, 8)} | {(mode, 4, warps): 16 for mode in (1, 2) for warps in (4, 8)} | {(1, 2, 8): 16, (1, 2, 4): 12}
+# (0: a result in 32 bit, 1: gated, 2: relu squared; tiles of eight rows; warps a block; a short K of its own) -> warps an SM
+ROOM = {(mode, 1, warps, 0): 32 for mode in (0, 1, 2) for warps in (4, 8)} | {(1, 1, 4, 0): 28, (0, 1, 4, 1): 32} \
+    | {(mode, 2, warps, 0): 24 for mode in (0, 2) for warps in (4, 8)} | {(0, 4, warps, 0): 24 for warps in (4, 8)} \
+    | {(mode, 4, warps, 0): 16 for mode in (1, 2) for warps in (4, 8)} | {(1, 2, 8, 0): 16, (1, 2, 4, 0): 12}
 
 
 @pytest.fixture(scope="module")
@@ -19,8 +20,8 @@ def registers(tmp_path_factory):
         pytest.skip(str(e))
     r = subprocess.run([nvcc, *build.NVCC_FLAGS, "-Xptxas", "-v", "-I", str(build.CSRC), "-c", str(build.CSRC / "experts_stream.cu"),
                         "-o", str(tmp_path_factory.mktemp("stream") / "x.o")], capture_output=True, text=True, check=True)
-    found = re.findall(r"Compiling entry function '\S*experts_stream_kernelILi(\d)ELi(\d)ELi(\d)E.*?Used (\d+) registers", r.stderr, re.S)
-    return {(int(a), int(b), int(c)): int(n) for a, b, c, n in found}
+    found = re.findall(r"Compiling entry function '\S*experts_stream_kernelILi(\d)ELi(\d)ELi(\d)ELb(\d)E.*?Used (\d+) registers", r.stderr, re.S)
+    return {(int(a), int(b), int(c), int(d)): int(n) for a, b, c, d, n in found}
 
 
 @pytest.mark.parametrize("instance", sorted(ROOM))
