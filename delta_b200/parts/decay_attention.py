@@ -94,16 +94,16 @@ class DecayAttention(Mixer):
         rows = dict(row_slot=ctx.row_slot, row_q_start=ctx.row_q_start, row_q_len=ctx.row_q_len)
         portions = not ctx.replayable and ctx.max_q_len >= PARALLEL_FROM
         # long portions: the recurrence is linear in the state, so a row's chunks run in parallel and are stitched together
-        chunk, long = ops.decay_attention_tiles_chunk(), ops.decay_attention_tc_chunk()
         tc = portions and ops.decay_attention_tc_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk, x.dtype)
+        long = ops.decay_attention_tc_chunk() if tc else 0
         if tc and tensor_cores_pay(ctx.host["q_lens"], long, H, ctx.sm_count):
             base, total, most = chunk_layout(ctx, long)
             work = self._chunks(ctx, total * H * dk * dv, tc)
             ops.decay_attention_tc(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, most, H=H, dk=dk, dv=dv, silu=True,
                                    err=ctx.err, **rows)
         elif (portions and ops.decay_attention_tiles_supported(dk, dv, qkvg.shape[1], 0, H * dk, 2 * H * dk)
-                and tiles_pay(ctx.host["q_lens"], chunk, H, ctx.sm_count)):
-            base, total, most = chunk_layout(ctx, chunk)
+                and tiles_pay(ctx.host["q_lens"], ops.decay_attention_tiles_chunk(), H, ctx.sm_count)):
+            base, total, most = chunk_layout(ctx, ops.decay_attention_tiles_chunk())
             work = self._chunks(ctx, total * H * ops.decay_attention_tiles_floats(dk, dv), tc)
             ops.decay_attention_tiles(qkvg, 0, H * dk, 2 * H * dk, self._decays, cache.state[STATE], o, work, base, total, most, H=H, dk=dk,
                                       dv=dv, silu=True, **rows)
