@@ -54,6 +54,7 @@ TWO_STAGES = ["s_full,", r"s_full \+ 8", "o_done,", r"o_done \+ 8"]
 
 
 @pytest.mark.parametrize("name, copies, products", [("gemm_rows_tc.cu", ["full0"], ["empty0"]),
+                                                    ("gemm_f32_tc.cu", ["wfull", "xfull"], ["xempty"]),
                                                     ("attention_rows_wide_tc.cu", ["q_full", "k_edge", "k_full"], ["s_full", "o_done"]),
                                                     ("attention_rows_tc.cu", ["q_full", "full,", r"full \+ 8", "v_edge"], TWO_STAGES),
                                                     ("attention_prefill_tc.cu", ["q_full", "full,", r"full \+ 8"], TWO_STAGES)])
